@@ -51,7 +51,10 @@ int tc_tile_for(int rows);
 TcPlan tc_plan(int w_tiles, int rows, int kb, bool may_split_k, bool dual, int sms);
 cudaError_t tc_launch(const TcPlan& plan, bool dual, const CUtensorMap* const* mw, const CUtensorMap& mx, TcArgs a, cudaStream_t s);
 constexpr int kTcMinRows = 9;  // below this the row-batched GEMV stages are used
-constexpr int kPrefillRows = 512;  // rows of a prefill pass on the batched path: every pass streams all the weights once
+// Rows of a prompt pass on the batched path.  Every pass streams all the weights once and is a chain of ~8 dependent
+// launches per layer, so few wide passes win: 256 GPT-2 prompts of 64 tokens took 32 passes of 512 rows at 0.74 ms, nearly
+// all of it launch latency; the wide models are bound by their products from 512 rows on and gain from fewer re-reads.
+constexpr int kPrefillRows = 2048, kPrefillRowsNarrow = 4096;  // d_model > 1024 / below
 
 // ---------------------------------------------------------------------------------------------- kernels
 
@@ -129,6 +132,13 @@ __global__ void __launch_bounds__(kThreads) k_lm_head(const GemvArgs p) {
         }
     }
     stage_gemv<WT, EPI_HEAD>(p, blockIdx.x, gridDim.x, smem + kRedFloats, smem);
+}
+
+// The hidden state of the last row of every sequence that ends in a prompt pass: ends[i] = (row, sequence).
+__global__ void k_gather_last(const float* hidden, const int4* ends, float* out, int d) {
+    const int4 e = ends[blockIdx.x];
+    for (int k = threadIdx.x; k < d / 4; k += blockDim.x)
+        reinterpret_cast<float4*>(out + (size_t)e.y * d)[k] = reinterpret_cast<const float4*>(hidden + (size_t)e.x * d)[k];
 }
 
 __global__ void k_bump(RowState rs, int rows) {
@@ -342,6 +352,10 @@ Engine::~Engine() {
     if (ev_begin_) cudaEventDestroy(ev_begin_);
     if (ev_end_) cudaEventDestroy(ev_end_);
     for (void* p : owned_) cudaFree(p);
+    for (auto& slot : pass_slots_) {
+        if (slot.copied) cudaEventDestroy(slot.copied);
+        if (slot.host) cudaFreeHost(slot.host);
+    }
     if (h_rows_block_) cudaFreeHost(h_rows_block_);
     if (h_next_) cudaFreeHost(h_next_);
     if (h_mega_ctl_) cudaFreeHost(h_mega_ctl_);
@@ -410,7 +424,12 @@ int32_t Engine::init() {
     m_.max_seq = cfg_.max_seq; m_.q_dim = m_.n_head * m_.head_dim; m_.kv_dim = m_.n_kv_head * m_.head_dim;
     m_.n_seq = cfg_.max_batch; m_.eps = cfg_.norm_eps; m_.eos_token = cfg_.eos_token;
 
-    max_rows_ = std::max(cfg_.max_batch, kPrefillRows);  // rows of one pass: sequences of a batch, or positions of a prefill chunk
+    // rows of one pass: sequences of a batch, or positions of a prompt pass (never more than the engine can hold)
+    prefill_rows_ = (int)std::min<long long>(m_.d_model <= 1024 ? kPrefillRowsNarrow : kPrefillRows, ((long long)cfg_.max_batch * m_.max_seq + 63) / 64 * 64);
+    max_rows_ = std::max(cfg_.max_batch, prefill_rows_);
+    // the split-KV attention kernel serves the row-wise path and passes with fewer (row, head) pairs than SMs
+    const bool rows_kernel = m_.head_dim == 32 || m_.head_dim == 64 || m_.head_dim == 128;
+    const int att_rows = rows_kernel ? std::min(max_rows_, std::max(std::max(cfg_.max_batch, 8), sm_count_ / m_.n_head + 1)) : max_rows_;
     n_splits_ = (m_.max_seq + kAttSplitTokens - 1) / kAttSplitTokens;
     out_stride_ = m_.max_seq;
 
@@ -418,8 +437,8 @@ int32_t Engine::init() {
     if ((rc = dev_alloc(owned_, &act_.q, (size_t)max_rows_ * m_.q_dim))) return rc;
     if ((rc = dev_alloc(owned_, &act_.ctx, (size_t)max_rows_ * m_.q_dim))) return rc;
     if ((rc = dev_alloc(owned_, &act_.act, (size_t)max_rows_ * m_.hidden))) return rc;
-    if ((rc = dev_alloc(owned_, &act_.att_part, (size_t)max_rows_ * m_.n_head * n_splits_ * (m_.head_dim + 2)))) return rc;
-    if ((rc = dev_alloc(owned_, &act_.att_ticket, (size_t)max_rows_ * m_.n_head))) return rc;
+    if ((rc = dev_alloc(owned_, &act_.att_part, (size_t)att_rows * m_.n_head * n_splits_ * (m_.head_dim + 2)))) return rc;
+    if ((rc = dev_alloc(owned_, &act_.att_ticket, (size_t)att_rows * m_.n_head))) return rc;
     act_.logits = nullptr;
     act_.debug = nullptr;
     act_.debug_layer = -1;
@@ -427,7 +446,9 @@ int32_t Engine::init() {
     if ((rc = dev_alloc(owned_, &kv_.k, kv_elems))) return rc;
     if ((rc = dev_alloc(owned_, &kv_.v, kv_elems))) return rc;
 
+    att_ticket_words_ = (size_t)att_rows * m_.n_head;
     if ((rc = dev_alloc(owned_, &d_rows_block_, (size_t)6 * max_rows_))) return rc;
+    if ((rc = dev_alloc(owned_, &d_runs_, (size_t)2 * max_rows_))) return rc;
     rs_.seq = d_rows_block_;
     rs_.pos = d_rows_block_ + max_rows_;
     rs_.tok = reinterpret_cast<uint32_t*>(d_rows_block_ + 2 * max_rows_);
@@ -440,6 +461,10 @@ int32_t Engine::init() {
     if ((rc = dev_alloc(owned_, &rs_.best, (size_t)max_rows_))) return rc;
     if ((rc = dev_alloc(owned_, &rs_.ticket, 4))) return rc;
     ESP_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&h_rows_block_), sizeof(int) * 6 * max_rows_));
+    for (auto& slot : pass_slots_) {
+        ESP_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&slot.host), (sizeof(int) * 6 + sizeof(int4) * 2) * (size_t)max_rows_));
+        ESP_CUDA_TRY(cudaEventCreateWithFlags(&slot.copied, cudaEventDisableTiming));
+    }
     ESP_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&h_next_), sizeof(uint32_t) * max_rows_));
     h_visible_.assign(cfg_.max_batch, 0);
 
@@ -720,9 +745,8 @@ int32_t Engine::finalize() {
     if (n_qk != 0 && n_qk != m_.n_layer) return fail(ESP_CUDA_ERR_INVALID_WEIGHTS, "q_norm/k_norm must be present in every layer or in none");
     qk_norm_ = n_qk > 0;
     if (qk_norm_ && tp_size_ > 1) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "per-head q/k norm is not available with tensor parallelism");
-    // full logits are kept for rows that run the head: sequences of a batch (or the two rows of a verify pass), every
-    // row of a pass only when the engine was asked to keep logits
-    const int logit_rows = (cfg_.flags & ESP_CUDA_FLAG_KEEP_LOGITS) ? max_rows_ : std::max(cfg_.max_batch, 2);
+    // full logits are kept for rows that run the head: sequences of a batch, or the rows of a verify pass
+    const int logit_rows = std::max(cfg_.max_batch, 8);
     if ((rc = dev_alloc(owned_, &act_.logits, (size_t)logit_rows * m_.vocab))) return rc;
     size_t dbg = (size_t)m_.q_dim * 2 + 2 * m_.kv_dim + 2 * m_.d_model + m_.hidden;
     if ((rc = dev_alloc(owned_, &d_debug_, dbg))) return rc;
@@ -878,7 +902,10 @@ int32_t Engine::submit(int rows, int mode) {
         int32_t rc = tc_operands();  // before any capture: it allocates
         if (rc) return rc;
     }
-    const bool direct = (cfg_.flags & ESP_CUDA_FLAG_NO_GRAPH) || debug_layer_ >= 0;
+    // Prompt passes come in any length: launching their kernels directly takes less time than they run for, and a graph
+    // per length would have to be captured and instantiated first (milliseconds).
+    const bool prompt = rows > 1 && !(mode & STEP_HEAD);
+    const bool direct = (cfg_.flags & ESP_CUDA_FLAG_NO_GRAPH) || debug_layer_ >= 0 || prompt;
     if (direct) {
         bool profile = (cfg_.flags & ESP_CUDA_FLAG_NO_GRAPH) && (mode & STEP_FORWARD) && (mode & STEP_HEAD);
         if (profile && prof_events_.empty()) {
@@ -931,35 +958,32 @@ int32_t Engine::upload_rows(int rows, const int* seq, const int* pos, const uint
     // the pinned block may still be in flight from the previous call
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
     int* h = h_rows_block_;
-    for (int r = 0; r < max_rows_; r++) {
-        bool in = r < rows;
-        h[r] = in ? seq[r] : 0;
-        h[max_rows_ + r] = in ? pos[r] : 0;
-        h[2 * max_rows_ + r] = in && tok ? (int)tok[r] : 0;
-        h[3 * max_rows_ + r] = in ? (active ? active[r] : 1) : 0;
-        h[4 * max_rows_ + r] = 0;
-        h[5 * max_rows_ + r] = in && limit ? limit[r] : 0;
+    for (int r = 0; r < rows; r++) {
+        h[r] = seq[r];
+        h[rows + r] = pos[r];
+        h[2 * rows + r] = tok ? (int)tok[r] : 0;
+        h[3 * rows + r] = active ? active[r] : 1;
+        h[4 * rows + r] = 0;
+        h[5 * rows + r] = limit ? limit[r] : 0;
     }
     (void)zero_out_counts;
-    ESP_CUDA_TRY(cudaMemcpyAsync(d_rows_block_, h, sizeof(int) * 6 * max_rows_, cudaMemcpyHostToDevice, stream_));
+    ESP_CUDA_TRY(cudaMemcpy2DAsync(d_rows_block_, sizeof(int) * max_rows_, h, sizeof(int) * rows, sizeof(int) * rows, 6, cudaMemcpyHostToDevice, stream_));
     return ESP_CUDA_OK;
 }
 
 int32_t Engine::reset() {
     int32_t rc = check_ready("reset");
     if (rc) return rc;
-    // reset() zeroes the caches and the hidden state (Engine.swift:613-635)
-    size_t kv_bytes = (size_t)m_.n_layer * m_.n_seq * m_.n_kv_head * m_.max_seq * m_.head_dim * sizeof(__half);
-    ESP_CUDA_TRY(cudaMemsetAsync(kv_.k, 0, kv_bytes, stream_));
-    ESP_CUDA_TRY(cudaMemsetAsync(kv_.v, 0, kv_bytes, stream_));
-    ESP_CUDA_TRY(cudaMemsetAsync(act_.hidden, 0, sizeof(float) * (size_t)max_rows_ * m_.d_model, stream_));
+    // reset() empties the caches and zeroes the hidden state (Engine.swift:613-635).  The caches themselves are not
+    // cleared: no kernel reads a slot at or beyond the visible count, and every slot is written before it becomes visible.
+    // (Clearing them was 9.7 GB of stores, 1.4 ms, in front of every prompt of a 256-sequence GPT-2 engine.)
+    ESP_CUDA_TRY(cudaMemsetAsync(act_.hidden, 0, sizeof(float) * (size_t)cfg_.max_batch * m_.d_model, stream_));
     ESP_CUDA_TRY(cudaMemsetAsync(rs_.best, 0, sizeof(unsigned long long) * max_rows_, stream_));
     ESP_CUDA_TRY(cudaMemsetAsync(rs_.ticket, 0, 16, stream_));
-    ESP_CUDA_TRY(cudaMemsetAsync(act_.att_ticket, 0, sizeof(unsigned int) * (size_t)max_rows_ * m_.n_head, stream_));
+    ESP_CUDA_TRY(cudaMemsetAsync(act_.att_ticket, 0, sizeof(unsigned int) * att_ticket_words_, stream_));
     // a bounded wait of the batched or tensor-parallel kernels that ran out left its code here and makes every later
     // kernel skip its waits: reset() is the documented way back (on a tensor-parallel group every rank must reset)
     if (d_tc_error_) ESP_CUDA_TRY(cudaMemsetAsync(d_tc_error_, 0, sizeof(int), stream_));
-    ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
     std::fill(h_visible_.begin(), h_visible_.end(), 0);
     for (auto& c : checkpoints_) c.visible = -1;
     pending_verify_ = 0;
@@ -988,15 +1012,7 @@ int32_t Engine::feed_rows(int rows, const int* seq, const uint32_t* tok, bool wi
     }
     int32_t rc = upload_rows(rows, seq, pos.data(), tok, nullptr, nullptr, true);
     if (rc) return rc;
-    // A prompt pass whose 64-row tiles each hold consecutive positions of one sequence takes the tiled tensor-core
-    // attention (prefill_attention.cuh); the choice is part of the graph key.
-    int tiled = 0;
-    if (tc_ready_ && rows >= 32 && !with_head && (m_.head_dim == 32 || m_.head_dim == 64 || m_.head_dim == 128)) {
-        tiled = STEP_TILED_ATT;
-        for (int r = 1; r < rows && tiled; r++)
-            if (r % kPfRows != 0 && (seq[r] != seq[r - 1] || pos[r] != pos[r - 1] + 1)) tiled = 0;
-    }
-    if ((rc = submit(rows, STEP_FORWARD | (with_head ? STEP_HEAD : 0) | tiled))) return rc;
+    if ((rc = submit(rows, STEP_FORWARD | (with_head ? STEP_HEAD : 0)))) return rc;
     if (with_head) ESP_CUDA_TRY(cudaMemcpyAsync(h_next_, rs_.next, sizeof(uint32_t) * rows, cudaMemcpyDeviceToHost, stream_));
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
     if (tc_ready_ && (rows >= kTcMinRows || tp_size_ > 1)) {
@@ -1037,23 +1053,78 @@ int32_t Engine::decode_step(uint32_t token, uint32_t* next) {
     return feed_rows(1, &seq, &token, true, next);
 }
 
+// One prompt pass over `rows` rows (seq[r], tok[r]), enqueued without waiting for it.  `last_of`: for every sequence that
+// ends in this pass its last row, or -1; that row's hidden state goes to d_last_hidden_[sequence].  The rows' control
+// words, the list of runs (at most kPfRows consecutive positions of one sequence: the tiles of the prompt attention)
+// and the list of last rows travel in a pinned slot; two slots alternate, so the host prepares a pass while the device
+// works on the one before it.
+int32_t Engine::enqueue_pass(int rows, const int* seq, const uint32_t* tok, const std::vector<int2>& ends) {
+    if (force_failure_enabled()) return fail(ESP_CUDA_ERR_FORCED_FAILURE, "forced failure is enabled");
+    PassSlot& slot = pass_slots_[pass_slot_ ^= 1];
+    ESP_CUDA_TRY(cudaEventSynchronize(slot.copied));
+    int* h = slot.host;
+    int4* runs = reinterpret_cast<int4*>(h + (size_t)6 * max_rows_);
+    int4* last = runs + max_rows_;
+    int n_runs = 0;
+    for (int r = 0; r < rows; r++) {
+        const int s = seq[r], pos = h_visible_[s];
+        const bool full = pos >= m_.max_seq;
+        if (full || tok[r] >= (uint32_t)vocab_global_) {  // advance guard and token guard, Engine.swift:673-677, :687-689
+            std::ostringstream os;
+            if (full) os << "position " << pos << " exceeds context " << m_.max_seq;
+            else os << "token " << tok[r] << " is outside vocab " << vocab_global_;
+            while (r-- > 0) h_visible_[seq[r]]--;
+            return fail(ESP_CUDA_ERR_OUT_OF_RANGE, os.str());
+        }
+        h_visible_[s]++;
+        h[r] = s; h[rows + r] = pos; h[2 * rows + r] = (int)tok[r]; h[3 * rows + r] = 1; h[4 * rows + r] = 0; h[5 * rows + r] = 0;
+        if (n_runs && runs[n_runs - 1].z == s && runs[n_runs - 1].y < kPfRows) runs[n_runs - 1].y++;
+        else runs[n_runs++] = make_int4(r, 1, s, pos);
+    }
+    for (size_t i = 0; i < ends.size(); i++) last[i] = make_int4(ends[i].x, ends[i].y, 0, 0);
+    ESP_CUDA_TRY(cudaMemcpy2DAsync(d_rows_block_, sizeof(int) * max_rows_, h, sizeof(int) * rows, sizeof(int) * rows, 6, cudaMemcpyHostToDevice, stream_));
+    ESP_CUDA_TRY(cudaMemcpyAsync(d_runs_, runs, sizeof(int4) * n_runs, cudaMemcpyHostToDevice, stream_));
+    if (!ends.empty()) ESP_CUDA_TRY(cudaMemcpyAsync(d_runs_ + max_rows_, last, sizeof(int4) * ends.size(), cudaMemcpyHostToDevice, stream_));
+    ESP_CUDA_TRY(cudaEventRecord(slot.copied, stream_));
+    // runs of several positions take the tiled tensor-core attention (prefill_attention.cuh)
+    n_runs_ = n_runs;
+    const int tiled = tc_ready_ && rows >= kTcMinRows && rows >= 4 * n_runs && (m_.head_dim == 32 || m_.head_dim == 64 || m_.head_dim == 128) ? STEP_TILED_ATT : 0;
+    int32_t rc = submit(rows, STEP_FORWARD | tiled);
+    if (rc) return rc;
+    if (!ends.empty()) {
+        k_gather_last<<<(unsigned)ends.size(), 256, 0, stream_>>>(act_.hidden, d_runs_ + max_rows_, d_last_hidden_, m_.d_model);
+        ESP_CUDA_TRY(cudaGetLastError());
+    }
+    return ESP_CUDA_OK;
+}
+
+// Waits for the passes enqueued so far and reports a device-side wait that gave up.
+int32_t Engine::finish_passes() {
+    ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
+    if (!tc_ready_) return ESP_CUDA_OK;
+    int herr = 0;
+    ESP_CUDA_TRY(cudaMemcpy(&herr, d_tc_error_, sizeof(int), cudaMemcpyDeviceToHost));
+    if (herr) return fail(ESP_CUDA_ERR_TIMEOUT, herr == 8 ? "peer all-reduce gave up waiting for another rank" : "tensor-core GEMM gave up waiting on a barrier");
+    return ESP_CUDA_OK;
+}
+
 int32_t Engine::prefill(const uint32_t* tokens, int32_t n) {
     int32_t rc = check_ready("prefill");
     if (rc) return rc;
     if (!tokens || n <= 0) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "Prompt tokens must not be empty");
     if ((rc = reset())) return rc;
     // the prompt is processed in chunks of rows that share sequence 0 at consecutive positions
-    const int chunk = std::min(max_rows_, tc_ready_ ? kPrefillRows : 8);
-    std::vector<int> seq(chunk, 0);
+    const int chunk = tc_ready_ ? prefill_rows_ : 8;
+    std::vector<int> seq(std::min(chunk, n), 0);
+    const std::vector<int2> none;
     for (int i = 0; i < n; i += chunk) {
-        int c = std::min(chunk, n - i);
-        if ((rc = feed_rows(c, seq.data(), tokens + i, false, nullptr))) return rc;
+        const int c = std::min(chunk, n - i);
+        if ((rc = enqueue_pass(c, seq.data(), tokens + i, none))) { cudaStreamSynchronize(stream_); return rc; }
         if (c > 1)  // the last row's hidden state is the sequence's lastHidden
             ESP_CUDA_TRY(cudaMemcpyAsync(act_.hidden, act_.hidden + (size_t)(c - 1) * m_.d_model, sizeof(float) * m_.d_model,
                                          cudaMemcpyDeviceToDevice, stream_));
     }
-    ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
-    return ESP_CUDA_OK;
+    return finish_passes();
 }
 
 int32_t Engine::select_greedy(uint32_t* token) {
@@ -1075,19 +1146,18 @@ int32_t Engine::get_logits(int32_t seq, float* out, int32_t vocab) {
     if (tp_size_ > 1) return fail(ESP_CUDA_ERR_STATE, "get_logits: a tensor-parallel rank holds only its vocabulary shard");
     if (!out || vocab != m_.vocab) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "get_logits: output must hold exactly vocab floats");
     if (seq < 0 || seq >= m_.n_seq) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "sequence index out of range");
-    int rows = seq + 1;
-    std::vector<int> s(rows), p(rows), a(rows, 0);
-    for (int r = 0; r < rows; r++) { s[r] = r; p[r] = h_visible_[r]; }
-    a[seq] = 1;
-    if ((rc = upload_rows(rows, s.data(), p.data(), nullptr, a.data(), nullptr, true))) return rc;
-    uint32_t saved = cfg_.flags;
-    int saved_dbg = debug_layer_;
+    // one row: sequence seq's hidden state is handed to the head as row 0
+    int row_seq = seq, pos = h_visible_[seq];
+    if ((rc = upload_rows(1, &row_seq, &pos, nullptr, nullptr, nullptr, true))) return rc;
+    const uint32_t saved = cfg_.flags;
+    float* const hidden = act_.hidden;
     cfg_.flags |= ESP_CUDA_FLAG_KEEP_LOGITS | ESP_CUDA_FLAG_NO_GRAPH;
-    rc = launch_step(rows, STEP_HEAD, stream_, false);
+    act_.hidden = hidden + (size_t)seq * m_.d_model;
+    rc = launch_step(1, STEP_HEAD, stream_, false);
     cfg_.flags = saved;
-    debug_layer_ = saved_dbg;
+    act_.hidden = hidden;
     if (rc) return rc;
-    ESP_CUDA_TRY(cudaMemcpyAsync(out, act_.logits + (size_t)seq * m_.vocab, sizeof(float) * m_.vocab, cudaMemcpyDeviceToHost, stream_));
+    ESP_CUDA_TRY(cudaMemcpyAsync(out, act_.logits, sizeof(float) * m_.vocab, cudaMemcpyDeviceToHost, stream_));
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
     return ESP_CUDA_OK;
 }
@@ -1162,7 +1232,7 @@ int32_t Engine::prefill_batch(const uint32_t* tokens, int32_t n_seq, int32_t len
     if (!tokens || len <= 0) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "Prompt tokens must not be empty");
     if (n_seq < 1 || n_seq > cfg_.max_batch) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "n_seq exceeds max_batch");
     if ((rc = reset())) return rc;
-    // Rows are filled sequence by sequence: a pass of the tensor-core path holds up to kPrefillRows consecutive
+    // Rows are filled sequence by sequence: a pass of the tensor-core path holds up to prefill_rows_ consecutive
     // positions, long runs of one sequence first (every pass streams all the weights once, and runs of consecutive
     // positions are what the tiled attention kernel wants).  Without that path a pass is one position of every sequence.
     if (!tc_ready_) {
@@ -1175,36 +1245,28 @@ int32_t Engine::prefill_batch(const uint32_t* tokens, int32_t n_seq, int32_t len
         }
         return ESP_CUDA_OK;
     }
-    const int budget = std::min(max_rows_, kPrefillRows);
     if (!d_last_hidden_ && (rc = dev_alloc(owned_, &d_last_hidden_, (size_t)cfg_.max_batch * m_.d_model))) return rc;
     std::vector<int> seq;
     std::vector<uint32_t> tok;
-    std::vector<std::pair<int, int>> ends;  // (row, sequence) of every sequence that ends in the pass being built
-    auto flush = [&]() -> int32_t {
-        if (seq.empty()) return ESP_CUDA_OK;
-        int32_t r = feed_rows((int)seq.size(), seq.data(), tok.data(), false, nullptr);
-        if (r) return r;
-        for (auto& e : ends)  // the sequence's last hidden state, before the next pass overwrites the rows
-            ESP_CUDA_TRY(cudaMemcpyAsync(d_last_hidden_ + (size_t)e.second * m_.d_model, act_.hidden + (size_t)e.first * m_.d_model, sizeof(float) * m_.d_model,
-                                         cudaMemcpyDeviceToDevice, stream_));
-        seq.clear(); tok.clear(); ends.clear();
-        return ESP_CUDA_OK;
-    };
+    std::vector<int2> ends;  // (row, sequence) of every sequence that ends in the pass being built
+    seq.reserve(prefill_rows_);
+    tok.reserve(prefill_rows_);
     for (int s = 0; s < n_seq; s++) {
-        int t = 0;
-        while (t < len) {
-            const int take = std::min(len - t, budget - (int)seq.size());
-            for (int j = 0; j < take; j++) { seq.push_back(s); tok.push_back(tokens[(size_t)s * len + t + j]); }
+        for (int t = 0; t < len;) {
+            const int take = std::min(len - t, prefill_rows_ - (int)seq.size());
+            seq.insert(seq.end(), take, s);
+            tok.insert(tok.end(), tokens + (size_t)s * len + t, tokens + (size_t)s * len + t + take);
             t += take;
-            if (t == len) ends.emplace_back((int)seq.size() - 1, s);
-            if ((int)seq.size() == budget && (rc = flush())) return rc;
+            if (t == len) ends.push_back(make_int2((int)seq.size() - 1, s));
+            if ((int)seq.size() == prefill_rows_ || (s == n_seq - 1 && t == len)) {
+                if ((rc = enqueue_pass((int)seq.size(), seq.data(), tok.data(), ends))) { cudaStreamSynchronize(stream_); return rc; }
+                seq.clear(); tok.clear(); ends.clear();
+            }
         }
     }
-    if ((rc = flush())) return rc;
     // row s must hold the last hidden state of sequence s (decode passes have one row per sequence)
     ESP_CUDA_TRY(cudaMemcpyAsync(act_.hidden, d_last_hidden_, sizeof(float) * (size_t)n_seq * m_.d_model, cudaMemcpyDeviceToDevice, stream_));
-    ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
-    return ESP_CUDA_OK;
+    return finish_passes();
 }
 
 int32_t Engine::decode_step_batch(const uint32_t* tokens, int32_t n_seq, uint32_t* next) {
@@ -1320,7 +1382,7 @@ int32_t Engine::decode_loop(int32_t n_seq, int32_t count, uint32_t* out_tokens, 
     ESP_CUDA_TRY(cudaEventRecord(ev_end_, stream_));
     timings_.kernel_launches = launches_by_key_.count(n_seq * 16 + (STEP_HEAD | STEP_FEEDBACK)) ? launches_by_key_[n_seq * 16 + (STEP_HEAD | STEP_FEEDBACK)] : 1;
     if (max_lim > 1) timings_.kernel_launches += (max_lim - 1) * launches_last_step_;
-    ESP_CUDA_TRY(cudaMemcpyAsync(h_rows_block_, d_rows_block_, sizeof(int) * 6 * max_rows_, cudaMemcpyDeviceToHost, stream_));
+    ESP_CUDA_TRY(cudaMemcpy2DAsync(h_rows_block_, sizeof(int) * max_rows_, d_rows_block_, sizeof(int) * max_rows_, sizeof(int) * n_seq, 6, cudaMemcpyDeviceToHost, stream_));
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
     if (tc_ready_ && (n_seq >= kTcMinRows || tp_size_ > 1)) {  // bounded device waits report here
         int herr = 0;
@@ -1339,13 +1401,16 @@ int32_t Engine::decode_loop(int32_t n_seq, int32_t count, uint32_t* out_tokens, 
             prev = step_events_[i];
         }
     }
+    int most = 0;
     for (int s = 0; s < n_seq; s++) {
-        int n = std::min(h_rows_block_[4 * max_rows_ + s], lim[s]);
+        const int n = std::min(h_rows_block_[4 * max_rows_ + s], lim[s]);
         if (n_out) n_out[s] = n;
         h_visible_[s] = h_rows_block_[max_rows_ + s];
-        if (n > 0 && out_tokens)
-            ESP_CUDA_TRY(cudaMemcpy(out_tokens + (size_t)s * out_stride, rs_.out + (size_t)s * out_stride_, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
+        most = std::max(most, n);
     }
+    // one copy for all sequences: `most` tokens of each (what lies behind a sequence's own count is unspecified)
+    if (most > 0 && out_tokens)
+        ESP_CUDA_TRY(cudaMemcpy2D(out_tokens, sizeof(uint32_t) * out_stride, rs_.out, sizeof(uint32_t) * out_stride_, sizeof(uint32_t) * most, n_seq, cudaMemcpyDeviceToHost));
     return ESP_CUDA_OK;
 }
 
@@ -1607,7 +1672,7 @@ int32_t Engine::all_reduce(const void* send, void* recv, size_t count, bool sum_
 
 int32_t Engine::build_tc() {
     tc_ready_ = false;
-    if (max_rows_ > kPrefillRows) return ESP_CUDA_OK;
+    if (cfg_.max_batch > 512) return ESP_CUDA_OK;
     if (m_.d_model % 64 || m_.q_dim % 64 || m_.hidden % 64 || m_.kv_dim % 16) return ESP_CUDA_OK;
     const int t0 = tensors_.at("lm_head").type;
     if (t0 != ESP_CUDA_F16 && t0 != ESP_CUDA_BF16 && t0 != ESP_CUDA_Q8_0 && t0 != ESP_CUDA_Q4_0) return ESP_CUDA_OK;
@@ -1806,9 +1871,9 @@ int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
             launches++;
             if ((mode & STEP_TILED_ATT) && att_ok_hd) {
                 PrefillAttArgs pa{};
-                pa.m = m_; pa.rs = rs_; pa.kv = kv_; pa.q = act_.q; pa.ctx16 = xh_q_; pa.bf16 = tc_bf16_; pa.layer = l; pa.rows = rows;
+                pa.m = m_; pa.rs = rs_; pa.kv = kv_; pa.q = act_.q; pa.ctx16 = xh_q_; pa.bf16 = tc_bf16_; pa.layer = l; pa.runs = d_runs_;
                 pa.debug = cap ? dbg + q + 2 * kv : nullptr;
-                const dim3 grid((rows + kPfRows - 1) / kPfRows, m_.n_head);
+                const dim3 grid(n_runs_, m_.n_head);
                 if (m_.head_dim == 32) ESP_CUDA_TRY(launch_pdl(k_attention_prefill<32>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<32>(), s, pa));
                 else if (m_.head_dim == 64) ESP_CUDA_TRY(launch_pdl(k_attention_prefill<64>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<64>(), s, pa));
                 else ESP_CUDA_TRY(launch_pdl(k_attention_prefill<128>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<128>(), s, pa));

@@ -105,6 +105,8 @@ private:
     int32_t tc_operands();  // weight maps (and a quantised model's fp16 expansion), built on first use of the batched path
     int32_t all_reduce(const void* send, void* recv, size_t count, bool sum_f32, cudaStream_t s);
     const CUtensorMap* activation_map(const uint16_t* buf, int K, int tile);
+    int32_t enqueue_pass(int rows, const int* seq, const uint32_t* tok, const std::vector<int2>& ends);  // one prompt pass, not waited for
+    int32_t finish_passes();
     int32_t feed_rows(int rows, const int* seq, const uint32_t* tok, bool with_head, uint32_t* next_out);
     Weight weight_of(const DeviceTensor& t) const;
     LayerWeights layer_weights(int l) const;
@@ -122,6 +124,8 @@ private:
     bool finalized_ = false;
     bool qk_norm_ = false;  // every layer has per-head q_norm / k_norm weights (Qwen3)
     int max_rows_ = 0;
+    int prefill_rows_ = 0;  // rows of a prompt pass of the batched path
+    size_t att_ticket_words_ = 0;
     int n_splits_ = 1;
     int sm_count_ = 148;
 
@@ -135,6 +139,15 @@ private:
     int* d_rows_block_ = nullptr;  // [6][max_rows] seq,pos,tok,active,n_out,limit
     int* h_rows_block_ = nullptr;  // pinned
     uint32_t* h_next_ = nullptr;   // pinned [max_rows]
+    // prompt passes: two pinned slots of row-control words, run list and last-row list
+    struct PassSlot {
+        int* host = nullptr;
+        cudaEvent_t copied = nullptr;
+    };
+    PassSlot pass_slots_[2];
+    int pass_slot_ = 0;
+    int4* d_runs_ = nullptr;       // [max_rows] runs of consecutive positions {first row, rows, sequence, first position}, then [max_rows] last rows
+    int n_runs_ = 0;               // runs of the pass being launched
     float2* d_rope_ = nullptr;
     float* d_debug_ = nullptr;
     int debug_layer_ = -1;

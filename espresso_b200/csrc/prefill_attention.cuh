@@ -28,7 +28,7 @@ struct PrefillAttArgs {
     uint16_t* ctx16;   // [rows][q_dim] fp16/bf16
     int bf16;
     int layer;
-    int rows;
+    const int4* runs;  // one per row tile: {first row, rows (at most kPfRows), sequence, first position}
     float* debug;      // optional fp32 capture of row 0's context, or null
 };
 
@@ -62,16 +62,14 @@ __device__ __forceinline__ uint32_t pf_pack(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// grid = (row tiles, query heads).  The host launches this kernel only for passes in which every tile's rows are
-// active, belong to one sequence and sit at consecutive positions (Engine::upload_rows checks it).
+// grid = (runs, query heads): a run is a row tile that belongs to one sequence and sits at consecutive positions; the host
+// cuts a pass into runs wherever its sequences begin, so prompts of any length take this kernel (Engine::enqueue_pass).
 template <int HD>
 __global__ void __launch_bounds__(kPfThreads) k_attention_prefill(const PrefillAttArgs p) {
     extern __shared__ __align__(128) uint8_t pf_smem[];
     const ModelDims& m = p.m;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int row0 = blockIdx.x * kPfRows;
-    const int n_rows = min(kPfRows, p.rows - row0);
     const int head = blockIdx.y;
     const int kvh = head / (m.n_head / m.n_kv_head);
     constexpr int kChunks = HD / 8;   // 16-byte chunks per row
@@ -82,7 +80,8 @@ __global__ void __launch_bounds__(kPfThreads) k_attention_prefill(const PrefillA
     const uint32_t sV = sK + 2 * kPfCols * HD * 2;             // two stages
     pdl_launch_dependents();
     pdl_wait();
-    const int seq = p.rs.seq[row0], pos0 = p.rs.pos[row0];
+    const int4 run = p.runs[blockIdx.x];
+    const int row0 = run.x, n_rows = run.y, seq = run.z, pos0 = run.w;
     const int last_pos = pos0 + n_rows - 1;                    // newest visible position of the tile
     const int n_tiles = last_pos / kPfCols + 1;
     const __half* Kbase = p.kv.k + p.kv.offset(m, p.layer, seq, kvh, 0);
