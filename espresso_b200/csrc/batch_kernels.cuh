@@ -2,8 +2,6 @@
 // kernels prepare its 16-bit operand rows and apply what the GEMV path fuses into its epilogues:
 //   k_prep_rows    (embedding) -> RMSNorm / LayerNorm / none -> fp16 or bf16 operand rows
 //   k_rope_append  half-split RoPE on q (in place) and k, KV-cache append of k and v
-//   k_act_rows     SiLU(gate) * up  or  GELU(up)  -> 16-bit operand rows of the down projection
-//   k_attention_rows  attention for many rows at once: one warp per (row, head), 16-bit context rows out
 //   k_head_done    turns the packed per-row maxima of the LM-head GEMM into tokens (head_finalize)
 // Every kernel here is launched with programmatic stream serialization: it lets its successor start early and
 // waits for its predecessor before it touches global memory.
@@ -15,6 +13,27 @@ namespace esp {
 
 __device__ __forceinline__ uint16_t to_16bit(float v, int bf16) {
     return bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+}
+
+// 16-bit parts of a value: part 0 is the rounded value, the next ones the rounded remainders (fp16 parts saturate).
+__device__ __forceinline__ uint16_t part16(float& v, int bf16) {
+    if (bf16) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(v);
+        v -= __bfloat162float(h);
+        return __bfloat16_as_ushort(h);
+    }
+    unsigned short h;
+    asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(h) : "f"(v));
+    v -= __half2float(__ushort_as_half(h));
+    return h;
+}
+// Four values of row r -> their parts at columns k..k+3 of operand rows r, r + 8, r + 16.
+__device__ __forceinline__ void store_parts4(uint16_t* buf, int ld, int r, int k, float4 v, int parts, int bf16) {
+    for (int j = 0; j < parts; j++) {
+        const uint32_t lo = part16(v.x, bf16) | ((uint32_t)part16(v.y, bf16) << 16);
+        const uint32_t hi = part16(v.z, bf16) | ((uint32_t)part16(v.w, bf16) << 16);
+        *reinterpret_cast<uint2*>(buf + (size_t)(r + 8 * j) * ld + k) = make_uint2(lo, hi);
+    }
 }
 
 struct PrepArgs {
@@ -32,6 +51,7 @@ struct PrepArgs {
     const float* b;
     uint16_t* dst;            // [rows][K] fp16/bf16
     int bf16;
+    int parts;                // 16-bit parts per value (see stream_gemm.cuh): part j of row r goes to row r + 8 j
     float* zero[4];           // optional fp32 rows to clear ([rows][zero_n[i]]): outputs that K-sliced products add into
     int zero_n[4];
 };
@@ -134,9 +154,7 @@ __global__ void __launch_bounds__(kThreads) k_prep_rows(const PrepArgs p) {
                 o = make_float4((o.x - mean) * inv * g.x + b.x, (o.y - mean) * inv * g.y + b.y, (o.z - mean) * inv * g.z + b.z,
                                 (o.w - mean) * inv * g.w + b.w);
             }
-            reinterpret_cast<uint2*>(dst)[idx] =
-                make_uint2((uint32_t)to_16bit(o.x, p.bf16) | ((uint32_t)to_16bit(o.y, p.bf16) << 16),
-                           (uint32_t)to_16bit(o.z, p.bf16) | ((uint32_t)to_16bit(o.w, p.bf16) << 16));
+            store_parts4(p.dst, K, r, 4 * idx, o, p.parts, p.bf16);
         }
         return;
     }
@@ -167,7 +185,7 @@ __global__ void __launch_bounds__(kThreads) k_prep_rows(const PrepArgs p) {
         float v = x;
         if (p.norm == NORM_RMS) v = (x * inv) * p.g[k];
         else if (p.norm == NORM_LAYER) v = (x - mean) * inv * p.g[k] + p.b[k];
-        dst[k] = to_16bit(v, p.bf16);
+        for (int j = 0; j < p.parts; j++) dst[(size_t)8 * j * K + k] = part16(v, p.bf16);
     }
 }
 
@@ -256,202 +274,10 @@ __global__ void __launch_bounds__(kThreads) k_rope_append(const RopeArgs p) {
     }
 }
 
-struct ActArgs {
-    RowState rs;
-    const float* gate;  // [rows][h] (GELU: the biased up projection)
-    const float* up;    // [rows][h] or null for GELU
-    uint16_t* dst;      // [rows][h]
-    int h;
-    int bf16;
-    float* debug;       // optional fp32 capture of row 0
-};
-
-__global__ void __launch_bounds__(kThreads) k_act_rows(const ActArgs p) {
-    const int r = blockIdx.y;
-    pdl_launch_dependents();
-    pdl_wait();
-    if (!p.rs.active[r]) return;
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i >= p.h) return;
-    const float g = p.gate[(size_t)r * p.h + i];
-    const float v = p.up ? silu_f(g) * p.up[(size_t)r * p.h + i] : gelu_f(g);
-    p.dst[(size_t)r * p.h + i] = to_16bit(v, p.bf16);
-    if (p.debug && r == 0) p.debug[i] = v;
-}
-
 __global__ void k_head_done(const GemvArgs p) {
     pdl_launch_dependents();
     pdl_wait();
-    head_finalize(p);
-}
-
-struct AttRowsArgs {
-    ModelDims m;
-    RowState rs;
-    KvLayout kv;
-    const float* q;    // [rows][q_dim] fp32, RoPE applied
-    uint16_t* ctx16;   // [rows][q_dim] fp16/bf16: operand rows of the output projection
-    int bf16;
-    int layer;
-    int rows;
-    float* debug;      // optional fp32 capture of row 0's context (already offset), or null
-};
-
-constexpr int kAttRowsWarps = 4;
-
-__device__ __forceinline__ void halves16_to_float(const uint4& a, const uint4& b, float (&f)[16]) {
-    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-        f[2 * i] = t.x;
-        f[2 * i + 1] = t.y;
-    }
-}
-
-// Attention of one new token per row against its sequence's cache, for many rows: one warp per (row, head).
-// HD / 16 lanes share a cache position (16 channels each), so a warp covers 32 / (HD / 16) positions per pass and
-// every load instruction reads whole 128-byte (or longer) cache rows.  Each lane group keeps its own running
-// (max, sum, context) over the positions it visits; the groups are merged once at the end.  Softmax in fp32 as in
-// decodeContext (Sources/RealModelInference/RealModelInferenceEngine.swift:6560-6640), evaluated online.
-// SPLIT = 2: two warps share one (row, head) and take alternate blocks of positions (twice the cache bytes in
-// flight when there are few (row, head) pairs and long contexts); the second warp hands its (max, sum, context) to the
-// first through shared memory.  Needs n_head % 4 == 0 so that a CTA (4 heads x SPLIT warps) never straddles two rows.
-template <int HD, int SPLIT>
-__global__ void __launch_bounds__(kAttRowsWarps * 32 * SPLIT) k_attention_rows(const AttRowsArgs p) {
-    constexpr int LPP = HD / 16;   // lanes per position
-    constexpr int G = 32 / LPP;    // positions per pass of one warp
-    __shared__ float s_merge[SPLIT > 1 ? kAttRowsWarps * LPP * 18 : 1];
-    pdl_launch_dependents();
-    pdl_wait();
-    const ModelDims& m = p.m;
-    const int lane = threadIdx.x & 31;
-    const int warp_in_cta = threadIdx.x >> 5;
-    const int split = SPLIT > 1 ? warp_in_cta / kAttRowsWarps : 0;
-    const int w = blockIdx.x * kAttRowsWarps + (SPLIT > 1 ? warp_in_cta % kAttRowsWarps : warp_in_cta);
-    if (w >= p.rows * m.n_head) return;
-    const int r = w / m.n_head, head = w - r * m.n_head;
-    // the three row-state words are requested together (one memory round trip, not three)
-    const int row_active = p.rs.active[r], row_pos = p.rs.pos[r], row_seq = p.rs.seq[r];
-    const int sub = lane % LPP, slot = lane / LPP;
-    float q[16];  // this lane's 16 channels of the query, requested with the row state
-    {
-        const float4* qp = reinterpret_cast<const float4*>(p.q + (size_t)r * m.q_dim + (size_t)head * HD + sub * 16);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float4 t = qp[i];
-            q[4 * i] = t.x; q[4 * i + 1] = t.y; q[4 * i + 2] = t.z; q[4 * i + 3] = t.w;
-        }
-    }
-    if (!row_active) return;
-    const int visible = row_pos + 1;
-    const int kvh = head / (m.n_head / m.n_kv_head);
-    const size_t base = p.kv.offset(m, p.layer, row_seq, kvh, 0) + (size_t)sub * 16;
-    const __half* K = p.kv.k + base;
-    const __half* V = p.kv.v + base;
-    const float scale = 1.0f / sqrtf((float)HD);
-    float mx = -INFINITY, sum = 0.f, acc[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) acc[i] = 0.f;
-
-    auto load = [&](int t0, uint4 (&k)[2][2], uint4 (&v)[2][2]) {
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int t = t0 + u * G + slot;
-            if (t < visible) {
-                const uint4* kp = reinterpret_cast<const uint4*>(K + (size_t)t * HD);
-                const uint4* vp = reinterpret_cast<const uint4*>(V + (size_t)t * HD);
-                // through L1: with grouped-query attention the warps of a CTA are the query heads of one KV head and
-                // walk the same rows almost in step, so three of four reads are L1 hits (the cache is only read here)
-                k[u][0] = __ldg(kp); k[u][1] = __ldg(kp + 1);
-                v[u][0] = __ldg(vp); v[u][1] = __ldg(vp + 1);
-            } else {
-                k[u][0] = k[u][1] = v[u][0] = v[u][1] = make_uint4(0, 0, 0, 0);
-            }
-        }
-    };
-    auto compute = [&](int t0, const uint4 (&k)[2][2], const uint4 (&v)[2][2]) {
-        float s[2];
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            float kf[16];
-            halves16_to_float(k[u][0], k[u][1], kf);
-            float d = 0.f;
-#pragma unroll
-            for (int i = 0; i < 16; i++) d = fmaf(kf[i], q[i], d);
-#pragma unroll
-            for (int o = 1; o < LPP; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            s[u] = (t0 + u * G + slot < visible) ? d * scale : -INFINITY;
-        }
-        const float mn = fmaxf(mx, fmaxf(s[0], s[1]));
-        if (mn == -INFINITY) return;  // nothing visible in this lane group yet
-        const float corr = expf(mx - mn);  // exp(-inf) = 0 on the first visit
-        const float p0 = expf(s[0] - mn), p1 = expf(s[1] - mn);
-        mx = mn;
-        sum = sum * corr + p0 + p1;
-        float v0[16], v1[16];
-        halves16_to_float(v[0][0], v[0][1], v0);
-        halves16_to_float(v[1][0], v[1][1], v1);
-#pragma unroll
-        for (int i = 0; i < 16; i++) acc[i] = fmaf(p1, v1[i], fmaf(p0, v0[i], acc[i] * corr));
-    };
-
-    uint4 ka[2][2], va[2][2], kb[2][2], vb[2][2];
-    const int first = split * 4 * G;  // warps of one (row, head) take alternate blocks of 4 G positions
-    load(first, ka, va);
-    for (int t0 = first; t0 < visible; t0 += 4 * G * SPLIT) {
-        load(t0 + 2 * G, kb, vb);
-        compute(t0, ka, va);
-        load(t0 + 4 * G * SPLIT, ka, va);
-        compute(t0 + 2 * G, kb, vb);
-    }
-    // merge the lane groups
-#pragma unroll
-    for (int o = LPP; o < 32; o <<= 1) {
-        const float mo = __shfl_xor_sync(0xffffffffu, mx, o);
-        const float so = __shfl_xor_sync(0xffffffffu, sum, o);
-        const float mn = fmaxf(mx, mo);
-        const float c1 = mx == -INFINITY ? 0.f : expf(mx - mn);
-        const float c2 = mo == -INFINITY ? 0.f : expf(mo - mn);
-        sum = sum * c1 + so * c2;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const float ao = __shfl_xor_sync(0xffffffffu, acc[i], o);
-            acc[i] = acc[i] * c1 + ao * c2;
-        }
-        mx = mn;
-    }
-    if (SPLIT > 1) {  // (the whole CTA works on one row, so every warp reaches this barrier)
-        float* mine = s_merge + ((warp_in_cta % kAttRowsWarps) * LPP + sub) * 18;
-        if (split == 1 && slot == 0) {
-            mine[0] = mx; mine[1] = sum;
-#pragma unroll
-            for (int i = 0; i < 16; i++) mine[2 + i] = acc[i];
-        }
-        __syncthreads();
-        if (split == 0 && slot == 0) {
-            const float mo = mine[0], so = mine[1];
-            const float mn = fmaxf(mx, mo);
-            const float c1 = mx == -INFINITY ? 0.f : expf(mx - mn);
-            const float c2 = mo == -INFINITY ? 0.f : expf(mo - mn);
-            sum = sum * c1 + so * c2;
-#pragma unroll
-            for (int i = 0; i < 16; i++) acc[i] = acc[i] * c1 + mine[2 + i] * c2;
-        }
-    }
-    if (slot == 0 && split == 0) {
-        const float inv = sum > 0.f ? 1.0f / sum : 0.f;
-        uint32_t packed[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const float a0 = acc[2 * i] * inv, a1 = acc[2 * i + 1] * inv;
-            packed[i] = (uint32_t)to_16bit(a0, p.bf16) | ((uint32_t)to_16bit(a1, p.bf16) << 16);
-            if (p.debug && r == 0) { p.debug[head * HD + sub * 16 + 2 * i] = a0; p.debug[head * HD + sub * 16 + 2 * i + 1] = a1; }
-        }
-        uint4* dst = reinterpret_cast<uint4*>(p.ctx16 + (size_t)r * m.q_dim + (size_t)head * HD + sub * 16);
-        dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-    }
+    head_finalize(p.m, p.rows, p.rs, p.finalize_mode);
 }
 
 __global__ void k_copy_debug(const float* src, float* dst, int n) {

@@ -871,26 +871,25 @@ __device__ __forceinline__ unsigned long long pack_best(float v, int idx) {
 // Runs once per head pass, by the last CTA to finish: turns the packed maxima into tokens and, in the
 // device-driven loop, applies the reference's emission rules (Llama: emit EOS then stop, Engine.swift:6385-6388;
 // GPT-2: stop on 50256 without emitting, :4920-4922; stop at the emission limit or when the context is full).
-__device__ inline void head_finalize(const GemvArgs& p) {
-    const ModelDims& m = p.m;
-    for (int r = threadIdx.x; r < p.rows; r += blockDim.x) {
-        unsigned long long key = p.rs.best[r];
-        p.rs.best[r] = 0ull;
-        if (!p.rs.active[r]) continue;
+__device__ inline void head_finalize(const ModelDims& m, int rows, const RowState& rs, int mode) {
+    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+        unsigned long long key = rs.best[r];
+        rs.best[r] = 0ull;
+        if (!rs.active[r]) continue;
         uint32_t tokn = min(0xffffffffu - (uint32_t)(key & 0xffffffffull), (uint32_t)(m.vocab - 1));  // in range even if every logit was NaN
-        p.rs.next[r] = tokn;
-        int pos = p.rs.pos[r];
-        if (p.finalize_mode & 2) { pos += 1; p.rs.pos[r] = pos; }
-        if (p.finalize_mode & 1) {
+        rs.next[r] = tokn;
+        int pos = rs.pos[r];
+        if (mode & 2) { pos += 1; rs.pos[r] = pos; }
+        if (mode & 1) {
             bool emit = true, stop = false;
             if (m.arch == ARCH_GPT2) { if (tokn == GPT2_EOS) { emit = false; stop = true; } }
             else if (m.eos_token >= 0 && tokn == (uint32_t)m.eos_token) stop = true;
-            int n = p.rs.n_out[r];
-            if (emit) { p.rs.out[(size_t)r * p.rs.out_stride + n] = tokn; n++; p.rs.n_out[r] = n; }
+            int n = rs.n_out[r];
+            if (emit) { rs.out[(size_t)r * rs.out_stride + n] = tokn; n++; rs.n_out[r] = n; }
             // `pos` tokens are visible; with the token just emitted the sequence holds pos + 1 tokens
-            if (n >= p.rs.limit[r] || pos + 1 >= m.max_seq) stop = true;
-            p.rs.tok[r] = tokn;
-            if (stop) p.rs.active[r] = 0;
+            if (n >= rs.limit[r] || pos + 1 >= m.max_seq) stop = true;
+            rs.tok[r] = tokn;
+            if (stop) rs.active[r] = 0;
         }
     }
 }
@@ -1006,17 +1005,11 @@ __device__ void stage_gemv(const GemvArgs& p, int cta, int n_cta, float* xs, flo
         __syncthreads();
         if (s_ticket == (unsigned)(n_cta - 1)) {
             __threadfence();
-            head_finalize(p);
+            head_finalize(m, p.rows, p.rs, p.finalize_mode);
             __syncthreads();
             if (threadIdx.x == 0) *p.rs.ticket = 0u;
         }
     }
-}
-
-// Advance the position of every active row by one (the token just processed becomes visible).
-__device__ __forceinline__ void bump_positions(const RowState& rs, int rows) {
-    for (int r = threadIdx.x; r < rows; r += blockDim.x)
-        if (rs.active[r]) rs.pos[r] += 1;
 }
 
 }  // namespace esp

@@ -3,8 +3,10 @@
 #include "engine.h"
 #include "batch_kernels.cuh"
 #include "tc_gemm.cuh"
+#include "stream_gemm.cuh"
 #include "spec_kernel.cuh"
 #include "prefill_attention.cuh"
+#include "decode_attention.cuh"
 
 #include <dlfcn.h>
 #include <nccl.h>
@@ -50,6 +52,18 @@ int32_t tc_make_map(CUtensorMap* map, const void* base, bool bf16, uint64_t rows
 int tc_tile_for(int rows);
 TcPlan tc_plan(int w_tiles, int rows, int kb, bool may_split_k, bool dual, int sms);
 cudaError_t tc_launch(const TcPlan& plan, bool dual, const CUtensorMap* const* mw, const CUtensorMap& mx, TcArgs a, cudaStream_t s);
+// tensor-parallel NCCL fallback: the residual joins rank 0's partial sum
+__global__ void k_add_rows(float* dst, const float* src, int n4) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n4) return;
+    float4 a = reinterpret_cast<float4*>(dst)[i];
+    const float4 b = reinterpret_cast<const float4*>(src)[i];
+    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+    reinterpret_cast<float4*>(dst)[i] = a;
+}
+SgPlan sg_plan(int w_tiles, int rows, int kb, int parts, bool may_split, int sms);
+cudaError_t sg_launch(const SgPlan& plan, int epilogue, const CUtensorMap* const* mw, const CUtensorMap& mx, SgArgs a, cudaStream_t s);
+constexpr int kSgMaxRows = 256;  // rows of a pass that take the streamed products; wider prompt passes take k_gemm_tc
 constexpr int kTcMinRows = 9;  // below this the row-batched GEMV stages are used
 // Rows of a prompt pass on the batched path.  Every pass streams all the weights once and is a chain of ~8 dependent
 // launches per layer, so few wide passes win: 256 GPT-2 prompts of 64 tokens took 32 passes of 512 rows at 0.74 ms, nearly
@@ -144,7 +158,8 @@ __global__ void k_gather_last(const float* hidden, const int4* ends, float* out,
 __global__ void k_bump(RowState rs, int rows) {
     pdl_launch_dependents();
     pdl_wait();
-    bump_positions(rs, rows);
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < rows && rs.active[r]) rs.pos[r] += 1;
 }
 
 // GGUF blocks (array of structs, file order) -> the split layout of esp::Weight.
@@ -279,6 +294,16 @@ static void raise_smem_limits_on_current_device() {
     ESP_SET_ALL(WT_F16) ESP_SET_ALL(WT_BF16) ESP_SET_ALL(WT_Q8_0) ESP_SET_ALL(WT_Q4_0)
 #undef ESP_SET_ALL
 #undef ESP_SET
+    // The kernels of a pass must agree on the split of an SM's memory into L1 and shared memory: a kernel that wants another
+    // split waits until the SM is empty, and nothing of its prologue overlaps its predecessor.
+#define ESP_CARVE(k) cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)
+    ESP_CARVE(k_attention); ESP_CARVE(k_prep_rows); ESP_CARVE(k_embed_rows); ESP_CARVE(k_rope_append); ESP_CARVE(k_head_done); ESP_CARVE(k_bump);
+#define ESP_DA(HD)                                                                                                         \
+    ESP_CARVE((k_attention_decode<HD, 2>)); ESP_CARVE((k_attention_decode<HD, 4>)); ESP_CARVE((k_attention_decode<HD, 8>)); \
+    cudaFuncSetAttribute(k_attention_decode<HD, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, da_smem_floats(HD, 8, 8) * 4);
+    ESP_DA(32) ESP_DA(64) ESP_DA(128)
+#undef ESP_DA
+#undef ESP_CARVE
     cudaFuncSetAttribute(k_attention_prefill<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem_bytes<32>());
     cudaFuncSetAttribute(k_attention_prefill<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem_bytes<64>());
     cudaFuncSetAttribute(k_attention_prefill<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem_bytes<128>());
@@ -758,6 +783,15 @@ int32_t Engine::finalize() {
     }
     if (tp_size_ > 1 && tc_ready_ && (rc = tp_peer_setup())) return rc;
     if ((rc = build_mega())) return rc;
+    layer_tensors_.resize(m_.n_layer);
+    for (int l = 0; l < m_.n_layer; l++) {
+        const std::string p = "layers/" + std::to_string(l) + "/";
+        auto T = [&](const char* n) -> const DeviceTensor* { auto it = tensors_.find(p + n); return it == tensors_.end() ? nullptr : &it->second; };
+        LayerTensors& t = layer_tensors_[l];
+        t.wq = T("wq"); t.wk = T("wk"); t.wv = T("wv"); t.wo = T("wo"); t.w1 = T("w1"); t.w2 = T("w2"); t.w3 = T("w3");
+        t.w = layer_weights(l);
+        if (qk_norm_) { t.q_norm = T("q_norm")->f32; t.k_norm = T("k_norm")->f32; }
+    }
     finalized_ = true;
     return reset();
 }
@@ -802,6 +836,7 @@ int32_t Engine::check_ready(const char* what) const {
 // row; STEP_HEAD runs final norm + LM head + argmax; STEP_FEEDBACK makes the head emit and feed back its token.
 int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
     if (tp_size_ > 1 && !tc_ready_) return fail(ESP_CUDA_ERR_STATE, "tensor parallelism needs 16-bit weights with 64-aligned shard sizes");
+    if (stream_path(rows)) return launch_step_stream(rows, mode, s, profile);
     if (tc_ready_ && (rows >= kTcMinRows || tp_size_ > 1)) return launch_step_tc(rows, mode, s);
     const bool gpt2 = m_.arch == ARCH_GPT2;
     const int cap = sm_count_ * 2;  // one wave: the stage kernels hold ~120 registers, two CTAs per SM
@@ -888,7 +923,7 @@ int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
         ESP_CUDA_TRY(launch_gemv(EPI_HEAD, lh.type, dim3(grid), gemv_smem(lh.type, m_.d_model, false), s, ga));
         launches++;
     } else if (mode & STEP_FORWARD) {
-        ESP_CUDA_TRY(launch_pdl(k_bump, dim3(1), dim3(64), 0, s, rs_, rows));
+        ESP_CUDA_TRY(launch_pdl(k_bump, dim3((rows + 63) / 64), dim3(64), 0, s, rs_, rows));
         launches++;
     }
     mark();
@@ -898,7 +933,7 @@ int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
 
 int32_t Engine::submit(int rows, int mode) {
     if (force_failure_enabled()) return fail(ESP_CUDA_ERR_FORCED_FAILURE, "forced failure is enabled");
-    if (tc_ready_ && !tc_operands_ready_ && (rows >= kTcMinRows || tp_size_ > 1)) {
+    if (tc_ready_ && !tc_operands_ready_ && (stream_path(rows) || rows >= kTcMinRows)) {
         int32_t rc = tc_operands();  // before any capture: it allocates
         if (rc) return rc;
     }
@@ -1015,7 +1050,7 @@ int32_t Engine::feed_rows(int rows, const int* seq, const uint32_t* tok, bool wi
     if ((rc = submit(rows, STEP_FORWARD | (with_head ? STEP_HEAD : 0)))) return rc;
     if (with_head) ESP_CUDA_TRY(cudaMemcpyAsync(h_next_, rs_.next, sizeof(uint32_t) * rows, cudaMemcpyDeviceToHost, stream_));
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
-    if (tc_ready_ && (rows >= kTcMinRows || tp_size_ > 1)) {
+    if (tc_ready_) {
         int herr = 0;
         ESP_CUDA_TRY(cudaMemcpy(&herr, d_tc_error_, sizeof(int), cudaMemcpyDeviceToHost));
         if (herr) return fail(ESP_CUDA_ERR_TIMEOUT, herr == 8 ? "peer all-reduce gave up waiting for another rank" : "tensor-core GEMM gave up waiting on a barrier");
@@ -1384,7 +1419,7 @@ int32_t Engine::decode_loop(int32_t n_seq, int32_t count, uint32_t* out_tokens, 
     if (max_lim > 1) timings_.kernel_launches += (max_lim - 1) * launches_last_step_;
     ESP_CUDA_TRY(cudaMemcpy2DAsync(h_rows_block_, sizeof(int) * max_rows_, d_rows_block_, sizeof(int) * max_rows_, sizeof(int) * n_seq, 6, cudaMemcpyDeviceToHost, stream_));
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
-    if (tc_ready_ && (n_seq >= kTcMinRows || tp_size_ > 1)) {  // bounded device waits report here
+    if (tc_ready_) {  // bounded device waits report here
         int herr = 0;
         ESP_CUDA_TRY(cudaMemcpy(&herr, d_tc_error_, sizeof(int), cudaMemcpyDeviceToHost));
         if (herr) return fail(ESP_CUDA_ERR_TIMEOUT, herr == 8 ? "peer all-reduce gave up waiting for another rank" : "tensor-core GEMM gave up waiting on a barrier");
@@ -1689,6 +1724,7 @@ int32_t Engine::build_tc() {
     }
     if (quantised && (cfg_.flags & ESP_CUDA_FLAG_NO_TC_SHADOW)) return ESP_CUDA_OK;
     tc_bf16_ = t0 == ESP_CUDA_BF16;
+    tc_quant_ = quantised;
     tc_mats_ = mats;
     tc_operands_ready_ = false;
     // 16-bit matrices get their TMA maps now.  A quantised model's fp16 expansion (what batches and prefill chunks
@@ -1698,7 +1734,7 @@ int32_t Engine::build_tc() {
         int32_t rc0 = tc_operands();
         if (rc0) return rc0;
     }
-    tc_rows_alloc_ = (max_rows_ + 15) / 16 * 16;
+    tc_rows_alloc_ = std::max((max_rows_ + 15) / 16 * 16, 32);  // (32: three 16-bit parts of up to eight rows)
     int32_t rc;
     if ((rc = dev_alloc(owned_, &xh_d_, (size_t)tc_rows_alloc_ * m_.d_model))) return rc;
     if ((rc = dev_alloc(owned_, &xh_q_, (size_t)tc_rows_alloc_ * m_.q_dim))) return rc;
@@ -1707,6 +1743,7 @@ int32_t Engine::build_tc() {
     if ((rc = dev_alloc(owned_, &vraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &up_, (size_t)max_rows_ * m_.hidden))) return rc;
     if ((rc = dev_alloc(owned_, &d_tc_error_, 4))) return rc;
+    if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, kSgMaxRows) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
     if (tp_size_ > 1 && (rc = dev_alloc(owned_, &tp_partial_, (size_t)max_rows_ * m_.d_model))) return rc;
     ESP_CUDA_TRY(cudaDeviceSynchronize());
     tc_ready_ = true;
@@ -1730,6 +1767,7 @@ int32_t Engine::tc_operands() {
         }
         int32_t rc = tc_make_map(&t.map, base, tc_bf16_, t.rows, t.cols, kTcHalf);
         if (rc) return rc;
+        if ((rc = tc_make_map(&t.map64, base, tc_bf16_, t.rows, t.cols, kSgHalf))) return rc;
         t.has_map = true;
     }
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
@@ -1748,6 +1786,204 @@ const CUtensorMap* Engine::activation_map(const uint16_t* buf, int K, int tile) 
     return &it->second;
 }
 
+// Decode attention (head_dim 32, 64 or 128).  Warps per (row, KV head): as many of 8, 4, 2 as keep every pair resident at
+// once (registers allow 16 warps per SM, 8 at head_dim 128).  Pairs too few to fill the SMs share long contexts among the
+// CTAs of a cluster, which costs nothing while the context fits the first one.
+int32_t Engine::launch_attention_decode(const DecodeAttArgs& a, int rows, cudaStream_t s) {
+    const int hd = m_.head_dim, qpk = m_.n_head / m_.n_kv_head, groups = (qpk + kDaHeads - 1) / kDaHeads;
+    const int pairs = m_.n_kv_head * groups * rows, resident = (hd == 128 ? 8 : 16) * sm_count_;
+    int nw = 8, ranks = 1;
+    while (nw > 2 && pairs * nw > resident) nw /= 2;
+    while (nw == 8 && ranks < 8 && pairs * ranks * 2 <= 2 * sm_count_ && ranks * nw * kDaBlock < m_.max_seq) ranks *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(m_.n_kv_head * groups, rows, ranks);
+    cfg.blockDim = dim3(nw * 32);
+    cfg.dynamicSmemBytes = sizeof(float) * da_smem_floats(hd, nw, ranks);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = ranks;
+    cfg.attrs = attr;
+    cfg.numAttrs = ranks > 1 ? 2 : 1;
+#define ESP_ATT(HD)                                                                              \
+    ESP_CUDA_TRY(nw == 8 ? cudaLaunchKernelEx(&cfg, k_attention_decode<HD, 8>, a)                \
+                 : nw == 4 ? cudaLaunchKernelEx(&cfg, k_attention_decode<HD, 4>, a) : cudaLaunchKernelEx(&cfg, k_attention_decode<HD, 2>, a))
+    if (hd == 32) ESP_ATT(32);
+    else if (hd == 64) ESP_ATT(64);
+    else ESP_ATT(128);
+#undef ESP_ATT
+    return ESP_CUDA_OK;
+}
+
+bool Engine::stream_path(int rows) const {
+    // A quantised model's single rows stay on the kernels that read the GGUF blocks themselves (the persistent kernel and the
+    // row-wise GEMVs): an engine that only ever decodes one sequence then never builds the fp16 expansion.
+    return tc_ready_ && rows <= kSgMaxRows && !(tc_quant_ && rows == 1);
+}
+
+// One pass over the model for up to kSgMaxRows rows with the streamed products (stream_gemm.cuh): per layer q/k/v (norm,
+// bias, RoPE and cache append inside), attention, Wo + residual, FFN up (norm and activation inside), W2 + residual.
+int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool profile) {
+    const bool gpt2 = m_.arch == ARCH_GPT2;
+    tp_parity_ = 0;  // a step holds an even number of all-reduces: every step starts on partial buffer 0
+    int launches = 0;
+    float* dbg = debug_layer_ >= 0 ? d_debug_ : nullptr;
+    const int q = m_.q_dim, kv = m_.kv_dim, d = m_.d_model, h = m_.hidden, hd = m_.head_dim;
+    const int parts = rows <= 8 ? (tc_bf16_ ? 3 : 2) : 1;
+    const int stat_tiles = (d + kSgRows - 1) / kSgRows;
+    // The operand is staged from the residual stream inside the product where the rows are few: at 5 rows that costs 1.3 us
+    // against 3 for a norm kernel, at 64 rows it is three times slower than the product itself (every weight tile repeats it).
+    // Tensor-parallel ranks, whose stream is summed by another kernel, get the norm kernel.
+    const bool fuse_norm = tp_size_ <= 1 && rows <= 16;
+    auto tiles_of = [](int M) { return (M + kSgRows - 1) / kSgRows; };
+    auto halves_of = [](int M) { return (M + kSgHalf - 1) / kSgHalf; };
+    size_t ev = 0;
+    auto mark = [&]() { if (profile && ev < prof_events_.size()) cudaEventRecord(prof_events_[ev++], s); };
+    auto prep = [&](const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst) -> int32_t {
+        PrepArgs p{};
+        p.m = m_; p.rs = rs_; p.src = src; p.K = K; p.norm = norm; p.g = g; p.b = b; p.dst = dst; p.bf16 = tc_bf16_; p.parts = parts;
+        ESP_CUDA_TRY(launch_pdl(k_prep_rows, dim3(rows), dim3(kThreads), 0, s, p));
+        launches++;
+        return ESP_CUDA_OK;
+    };
+    struct Part { const DeviceTensor* W; float* out; int ldo; const float* bias; };
+    struct Norm { const float *g, *b; };
+    // norm != null: the operand is the normalised residual stream (fused, or through xbuf); else the 16-bit rows of xbuf
+    auto gemm = [&](std::initializer_list<Part> ps, int w_tiles, const uint16_t* xbuf, const Norm* norm, int epilogue, SgArgs a) -> int32_t {
+        const int K = ps.begin()->W->cols;
+        const SgPlan plan = sg_plan(w_tiles, rows, K / kTcBlockK, parts, epilogue != SG_HEAD, sm_count_);
+        const CUtensorMap* maps[3] = {&ps.begin()->W->map64, &ps.begin()->W->map64, &ps.begin()->W->map64};
+        int g = 0;
+        for (const Part& pt : ps) {
+            if (!pt.W->has_map || pt.W->cols != K) return fail(ESP_CUDA_ERR_CUDA, "tensor map missing for the batched path");
+            maps[g] = &pt.W->map64;
+            a.g[g].M = pt.W->rows; a.g[g].out = pt.out; a.g[g].ldo = pt.ldo; a.g[g].bias = pt.bias;
+            g++;
+        }
+        a.n_groups = g; a.K = K; a.rows = rows; a.bf16 = tc_bf16_; a.error = d_tc_error_; a.m = m_; a.rs = rs_; a.kv = kv_; a.eps = m_.eps;
+        if (norm) {
+            a.hidden = act_.hidden; a.stat = row_stat_; a.stat_tiles = stat_tiles; a.norm = gpt2 ? NORM_LAYER : NORM_RMS; a.norm_g = norm->g; a.norm_b = norm->b;
+        }
+        const CUtensorMap* mx = norm ? maps[0] : activation_map(xbuf, K, plan.n_cols);
+        if (!mx) return fail(ESP_CUDA_ERR_CUDA, "tensor map missing for the batched path");
+        ESP_CUDA_TRY(sg_launch(plan, epilogue, maps, *mx, a, s));
+        launches++;
+        return ESP_CUDA_OK;
+    };
+    // hidden += W . x (+ bias)
+    auto project = [&](const DeviceTensor& W, const uint16_t* xbuf, const float* bias) -> int32_t {
+        SgArgs a{};
+        if (tp_size_ <= 1) {
+            a.stat_out = fuse_norm ? row_stat_ : nullptr;
+            return gemm({{&W, act_.hidden, d, bias}}, tiles_of(d), xbuf, nullptr, SG_RESIDUAL, a);
+        }
+        // W holds this rank's slice of the input dimension: the product is a partial sum (rank 0's carries the bias).  Every
+        // row is written, inactive ones too: the sum reads them all.
+        float* partial = tp_current_partial();
+        a.all_rows = 1;
+        int32_t rc = gemm({{&W, partial, d, tp_rank_ == 0 ? bias : nullptr}}, tiles_of(d), xbuf, nullptr, SG_STORE, a);
+        if (rc) return rc;
+        if (tp_peer_ready_) { launches++; return tp_sum_peers(act_.hidden, rows, s); }
+        if (tp_rank_ == 0) {  // NCCL: rank 0's partial also carries the residual
+            k_add_rows<<<(rows * d / 4 + 255) / 256, 256, 0, s>>>(partial, act_.hidden, rows * d / 4);
+            launches++;
+        }
+        return all_reduce(partial, act_.hidden, (size_t)rows * d, true, s);
+    };
+    auto copy_dbg = [&](const float* src, int offset, int n) {
+        if (dbg) { k_copy_debug<<<(n + 255) / 256, 256, 0, s>>>(src, dbg + offset, n); launches++; }
+    };
+    const bool att_ok_hd = hd == 32 || hd == 64 || hd == 128;
+    const bool fuse_qkv = !qk_norm_ && att_ok_hd && kv % kSgHalf == 0;  // whole heads per 64-row half (a 128-wide head: per tile)
+    int32_t rc;
+    mark();
+    if (mode & STEP_FORWARD) {
+        const DeviceTensor& te = tensors_.at("embeddings/token");
+        EmbedArgs ea{};
+        ea.m = m_; ea.rs = rs_; ea.hidden = act_.hidden; ea.stat = row_stat_; ea.stat_tiles = stat_tiles;
+        ea.tok_emb = static_cast<const uint16_t*>(te.data);
+        ea.pos_emb = gpt2 ? static_cast<const uint16_t*>(tensors_.at("embeddings/position").data) : nullptr;
+        ea.emb_type = te.type == ESP_CUDA_BF16 ? WT_BF16 : WT_F16;
+        ESP_CUDA_TRY(launch_pdl(k_embed_rows, dim3(rows), dim3(kThreads), 0, s, ea));
+        launches++;
+        for (int l = 0; l < m_.n_layer; l++) {
+            const LayerTensors& t = layer_tensors_[l];
+            const LayerWeights& lw = t.w;
+            const bool cap = dbg && l == debug_layer_;
+            const Norm n1{lw.norm1_g, lw.norm1_b}, n2{lw.norm2_g, lw.norm2_b};
+            if (!fuse_norm && (rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, n1.g, n1.b, xh_d_))) return rc;
+            SgArgs qa{};
+            qa.rope = gpt2 ? nullptr : d_rope_; qa.layer = l; qa.debug = cap ? dbg : nullptr;
+            if ((rc = gemm({{t.wq, act_.q, q, lw.bq}, {t.wk, kraw_, kv, lw.bk}, {t.wv, vraw_, kv, lw.bv}}, (halves_of(q) + 2 * halves_of(kv) + 1) / 2, xh_d_,
+                           fuse_norm ? &n1 : nullptr, fuse_qkv ? SG_QKV : SG_STORE, qa)))
+                return rc;
+            if (!fuse_qkv) {
+                RopeArgs ra{};
+                ra.m = m_; ra.rs = rs_; ra.kv = kv_; ra.q = act_.q; ra.k_raw = kraw_; ra.v_raw = vraw_; ra.rope = gpt2 ? nullptr : d_rope_; ra.layer = l;
+                ra.debug = cap ? dbg : nullptr;
+                ra.q_norm = t.q_norm; ra.k_norm = t.k_norm;
+                ESP_CUDA_TRY(launch_pdl(k_rope_append, dim3(rows, (q / 2 + kv + kThreads - 1) / kThreads), dim3(kThreads), 0, s, ra));
+                launches++;
+            }
+            mark();
+            if (att_ok_hd) {
+                DecodeAttArgs da{};
+                da.m = m_; da.rs = rs_; da.kv = kv_; da.q = act_.q; da.ctx16 = xh_q_; da.bf16 = tc_bf16_; da.parts = parts; da.layer = l;
+                da.debug = cap ? dbg + q + 2 * kv : nullptr;
+                if ((rc = launch_attention_decode(da, rows, s))) return rc;
+                launches++;
+            } else {
+                AttArgs aa{};
+                aa.m = m_; aa.layer = l; aa.rows = rows; aa.n_splits = n_splits_; aa.rs = rs_; aa.a = act_; aa.kv = kv_;
+                aa.a.logits = nullptr; aa.a.debug = cap ? dbg : nullptr; aa.a.debug_layer = debug_layer_;
+                ESP_CUDA_TRY(launch_pdl(k_attention, dim3(m_.n_head, rows, n_splits_), dim3(kAttThreads), 0, s, aa));
+                launches++;
+                if ((rc = prep(act_.ctx, q, NORM_NONE, nullptr, nullptr, xh_q_))) return rc;
+            }
+            mark();
+            if ((rc = project(*t.wo, xh_q_, lw.bo))) return rc;
+            if (cap) copy_dbg(act_.hidden, 2 * q + 2 * kv, d);
+            if (!fuse_norm && (rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, n2.g, n2.b, xh_d_))) return rc;
+            SgArgs ua{};
+            ua.out16 = xh_h_; ua.ld16 = h; ua.debug = cap ? dbg + 2 * q + 2 * kv + d : nullptr;
+            if (gpt2) rc = gemm({{t.w1, nullptr, 0, lw.b1}}, tiles_of(h), xh_d_, fuse_norm ? &n2 : nullptr, SG_GELU, ua);
+            else rc = gemm({{t.w1, nullptr, 0, nullptr}, {t.w3, nullptr, 0, nullptr}}, halves_of(h), xh_d_, fuse_norm ? &n2 : nullptr, SG_SWIGLU, ua);
+            if (rc) return rc;
+            if ((rc = project(*t.w2, xh_h_, lw.b2))) return rc;
+            if (cap) copy_dbg(act_.hidden, 2 * q + 2 * kv + d + h, d);
+            mark();
+        }
+    }
+    if (mode & STEP_HEAD) {
+        const Norm nf{tensors_.at(gpt2 ? "final_norm_gamma" : "rms_final").f32, gpt2 ? tensors_.at("final_norm_beta").f32 : nullptr};
+        // (the head has hundreds of weight tiles and always takes the norm kernel)
+        if ((rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, nf.g, nf.b, xh_d_))) return rc;
+        const DeviceTensor& lh = tensors_.at("lm_head");
+        const int finalize = ((mode & STEP_FEEDBACK) ? 1 : 0) | ((mode & STEP_FORWARD) ? 2 : 0);
+        SgArgs ha{};
+        ha.logits = (cfg_.flags & ESP_CUDA_FLAG_KEEP_LOGITS) ? act_.logits : nullptr;
+        ha.row_offset = tp_rank_ * m_.vocab;
+        ha.finalize = tp_size_ > 1 ? -1 : finalize;
+        if ((rc = gemm({{&lh, nullptr, 0, nullptr}}, tiles_of(lh.rows), xh_d_, nullptr, SG_HEAD, ha))) return rc;
+        if (tp_size_ > 1) {
+            if ((rc = all_reduce(rs_.best, rs_.best, (size_t)rows, false, s))) return rc;  // max of (value, ~index) keys
+            GemvArgs fin{};
+            fin.m = m_; fin.m.vocab = vocab_global_; fin.rows = rows; fin.rs = rs_; fin.finalize_mode = finalize;
+            ESP_CUDA_TRY(launch_pdl(k_head_done, dim3(1), dim3(256), 0, s, fin));
+            launches++;
+        }
+    } else if (mode & STEP_FORWARD) {
+        ESP_CUDA_TRY(launch_pdl(k_bump, dim3((rows + 63) / 64), dim3(64), 0, s, rs_, rows));
+        launches++;
+    }
+    mark();
+    ESP_CUDA_TRY(cudaGetLastError());
+    launches_last_step_ = launches;
+    return ESP_CUDA_OK;
+}
+
 // One pass over the model for `rows` rows with the matrix products on the tensor cores: every weight matrix is
 // streamed once per pass whatever the row count.
 int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
@@ -1761,7 +1997,7 @@ int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
     auto prep = [&](const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst, bool from_emb, bool zero_qkv, bool zero_ffn = false,
                     float* zero_partial = nullptr) -> int32_t {
         PrepArgs p{};
-        p.m = m_; p.rs = rs_; p.src = src; p.hidden_out = act_.hidden; p.K = K; p.norm = norm; p.g = g; p.b = b; p.dst = dst; p.bf16 = tc_bf16_;
+        p.m = m_; p.rs = rs_; p.src = src; p.hidden_out = act_.hidden; p.K = K; p.norm = norm; p.g = g; p.b = b; p.dst = dst; p.bf16 = tc_bf16_; p.parts = 1;
         p.from_embedding = from_emb ? 1 : 0;
         if (from_emb) {
             const DeviceTensor& te = tensors_.at("embeddings/token");
@@ -1835,13 +2071,7 @@ int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
     auto copy_dbg = [&](const float* src, int offset, int n) {
         if (dbg) { k_copy_debug<<<(n + 255) / 256, 256, 0, s>>>(src, dbg + offset, n); launches++; }
     };
-    // (row, head) pairs for every SM: one warp each (two below ~28 warps per SM); fewer: the split-KV kernel of the GEMV
-    // path.  (Measured on 16 rows x 32 heads, contexts 128..384: 1.24 ms per step against 1.63 ms with the split-KV kernel
-    // and its extra conversion pass.)
     const bool att_ok_hd = m_.head_dim == 32 || m_.head_dim == 64 || m_.head_dim == 128;
-    // (a tensor-parallel rank holds 1/size of the heads: the choice follows the whole model's count, so that the ranks of a
-    // group keep the kernel a single GPU would use)
-    const bool att_rows = att_ok_hd && (long long)rows * m_.n_head * std::max(1, tp_size_) >= (long long)sm_count_;
     int32_t rc;
     if (mode & STEP_FORWARD) {
         const TcPlan plan_qkv = tc_plan(tiles_of(q) + 2 * tiles_of(kv), rows, d / kTcBlockK, true, false, sm_count_);
@@ -1878,23 +2108,11 @@ int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
                 else if (m_.head_dim == 64) ESP_CUDA_TRY(launch_pdl(k_attention_prefill<64>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<64>(), s, pa));
                 else ESP_CUDA_TRY(launch_pdl(k_attention_prefill<128>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<128>(), s, pa));
                 launches++;
-            } else if (att_rows) {
-                AttRowsArgs ar{};
-                ar.m = m_; ar.rs = rs_; ar.kv = kv_; ar.q = act_.q; ar.ctx16 = xh_q_; ar.bf16 = tc_bf16_; ar.layer = l; ar.rows = rows;
-                ar.debug = cap ? dbg + q + 2 * kv : nullptr;
-                const dim3 grid((rows * m_.n_head + kAttRowsWarps - 1) / kAttRowsWarps);
-                // few (row, head) pairs (less than ~28 warps per SM): two warps per pair, on alternate position blocks
-                const bool split2 = m_.n_head % kAttRowsWarps == 0 && (long long)rows * m_.n_head < 28LL * sm_count_;
-                const dim3 block(kAttRowsWarps * 32 * (split2 ? 2 : 1));
-#define ESP_ATT(HDV)                                                                                             \
-    do {                                                                                                         \
-        if (split2) ESP_CUDA_TRY(launch_pdl(k_attention_rows<HDV, 2>, grid, block, 0, s, ar));                   \
-        else ESP_CUDA_TRY(launch_pdl(k_attention_rows<HDV, 1>, grid, block, 0, s, ar));                          \
-    } while (0)
-                if (m_.head_dim == 32) ESP_ATT(32);
-                else if (m_.head_dim == 64) ESP_ATT(64);
-                else ESP_ATT(128);
-#undef ESP_ATT
+            } else if (att_ok_hd) {
+                DecodeAttArgs da{};
+                da.m = m_; da.rs = rs_; da.kv = kv_; da.q = act_.q; da.ctx16 = xh_q_; da.bf16 = tc_bf16_; da.parts = 1; da.layer = l;
+                da.debug = cap ? dbg + q + 2 * kv : nullptr;
+                if ((rc = launch_attention_decode(da, rows, s))) return rc;
                 launches++;
             } else {
                 AttArgs aa{};
@@ -1942,7 +2160,7 @@ int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
         ESP_CUDA_TRY(launch_pdl(k_head_done, dim3(1), dim3(256), 0, s, fin));
         launches++;
     } else if (mode & STEP_FORWARD) {
-        ESP_CUDA_TRY(launch_pdl(k_bump, dim3(1), dim3(64), 0, s, rs_, rows));
+        ESP_CUDA_TRY(launch_pdl(k_bump, dim3((rows + 63) / 64), dim3(64), 0, s, rs_, rows));
         launches++;
     }
     ESP_CUDA_TRY(cudaGetLastError());

@@ -28,9 +28,19 @@ struct DeviceTensor {
     int rows = 0, cols = 0;
     bool loaded = false;
     CUtensorMap map{};          // TMA map of a 16-bit matrix for the tensor-core path (128-row boxes)
+    CUtensorMap map64{};        // the same matrix in 64-row boxes (streamed products)
     bool has_map = false;
     __half* shadow16 = nullptr; // fp16 expansion of a quantised matrix: what the tensor-core path multiplies by
 };
+
+// A layer's tensors, looked up by name once.
+struct LayerTensors {
+    const DeviceTensor *wq = nullptr, *wk = nullptr, *wv = nullptr, *wo = nullptr, *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
+    const float *q_norm = nullptr, *k_norm = nullptr;
+    LayerWeights w{};
+};
+
+struct DecodeAttArgs;
 
 struct Checkpoint {
     int visible = 0;
@@ -101,6 +111,9 @@ private:
     int32_t submit(int rows, int mode);                  // graph replay or direct launch
     int32_t launch_step(int rows, int mode, cudaStream_t s, bool profile);
     int32_t launch_step_tc(int rows, int mode, cudaStream_t s);  // batched path: tensor-core GEMMs + element-wise stages
+    int32_t launch_step_stream(int rows, int mode, cudaStream_t s, bool profile);  // up to kSgMaxRows rows: streamed products, fused stages
+    bool stream_path(int rows) const;
+    int32_t launch_attention_decode(const DecodeAttArgs& a, int rows, cudaStream_t s);
     int32_t build_tc();
     int32_t tc_operands();  // weight maps (and a quantised model's fp16 expansion), built on first use of the batched path
     int32_t all_reduce(const void* send, void* recv, size_t count, bool sum_f32, cudaStream_t s);
@@ -184,10 +197,13 @@ private:
     bool tc_operands_ready_ = false;
     std::vector<std::string> tc_mats_;
     int tc_bf16_ = 0;
+    bool tc_quant_ = false;  // the operands are the fp16 expansion of a quantised model
+    std::vector<LayerTensors> layer_tensors_;
     int tc_rows_alloc_ = 0;
     uint16_t *xh_d_ = nullptr, *xh_q_ = nullptr, *xh_h_ = nullptr;  // 16-bit operand rows [tc_rows_alloc_][K]
     float *kraw_ = nullptr, *vraw_ = nullptr, *up_ = nullptr;
     float* d_last_hidden_ = nullptr;  // [max_batch][d_model] last hidden state per sequence while a batch of prompts is fed
+    float2* row_stat_ = nullptr;      // [rows][d_model / 128] statistics of the residual stream (streamed products)
     int* d_tc_error_ = nullptr;
     std::map<std::pair<const void*, int>, CUtensorMap> act_maps_;
 

@@ -139,17 +139,18 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 // Non-blocking test of a phase: the potentially blocking try_wait form costs about 0.25 us per call on this part even
 // when the phase has already completed, which a chunk-by-chunk consumer cannot afford.
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
+__device__ __forceinline__ bool mbar_test(uint32_t bar, unsigned parity) {
     unsigned ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) { return mbar_test(smem_u32(bar), parity); }
 // Weight chunks carry an evict-first L2 policy: they are used once per token, and keeping them out of the way
 // leaves the KV cache and the exchange words resident in L2.
 __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar, uint64_t policy) {

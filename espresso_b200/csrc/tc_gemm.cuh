@@ -98,6 +98,10 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
                  : "memory");
 }
 
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (64 x 16-bit) with the 128-byte
 // swizzle: 8-row groups are 1024 bytes apart (stride byte offset), the leading byte offset is unused (1).
 __device__ __forceinline__ uint64_t umma_smem_desc_sw128(const void* smem_tile) {
@@ -121,6 +125,15 @@ __device__ __forceinline__ uint32_t umma_idesc_f16(int n, int bf16) {
     d |= (uint32_t)(n >> 3) << 17;       // N / 8
     d |= (uint32_t)(kTcBatch >> 4) << 24;  // M / 16
     return d;
+}
+
+// True in one lane of a converged warp.  The loops that issue TMA copies and MMAs are run by the whole warp and elect a lane
+// only around the instructions: the same loop under `if (lane == 0)` took 1041 cycles per 64-wide K block (four MMAs and one
+// barrier wait) whatever the MMA's shape, against 509 (N = 256, the tensor pipe's own time) and ~320 (N <= 64) this way.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
 }
 
 __device__ __forceinline__ bool tc_wait(uint64_t* bar, unsigned parity, int* error) {
@@ -242,28 +255,32 @@ __global__ void __launch_bounds__(kTcThreads) k_gemm_tc(const __grid_constant__ 
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            for (int kb = 0; kb < num_kb; kb++) {
-                const int s = kb % kTcStages;
-                uint8_t* sx = tiles + (size_t)s * kTcStageBytes;
+        for (int kb = 0; kb < num_kb; kb++) {
+            const int s = kb % kTcStages;
+            uint8_t* sx = tiles + (size_t)s * kTcStageBytes;
+            if (kb >= kTcStages && !tc_wait(empty + s, ((kb / kTcStages) - 1) & 1, a.error)) break;
+            if (elect_one()) {
                 if (kb >= kTcStages) {
-                    if (!tc_wait(empty + s, ((kb / kTcStages) - 1) & 1, a.error)) break;
                     mbar_expect_tx(full + s, stage_tx);
                     tma_load_2d(sx + kTcXBytes, map_h0, (kb0 + kb) * kTcBlockK, m0_h0, full + s);
                     if (n_halves == 2) tma_load_2d(sx + kTcXBytes + kTcHalfBytes, map_h1, (kb0 + kb) * kTcBlockK, m0_h1, full + s);
                 }
                 tma_load_2d(sx, &map_x, (kb0 + kb) * kTcBlockK, n0, full + s);
             }
+            __syncwarp();
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_f16(n_halves * kTcHalf, a.bf16);
-            for (int kb = 0; kb < num_kb; kb++) {
-                const int s = kb % kTcStages;
-                if (!tc_wait(full + s, (kb / kTcStages) & 1, a.error)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint8_t* sx = tiles + (size_t)s * kTcStageBytes;
+        const uint32_t idesc = umma_idesc_f16(n_halves * kTcHalf, a.bf16);
+        bool ready = num_kb > 0 && mbar_try_wait(full, 0);
+        for (int kb = 0; kb < num_kb; kb++) {
+            const int s = kb % kTcStages;
+            if (!ready && !tc_wait(full + s, (kb / kTcStages) & 1, a.error)) break;
+            // the next block's barrier is tested before this block's MMAs: behind them the test would wait for their issue
+            ready = kb + 1 < num_kb && mbar_try_wait(full + (kb + 1) % kTcStages, ((kb + 1) / kTcStages) & 1);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint8_t* sx = tiles + (size_t)s * kTcStageBytes;
+            if (elect_one()) {
                 const uint64_t da = umma_smem_desc_sw128(sx), db = umma_smem_desc_sw128(sx + kTcXBytes);
 #pragma unroll
                 for (int k = 0; k < kTcBlockK / 16; k++) {
@@ -273,9 +290,10 @@ __global__ void __launch_bounds__(kTcThreads) k_gemm_tc(const __grid_constant__ 
                 // the stage may be refilled once these MMAs have read it
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(empty + s)) : "memory");
             }
-            // accumulator complete (or abandoned): release the epilogue either way
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(acc_ready)) : "memory");
+            __syncwarp();
         }
+        // accumulator complete (or abandoned): release the epilogue either way
+        if (elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(acc_ready)) : "memory");
     } else {
         // ---------------- epilogue: TMEM -> registers -> shared -> global ----------------
         const int ew = warp - 2;            // 0..7

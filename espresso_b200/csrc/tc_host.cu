@@ -1,7 +1,7 @@
 // Host side of the tensor-core GEMM: TMA tensor maps, launch dispatch over the batch tile width, and the
 // stand-alone entry point used for parity checks and tensor-pipe measurements.
 #include "engine.h"
-#include "tc_gemm.cuh"
+#include "stream_gemm.cuh"
 
 namespace esp {
 
@@ -110,6 +110,68 @@ cudaError_t tc_launch(const TcPlan& plan, bool dual, const CUtensorMap* const* m
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_gemm_tc, *mw[0], *mw[1], *mw[2], mx, a);
+}
+
+// Launch shape of a streamed product: w_tiles 128-row weight tiles, K of kb 64-wide blocks, `rows` batch rows in `parts`
+// 16-bit parts.  K slices: as many as fit two CTAs per SM with some room for the placement of clusters.  Measured (fp16, us
+// per launch in a warm chain; 1 slice -> rule): 2048 x 2048, 5 rows 13.8 -> 6.7 (8); 11264 x 2048 15.7 -> 11.5 (3);
+// 6144 x 4096, 1 row 30.7 -> 12.5 (5); 28672 x 4096 43 (1).  One slice more than the SMs can place costs a whole wave
+// (6144 x 4096 in 6 slices: 21.7).
+SgPlan sg_plan(int w_tiles, int rows, int kb, int parts, bool may_split, int sms) {
+    SgPlan p;
+    p.parts = parts;
+    p.n_cols = parts > 1 ? (parts == 2 ? 16 : 32) : std::min((rows + 15) / 16 * 16, kSgMaxCols);
+    p.col_tiles = parts > 1 ? 1 : (rows + p.n_cols - 1) / p.n_cols;
+    p.row_tiles = w_tiles;
+    // (several column tiles re-read the weights out of L2: 256 rows x 2304 x 768 takes 7.1 us in 144 CTAs, 7.7 in 216)
+    const int limit = p.col_tiles > 1 ? sms * 4 / 3 : sms * 9 / 5;
+    int want = may_split ? std::max(1, std::min(kSgMaxSplits, limit / std::max(1, w_tiles * p.col_tiles))) : 1;
+    want = std::min(want, std::max(1, kb / 2));
+    p.kb_per_split = (kb + want - 1) / want;
+    p.splits = (kb + p.kb_per_split - 1) / p.kb_per_split;
+    const int stage = kSgWBytes + p.n_cols * 128;
+    const int own = ((parts > 1 ? 8 : p.n_cols) + p.splits - 1) / p.splits;
+    const int exchange = p.splits * parts * own * kSgRows * 4;  // overlays the ring when there is one slice
+    const int room = kSgSmemBudget - 1024 - (p.splits > 1 ? exchange : 0);
+    p.stages = std::max(1, std::min(std::min(kSgMaxStages, p.kb_per_split), room / stage));
+    p.smem = (p.splits > 1 ? p.stages * stage + exchange : std::max(p.stages * stage, exchange)) + 1024;
+    return p;
+}
+
+static cudaError_t sg_configure() {
+    static std::mutex mu;
+    static bool configured[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev < 0 || dev >= 64 || configured[dev]) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(k_gemm_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgSmemBudget + 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_stream, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    configured[dev] = e == cudaSuccess;
+    return e;
+}
+
+// mw: 64-row maps of the group's matrices (unused slots repeat slot 0); mx: map of the operand rows with n_cols-row boxes
+// (ignored when the operand is staged from the residual stream).
+cudaError_t sg_launch(const SgPlan& plan, int epilogue, const CUtensorMap* const* mw, const CUtensorMap& mx, SgArgs a, cudaStream_t s) {
+    cudaError_t e = sg_configure();
+    if (e != cudaSuccess) return e;
+    int halves = 0;
+    for (int g = 0; g < a.n_groups; g++) { a.g[g].half0 = halves; halves += (a.g[g].M + kSgHalf - 1) / kSgHalf; }
+    a.kb_per_split = plan.kb_per_split; a.n_cols = plan.n_cols; a.parts = plan.parts; a.stages = plan.stages; a.epilogue = epilogue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(plan.col_tiles, plan.row_tiles, plan.splits);
+    cfg.blockDim = dim3(kSgThreads);
+    cfg.dynamicSmemBytes = plan.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = plan.splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = plan.splits > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, k_gemm_stream, *mw[0], *mw[1], *mw[2], mx, a);
 }
 
 __global__ void k_f32_to_16(const float* src, int64_t n, uint16_t* dst, int bf16) {
