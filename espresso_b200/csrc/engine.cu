@@ -1085,7 +1085,12 @@ int32_t Engine::decode_step(uint32_t token, uint32_t* next) {
     if (rc) return rc;
     if (!next) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "decode_step: null output");
     int seq = 0;
-    return feed_rows(1, &seq, &token, true, next);
+    if (!mega_usable() || (cfg_.flags & ESP_CUDA_FLAG_KEEP_LOGITS) || h_visible_[0] >= m_.max_seq || token >= (uint32_t)vocab_global_) return feed_rows(1, &seq, &token, true, next);  // (or its range errors)
+    // the persistent kernel for a single token: the layers take half the time of one launch per stage
+    if ((rc = launch_mega(1, &token, false))) return rc;
+    h_visible_[0]++;
+    *next = (uint32_t)(h_mega_ctl_[5] >> 32);
+    return ESP_CUDA_OK;
 }
 
 // One prompt pass over `rows` rows (seq[r], tok[r]), enqueued without waiting for it.  `last_of`: for every sequence that
@@ -1380,7 +1385,7 @@ int32_t Engine::decode_loop(int32_t n_seq, int32_t count, uint32_t* out_tokens, 
         if (n_out) n_out[s] = 0;
     }
     if (max_lim == 0) { if (device_ms) *device_ms = 0.f; return ESP_CUDA_OK; }
-    if (mega_ready_ && n_seq == 1 && debug_layer_ < 0 && !(cfg_.flags & (ESP_CUDA_FLAG_NO_MEGAKERNEL | ESP_CUDA_FLAG_NO_GRAPH))) {
+    if (n_seq == 1 && mega_usable()) {
         int emitted = 0;
         if ((rc = run_mega(lim[0], &emitted, device_ms, first_token_ms))) return rc;
         if (n_out) n_out[0] = emitted;
@@ -2331,9 +2336,10 @@ int32_t Engine::build_mega() {
     return ESP_CUDA_OK;
 }
 
-// Runs the greedy loop (at most n_steps emitted tokens; fewer when the end-of-sequence token comes up) of sequence 0
-// as one cooperative launch.  *emitted receives the number of tokens written to rs_.out.
-int32_t Engine::run_mega(int n_steps, int* emitted, float* device_ms, double* first_token_ms) {
+// Launches the persistent kernel for up to n_steps tokens of sequence 0 and waits for it: the greedy loop from the current
+// state, or (feed != null) starting with a forward pass for the token *feed at the current position.  h_mega_ctl_ then
+// holds {.., error, start, first token, {last token, tokens emitted}}.
+int32_t Engine::launch_mega(int n_steps, const uint32_t* feed, bool times) {
     MegaArgs a{};
     const MegaPlan& p = mega_plan_;
     a.m = m_; a.plan = p; a.pack = d_pack_; a.norms = d_norms_;
@@ -2345,19 +2351,31 @@ int32_t Engine::run_mega(int n_steps, int* emitted, float* device_ms, double* fi
     a.stamps = d_mega_ctl_ + 3;
     a.rs = rs_;
     a.trace = d_mega_trace_;
-    a.token_times = n_steps <= m_.max_seq + 1 ? d_token_times_ : nullptr;
+    a.token_times = times && n_steps <= m_.max_seq + 1 ? d_token_times_ : nullptr;
     token_times_n_ = 0;
     a.trace_cta = std::min(mega_trace_cta_, p.n_cta - 1);
     a.n_steps = n_steps;
+    a.first = feed ? 1 : 0;
+    a.tok0 = feed ? *feed : 0;
     a.pos0 = h_visible_[0];
     a.spin_limit = mega_spin_limit_;
+    // The arena is cleared when the tags have wrapped far enough to matter or a launch gave up half-way; otherwise every
+    // launch continues the numbering of the one before (clearing it cost two memory operations per streamed token).
+    const unsigned used = (unsigned)(n_steps + 1) * (unsigned)m_.n_layer;
+    if (mega_dirty_ || mega_tag_ > 0xffff0000u - used) {
+        ESP_CUDA_TRY(cudaMemsetAsync(d_mega_ctl_, 0, 8 * sizeof(unsigned long long), stream_));
+        ESP_CUDA_TRY(cudaMemsetAsync(d_mega_arena_, 0, mega_arena_words_ * sizeof(unsigned long long), stream_));
+        mega_tag_ = mega_cand_ = 0;
+    }
+    a.tag0 = mega_tag_;
+    a.cand0 = mega_cand_;
+    mega_tag_ += used;
+    mega_dirty_ = true;  // until this launch has come back without an error
     if (!ev_begin_) { ESP_CUDA_TRY(cudaEventCreate(&ev_begin_)); ESP_CUDA_TRY(cudaEventCreate(&ev_end_)); }
-    ESP_CUDA_TRY(cudaMemsetAsync(d_mega_ctl_, 0, 8 * sizeof(unsigned long long), stream_));
-    ESP_CUDA_TRY(cudaMemsetAsync(d_mega_arena_, 0, mega_arena_words_ * sizeof(unsigned long long), stream_));
-    ESP_CUDA_TRY(cudaEventRecord(ev_begin_, stream_));
+    if (times) ESP_CUDA_TRY(cudaEventRecord(ev_begin_, stream_));
     void* args[] = {&a};
     ESP_CUDA_TRY(cudaLaunchCooperativeKernel(mega_kernel_for(m_.head_dim, p.wt_layer), dim3(p.n_cta), dim3(kMegaThreads), args, (size_t)p.smem_bytes, stream_));
-    ESP_CUDA_TRY(cudaEventRecord(ev_end_, stream_));
+    if (times) ESP_CUDA_TRY(cudaEventRecord(ev_end_, stream_));
     ESP_CUDA_TRY(cudaMemcpyAsync(h_mega_ctl_, d_mega_ctl_, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream_));
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
     launches_last_step_ = 1;
@@ -2369,14 +2387,25 @@ int32_t Engine::run_mega(int n_steps, int* emitted, float* device_ms, double* fi
            << ": 3 = weight chunk, 4 = ring slot, 5/9 = layer output words, 6 = q/k/v words, 7 = attention sums, 8 = activation words, 10 = arg-max words)";
         return fail(ESP_CUDA_ERR_TIMEOUT, os.str());
     }
-    const int n = (int)h_mega_ctl_[5];
+    mega_cand_ = (a.cand0 + (unsigned)a.first + (unsigned)(h_mega_ctl_[5] & 0xffffffffull)) % 255u;  // right behind the last step that ran
+    mega_dirty_ = false;
+    return ESP_CUDA_OK;
+}
+
+// The greedy loop (at most n_steps emitted tokens; fewer when the end-of-sequence token comes up) of sequence 0 as one
+// cooperative launch.  *emitted receives the number of tokens written to rs_.out.
+int32_t Engine::run_mega(int n_steps, int* emitted, float* device_ms, double* first_token_ms) {
+    int32_t rc = launch_mega(n_steps, nullptr, true);
+    if (rc) return rc;
+    const int n = (int)(h_mega_ctl_[5] & 0xffffffffull);
     if (n < 1 || n > n_steps) return fail(ESP_CUDA_ERR_CUDA, "persistent decode kernel reported an impossible token count");
     if (emitted) *emitted = n;
-    token_times_n_ = a.token_times ? n : 0;
+    const bool have_times = n_steps <= m_.max_seq + 1;
+    token_times_n_ = have_times ? n : 0;
     if (device_ms) ESP_CUDA_TRY(cudaEventElapsedTime(device_ms, ev_begin_, ev_end_));
     if (first_token_ms) *first_token_ms = (double)(h_mega_ctl_[4] - h_mega_ctl_[3]) / 1e6;
     latencies_ms_.clear();
-    if (a.token_times) {
+    if (have_times) {
         std::vector<unsigned long long> tt((size_t)n);
         ESP_CUDA_TRY(cudaMemcpy(tt.data(), d_token_times_, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost));
         unsigned long long prev = h_mega_ctl_[3];  // kernel start
@@ -2384,6 +2413,10 @@ int32_t Engine::run_mega(int n_steps, int* emitted, float* device_ms, double* fi
     }
     h_visible_[0] += n - 1;
     return ESP_CUDA_OK;
+}
+
+bool Engine::mega_usable() const {
+    return mega_ready_ && debug_layer_ < 0 && !(cfg_.flags & (ESP_CUDA_FLAG_NO_MEGAKERNEL | ESP_CUDA_FLAG_NO_GRAPH));
 }
 
 static const void* spec_kernel_for(int head_dim) {

@@ -125,6 +125,8 @@ private:
     LayerWeights layer_weights(int l) const;
     size_t gemv_smem(int type, int K, bool with_tmp) const;
     int32_t build_mega();   // packs the weights for the persistent decode kernel when the model qualifies
+    int32_t launch_mega(int n_steps, const uint32_t* feed, bool times);
+    bool mega_usable() const;
     int32_t run_mega(int n_steps, int* emitted, float* device_ms, double* first_token_ms);
     int32_t ensure_norms2();  // the gain vectors twice over, as the two-position kernel reads them
     int32_t spec_prepare();   // plan, arena and result block of the two-position kernel
@@ -212,8 +214,10 @@ private:
     MegaPlan mega_plan_{};
     uint8_t* d_pack_ = nullptr;
     float* d_norms_ = nullptr;
-    unsigned long long* d_mega_arena_ = nullptr;  // exchange words and counted sums of the persistent kernel (zeroed per launch)
+    unsigned long long* d_mega_arena_ = nullptr;  // exchange words and counted sums of the persistent kernel
     size_t mega_arena_words_ = 0;
+    unsigned mega_tag_ = 0, mega_cand_ = 0;       // numbering of the exchanges, continued from launch to launch
+    bool mega_dirty_ = true;                      // the arena must be cleared before the next launch
     unsigned mega_spin_limit_ = kMegaSpinLimit;   // attempts per device-side wait (test hook: set_wait_limit)
     unsigned long long* d_mega_ctl_ = nullptr;  // [2] error (i32 in the upper half), [3..4] time stamps, [5] tokens emitted
     unsigned long long* h_mega_ctl_ = nullptr;  // pinned mirror

@@ -107,7 +107,7 @@ struct MegaArgs {
     const uint16_t* tok_emb;  // fp16 [vocab][d_model]
     const float2* rope;       // [max_seq][head_dim/2]
     KvLayout kv;
-    // exchange arena (zero at launch)
+    // exchange arena (zero before the first launch; tags keep launches apart, the counted sums are zeroed at the end)
     unsigned long long* x_words;    // [d_model] tagged: output of a layer
     unsigned long long* act_words;  // [hidden] or [n_cta][act_wpc]; tagged: FFN activation
     unsigned long long* qkv_words;  // [n_kv_head][2 * group_items] tagged: post-RoPE q / k / v of one token
@@ -115,12 +115,16 @@ struct MegaArgs {
     unsigned long long* cand_words; // [n_cta][kMegaCandStride] {logit bits, index, 8-bit tag} of each CTA's best row in word 0
     float* hidden_io;         // [d_model] last hidden state of the sequence (in and out)
     int* error;               // [1] 0 = ok
-    unsigned long long* stamps; // [3] globaltimer at kernel start and when the first token is known; number of tokens emitted
+    unsigned long long* stamps; // [3] globaltimer at kernel start and when the first token is known; {last token : 32}{number of tokens emitted : 32}
     unsigned long long* token_times; // optional [n_steps] globaltimer (ns) at which each token became known, or null
     long long* trace;         // optional [kMegaTraceLayer*L + kMegaTraceHead] SM clock stamps of the last step taken by CTA `trace_cta`, or null
     int trace_cta;
     RowState rs;              // row 0 carries pos / tok / n_out / out
     int n_steps;              // tokens to emit at most (>= 1)
+    int first;                // 0: the loop starts with the head (the state holds the last hidden vector); 1: with a forward pass for `tok0`
+    uint32_t tok0;
+    unsigned tag0;            // added to every sequence tag, and cand0 to the candidates' step count: the arena is never cleared
+    unsigned cand0;           // between launches, so the words of earlier launches must not look like this one's
     int pos0;                 // visible tokens at launch
     unsigned spin_limit;      // attempts per wait
 };
@@ -1034,9 +1038,9 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
             auto issue_stage = [&](long long off, int items, int per_chunk, int item_bytes) {
                 for (int i0 = 0; i0 < items; i0 += per_chunk) issue(off + (long long)i0 * item_bytes, min(per_chunk, items - i0) * item_bytes);
             };
-            for (int step = 0; step < a.n_steps; step++) {
+            for (int step = a.first; step < a.first + a.n_steps; step++) {
 #ifdef MEGA_FINE_TRACE
-                p_step = step;
+                p_step = step - a.first;
 #endif
                 if (step > 0) {
                     for (int l = 0; l < L; l++) {
@@ -1076,7 +1080,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         if (lane == 0) {
             auto chunks_of = [](int items, int per_chunk) { return (items + per_chunk - 1) / per_chunk; };
             const unsigned per_layer = (w.in_group ? chunks_of(w.s1_n, p.s1_ipc) + chunks_of(p.rpb, p.s2_rpc) : 0) + chunks_of(w.h_n, p.s3a_ipc) + chunks_of(w.d_n, p.s3b_rpc);
-            const unsigned total = (unsigned)a.n_steps * chunks_of(w.v_n, p.head_rpc) + (unsigned)(a.n_steps - 1) * L * per_layer;
+            const unsigned total = (unsigned)a.n_steps * chunks_of(w.v_n, p.head_rpc) + (unsigned)(a.n_steps - 1 + a.first) * L * per_layer;
             MegaCursor k;
             for (unsigned i = 0; i < total; i++) {
                 unsigned spins = 0;
@@ -1107,12 +1111,12 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
 #endif
     int n_stamp = 0;
     auto stamp = [&](int step) {
-        if (a.trace && (int)blockIdx.x == a.trace_cta && tid == 0 && step == a.n_steps - 1) a.trace[n_stamp++] = clock64();
+        if (a.trace && (int)blockIdx.x == a.trace_cta && tid == 0 && step == a.first + a.n_steps - 1) a.trace[n_stamp++] = clock64();
     };
     MegaCursor c;        // ring position, advances in lock step with the producer's
     unsigned n_chunk = 0;  // chunks consumed so far
     int pos = a.pos0;    // visible tokens
-    uint32_t tok = 0;
+    uint32_t tok = a.tok0;
     int emitted = 0;
     int par = 0;         // which half of s.partial the next chunk's sums go to
     constexpr int half = HD / 2;
@@ -1174,12 +1178,12 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         return partial;
     };
 
-    for (int step = 0; step < a.n_steps; step++) {
+    for (int step = a.first; step < a.first + a.n_steps; step++) {
         if (step > 0) {
             const uint16_t* emb_row = a.tok_emb + (size_t)tok * d;
             if (tid < half) s.rope[tid] = a.rope[(size_t)pos * half + tid];  // published by the barrier of the first norm
             for (int l = 0; l < L; l++) {
-                const unsigned seq = (unsigned)((step - 1) * L + l + 1);  // tag of everything this layer publishes
+                const unsigned seq = a.tag0 + (unsigned)((step - 1) * L + l + 1);  // tag of everything this layer publishes
                 float inv = 0.f;
 #ifdef MEGA_FINE_TRACE
                 fine_layer = l; fine_step = step;
@@ -1359,7 +1363,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
             if (step == 0) {
                 for (int k = tid; k < d; k += kMegaConsumers) stage_x(s.xraw, d, head_digits, k, __ldcg(a.hidden_io + k), __ldg(fin_gain + k), ss);
             } else {
-                mega_read_words(a, s, a.x_words, d, (unsigned)(step * L), 9, fin_gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, head_digits, k, v0, v1, g0, g1, ss); });
+                mega_read_words(a, s, a.x_words, d, a.tag0 + (unsigned)(step * L), 9, fin_gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, head_digits, k, v0, v1, g0, g1, ss); });
             }
             release_pending();  // the W2 chunk of the last layer
             consumer_sync();  // the RMSNorm scale is positive: the arg-max does not need it
@@ -1383,7 +1387,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         // CTA-wide best (larger value first, then smaller index), published as one word per CTA:
         // [ordered logit bits : 32][0xffffff - index : 24][tag : 8].  The tag is the same in every word of a step, so the
         // largest word is the best candidate; 148 consecutive words are ten cache lines for every reader.
-        const unsigned long long tag8 = (unsigned long long)(step % 255 + 1);
+        const unsigned long long tag8 = (unsigned long long)((a.cand0 + (unsigned)step) % 255u + 1u);
         {
             unsigned long long k = best_i != 0x7fffffff ? ((unsigned long long)ordered_bits(best_v) << 32) | ((unsigned long long)(0xffffffu - (unsigned)best_i) << 8) : 0ull;
 #pragma unroll
@@ -1430,13 +1434,13 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
 #ifdef MEGA_FINE_TRACE
         if (a.trace && tid == 0 && step == a.n_steps - 1) { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); a.trace[800 + blockIdx.x] = (long long)t; }
 #endif
-        emitted = step + 1;
+        emitted = step - a.first + 1;
         if (blockIdx.x == 0 && tid == 0) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (step == 0) a.stamps[1] = t;
-            a.rs.out[step] = tok;
-            if (a.token_times) a.token_times[step] = t;
+            if (emitted == 1) a.stamps[1] = t;
+            a.rs.out[emitted - 1] = tok;
+            if (a.token_times) a.token_times[emitted - 1] = t;
         }
         // Llama rule: the end-of-sequence token is emitted, then the loop stops (every CTA sees the same token)
         const bool eos = m.eos_token >= 0 && tok == (uint32_t)m.eos_token;
@@ -1453,9 +1457,12 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
             a.rs.tok[0] = tok;
             a.rs.next[0] = tok;
             a.rs.n_out[0] = emitted;
-            a.stamps[2] = (unsigned long long)emitted;
+            a.stamps[2] = (unsigned long long)emitted | ((unsigned long long)tok << 32);
         }
     }
+    // The counted sums go back to zero for the next launch: the token exchange above proves that every contribution has
+    // arrived and every CTA has read the last layer's totals.
+    for (int k = w.d_begin + tid; k < w.d_begin + w.d_n; k += kMegaConsumers) a.mid_sums[k] = 0ull;
 }
 
 // ------------------------------------------------------------------------------------------------ pack builder
