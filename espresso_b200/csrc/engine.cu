@@ -3,7 +3,7 @@
 #include "engine.h"
 #include "batch_kernels.cuh"
 #include "tc_gemm.cuh"
-#include "stream_gemm.cuh"
+#include "pair_gemm.cuh"
 #include "spec_kernel.cuh"
 #include "prefill_attention.cuh"
 #include "decode_attention.cuh"
@@ -49,9 +49,7 @@ static int32_t fail(int32_t code, const std::string& msg) {
 }
 
 int32_t tc_make_map(CUtensorMap* map, const void* base, bool bf16, uint64_t rows, uint64_t cols, uint32_t box_rows);
-int tc_tile_for(int rows);
-TcPlan tc_plan(int w_tiles, int rows, int kb, bool may_split_k, bool dual, int sms);
-cudaError_t tc_launch(const TcPlan& plan, bool dual, const CUtensorMap* const* mw, const CUtensorMap& mx, TcArgs a, cudaStream_t s);
+cudaError_t pg_launch(const CUtensorMap* const* mw, const CUtensorMap& mx, PgArgs a, int sms, cudaStream_t s);
 // tensor-parallel NCCL fallback: the residual joins rank 0's partial sum
 __global__ void k_add_rows(float* dst, const float* src, int n4) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -837,7 +835,7 @@ int32_t Engine::check_ready(const char* what) const {
 int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
     if (tp_size_ > 1 && !tc_ready_) return fail(ESP_CUDA_ERR_STATE, "tensor parallelism needs 16-bit weights with 64-aligned shard sizes");
     if (stream_path(rows)) return launch_step_stream(rows, mode, s, profile);
-    if (tc_ready_ && (rows >= kTcMinRows || tp_size_ > 1)) return launch_step_tc(rows, mode, s);
+    if (tc_ready_ && rows > kSgMaxRows) return launch_step_wide(rows, mode, s);
     const bool gpt2 = m_.arch == ARCH_GPT2;
     const int cap = sm_count_ * 2;  // one wave: the stage kernels hold ~120 registers, two CTAs per SM
     int launches = 0;
@@ -1581,26 +1579,6 @@ __global__ void __launch_bounds__(256) k_tp_sum_peers(const TpSumArgs a) {
     }
 }
 
-// SiLU(gate) * up over fp32 rows -> the 16-bit operand rows of the W2 product.  Used where the gate and up products are
-// cut along K (a narrow tensor-parallel shard), so that their sums are complete only after the product kernel.
-struct SwigluArgs {
-    const float* gate;  // [rows][hidden]
-    const float* up;
-    uint16_t* dst;      // [rows][hidden]
-    float* debug;       // optional fp32 capture of row 0
-    int hidden, n4, bf16;
-};
-__global__ void __launch_bounds__(256) k_swiglu_rows(const SwigluArgs a) {
-    pdl_launch_dependents();
-    pdl_wait();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n4; i += gridDim.x * blockDim.x) {
-        const float4 g = __ldcg(reinterpret_cast<const float4*>(a.gate) + i), u = __ldcg(reinterpret_cast<const float4*>(a.up) + i);
-        const float v0 = silu_fast(g.x) * u.x, v1 = silu_fast(g.y) * u.y, v2 = silu_fast(g.z) * u.z, v3 = silu_fast(g.w) * u.w;
-        reinterpret_cast<uint2*>(a.dst)[i] = make_uint2(pack16x2(v0, v1, a.bf16), pack16x2(v2, v3, a.bf16));
-        if (a.debug && 4 * i < a.hidden) *reinterpret_cast<float4*>(a.debug + 4 * i) = make_float4(v0, v1, v2, v3);
-    }
-}
-
 // {all-reduces over peer memory, ns from arrival to the last sum, ns of that spent waiting for the peers} since the
 // previous call (zeros when the group uses NCCL).
 int32_t Engine::tp_sum_stats(unsigned long long* out3) {
@@ -1746,7 +1724,6 @@ int32_t Engine::build_tc() {
     if ((rc = dev_alloc(owned_, &xh_h_, (size_t)tc_rows_alloc_ * m_.hidden))) return rc;
     if ((rc = dev_alloc(owned_, &kraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &vraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
-    if ((rc = dev_alloc(owned_, &up_, (size_t)max_rows_ * m_.hidden))) return rc;
     if ((rc = dev_alloc(owned_, &d_tc_error_, 4))) return rc;
     if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, kSgMaxRows) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
     if (tp_size_ > 1 && (rc = dev_alloc(owned_, &tp_partial_, (size_t)max_rows_ * m_.d_model))) return rc;
@@ -1770,7 +1747,7 @@ int32_t Engine::tc_operands() {
             ESP_CUDA_TRY(cudaGetLastError());
             base = t.shadow16;
         }
-        int32_t rc = tc_make_map(&t.map, base, tc_bf16_, t.rows, t.cols, kTcHalf);
+        int32_t rc = tc_make_map(&t.map, base, tc_bf16_, t.rows, t.cols, 128);
         if (rc) return rc;
         if ((rc = tc_make_map(&t.map64, base, tc_bf16_, t.rows, t.cols, kSgHalf))) return rc;
         t.has_map = true;
@@ -1826,6 +1803,40 @@ bool Engine::stream_path(int rows) const {
     // A quantised model's single rows stay on the kernels that read the GGUF blocks themselves (the persistent kernel and the
     // row-wise GEMVs): an engine that only ever decodes one sequence then never builds the fp16 expansion.
     return tc_ready_ && rows <= kSgMaxRows && !(tc_quant_ && rows == 1);
+}
+
+// Final norm, LM head and arg-max of `rows` rows; the last CTA turns the maxima into tokens.
+int32_t Engine::launch_head_stream(int rows, int mode, int parts, cudaStream_t s, int& launches) {
+    const bool gpt2 = m_.arch == ARCH_GPT2;
+    // (the head has hundreds of weight tiles and always takes the norm kernel)
+    PrepArgs p{};
+    p.m = m_; p.rs = rs_; p.src = act_.hidden; p.K = m_.d_model; p.norm = gpt2 ? NORM_LAYER : NORM_RMS; p.dst = xh_d_; p.bf16 = tc_bf16_; p.parts = parts;
+    p.g = tensors_.at(gpt2 ? "final_norm_gamma" : "rms_final").f32;
+    p.b = gpt2 ? tensors_.at("final_norm_beta").f32 : nullptr;
+    ESP_CUDA_TRY(launch_pdl(k_prep_rows, dim3(rows), dim3(kThreads), 0, s, p));
+    const DeviceTensor& lh = tensors_.at("lm_head");
+    if (!lh.has_map) return fail(ESP_CUDA_ERR_CUDA, "tensor map missing for the batched path");
+    const int finalize = ((mode & STEP_FEEDBACK) ? 1 : 0) | ((mode & STEP_FORWARD) ? 2 : 0);
+    const SgPlan plan = sg_plan((lh.rows + kSgRows - 1) / kSgRows, rows, m_.d_model / kTcBlockK, parts, false, sm_count_);
+    const CUtensorMap* mx = activation_map(xh_d_, m_.d_model, plan.n_cols);
+    if (!mx) return fail(ESP_CUDA_ERR_CUDA, "tensor map missing for the batched path");
+    const CUtensorMap* maps[3] = {&lh.map64, &lh.map64, &lh.map64};
+    SgArgs a{};
+    a.n_groups = 1; a.g[0].M = lh.rows; a.K = m_.d_model; a.rows = rows; a.bf16 = tc_bf16_; a.error = d_tc_error_; a.m = m_; a.rs = rs_; a.eps = m_.eps;
+    a.logits = (cfg_.flags & ESP_CUDA_FLAG_KEEP_LOGITS) ? act_.logits : nullptr;
+    a.row_offset = tp_rank_ * m_.vocab;
+    a.finalize = tp_size_ > 1 ? -1 : finalize;
+    ESP_CUDA_TRY(sg_launch(plan, SG_HEAD, maps, *mx, a, s));
+    launches += 2;
+    if (tp_size_ > 1) {
+        int32_t rc = all_reduce(rs_.best, rs_.best, (size_t)rows, false, s);  // max of (value, ~index) keys
+        if (rc) return rc;
+        GemvArgs fin{};
+        fin.m = m_; fin.m.vocab = vocab_global_; fin.rows = rows; fin.rs = rs_; fin.finalize_mode = finalize;
+        ESP_CUDA_TRY(launch_pdl(k_head_done, dim3(1), dim3(256), 0, s, fin));
+        launches++;
+    }
+    return ESP_CUDA_OK;
 }
 
 // One pass over the model for up to kSgMaxRows rows with the streamed products (stream_gemm.cuh): per layer q/k/v (norm,
@@ -1962,23 +1973,7 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
         }
     }
     if (mode & STEP_HEAD) {
-        const Norm nf{tensors_.at(gpt2 ? "final_norm_gamma" : "rms_final").f32, gpt2 ? tensors_.at("final_norm_beta").f32 : nullptr};
-        // (the head has hundreds of weight tiles and always takes the norm kernel)
-        if ((rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, nf.g, nf.b, xh_d_))) return rc;
-        const DeviceTensor& lh = tensors_.at("lm_head");
-        const int finalize = ((mode & STEP_FEEDBACK) ? 1 : 0) | ((mode & STEP_FORWARD) ? 2 : 0);
-        SgArgs ha{};
-        ha.logits = (cfg_.flags & ESP_CUDA_FLAG_KEEP_LOGITS) ? act_.logits : nullptr;
-        ha.row_offset = tp_rank_ * m_.vocab;
-        ha.finalize = tp_size_ > 1 ? -1 : finalize;
-        if ((rc = gemm({{&lh, nullptr, 0, nullptr}}, tiles_of(lh.rows), xh_d_, nullptr, SG_HEAD, ha))) return rc;
-        if (tp_size_ > 1) {
-            if ((rc = all_reduce(rs_.best, rs_.best, (size_t)rows, false, s))) return rc;  // max of (value, ~index) keys
-            GemvArgs fin{};
-            fin.m = m_; fin.m.vocab = vocab_global_; fin.rows = rows; fin.rs = rs_; fin.finalize_mode = finalize;
-            ESP_CUDA_TRY(launch_pdl(k_head_done, dim3(1), dim3(256), 0, s, fin));
-            launches++;
-        }
+        if ((rc = launch_head_stream(rows, mode, parts, s, launches))) return rc;
     } else if (mode & STEP_FORWARD) {
         ESP_CUDA_TRY(launch_pdl(k_bump, dim3((rows + 63) / 64), dim3(64), 0, s, rs_, rows));
         launches++;
@@ -1989,18 +1984,23 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
     return ESP_CUDA_OK;
 }
 
-// One pass over the model for `rows` rows with the matrix products on the tensor cores: every weight matrix is
-// streamed once per pass whatever the row count.
-int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
+int32_t Engine::launch_attention_prefill(const PrefillAttArgs& pa, cudaStream_t s) {
+    const dim3 grid(n_runs_, m_.n_head);
+    if (m_.head_dim == 32) ESP_CUDA_TRY(launch_pdl(k_attention_prefill<32>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<32>(), s, pa));
+    else if (m_.head_dim == 64) ESP_CUDA_TRY(launch_pdl(k_attention_prefill<64>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<64>(), s, pa));
+    else ESP_CUDA_TRY(launch_pdl(k_attention_prefill<128>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<128>(), s, pa));
+    return ESP_CUDA_OK;
+}
+
+// One pass over the model for more rows than the streamed products take (prompt passes, very wide batches): products on SM
+// pairs (pair_gemm.cuh), element-wise stages between them.
+int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
     const bool gpt2 = m_.arch == ARCH_GPT2;
-    if (!tc_tile_for(rows)) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "too many rows for one tensor-core pass");
     tp_parity_ = 0;  // a step holds an even number of all-reduces: every step starts on partial buffer 0
     int launches = 0;
     float* dbg = debug_layer_ >= 0 ? d_debug_ : nullptr;
-    const int q = m_.q_dim, kv = m_.kv_dim, d = m_.d_model, h = m_.hidden;
-    auto tiles_of = [](int M) { return (M + kTcHalf - 1) / kTcHalf; };
-    auto prep = [&](const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst, bool from_emb, bool zero_qkv, bool zero_ffn = false,
-                    float* zero_partial = nullptr) -> int32_t {
+    const int q = m_.q_dim, kv = m_.kv_dim, d = m_.d_model, h = m_.hidden, hd = m_.head_dim;
+    auto prep = [&](const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst, bool from_emb = false) -> int32_t {
         PrepArgs p{};
         p.m = m_; p.rs = rs_; p.src = src; p.hidden_out = act_.hidden; p.K = K; p.norm = norm; p.g = g; p.b = b; p.dst = dst; p.bf16 = tc_bf16_; p.parts = 1;
         p.from_embedding = from_emb ? 1 : 0;
@@ -2010,28 +2010,16 @@ int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
             p.pos_emb = gpt2 ? static_cast<const uint16_t*>(tensors_.at("embeddings/position").data) : nullptr;
             p.emb_type = te.type == ESP_CUDA_BF16 ? WT_BF16 : WT_F16;
         }
-        if (zero_qkv) {
-            p.zero[0] = act_.q; p.zero_n[0] = q;
-            p.zero[1] = kraw_; p.zero_n[1] = kv;
-            p.zero[2] = vraw_; p.zero_n[2] = kv;
-        }
-        if (zero_ffn) {
-            p.zero[0] = act_.act; p.zero_n[0] = h;
-            p.zero[1] = up_; p.zero_n[1] = h;
-        }
-        if (zero_partial) { p.zero[3] = zero_partial; p.zero_n[3] = d; }
         ESP_CUDA_TRY(launch_pdl(k_prep_rows, dim3(rows), dim3(kThreads), 0, s, p));
         launches++;
         return ESP_CUDA_OK;
     };
     struct Part { const DeviceTensor* W; float* out; int ldo; const float* bias; };
-    // one launch over up to three weight matrices that read the same operand rows
-    auto gemm = [&](const TcPlan& plan, bool dual, std::initializer_list<Part> parts, const uint16_t* xbuf, int epi, uint16_t* out16, int ld16,
-                    float* capture) -> int32_t {
+    auto gemm = [&](std::initializer_list<Part> parts, const uint16_t* xbuf, int epi, uint16_t* out16, int ld16, float* capture, bool all_rows = false) -> int32_t {
         const int K = parts.begin()->W->cols;
-        const CUtensorMap* mx = activation_map(xbuf, K, plan.x_rows);
+        const CUtensorMap* mx = activation_map(xbuf, K, 128);
         if (!mx) return fail(ESP_CUDA_ERR_CUDA, "tensor map missing for the batched path");
-        TcArgs a{};
+        PgArgs a{};
         const CUtensorMap* maps[3] = {&parts.begin()->W->map, &parts.begin()->W->map, &parts.begin()->W->map};
         int g = 0;
         for (const Part& pt : parts) {
@@ -2040,78 +2028,48 @@ int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
             a.g[g].M = pt.W->rows; a.g[g].out = pt.out; a.g[g].ldo = pt.ldo; a.g[g].bias = pt.bias;
             g++;
         }
-        a.n_groups = dual ? 1 : g;
-        a.K = K; a.n_valid = rows; a.epilogue = epi; a.active = rs_.active; a.error = d_tc_error_; a.bf16 = tc_bf16_;
-        a.out16 = out16; a.ld16 = ld16; a.debug = capture;
-        a.row_offset = epi == TC_HEAD ? tp_rank_ * m_.vocab : 0;
-        if (epi == TC_HEAD) { a.best = rs_.best; a.logits = (cfg_.flags & ESP_CUDA_FLAG_KEEP_LOGITS) ? act_.logits : nullptr; }
-        ESP_CUDA_TRY(tc_launch(plan, dual, maps, *mx, a, s));
+        a.n_groups = g; a.K = K; a.rows = rows; a.epilogue = epi; a.bf16 = tc_bf16_; a.out16 = out16; a.ld16 = ld16; a.debug = capture; a.error = d_tc_error_;
+        a.active = all_rows ? nullptr : rs_.active;
+        ESP_CUDA_TRY(pg_launch(maps, *mx, a, sm_count_, s));
         launches++;
         return ESP_CUDA_OK;
     };
-    // hidden += W . x (+ bias).  Tensor parallel: W holds this rank's slice of the input dimension, so the product
-    // is a partial sum; rank 0's partial also carries the residual and the bias, and one all-reduce leaves the
-    // new residual stream on every rank.
+    // hidden += W . x (+ bias); tensor parallel as in launch_step_stream
     auto project = [&](const DeviceTensor& W, const uint16_t* xbuf, const float* bias) -> int32_t {
-        const TcPlan plan = tc_plan(tiles_of(W.rows), rows, W.cols / kTcBlockK, true, false, sm_count_);
-        if (tp_size_ <= 1) return gemm(plan, false, {{&W, act_.hidden, d, bias}}, xbuf, TC_RESIDUAL, nullptr, 0, nullptr);
-        int32_t prc;
+        if (tp_size_ <= 1) return gemm({{&W, act_.hidden, d, bias}}, xbuf, PG_RESIDUAL, nullptr, 0, nullptr);
         float* partial = tp_current_partial();
-        if (tp_peer_ready_) {
-            // peer-memory sum: every rank's partial is the bare product (rank 0's carries the bias), cleared by the norm
-            // kernel before it where K slices add into it; the sum kernel adds the partials to the residual stream
-            if ((prc = gemm(plan, false, {{&W, partial, d, tp_rank_ == 0 ? bias : nullptr}}, xbuf, TC_STORE, nullptr, 0, nullptr))) return prc;
-            launches++;
-            return tp_sum_peers(act_.hidden, rows, s);
-        }
+        int32_t rc = gemm({{&W, partial, d, tp_rank_ == 0 ? bias : nullptr}}, xbuf, PG_STORE, nullptr, 0, nullptr, true);
+        if (rc) return rc;
+        if (tp_peer_ready_) { launches++; return tp_sum_peers(act_.hidden, rows, s); }
         if (tp_rank_ == 0) {
-            ESP_CUDA_TRY(cudaMemcpyAsync(partial, act_.hidden, sizeof(float) * (size_t)rows * d, cudaMemcpyDeviceToDevice, s));
-            if ((prc = gemm(plan, false, {{&W, partial, d, bias}}, xbuf, TC_RESIDUAL, nullptr, 0, nullptr))) return prc;
-        } else {
-            if (plan.splits > 1) ESP_CUDA_TRY(cudaMemsetAsync(partial, 0, sizeof(float) * (size_t)rows * d, s));
-            if ((prc = gemm(plan, false, {{&W, partial, d, nullptr}}, xbuf, TC_STORE, nullptr, 0, nullptr))) return prc;
+            k_add_rows<<<(rows * d / 4 + 255) / 256, 256, 0, s>>>(partial, act_.hidden, rows * d / 4);
+            launches++;
         }
         return all_reduce(partial, act_.hidden, (size_t)rows * d, true, s);
     };
     auto copy_dbg = [&](const float* src, int offset, int n) {
         if (dbg) { k_copy_debug<<<(n + 255) / 256, 256, 0, s>>>(src, dbg + offset, n); launches++; }
     };
-    const bool att_ok_hd = m_.head_dim == 32 || m_.head_dim == 64 || m_.head_dim == 128;
+    const bool att_ok_hd = hd == 32 || hd == 64 || hd == 128;
     int32_t rc;
     if (mode & STEP_FORWARD) {
-        const TcPlan plan_qkv = tc_plan(tiles_of(q) + 2 * tiles_of(kv), rows, d / kTcBlockK, true, false, sm_count_);
-        const TcPlan plan_up = tc_plan(tiles_of(h), rows, d / kTcBlockK, false, !gpt2, sm_count_);
-        // The fused gate/up product (activation in the epilogue) cannot be cut along K.  Where its weight tiles cover less
-        // than half of the SMs (a narrow tensor-parallel shard, a small model) the rest would idle while each CTA streams
-        // its tile at one SM's pace; there the two matrices run as a K-sliced grouped product into fp32 rows, and a small
-        // kernel applies SiLU(gate) * up.
-        const bool split_up = !gpt2 && 2 * tiles_of(h) * ((rows + kTcBatch - 1) / kTcBatch) <= sm_count_ && (h & 3) == 0;
-        const TcPlan plan_up2 = tc_plan(2 * tiles_of(h), rows, d / kTcBlockK, true, false, sm_count_);
         for (int l = 0; l < m_.n_layer; l++) {
-            const std::string pre = "layers/" + std::to_string(l) + "/";
-            const LayerWeights lw = layer_weights(l);
+            const LayerTensors& t = layer_tensors_[l];
+            const LayerWeights& lw = t.w;
             const bool cap = dbg && l == debug_layer_;
-            if ((rc = prep(l == 0 ? nullptr : act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, lw.norm1_g, lw.norm1_b, xh_d_, l == 0, plan_qkv.splits > 1, false,
-                           tp_peer_ready_ ? tp_current_partial() : nullptr)))
-                return rc;
-            if ((rc = gemm(plan_qkv, false,
-                           {{&tensors_.at(pre + "wq"), act_.q, q, lw.bq}, {&tensors_.at(pre + "wk"), kraw_, kv, lw.bk}, {&tensors_.at(pre + "wv"), vraw_, kv, lw.bv}},
-                           xh_d_, TC_STORE, nullptr, 0, nullptr)))
-                return rc;
+            if ((rc = prep(l == 0 ? nullptr : act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, lw.norm1_g, lw.norm1_b, xh_d_, l == 0))) return rc;
+            if ((rc = gemm({{t.wq, act_.q, q, lw.bq}, {t.wk, kraw_, kv, lw.bk}, {t.wv, vraw_, kv, lw.bv}}, xh_d_, PG_STORE, nullptr, 0, nullptr))) return rc;
             RopeArgs ra{};
             ra.m = m_; ra.rs = rs_; ra.kv = kv_; ra.q = act_.q; ra.k_raw = kraw_; ra.v_raw = vraw_; ra.rope = gpt2 ? nullptr : d_rope_; ra.layer = l;
             ra.debug = cap ? dbg : nullptr;
-            if (qk_norm_) { ra.q_norm = tensors_.at(pre + "q_norm").f32; ra.k_norm = tensors_.at(pre + "k_norm").f32; }
+            ra.q_norm = t.q_norm; ra.k_norm = t.k_norm;
             ESP_CUDA_TRY(launch_pdl(k_rope_append, dim3(rows, (q / 2 + kv + kThreads - 1) / kThreads), dim3(kThreads), 0, s, ra));
             launches++;
             if ((mode & STEP_TILED_ATT) && att_ok_hd) {
                 PrefillAttArgs pa{};
-                pa.m = m_; pa.rs = rs_; pa.kv = kv_; pa.q = act_.q; pa.ctx16 = xh_q_; pa.bf16 = tc_bf16_; pa.layer = l; pa.runs = d_runs_;
+                pa.m = m_; pa.kv = kv_; pa.q = act_.q; pa.ctx16 = xh_q_; pa.bf16 = tc_bf16_; pa.layer = l; pa.runs = d_runs_;
                 pa.debug = cap ? dbg + q + 2 * kv : nullptr;
-                const dim3 grid(n_runs_, m_.n_head);
-                if (m_.head_dim == 32) ESP_CUDA_TRY(launch_pdl(k_attention_prefill<32>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<32>(), s, pa));
-                else if (m_.head_dim == 64) ESP_CUDA_TRY(launch_pdl(k_attention_prefill<64>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<64>(), s, pa));
-                else ESP_CUDA_TRY(launch_pdl(k_attention_prefill<128>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<128>(), s, pa));
+                if ((rc = launch_attention_prefill(pa, s))) return rc;
                 launches++;
             } else if (att_ok_hd) {
                 DecodeAttArgs da{};
@@ -2125,45 +2083,21 @@ int32_t Engine::launch_step_tc(int rows, int mode, cudaStream_t s) {
                 aa.a.logits = nullptr; aa.a.debug = cap ? dbg : nullptr; aa.a.debug_layer = debug_layer_;
                 ESP_CUDA_TRY(launch_pdl(k_attention, dim3(m_.n_head, rows, n_splits_), dim3(kAttThreads), 0, s, aa));
                 launches++;
-                if ((rc = prep(act_.ctx, q, NORM_NONE, nullptr, nullptr, xh_q_, false, false))) return rc;
+                if ((rc = prep(act_.ctx, q, NORM_NONE, nullptr, nullptr, xh_q_))) return rc;
             }
-            if ((rc = project(tensors_.at(pre + "wo"), xh_q_, lw.bo))) return rc;
+            if ((rc = project(*t.wo, xh_q_, lw.bo))) return rc;
             if (cap) copy_dbg(act_.hidden, 2 * q + 2 * kv, d);
-            if ((rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, lw.norm2_g, lw.norm2_b, xh_d_, false, false, split_up && plan_up2.splits > 1,
-                           tp_peer_ready_ ? tp_current_partial() : nullptr)))
-                return rc;
-            // up projection with the activation in the epilogue: GELU(w1 x + b1), or SiLU(w1 x) * (w3 x) from two accumulators
+            if ((rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, lw.norm2_g, lw.norm2_b, xh_d_))) return rc;
             float* capture = cap ? dbg + 2 * q + 2 * kv + d : nullptr;
-            if (gpt2) {
-                if ((rc = gemm(plan_up, false, {{&tensors_.at(pre + "w1"), nullptr, 0, lw.b1}}, xh_d_, TC_GELU16, xh_h_, h, capture))) return rc;
-            } else if (split_up) {
-                if ((rc = gemm(plan_up2, false, {{&tensors_.at(pre + "w1"), act_.act, h, nullptr}, {&tensors_.at(pre + "w3"), up_, h, nullptr}}, xh_d_, TC_STORE,
-                               nullptr, 0, nullptr)))
-                    return rc;
-                SwigluArgs sa{};
-                sa.gate = act_.act; sa.up = up_; sa.dst = xh_h_; sa.debug = capture; sa.hidden = h; sa.n4 = rows * h / 4; sa.bf16 = tc_bf16_;
-                ESP_CUDA_TRY(launch_pdl(k_swiglu_rows, dim3(std::max(1, std::min(4 * sm_count_, (sa.n4 + 255) / 256))), dim3(256), 0, s, sa));
-                launches++;
-            } else if ((rc = gemm(plan_up, true, {{&tensors_.at(pre + "w1"), nullptr, 0, nullptr}, {&tensors_.at(pre + "w3"), nullptr, 0, nullptr}}, xh_d_,
-                                  TC_SWIGLU16, xh_h_, h, capture)))
-                return rc;
-            if ((rc = project(tensors_.at(pre + "w2"), xh_h_, lw.b2))) return rc;
+            if (gpt2) rc = gemm({{t.w1, nullptr, 0, lw.b1}}, xh_d_, PG_GELU, xh_h_, h, capture);
+            else rc = gemm({{t.w1, nullptr, 0, nullptr}, {t.w3, nullptr, 0, nullptr}}, xh_d_, PG_SWIGLU, xh_h_, h, capture);
+            if (rc) return rc;
+            if ((rc = project(*t.w2, xh_h_, lw.b2))) return rc;
             if (cap) copy_dbg(act_.hidden, 2 * q + 2 * kv + d + h, d);
         }
     }
-    GemvArgs fin{};
-    fin.m = m_; fin.rows = rows; fin.rs = rs_;
     if (mode & STEP_HEAD) {
-        if ((rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, tensors_.at(gpt2 ? "final_norm_gamma" : "rms_final").f32,
-                       gpt2 ? tensors_.at("final_norm_beta").f32 : nullptr, xh_d_, false, false))) return rc;
-        const DeviceTensor& lh = tensors_.at("lm_head");
-        const TcPlan plan_head = tc_plan(tiles_of(lh.rows), rows, d / kTcBlockK, false, false, sm_count_);
-        if ((rc = gemm(plan_head, false, {{&lh, nullptr, 0, nullptr}}, xh_d_, TC_HEAD, nullptr, 0, nullptr))) return rc;
-        if (tp_size_ > 1 && (rc = all_reduce(rs_.best, rs_.best, (size_t)rows, false, s))) return rc;  // max of (value, ~index) keys
-        fin.m.vocab = vocab_global_;
-        fin.finalize_mode = ((mode & STEP_FEEDBACK) ? 1 : 0) | ((mode & STEP_FORWARD) ? 2 : 0);
-        ESP_CUDA_TRY(launch_pdl(k_head_done, dim3(1), dim3(256), 0, s, fin));
-        launches++;
+        if ((rc = launch_head_stream(rows, mode, 1, s, launches))) return rc;
     } else if (mode & STEP_FORWARD) {
         ESP_CUDA_TRY(launch_pdl(k_bump, dim3((rows + 63) / 64), dim3(64), 0, s, rs_, rows));
         launches++;

@@ -41,6 +41,7 @@ struct LayerTensors {
 };
 
 struct DecodeAttArgs;
+struct PrefillAttArgs;
 
 struct Checkpoint {
     int visible = 0;
@@ -110,7 +111,9 @@ private:
                         const int* limit, bool zero_out_counts);
     int32_t submit(int rows, int mode);                  // graph replay or direct launch
     int32_t launch_step(int rows, int mode, cudaStream_t s, bool profile);
-    int32_t launch_step_tc(int rows, int mode, cudaStream_t s);  // batched path: tensor-core GEMMs + element-wise stages
+    int32_t launch_step_wide(int rows, int mode, cudaStream_t s);  // more rows: products on SM pairs, element-wise stages
+    int32_t launch_head_stream(int rows, int mode, int parts, cudaStream_t s, int& launches);
+    int32_t launch_attention_prefill(const PrefillAttArgs& pa, cudaStream_t s);
     int32_t launch_step_stream(int rows, int mode, cudaStream_t s, bool profile);  // up to kSgMaxRows rows: streamed products, fused stages
     bool stream_path(int rows) const;
     int32_t launch_attention_decode(const DecodeAttArgs& a, int rows, cudaStream_t s);
@@ -203,7 +206,7 @@ private:
     std::vector<LayerTensors> layer_tensors_;
     int tc_rows_alloc_ = 0;
     uint16_t *xh_d_ = nullptr, *xh_q_ = nullptr, *xh_h_ = nullptr;  // 16-bit operand rows [tc_rows_alloc_][K]
-    float *kraw_ = nullptr, *vraw_ = nullptr, *up_ = nullptr;
+    float *kraw_ = nullptr, *vraw_ = nullptr;
     float* d_last_hidden_ = nullptr;  // [max_batch][d_model] last hidden state per sequence while a batch of prompts is fed
     float2* row_stat_ = nullptr;      // [rows][d_model / 128] statistics of the residual stream (streamed products)
     int* d_tc_error_ = nullptr;

@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
 
     if (warp == 1) {
         // ---------------- MMA issuer (see elect_one for the shape of this loop) ----------------
-        const uint32_t idesc = umma_idesc_f16(a.n_cols, a.bf16);
+        const uint32_t idesc = umma_idesc_f16(kSgRows, a.n_cols, a.bf16);
         // Everything the loop needs is kept up by counting; the next stage's barrier is tested before this stage's MMAs.
         const uint64_t d_first = umma_smem_desc_sw128(tiles);
         const uint32_t d_step = (uint32_t)stage_bytes >> 4;

@@ -1,7 +1,7 @@
 // Host side of the tensor-core GEMM: TMA tensor maps, launch dispatch over the batch tile width, and the
 // stand-alone entry point used for parity checks and tensor-pipe measurements.
 #include "engine.h"
-#include "stream_gemm.cuh"
+#include "pair_gemm.cuh"
 
 namespace esp {
 
@@ -40,76 +40,6 @@ int32_t tc_make_map(CUtensorMap* map, const void* base, bool bf16, uint64_t rows
         return esp::fail(ESP_CUDA_ERR_CUDA, os.str());
     }
     return ESP_CUDA_OK;
-}
-
-// Rows of the activation TMA box for `rows` batch rows (one batch tile holds at most 128).
-int tc_tile_for(int rows) {
-    for (int t : {16, 32, 64, 128})
-        if (rows <= t) return t;
-    return 128;
-}
-
-// Launch shape for a product with `w_tiles` 128-row weight tiles, `rows` batch rows and `kb` 64-wide K blocks on
-// `sms` SMs.  A large matrix runs two weight tiles per CTA (256 weight rows per MMA) over all of K; a small one is
-// cut along K (a slice keeps at least 3 K blocks; wide batches take fewer slices, measured), and goes to one tile
-// per CTA, until the grid covers the SMs.
-TcPlan tc_plan(int w_tiles, int rows, int kb, bool may_split_k, bool dual, int sms) {
-    TcPlan p;
-    p.x_rows = tc_tile_for(std::min(rows, kTcBatch));
-    p.n_tiles = (rows + kTcBatch - 1) / kTcBatch;
-    auto shape = [&](int halves) {
-        p.halves = halves;
-        const int ctas = (dual ? w_tiles : (w_tiles + halves - 1) / halves) * p.n_tiles;
-        int want = may_split_k ? std::max(1, std::min(sms / std::max(1, ctas), kb / 3)) : 1;
-        want = std::min(want, std::max(4, 1024 / std::max(1, rows)));  // every slice adds rows x M floats with atomics
-        p.kb_per_split = (kb + want - 1) / want;
-        p.splits = (kb + p.kb_per_split - 1) / p.kb_per_split;
-        return ctas * p.splits;
-    };
-    if (shape(2) * 2 <= sms && !dual) shape(1);
-    return p;
-}
-
-static cudaError_t tc_configure() {
-    static bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmemBytes);
-        if (e != cudaSuccess) return e;
-        configured[dev] = true;
-    }
-    return cudaSuccess;
-}
-
-// mw: the weight maps of the group (unused slots repeat slot 0); map_x must have been built with box_rows ==
-// plan.x_rows.  The argument block's tile list, K slicing and box size are filled in here.
-cudaError_t tc_launch(const TcPlan& plan, bool dual, const CUtensorMap* const* mw, const CUtensorMap& mx, TcArgs a, cudaStream_t s) {
-    cudaError_t e = tc_configure();
-    if (e != cudaSuccess) return e;
-    int tiles = 0;
-    const int groups = dual ? 1 : a.n_groups;
-    for (int g = 0; g < groups; g++) {
-        a.g[g].tile0 = tiles;
-        tiles += (a.g[g].M + kTcHalf - 1) / kTcHalf;
-    }
-    a.n_tiles = tiles;
-    a.dual = dual ? 1 : 0;
-    a.halves = dual ? 2 : plan.halves;
-    a.x_rows = plan.x_rows;
-    a.kb_per_split = plan.kb_per_split;
-    a.atomic_out = plan.splits > 1 ? 1 : 0;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(plan.n_tiles, dual ? tiles : (tiles + a.halves - 1) / a.halves, plan.splits);
-    cfg.blockDim = dim3(kTcThreads);
-    cfg.dynamicSmemBytes = kTcSmemBytes;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_gemm_tc, *mw[0], *mw[1], *mw[2], mx, a);
 }
 
 // Launch shape of a streamed product: w_tiles 128-row weight tiles, K of kb 64-wide blocks, `rows` batch rows in `parts`
@@ -174,6 +104,41 @@ cudaError_t sg_launch(const SgPlan& plan, int epilogue, const CUtensorMap* const
     return cudaLaunchKernelEx(&cfg, k_gemm_stream, *mw[0], *mw[1], *mw[2], mx, a);
 }
 
+// mw: 128-row maps of the group's matrices (unused slots repeat slot 0); mx: map of the operand rows with 128-row boxes.
+cudaError_t pg_launch(const CUtensorMap* const* mw, const CUtensorMap& mx, PgArgs a, int sms, cudaStream_t s) {
+    static std::mutex mu;
+    static bool configured[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (dev >= 0 && dev < 64 && !configured[dev]) {
+            cudaError_t e = cudaFuncSetAttribute(k_gemm_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPgSmemBytes);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_pair, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+            if (e != cudaSuccess) return e;
+            configured[dev] = true;
+        }
+    }
+    int halves = 0;
+    const int groups = a.epilogue == PG_SWIGLU ? 1 : a.n_groups;
+    for (int g = 0; g < groups; g++) { a.g[g].half0 = halves; halves += (a.g[g].M + 127) / 128; }
+    a.tiles_w = a.epilogue == PG_SWIGLU ? halves : (halves + 1) / 2;
+    a.tiles_n = (a.rows + kPgRows - 1) / kPgRows;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * std::min(sms / 2, a.tiles_n * a.tiles_w));
+    cfg.blockDim = dim3(kPgThreads);
+    cfg.dynamicSmemBytes = kPgSmemBytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, k_gemm_pair, *mw[0], *mw[1], *mw[2], mx, a);
+}
+
 __global__ void k_f32_to_16(const float* src, int64_t n, uint16_t* dst, int bf16) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -190,6 +155,7 @@ int32_t gemm_tc_bench(int32_t type, const void* w, int32_t M, int32_t K, const f
     if (force_failure_enabled()) return esp::fail(ESP_CUDA_ERR_FORCED_FAILURE, "forced failure is enabled");
     ESP_CUDA_TRY(cudaSetDevice(device));
     const int alloc_rows = (N + 15) / 16 * 16;
+    const int ldo = (M + 3) / 4 * 4;  // the kernel stores four weight rows at a time
     std::vector<void*> owned;
     auto cleanup = [&] { for (void* p : owned) cudaFree(p); };
     auto body = [&]() -> int32_t {
@@ -199,7 +165,7 @@ int32_t gemm_tc_bench(int32_t type, const void* w, int32_t M, int32_t K, const f
         ESP_CUDA_TRY(cudaMalloc(&dw, (size_t)M * K * 2)); owned.push_back(dw);
         ESP_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&dx), sizeof(float) * (size_t)N * K)); owned.push_back(dx);
         ESP_CUDA_TRY(cudaMalloc(&dx16, (size_t)alloc_rows * K * 2)); owned.push_back(dx16);
-        ESP_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&dy), sizeof(float) * (size_t)N * M)); owned.push_back(dy);
+        ESP_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&dy), sizeof(float) * (size_t)N * ldo)); owned.push_back(dy);
         ESP_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(&derr), sizeof(int))); owned.push_back(derr);
         ESP_CUDA_TRY(cudaMemcpy(dw, w, (size_t)M * K * 2, cudaMemcpyDefault));
         ESP_CUDA_TRY(cudaMemcpy(dx, x, sizeof(float) * (size_t)N * K, cudaMemcpyDefault));
@@ -210,24 +176,18 @@ int32_t gemm_tc_bench(int32_t type, const void* w, int32_t M, int32_t K, const f
         ESP_CUDA_TRY(cudaGetLastError());
         CUtensorMap mw, mx;
         int32_t rc;
-        if ((rc = tc_make_map(&mw, dw, type == WT_BF16, M, K, kTcHalf))) return rc;
+        if ((rc = tc_make_map(&mw, dw, type == WT_BF16, M, K, kSgHalf))) return rc;
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        // the plan the decode engine would use for a product of this shape (K slices add into a zeroed output)
-        const TcPlan plan = tc_plan((M + kTcHalf - 1) / kTcHalf, N, K / kTcBlockK, true, false, sms);
-        if ((rc = tc_make_map(&mx, dx16, type == WT_BF16, alloc_rows, K, plan.x_rows))) return rc;
+        // the plan the decode engine would use for a product of this shape, with the batch rows rounded to 16 bits
+        const SgPlan plan = sg_plan((M + kSgRows - 1) / kSgRows, N, K / kTcBlockK, 1, true, sms);
+        if ((rc = tc_make_map(&mx, dx16, type == WT_BF16, alloc_rows, K, plan.n_cols))) return rc;
         const CUtensorMap* maps[3] = {&mw, &mw, &mw};
-        TcArgs a{};
+        SgArgs a{};
         a.n_groups = 1;
-        a.g[0].M = M; a.g[0].out = dy; a.g[0].ldo = M;
-        a.K = K; a.n_valid = N; a.epilogue = TC_STORE; a.error = derr; a.bf16 = type == WT_BF16;
-        auto launch = [&]() -> cudaError_t {
-            if (plan.splits > 1) {
-                cudaError_t e = cudaMemsetAsync(dy, 0, sizeof(float) * (size_t)N * M, nullptr);
-                if (e != cudaSuccess) return e;
-            }
-            return tc_launch(plan, false, maps, mx, a, nullptr);
-        };
+        a.g[0].M = M; a.g[0].out = dy; a.g[0].ldo = ldo;
+        a.K = K; a.rows = N; a.all_rows = 1; a.error = derr; a.bf16 = type == WT_BF16;
+        auto launch = [&]() -> cudaError_t { return sg_launch(plan, SG_STORE, maps, mx, a, nullptr); };
         for (int i = 0; i < warmup; i++) ESP_CUDA_TRY(launch());
         cudaEvent_t e0, e1;
         ESP_CUDA_TRY(cudaEventCreate(&e0));
@@ -246,7 +206,7 @@ int32_t gemm_tc_bench(int32_t type, const void* w, int32_t M, int32_t K, const f
         int herr = 0;
         ESP_CUDA_TRY(cudaMemcpy(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost));
         if (herr) return esp::fail(ESP_CUDA_ERR_TIMEOUT, "tensor-core GEMM gave up waiting on a barrier");
-        ESP_CUDA_TRY(cudaMemcpy(y, dy, sizeof(float) * (size_t)N * M, cudaMemcpyDeviceToHost));
+        ESP_CUDA_TRY(cudaMemcpy2D(y, sizeof(float) * M, dy, sizeof(float) * ldo, sizeof(float) * M, N, cudaMemcpyDeviceToHost));
         return ESP_CUDA_OK;
     };
     int32_t rc = body();
