@@ -15,169 +15,133 @@ __device__ __forceinline__ uint16_t to_16bit(float v, int bf16) {
     return bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
 }
 
-// 16-bit parts of a value: part 0 is the rounded value, the next ones the rounded remainders (fp16 parts saturate).
-__device__ __forceinline__ uint16_t part16(float& v, int bf16) {
+// 16-bit parts of two values: the rounded values packed into one word (fp16 parts saturate); x and y keep the remainders.
+__device__ __forceinline__ uint32_t part16x2(float& x, float& y, bool bf16) {
+    uint32_t d;
     if (bf16) {
-        const __nv_bfloat16 h = __float2bfloat16_rn(v);
-        v -= __bfloat162float(h);
-        return __bfloat16_as_ushort(h);
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(y), "f"(x));
+        x -= __uint_as_float(d << 16);
+        y -= __uint_as_float(d & 0xffff0000u);
+    } else {
+        asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(y), "f"(x));
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&d));
+        x -= f.x;
+        y -= f.y;
     }
-    unsigned short h;
-    asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(h) : "f"(v));
-    v -= __half2float(__ushort_as_half(h));
-    return h;
+    return d;
 }
 // Four values of row r -> their parts at columns k..k+3 of operand rows r, r + 8, r + 16.
-__device__ __forceinline__ void store_parts4(uint16_t* buf, int ld, int r, int k, float4 v, int parts, int bf16) {
+__device__ __forceinline__ void store_parts4(uint16_t* buf, int ld, int r, int k, float4 v, int parts, bool bf16) {
+    uint16_t* dst = buf + (size_t)r * ld + k;
+#pragma unroll 1
     for (int j = 0; j < parts; j++) {
-        const uint32_t lo = part16(v.x, bf16) | ((uint32_t)part16(v.y, bf16) << 16);
-        const uint32_t hi = part16(v.z, bf16) | ((uint32_t)part16(v.w, bf16) << 16);
-        *reinterpret_cast<uint2*>(buf + (size_t)(r + 8 * j) * ld + k) = make_uint2(lo, hi);
+        const uint32_t lo = part16x2(v.x, v.y, bf16), hi = part16x2(v.z, v.w, bf16);
+        *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
+        dst += (size_t)8 * ld;
     }
 }
 
 struct PrepArgs {
-    ModelDims m;
-    RowState rs;
-    const float* src;         // [rows][K] fp32, or null when from_embedding
-    float* hidden_out;        // from_embedding: the residual stream [rows][d_model] is initialised here
-    const uint16_t* tok_emb;  // from_embedding
-    const uint16_t* pos_emb;
-    int emb_type;
-    int from_embedding;
-    int K;
-    int norm;                 // NormKind
+    const int* active;
+    const float* src;  // [rows][K] fp32
+    int K;             // a multiple of 4
+    int norm;          // NormKind
+    float eps;
     const float* g;
     const float* b;
-    uint16_t* dst;            // [rows][K] fp16/bf16
+    uint16_t* dst;     // [rows][K] fp16/bf16
     int bf16;
-    int parts;                // 16-bit parts per value (see stream_gemm.cuh): part j of row r goes to row r + 8 j
+    int parts;         // 16-bit parts per value (see stream_gemm.cuh): part j of row r goes to row r + 8 j
 };
 
-// One CTA per row.  Rows of up to 8192 elements are held in registers (one global read, 16-byte accesses); longer
-// rows are re-read for every pass.
+// One CTA per row, the row in registers: VEC float4 per thread (VEC = 0: rows of more than 8192 elements, re-read for every
+// pass).  Bound by latency at few rows: one load round trip, one or two block reductions, one store; the code is kept short
+// because instruction fetch is a visible part of a launch this small.
+template <int VEC>
 __global__ void __launch_bounds__(kThreads) k_prep_rows(const PrepArgs p) {
     __shared__ float red[kRedFloats];
-    const int r = blockIdx.x;
+    constexpr int N = VEC ? VEC : 1;
+    const int r = blockIdx.x, K = p.K, nvec = K >> 2;
+    float4 g[N], b[N];
+    if (VEC && p.norm != NORM_NONE) {  // gains do not depend on the previous kernel
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int idx = threadIdx.x + i * kThreads;
+            g[i] = b[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (idx < nvec) {
+                g[i] = __ldg(reinterpret_cast<const float4*>(p.g) + idx);
+                if (p.norm == NORM_LAYER) b[i] = __ldg(reinterpret_cast<const float4*>(p.b) + idx);
+            }
+        }
+    }
     pdl_launch_dependents();
     pdl_wait();
-    // The row's state words and (when the row comes from the residual stream) its values are requested together;
-    // the check for an inactive row comes after the requests, so the chain is one memory round trip shorter.
-    const int row_active = p.rs.active[r];
-    const int K = p.K;
-    const float* src = p.src ? p.src + (size_t)r * K : nullptr;
-    const uint16_t* te = nullptr;
-    const uint16_t* pe = nullptr;
-    if (p.from_embedding) {
-        te = p.tok_emb + (size_t)p.rs.tok[r] * K;
-        if (p.pos_emb) pe = p.pos_emb + (size_t)p.rs.pos[r] * K;
-    }
-    uint16_t* dst = p.dst + (size_t)r * K;
-    constexpr int kVec = 8;  // float4 per thread held in registers
-    const bool fast = K % 4 == 0 && K / 4 <= kVec * kThreads;
-    float4 pre[kVec];
-    if (fast && !p.from_embedding) {
+    const int active = __ldcg(p.active + r);
+    const float4* src = reinterpret_cast<const float4*>(p.src + (size_t)r * K);
+    if constexpr (VEC > 0) {
+        float4 v[N];  // requested together with the row's state
 #pragma unroll
-        for (int i = 0; i < kVec; i++) {
+        for (int i = 0; i < N; i++) {
             const int idx = threadIdx.x + i * kThreads;
-            pre[i] = idx < K / 4 ? reinterpret_cast<const float4*>(src)[idx] : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[i] = idx < nvec ? __ldcg(src + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-    }
-    if (!row_active) return;
-    if (fast) {
-        const int nvec = K / 4;
-        float4 v[kVec];
-#pragma unroll
-        for (int i = 0; i < kVec; i++) {
-            const int idx = threadIdx.x + i * kThreads;
-            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (idx < nvec) {
-                if (!p.from_embedding) {
-                    v[i] = pre[i];
-                } else {
-                    const uint2 t = reinterpret_cast<const uint2*>(te)[idx];
-                    v[i] = make_float4(emb_to_float((uint16_t)(t.x & 0xffffu), p.emb_type), emb_to_float((uint16_t)(t.x >> 16), p.emb_type),
-                                       emb_to_float((uint16_t)(t.y & 0xffffu), p.emb_type), emb_to_float((uint16_t)(t.y >> 16), p.emb_type));
-                    if (pe) {
-                        const uint2 u = reinterpret_cast<const uint2*>(pe)[idx];
-                        v[i].x += emb_to_float((uint16_t)(u.x & 0xffffu), p.emb_type);
-                        v[i].y += emb_to_float((uint16_t)(u.x >> 16), p.emb_type);
-                        v[i].z += emb_to_float((uint16_t)(u.y & 0xffffu), p.emb_type);
-                        v[i].w += emb_to_float((uint16_t)(u.y >> 16), p.emb_type);
-                    }
-                    reinterpret_cast<float4*>(p.hidden_out + (size_t)r * K)[idx] = v[i];
-                }
-            }
-        }
+        if (!active) return;
         float inv = 1.f, mean = 0.f;
-        if (p.norm == NORM_RMS) {
-            float ss = 0.f;
-#pragma unroll
-            for (int i = 0; i < kVec; i++) ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, ss))));
-            ss = block_sum(ss, red);
-            inv = 1.0f / sqrtf(ss / (float)K + p.m.eps);
-        } else if (p.norm == NORM_LAYER) {
+        if (p.norm == NORM_LAYER) {
             float sm = 0.f;
 #pragma unroll
-            for (int i = 0; i < kVec; i++) sm += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+            for (int i = 0; i < N; i++) sm += (v[i].x + v[i].y) + (v[i].z + v[i].w);
             mean = block_sum(sm, red) / (float)K;
-            float vs = 0.f;
+        }
+        if (p.norm != NORM_NONE) {
+            float ss = 0.f;
 #pragma unroll
-            for (int i = 0; i < kVec; i++) {
-                if (threadIdx.x + i * kThreads < nvec) {
-                    const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
-                    vs = fmaf(a, a, fmaf(b, b, fmaf(c, c, fmaf(d, d, vs))));
-                }
+            for (int i = 0; i < N; i++) {
+                if (threadIdx.x + i * kThreads >= nvec) continue;
+                v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean;
+                ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, ss))));
             }
-            vs = block_sum(vs, red);
-            inv = 1.0f / sqrtf(vs / (float)K + p.m.eps);
+            ss = block_sum(ss, red);
+            inv = 1.0f / sqrtf(ss / (float)K + p.eps);
         }
 #pragma unroll
-        for (int i = 0; i < kVec; i++) {
+        for (int i = 0; i < N; i++) {
             const int idx = threadIdx.x + i * kThreads;
             if (idx >= nvec) continue;
-            float4 o = v[i];
-            if (p.norm == NORM_RMS) {
-                const float4 g = reinterpret_cast<const float4*>(p.g)[idx];
-                o = make_float4((o.x * inv) * g.x, (o.y * inv) * g.y, (o.z * inv) * g.z, (o.w * inv) * g.w);
-            } else if (p.norm == NORM_LAYER) {
-                const float4 g = reinterpret_cast<const float4*>(p.g)[idx];
-                const float4 b = reinterpret_cast<const float4*>(p.b)[idx];
-                o = make_float4((o.x - mean) * inv * g.x + b.x, (o.y - mean) * inv * g.y + b.y, (o.z - mean) * inv * g.z + b.z,
-                                (o.w - mean) * inv * g.w + b.w);
-            }
-            store_parts4(p.dst, K, r, 4 * idx, o, p.parts, p.bf16);
+            if (p.norm != NORM_NONE)
+                v[i] = make_float4(fmaf(v[i].x * inv, g[i].x, b[i].x), fmaf(v[i].y * inv, g[i].y, b[i].y), fmaf(v[i].z * inv, g[i].z, b[i].z), fmaf(v[i].w * inv, g[i].w, b[i].w));
+            store_parts4(p.dst, K, r, 4 * idx, v[i], p.parts, p.bf16);
         }
-        return;
-    }
-    auto raw = [&](int k) {
-        if (!p.from_embedding) return src[k];
-        float v = emb_to_float(te[k], p.emb_type);
-        if (pe) v += emb_to_float(pe[k], p.emb_type);
-        return v;
-    };
-    float inv = 1.f, mean = 0.f;
-    if (p.norm == NORM_RMS) {
-        float ss = 0.f;
-        for (int k = threadIdx.x; k < K; k += kThreads) { const float v = raw(k); ss = fmaf(v, v, ss); }
-        ss = block_sum(ss, red);
-        inv = 1.0f / sqrtf(ss / (float)K + p.m.eps);
-    } else if (p.norm == NORM_LAYER) {
-        float s = 0.f;
-        for (int k = threadIdx.x; k < K; k += kThreads) s += raw(k);
-        mean = block_sum(s, red) / (float)K;
-        float vs = 0.f;
-        for (int k = threadIdx.x; k < K; k += kThreads) { const float c = raw(k) - mean; vs = fmaf(c, c, vs); }
-        vs = block_sum(vs, red);
-        inv = 1.0f / sqrtf(vs / (float)K + p.m.eps);
-    }
-    for (int k = threadIdx.x; k < K; k += kThreads) {
-        const float x = raw(k);
-        if (p.from_embedding) p.hidden_out[(size_t)r * K + k] = x;
-        float v = x;
-        if (p.norm == NORM_RMS) v = (x * inv) * p.g[k];
-        else if (p.norm == NORM_LAYER) v = (x - mean) * inv * p.g[k] + p.b[k];
-        for (int j = 0; j < p.parts; j++) dst[(size_t)8 * j * K + k] = part16(v, p.bf16);
+    } else {
+        if (!active) return;
+        float inv = 1.f, mean = 0.f;
+        if (p.norm == NORM_LAYER) {
+            float sm = 0.f;
+#pragma unroll 1
+            for (int k = threadIdx.x; k < nvec; k += kThreads) { const float4 v = __ldcg(src + k); sm += (v.x + v.y) + (v.z + v.w); }
+            mean = block_sum(sm, red) / (float)K;
+        }
+        if (p.norm != NORM_NONE) {
+            float ss = 0.f;
+#pragma unroll 1
+            for (int k = threadIdx.x; k < nvec; k += kThreads) {
+                const float4 v = __ldcg(src + k);
+                const float x = v.x - mean, y = v.y - mean, z = v.z - mean, w = v.w - mean;
+                ss = fmaf(x, x, fmaf(y, y, fmaf(z, z, fmaf(w, w, ss))));
+            }
+            ss = block_sum(ss, red);
+            inv = 1.0f / sqrtf(ss / (float)K + p.eps);
+        }
+#pragma unroll 1
+        for (int k = threadIdx.x; k < nvec; k += kThreads) {
+            float4 v = __ldcg(src + k);
+            if (p.norm != NORM_NONE) {
+                const float4 gg = __ldg(reinterpret_cast<const float4*>(p.g) + k);
+                const float4 bb = p.norm == NORM_LAYER ? __ldg(reinterpret_cast<const float4*>(p.b) + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v = make_float4(fmaf((v.x - mean) * inv, gg.x, bb.x), fmaf((v.y - mean) * inv, gg.y, bb.y), fmaf((v.z - mean) * inv, gg.z, bb.z), fmaf((v.w - mean) * inv, gg.w, bb.w));
+            }
+            store_parts4(p.dst, K, r, 4 * k, v, p.parts, p.bf16);
+        }
     }
 }
 

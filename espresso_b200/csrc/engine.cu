@@ -295,7 +295,7 @@ static void raise_smem_limits_on_current_device() {
     // The kernels of a pass must agree on the split of an SM's memory into L1 and shared memory: a kernel that wants another
     // split waits until the SM is empty, and nothing of its prologue overlaps its predecessor.
 #define ESP_CARVE(k) cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)
-    ESP_CARVE(k_attention); ESP_CARVE(k_prep_rows); ESP_CARVE(k_embed_rows); ESP_CARVE(k_rope_append); ESP_CARVE(k_head_done); ESP_CARVE(k_bump);
+    ESP_CARVE(k_attention); ESP_CARVE(k_prep_rows<0>); ESP_CARVE(k_prep_rows<1>); ESP_CARVE(k_prep_rows<2>); ESP_CARVE(k_prep_rows<4>); ESP_CARVE(k_prep_rows<8>); ESP_CARVE(k_embed_rows); ESP_CARVE(k_rope_append); ESP_CARVE(k_head_done); ESP_CARVE(k_bump);
 #define ESP_DA(HD)                                                                                                         \
     ESP_CARVE((k_attention_decode<HD, 2>)); ESP_CARVE((k_attention_decode<HD, 4>)); ESP_CARVE((k_attention_decode<HD, 8>)); \
     cudaFuncSetAttribute(k_attention_decode<HD, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, da_smem_floats(HD, 8, 8) * 4);
@@ -1805,15 +1805,33 @@ bool Engine::stream_path(int rows) const {
     return tc_ready_ && rows <= kSgMaxRows && !(tc_quant_ && rows == 1);
 }
 
+int32_t Engine::launch_embed(int rows, float2* stat, cudaStream_t s) {
+    const DeviceTensor& te = tensors_.at("embeddings/token");
+    EmbedArgs ea{};
+    ea.m = m_; ea.rs = rs_; ea.hidden = act_.hidden; ea.stat = stat; ea.stat_tiles = (m_.d_model + kSgRows - 1) / kSgRows;
+    ea.tok_emb = static_cast<const uint16_t*>(te.data);
+    ea.pos_emb = m_.arch == ARCH_GPT2 ? static_cast<const uint16_t*>(tensors_.at("embeddings/position").data) : nullptr;
+    ea.emb_type = te.type == ESP_CUDA_BF16 ? WT_BF16 : WT_F16;
+    ESP_CUDA_TRY(launch_pdl(k_embed_rows, dim3(rows), dim3(kThreads), 0, s, ea));
+    return ESP_CUDA_OK;
+}
+
+// Rows of src (normalised) -> 16-bit operand rows.
+int32_t Engine::launch_prep(int rows, const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst, int parts, cudaStream_t s) {
+    const PrepArgs p{rs_.active, src, K, norm, m_.eps, g, b, dst, tc_bf16_, parts};
+    const int per = (K / 4 + kThreads - 1) / kThreads;
+    auto kern = per <= 1 ? k_prep_rows<1> : per <= 2 ? k_prep_rows<2> : per <= 4 ? k_prep_rows<4> : per <= 8 ? k_prep_rows<8> : k_prep_rows<0>;
+    ESP_CUDA_TRY(launch_pdl(kern, dim3(rows), dim3(kThreads), 0, s, p));
+    return ESP_CUDA_OK;
+}
+
 // Final norm, LM head and arg-max of `rows` rows; the last CTA turns the maxima into tokens.
 int32_t Engine::launch_head_stream(int rows, int mode, int parts, cudaStream_t s, int& launches) {
     const bool gpt2 = m_.arch == ARCH_GPT2;
     // (the head has hundreds of weight tiles and always takes the norm kernel)
-    PrepArgs p{};
-    p.m = m_; p.rs = rs_; p.src = act_.hidden; p.K = m_.d_model; p.norm = gpt2 ? NORM_LAYER : NORM_RMS; p.dst = xh_d_; p.bf16 = tc_bf16_; p.parts = parts;
-    p.g = tensors_.at(gpt2 ? "final_norm_gamma" : "rms_final").f32;
-    p.b = gpt2 ? tensors_.at("final_norm_beta").f32 : nullptr;
-    ESP_CUDA_TRY(launch_pdl(k_prep_rows, dim3(rows), dim3(kThreads), 0, s, p));
+    int32_t prc = launch_prep(rows, act_.hidden, m_.d_model, gpt2 ? NORM_LAYER : NORM_RMS, tensors_.at(gpt2 ? "final_norm_gamma" : "rms_final").f32,
+                              gpt2 ? tensors_.at("final_norm_beta").f32 : nullptr, xh_d_, parts, s);
+    if (prc) return prc;
     const DeviceTensor& lh = tensors_.at("lm_head");
     if (!lh.has_map) return fail(ESP_CUDA_ERR_CUDA, "tensor map missing for the batched path");
     const int finalize = ((mode & STEP_FEEDBACK) ? 1 : 0) | ((mode & STEP_FORWARD) ? 2 : 0);
@@ -1858,11 +1876,8 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
     size_t ev = 0;
     auto mark = [&]() { if (profile && ev < prof_events_.size()) cudaEventRecord(prof_events_[ev++], s); };
     auto prep = [&](const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst) -> int32_t {
-        PrepArgs p{};
-        p.m = m_; p.rs = rs_; p.src = src; p.K = K; p.norm = norm; p.g = g; p.b = b; p.dst = dst; p.bf16 = tc_bf16_; p.parts = parts;
-        ESP_CUDA_TRY(launch_pdl(k_prep_rows, dim3(rows), dim3(kThreads), 0, s, p));
         launches++;
-        return ESP_CUDA_OK;
+        return launch_prep(rows, src, K, norm, g, b, dst, parts, s);
     };
     struct Part { const DeviceTensor* W; float* out; int ldo; const float* bias; };
     struct Norm { const float *g, *b; };
@@ -1916,13 +1931,7 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
     int32_t rc;
     mark();
     if (mode & STEP_FORWARD) {
-        const DeviceTensor& te = tensors_.at("embeddings/token");
-        EmbedArgs ea{};
-        ea.m = m_; ea.rs = rs_; ea.hidden = act_.hidden; ea.stat = row_stat_; ea.stat_tiles = stat_tiles;
-        ea.tok_emb = static_cast<const uint16_t*>(te.data);
-        ea.pos_emb = gpt2 ? static_cast<const uint16_t*>(tensors_.at("embeddings/position").data) : nullptr;
-        ea.emb_type = te.type == ESP_CUDA_BF16 ? WT_BF16 : WT_F16;
-        ESP_CUDA_TRY(launch_pdl(k_embed_rows, dim3(rows), dim3(kThreads), 0, s, ea));
+        if ((rc = launch_embed(rows, row_stat_, s))) return rc;
         launches++;
         for (int l = 0; l < m_.n_layer; l++) {
             const LayerTensors& t = layer_tensors_[l];
@@ -2000,19 +2009,9 @@ int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
     int launches = 0;
     float* dbg = debug_layer_ >= 0 ? d_debug_ : nullptr;
     const int q = m_.q_dim, kv = m_.kv_dim, d = m_.d_model, h = m_.hidden, hd = m_.head_dim;
-    auto prep = [&](const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst, bool from_emb = false) -> int32_t {
-        PrepArgs p{};
-        p.m = m_; p.rs = rs_; p.src = src; p.hidden_out = act_.hidden; p.K = K; p.norm = norm; p.g = g; p.b = b; p.dst = dst; p.bf16 = tc_bf16_; p.parts = 1;
-        p.from_embedding = from_emb ? 1 : 0;
-        if (from_emb) {
-            const DeviceTensor& te = tensors_.at("embeddings/token");
-            p.tok_emb = static_cast<const uint16_t*>(te.data);
-            p.pos_emb = gpt2 ? static_cast<const uint16_t*>(tensors_.at("embeddings/position").data) : nullptr;
-            p.emb_type = te.type == ESP_CUDA_BF16 ? WT_BF16 : WT_F16;
-        }
-        ESP_CUDA_TRY(launch_pdl(k_prep_rows, dim3(rows), dim3(kThreads), 0, s, p));
+    auto prep = [&](const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst) -> int32_t {
         launches++;
-        return ESP_CUDA_OK;
+        return launch_prep(rows, src, K, norm, g, b, dst, 1, s);
     };
     struct Part { const DeviceTensor* W; float* out; int ldo; const float* bias; };
     auto gemm = [&](std::initializer_list<Part> parts, const uint16_t* xbuf, int epi, uint16_t* out16, int ld16, float* capture, bool all_rows = false) -> int32_t {
@@ -2053,11 +2052,13 @@ int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
     const bool att_ok_hd = hd == 32 || hd == 64 || hd == 128;
     int32_t rc;
     if (mode & STEP_FORWARD) {
+        if ((rc = launch_embed(rows, nullptr, s))) return rc;
+        launches++;
         for (int l = 0; l < m_.n_layer; l++) {
             const LayerTensors& t = layer_tensors_[l];
             const LayerWeights& lw = t.w;
             const bool cap = dbg && l == debug_layer_;
-            if ((rc = prep(l == 0 ? nullptr : act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, lw.norm1_g, lw.norm1_b, xh_d_, l == 0))) return rc;
+            if ((rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, lw.norm1_g, lw.norm1_b, xh_d_))) return rc;
             if ((rc = gemm({{t.wq, act_.q, q, lw.bq}, {t.wk, kraw_, kv, lw.bk}, {t.wv, vraw_, kv, lw.bv}}, xh_d_, PG_STORE, nullptr, 0, nullptr))) return rc;
             RopeArgs ra{};
             ra.m = m_; ra.rs = rs_; ra.kv = kv_; ra.q = act_.q; ra.k_raw = kraw_; ra.v_raw = vraw_; ra.rope = gpt2 ? nullptr : d_rope_; ra.layer = l;

@@ -113,6 +113,8 @@ private:
     int32_t launch_step(int rows, int mode, cudaStream_t s, bool profile);
     int32_t launch_step_wide(int rows, int mode, cudaStream_t s);  // more rows: products on SM pairs, element-wise stages
     int32_t launch_head_stream(int rows, int mode, int parts, cudaStream_t s, int& launches);
+    int32_t launch_embed(int rows, float2* stat, cudaStream_t s);
+    int32_t launch_prep(int rows, const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst, int parts, cudaStream_t s);
     int32_t launch_attention_prefill(const PrefillAttArgs& pa, cudaStream_t s);
     int32_t launch_step_stream(int rows, int mode, cudaStream_t s, bool profile);  // up to kSgMaxRows rows: streamed products, fused stages
     bool stream_path(int rows) const;

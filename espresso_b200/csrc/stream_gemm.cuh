@@ -140,68 +140,67 @@ __device__ __forceinline__ void sg_norm_rows(const SgArgs& a, SgNormPre& p, int 
     }
 }
 // Normalises and stores rows r0 .. r0 + 15 (128-byte rows, 16-byte chunks XOR-swizzled by the row).
+template <bool BF16>
 __device__ __forceinline__ void sg_norm_store(const SgArgs& a, const SgNormPre& p, uint8_t* sx, const float2* stat, int r0, int rows, int lane) {
     const int c = lane & 7;
     const float g[8] = {p.g[0].x, p.g[0].y, p.g[0].z, p.g[0].w, p.g[1].x, p.g[1].y, p.g[1].z, p.g[1].w};
     const float b[8] = {p.b[0].x, p.b[0].y, p.b[0].z, p.b[0].w, p.b[1].x, p.b[1].y, p.b[1].z, p.b[1].w};
 #pragma unroll
     for (int u = 0; u < 4; u++) {
-        const int r = r0 + u * 4 + (lane >> 3);
-        if (r >= rows) continue;
+        if (r0 + u * 4 >= rows) break;  // (the whole warp)
+        const int r = min(r0 + u * 4 + (lane >> 3), rows - 1);  // rows past the end repeat the last one
+        const bool mine = r0 + u * 4 + (lane >> 3) < rows;
         const float2 st = stat[r];  // (mean or 0, 1 / sqrt(variance + eps))
         float y[8] = {p.v[u][0].x, p.v[u][0].y, p.v[u][0].z, p.v[u][0].w, p.v[u][1].x, p.v[u][1].y, p.v[u][1].z, p.v[u][1].w};
 #pragma unroll
         for (int i = 0; i < 8; i++) y[i] = (y[i] - st.x) * st.y * g[i] + b[i];
+        uint8_t* dst = sx + r * 128 + ((c ^ (r & 7)) << 4);  // (part j: eight rows further down, the same swizzle)
+#pragma unroll 1
         for (int j = 0; j < a.parts; j++) {
-            uint32_t w[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) w[i] = part16(y[2 * i], a.bf16) | ((uint32_t)part16(y[2 * i + 1], a.bf16) << 16);
-            const int row = r + 8 * j;
-            *reinterpret_cast<uint4*>(sx + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+            const uint4 w = make_uint4(part16x2(y[0], y[1], BF16), part16x2(y[2], y[3], BF16), part16x2(y[4], y[5], BF16), part16x2(y[6], y[7], BF16));
+            if (mine) *reinterpret_cast<uint4*>(dst + j * 1024) = w;
         }
     }
 }
 
-// (mean, 1 / sqrt(var + eps)) of every row from its per-128-column statistics; RMSNorm: mean 0, mean square.  The stage warps
-// share the rows; the caller synchronises them.
+// (mean, 1 / sqrt(var + eps)) of every row from its per-128-column statistics; RMSNorm: mean 0, mean square.  Eight lanes per
+// row, four rows per stage warp, one round trip; the caller synchronises the warps.
 __device__ __forceinline__ void sg_row_stats(const SgArgs& a, float2* stat, int n0, int rows, int xw, int lane) {
     const float inv_k = 1.0f / (float)a.K;
-    for (int r0 = xw; r0 < rows; r0 += 3 * kSgXWarps) {
-        float2 v[3][2];
+    const int l = lane & 7, tiles = a.stat_tiles;
+    auto n_of = [&](int t) { return (float)min(kSgRows, a.K - t * kSgRows); };
+    auto sum8 = [](float v) {
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        return v + __shfl_xor_sync(0xffffffffu, v, 4);
+    };
+#pragma unroll 1
+    for (int r0 = xw * 4; r0 < rows; r0 += 4 * kSgXWarps) {
+        const int r = min(r0 + (lane >> 3), rows - 1);
+        const float2* src = a.stat + (size_t)(n0 + r) * tiles;
+        float2 v[4];
 #pragma unroll
-        for (int i = 0; i < 3; i++)
+        for (int i = 0; i < 4; i++) v[i] = l + 8 * i < tiles ? __ldcg(src + l + 8 * i) : make_float2(0.f, 0.f);
+        float mean = 0.f;
+        if (a.norm == NORM_LAYER) {
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int r = r0 + i * kSgXWarps, t = lane + 32 * h;
-                v[i][h] = make_float2(0.f, 0.f);
-                if (r < rows && t < a.stat_tiles) v[i][h] = __ldcg(a.stat + (size_t)(n0 + r) * a.stat_tiles + t);
-            }
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-            const int r = r0 + i * kSgXWarps;
-            if (r >= rows) break;
-            const float2* src = a.stat + (size_t)(n0 + r) * a.stat_tiles;
-            auto n_of = [&](int t) { return (float)max(0, min(kSgRows, a.K - t * kSgRows)); };
-            float mean = 0.f;
-            if (a.norm == NORM_LAYER) {
-                float sum = fmaf(v[i][0].x, n_of(lane), v[i][1].x * n_of(lane + 32));
-                for (int t = lane + 64; t < a.stat_tiles; t += 32) sum = fmaf(__ldcg(&src[t].x), n_of(t), sum);
-                mean = warp_sum(sum) * inv_k;
-            }
-            float ss = 0.f;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const float d = v[i][h].x - mean;
-                ss += fmaf(d * d, n_of(lane + 32 * h), v[i][h].y);
-            }
-            for (int t = lane + 64; t < a.stat_tiles; t += 32) {
-                const float2 s = __ldcg(src + t);
-                const float d = s.x - mean;
-                ss += fmaf(d * d, n_of(t), s.y);
-            }
-            ss = warp_sum(ss);
-            if (lane == 0) stat[r] = make_float2(mean, 1.0f / sqrtf(ss / (float)a.K + a.eps));
+            for (int i = 0; i < 4; i++)
+                if (l + 8 * i < tiles) mean = fmaf(v[i].x, n_of(l + 8 * i), mean);
+#pragma unroll 1
+            for (int t = l + 32; t < tiles; t += 8) mean = fmaf(__ldcg(&src[t].x), n_of(t), mean);
+            mean = sum8(mean) * inv_k;
         }
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (l + 8 * i < tiles) ss += fmaf((v[i].x - mean) * (v[i].x - mean), n_of(l + 8 * i), v[i].y);
+#pragma unroll 1
+        for (int t = l + 32; t < tiles; t += 8) {
+            const float2 s = __ldcg(src + t);
+            ss += fmaf((s.x - mean) * (s.x - mean), n_of(t), s.y);
+        }
+        ss = sum8(ss);
+        if (l == 0 && r0 + (lane >> 3) < rows) stat[r] = make_float2(mean, rsqrtf(fmaf(ss, inv_k, a.eps)));
     }
 }
 
@@ -237,7 +236,7 @@ __device__ __forceinline__ SgRowPre sg_row_prefetch(const SgArgs& a, int row, in
 // What happens to complete sums: lane l of the calling warp holds v = four consecutive weight rows of batch row `row`
 // (lanes 0..15: half 0 of the tile, 16..31: half 1), first of them m0 of matrix gi; ok = false past the matrix' end (nothing is
 // stored; the warp's exchanges still take place).
-template <int EPI>
+template <int EPI, bool BF16>
 __device__ __forceinline__ void sg_epilogue_row(const SgArgs& a, int row, float4 v, const SgRowPre& pre, int4 ctl, float4 bias, int lane, int gi, int m0, bool ok) {
 #define ESP_SG_G(field) (gi == 0 ? a.g[0].field : gi == 1 ? a.g[1].field : a.g[2].field)
     v.x += bias.x; v.y += bias.y; v.z += bias.z; v.w += bias.w;
@@ -281,18 +280,16 @@ __device__ __forceinline__ void sg_epilogue_row(const SgArgs& a, int row, float4
             }
         }
     } else if constexpr (EPI == SG_GELU) {
-        if (a.parts == 1) v = make_float4(gelu_fast(v.x), gelu_fast(v.y), gelu_fast(v.z), gelu_fast(v.w));
-        else v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
-        if (ok) store_parts4(a.out16, a.ld16, row, m0, v, a.parts, a.bf16);
+        v = make_float4(gelu_fast(v.x), gelu_fast(v.y), gelu_fast(v.z), gelu_fast(v.w));
+        if (ok) store_parts4(a.out16, a.ld16, row, m0, v, a.parts, BF16);
         if (ok && dbg) *reinterpret_cast<float4*>(a.debug + m0) = v;
     } else if constexpr (EPI == SG_SWIGLU) {  // lanes 0..15 hold the gate values, 16..31 the up values of the same hidden units
         float4 u;
         u.x = __shfl_xor_sync(0xffffffffu, v.x, 16); u.y = __shfl_xor_sync(0xffffffffu, v.y, 16);
         u.z = __shfl_xor_sync(0xffffffffu, v.z, 16); u.w = __shfl_xor_sync(0xffffffffu, v.w, 16);
-        if (a.parts == 1) v = make_float4(silu_fast(v.x) * u.x, silu_fast(v.y) * u.y, silu_fast(v.z) * u.z, silu_fast(v.w) * u.w);
-        else v = make_float4(silu_f(v.x) * u.x, silu_f(v.y) * u.y, silu_f(v.z) * u.z, silu_f(v.w) * u.w);
+        v = make_float4(silu_fast(v.x) * u.x, silu_fast(v.y) * u.y, silu_fast(v.z) * u.z, silu_fast(v.w) * u.w);
         if (ok && lane < 16) {
-            store_parts4(a.out16, a.ld16, row, m0, v, a.parts, a.bf16);
+            store_parts4(a.out16, a.ld16, row, m0, v, a.parts, BF16);
             if (dbg) *reinterpret_cast<float4*>(a.debug + m0) = v;
         }
     }
@@ -305,7 +302,7 @@ struct SgFinish {
     int rows, n0, splits, own, r_first, r_step, lane, gi, m0;
     bool valid;
 };
-template <int EPI>
+template <int EPI, bool BF16>
 __device__ __forceinline__ void sg_finish_rows(const SgArgs& a, const SgFinish& f, SgRowPre now, float4 bias) {
     const float* src = f.sums;
     const int n_parts = f.splits * a.parts, stride = f.own * kSgRows;
@@ -320,7 +317,7 @@ __device__ __forceinline__ void sg_finish_rows(const SgArgs& a, const SgFinish& 
             const float4 t = *reinterpret_cast<const float4*>(src + (size_t)i * stride);
             v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
         }
-        if (ctl.x) sg_epilogue_row<EPI>(a, f.n0 + r, v, now, ctl, bias, f.lane, f.gi, f.m0, f.valid);
+        if (ctl.x) sg_epilogue_row<EPI, BF16>(a, f.n0 + r, v, now, ctl, bias, f.lane, f.gi, f.m0, f.valid);
         now = next;
         src += (kSgThreads / 32) * kSgRows;  // the warp's next own row
     }
@@ -338,19 +335,29 @@ __device__ __forceinline__ void sg_head_rows(const SgArgs& a, const float* part,
         const float* src = part + r * kSgRows;
         float bv = -INFINITY;
         int bi = 0x7fffffff;
+        const int last0 = a.g[0].M - m_h0, last1 = a.g[0].M - m_h1 + kSgHalf;  // valid sums of the halves end here
 #pragma unroll 4
         for (int i = 0; i < count; i++) {
             const int e = sub + (((i + r) & (count - 1)) << lg);
             float x = src[e];
-            for (int j = 1; j < a.parts; j++) x += src[e + j * own * kSgRows];
+            if (a.parts > 1) x += src[e + own * kSgRows];
+            if (a.parts > 2) x += src[e + 2 * own * kSgRows];
             const int m = (e < kSgHalf ? m_h0 : m_h1 - kSgHalf) + e;
-            if (m < a.g[0].M) {
-                if (x > bv || (x == bv && m < bi)) { bv = x; bi = m; }  // (a NaN logit is never chosen)
-                if (a.logits) a.logits[(size_t)(n0 + r) * a.g[0].M + m] = x;
+            const bool better = x > bv || (x == bv && m < bi);  // (a NaN logit is never chosen)
+            if (better && e < (e < kSgHalf ? last0 : last1)) { bv = x; bi = m; }
+        }
+        if (a.logits) {
+#pragma unroll 1
+            for (int e = sub; e < kSgRows; e += tpr) {
+                float x = src[e];
+#pragma unroll 1
+                for (int j = 1; j < a.parts; j++) x += src[e + j * own * kSgRows];
+                if (e < (e < kSgHalf ? last0 : last1)) a.logits[(size_t)(n0 + r) * a.g[0].M + (e < kSgHalf ? m_h0 : m_h1 - kSgHalf) + e] = x;
             }
         }
         if (bi != 0x7fffffff) key = pack_best(bv, bi + a.row_offset);
     }
+#pragma unroll 1
     for (int o = 1; o < tpr; o <<= 1) key = max(key, __shfl_xor_sync(0xffffffffu, key, o));
     if (sub == 0 && key) atomicMax(a.rs.best + n0 + r, key);
 }
@@ -380,7 +387,7 @@ struct EmbedArgs {
     const uint16_t* pos_emb;  // GPT-2, else null
     int emb_type;
     float* hidden;            // [rows][d_model]
-    float2* stat;             // [rows][stat_tiles]
+    float2* stat;             // [rows][stat_tiles], or null
     int stat_tiles;
 };
 // hidden = token embedding (+ position embedding) and its per-128-column statistics; one CTA per row, a warp per tile.
@@ -406,14 +413,17 @@ __global__ void __launch_bounds__(kThreads) k_embed_rows(const EmbedArgs p) {
             }
             *reinterpret_cast<float4*>(p.hidden + (size_t)r * d + k) = v;
         }
+        if (!p.stat) continue;
         const float2 st = tile_stat(v, ok, min(kSgRows, d - t * kSgRows), p.m.arch == ARCH_LLAMA);
         if (lane == 0) p.stat[(size_t)r * p.stat_tiles + t] = st;
     }
 }
 
 // grid = (column tiles, row tiles, K slices), cluster = (1, 1, K slices).
-// One kernel for all epilogues: the kernels of a pass alternate, and five large instances would not stay in the instruction
-// cache together (1.1B shape, 5 rows: 1079 us per step with an instance per epilogue, 800 with one kernel).
+// One kernel for all epilogues, and small on purpose: with a few hundred instructions per warp and launch, instruction fetch
+// was most of the time (no_instruction 7 to 12 of 15 stall cycles per issue at 137 KB of code; an instance per epilogue was
+// slower still: 1079 against 800 us per step of the 1.1B shape at 5 rows).  Hence rolled loops wherever they are not hot.
+template <bool BF16>
 __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                                                                const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x,
                                                                const __grid_constant__ SgArgs a) {
@@ -462,6 +472,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
     };
 
     if (threadIdx.x == 0) {
+#pragma unroll 1
         for (int s = 0; s < stages; s++) { mbar_init(s_full + s, norm ? 2 : 1); mbar_init(s_empty + s, 1); }
         mbar_init(&s_acc, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -496,6 +507,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
     pdl_wait();
     const uint32_t acc = s_tmem;
     if (warp == 0) {  // read by the epilogue, several barriers later
+#pragma unroll 1
         for (int r = lane; r < rows; r += 32) {
             const bool kv_rows = a.epilogue == SG_QKV;
             s_ctl[r] = make_int4(a.all_rows ? 1 : __ldcg(a.rs.active + n0 + r), kv_rows ? __ldcg(a.rs.pos + n0 + r) : 0, kv_rows ? __ldcg(a.rs.seq + n0 + r) : 0, 0);
@@ -504,7 +516,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
 
     if (warp == 1) {
         // ---------------- MMA issuer (see elect_one for the shape of this loop) ----------------
-        const uint32_t idesc = umma_idesc_f16(kSgRows, a.n_cols, a.bf16);
+        const uint32_t idesc = umma_idesc_f16(kSgRows, a.n_cols, BF16);
         // Everything the loop needs is kept up by counting; the next stage's barrier is tested before this stage's MMAs.
         const uint64_t d_first = umma_smem_desc_sw128(tiles);
         const uint32_t d_step = (uint32_t)stage_bytes >> 4;
@@ -540,14 +552,14 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
             asm volatile("bar.sync 2, %0;" ::"n"(kSgXWarps * 32) : "memory");
         }
         if (feeds) {
+            uint32_t phase = 1;
+#pragma unroll 1
             for (int kb = xw; kb < num_kb; kb += stages) {
                 const int k0 = (kb0 + kb) * kTcBlockK;
+                phase ^= 1u;
                 if (kb >= stages) {
-                    if (norm) {
-                        sg_norm_gains(a, pre_x, k0, lane);
-                        sg_norm_rows(a, pre_x, n0, 0, rows, k0, lane);
-                    }
-                    if (!tc_wait(s_empty + xw, ((kb / stages) - 1) & 1, a.error)) break;
+                    if (norm) sg_norm_gains(a, pre_x, k0, lane);
+                    if (!tc_wait(s_empty + xw, phase ^ 1u, a.error)) break;
                     if (elect_one()) load_w(kb, xw);
                 }
                 if (!norm) {
@@ -555,10 +567,10 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
                     __syncwarp();
                     continue;
                 }
-                sg_norm_store(a, pre_x, sw + kSgWBytes, s_stat, 0, rows, lane);
-                for (int r0 = 16; r0 < rows; r0 += 16) {
-                    sg_norm_rows(a, pre_x, n0, r0, rows, k0, lane);
-                    sg_norm_store(a, pre_x, sw + kSgWBytes, s_stat, r0, rows, lane);
+#pragma unroll 1
+                for (int r0 = 0; r0 < rows; r0 += 16) {
+                    if (kb >= stages || r0 > 0) sg_norm_rows(a, pre_x, n0, r0, rows, k0, lane);
+                    sg_norm_store<BF16>(a, pre_x, sw + kSgWBytes, s_stat, r0, rows, lane);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
@@ -579,6 +591,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
     if (!ok) {
         // a wait gave up (the results are void): the copies still in flight must land before the CTA may leave
         if (threadIdx.x == 0)
+#pragma unroll 1
             for (int kb = max(0, num_kb - stages); kb < num_kb; kb++) {
                 unsigned spins = 0;
                 while (!mbar_try_wait(s_full + kb % stages, (kb / stages) & 1) && ++spins < kTcSpinLimit / 64) {}
@@ -608,11 +621,11 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
     const float* const sums = part + warp * kSgRows + lane * 4;
     const SgFinish f{sums, s_ctl, rows, n0, splits, own, r_first, r_step, lane, gi, m0, valid};
     switch (a.epilogue) {
-        case SG_STORE: sg_finish_rows<SG_STORE>(a, f, ahead, bias4); break;
-        case SG_RESIDUAL: sg_finish_rows<SG_RESIDUAL>(a, f, ahead, bias4); break;
-        case SG_QKV: sg_finish_rows<SG_QKV>(a, f, ahead, bias4); break;
-        case SG_GELU: sg_finish_rows<SG_GELU>(a, f, ahead, bias4); break;
-        case SG_SWIGLU: sg_finish_rows<SG_SWIGLU>(a, f, ahead, bias4); break;
+        case SG_STORE: sg_finish_rows<SG_STORE, BF16>(a, f, ahead, bias4); break;
+        case SG_RESIDUAL: sg_finish_rows<SG_RESIDUAL, BF16>(a, f, ahead, bias4); break;
+        case SG_QKV: sg_finish_rows<SG_QKV, BF16>(a, f, ahead, bias4); break;
+        case SG_GELU: sg_finish_rows<SG_GELU, BF16>(a, f, ahead, bias4); break;
+        case SG_SWIGLU: sg_finish_rows<SG_SWIGLU, BF16>(a, f, ahead, bias4); break;
         default: sg_head_rows(a, part, s_ctl, rows, n0, own, m_h0, m_h1); break;  // (never sliced along K)
     }
     if (a.epilogue == SG_HEAD && a.finalize >= 0) {

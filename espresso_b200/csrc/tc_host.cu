@@ -75,8 +75,11 @@ static cudaError_t sg_configure() {
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lock(mu);
     if (dev < 0 || dev >= 64 || configured[dev]) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgSmemBudget + 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_stream, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaError_t e = cudaSuccess;
+    for (auto k : {k_gemm_stream<false>, k_gemm_stream<true>}) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSgSmemBudget + 1024);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    }
     configured[dev] = e == cudaSuccess;
     return e;
 }
@@ -101,7 +104,7 @@ cudaError_t sg_launch(const SgPlan& plan, int epilogue, const CUtensorMap* const
     attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = plan.splits;
     cfg.attrs = attr;
     cfg.numAttrs = plan.splits > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k_gemm_stream, *mw[0], *mw[1], *mw[2], mx, a);
+    return cudaLaunchKernelEx(&cfg, a.bf16 ? k_gemm_stream<true> : k_gemm_stream<false>, *mw[0], *mw[1], *mw[2], mx, a);
 }
 
 // mw: 128-row maps of the group's matrices (unused slots repeat slot 0); mx: map of the operand rows with 128-row boxes.
