@@ -61,7 +61,10 @@ __global__ void k_add_rows(float* dst, const float* src, int n4) {
 }
 SgPlan sg_plan(int w_tiles, int rows, int kb, int parts, bool may_split, int sms);
 cudaError_t sg_launch(const SgPlan& plan, int epilogue, const CUtensorMap* const* mw, const CUtensorMap& mx, SgArgs a, cudaStream_t s);
-constexpr int kSgMaxRows = 256;  // rows of a pass that take the streamed products; wider prompt passes take k_gemm_tc
+// Rows of a pass that take the streamed products; wider passes take the products on SM pairs.  Measured crossings (prompt pass,
+// us, streamed / pairs): 1.1B 256 rows 2181 / 2602, 400 rows 3246 / 2930; GPT-2 400 rows 1056 / 1078; 8B (4 layers) 128 rows
+// 716 / 959, 192 rows 942 / 974, 256 rows 1188 / 992.
+constexpr int kSgMaxRows = 320, kSgMaxRowsWide = 192;  // d_model <= 2048 / above
 constexpr int kTcMinRows = 9;  // below this the row-batched GEMV stages are used
 // Rows of a prompt pass on the batched path.  Every pass streams all the weights once and is a chain of ~8 dependent
 // launches per layer, so few wide passes win: 256 GPT-2 prompts of 64 tokens took 32 passes of 512 rows at 0.74 ms, nearly
@@ -835,7 +838,7 @@ int32_t Engine::check_ready(const char* what) const {
 int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
     if (tp_size_ > 1 && !tc_ready_) return fail(ESP_CUDA_ERR_STATE, "tensor parallelism needs 16-bit weights with 64-aligned shard sizes");
     if (stream_path(rows)) return launch_step_stream(rows, mode, s, profile);
-    if (tc_ready_ && rows > kSgMaxRows) return launch_step_wide(rows, mode, s);
+    if (tc_ready_ && rows > sg_max_rows_) return launch_step_wide(rows, mode, s);
     const bool gpt2 = m_.arch == ARCH_GPT2;
     const int cap = sm_count_ * 2;  // one wave: the stage kernels hold ~120 registers, two CTAs per SM
     int launches = 0;
@@ -1708,6 +1711,7 @@ int32_t Engine::build_tc() {
     if (quantised && (cfg_.flags & ESP_CUDA_FLAG_NO_TC_SHADOW)) return ESP_CUDA_OK;
     tc_bf16_ = t0 == ESP_CUDA_BF16;
     tc_quant_ = quantised;
+    sg_max_rows_ = m_.d_model <= 2048 ? kSgMaxRows : kSgMaxRowsWide;
     tc_mats_ = mats;
     tc_operands_ready_ = false;
     // 16-bit matrices get their TMA maps now.  A quantised model's fp16 expansion (what batches and prefill chunks
@@ -1725,7 +1729,7 @@ int32_t Engine::build_tc() {
     if ((rc = dev_alloc(owned_, &kraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &vraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &d_tc_error_, 4))) return rc;
-    if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, kSgMaxRows) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
+    if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, sg_max_rows_) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
     if (tp_size_ > 1 && (rc = dev_alloc(owned_, &tp_partial_, (size_t)max_rows_ * m_.d_model))) return rc;
     ESP_CUDA_TRY(cudaDeviceSynchronize());
     tc_ready_ = true;
@@ -1802,7 +1806,7 @@ int32_t Engine::launch_attention_decode(const DecodeAttArgs& a, int rows, cudaSt
 bool Engine::stream_path(int rows) const {
     // A quantised model's single rows stay on the kernels that read the GGUF blocks themselves (the persistent kernel and the
     // row-wise GEMVs): an engine that only ever decodes one sequence then never builds the fp16 expansion.
-    return tc_ready_ && rows <= kSgMaxRows && !(tc_quant_ && rows == 1);
+    return tc_ready_ && rows <= sg_max_rows_ && !(tc_quant_ && rows == 1);
 }
 
 int32_t Engine::launch_embed(int rows, float2* stat, cudaStream_t s) {
@@ -2014,7 +2018,7 @@ int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
         return launch_prep(rows, src, K, norm, g, b, dst, 1, s);
     };
     struct Part { const DeviceTensor* W; float* out; int ldo; const float* bias; };
-    auto gemm = [&](std::initializer_list<Part> parts, const uint16_t* xbuf, int epi, uint16_t* out16, int ld16, float* capture, bool all_rows = false) -> int32_t {
+    auto gemm = [&](std::initializer_list<Part> parts, const uint16_t* xbuf, int epi, uint16_t* out16, int ld16, float* capture, bool all_rows = false, int layer = 0) -> int32_t {
         const int K = parts.begin()->W->cols;
         const CUtensorMap* mx = activation_map(xbuf, K, 128);
         if (!mx) return fail(ESP_CUDA_ERR_CUDA, "tensor map missing for the batched path");
@@ -2029,6 +2033,7 @@ int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
         }
         a.n_groups = g; a.K = K; a.rows = rows; a.epilogue = epi; a.bf16 = tc_bf16_; a.out16 = out16; a.ld16 = ld16; a.debug = capture; a.error = d_tc_error_;
         a.active = all_rows ? nullptr : rs_.active;
+        a.m = m_; a.rs = rs_; a.kv = kv_; a.rope = gpt2 ? nullptr : d_rope_; a.layer = layer;
         ESP_CUDA_TRY(pg_launch(maps, *mx, a, sm_count_, s));
         launches++;
         return ESP_CUDA_OK;
@@ -2059,13 +2064,18 @@ int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
             const LayerWeights& lw = t.w;
             const bool cap = dbg && l == debug_layer_;
             if ((rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, lw.norm1_g, lw.norm1_b, xh_d_))) return rc;
-            if ((rc = gemm({{t.wq, act_.q, q, lw.bq}, {t.wk, kraw_, kv, lw.bk}, {t.wv, vraw_, kv, lw.bv}}, xh_d_, PG_STORE, nullptr, 0, nullptr))) return rc;
-            RopeArgs ra{};
-            ra.m = m_; ra.rs = rs_; ra.kv = kv_; ra.q = act_.q; ra.k_raw = kraw_; ra.v_raw = vraw_; ra.rope = gpt2 ? nullptr : d_rope_; ra.layer = l;
-            ra.debug = cap ? dbg : nullptr;
-            ra.q_norm = t.q_norm; ra.k_norm = t.k_norm;
-            ESP_CUDA_TRY(launch_pdl(k_rope_append, dim3(rows, (q / 2 + kv + kThreads - 1) / kThreads), dim3(kThreads), 0, s, ra));
-            launches++;
+            const bool fuse_qkv = !qk_norm_ && att_ok_hd;  // (head_dim 32, 64 or 128: whole heads per 128-row half)
+            if ((rc = gemm({{t.wq, act_.q, q, lw.bq}, {t.wk, kraw_, kv, lw.bk}, {t.wv, vraw_, kv, lw.bv}}, xh_d_, fuse_qkv ? PG_QKV : PG_STORE, nullptr, 0,
+                           cap && fuse_qkv ? dbg : nullptr, false, l)))
+                return rc;
+            if (!fuse_qkv) {
+                RopeArgs ra{};
+                ra.m = m_; ra.rs = rs_; ra.kv = kv_; ra.q = act_.q; ra.k_raw = kraw_; ra.v_raw = vraw_; ra.rope = gpt2 ? nullptr : d_rope_; ra.layer = l;
+                ra.debug = cap ? dbg : nullptr;
+                ra.q_norm = t.q_norm; ra.k_norm = t.k_norm;
+                ESP_CUDA_TRY(launch_pdl(k_rope_append, dim3(rows, (q / 2 + kv + kThreads - 1) / kThreads), dim3(kThreads), 0, s, ra));
+                launches++;
+            }
             if ((mode & STEP_TILED_ATT) && att_ok_hd) {
                 PrefillAttArgs pa{};
                 pa.m = m_; pa.kv = kv_; pa.q = act_.q; pa.ctx16 = xh_q_; pa.bf16 = tc_bf16_; pa.layer = l; pa.runs = d_runs_;

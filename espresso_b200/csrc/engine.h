@@ -204,6 +204,7 @@ private:
     bool tc_operands_ready_ = false;
     std::vector<std::string> tc_mats_;
     int tc_bf16_ = 0;
+    int sg_max_rows_ = 0;    // widest pass of the streamed products
     bool tc_quant_ = false;  // the operands are the fp16 expansion of a quantised model
     std::vector<LayerTensors> layer_tensors_;
     int tc_rows_alloc_ = 0;

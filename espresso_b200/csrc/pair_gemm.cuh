@@ -7,32 +7,34 @@
 //
 // Persistent: one CTA per SM, tiles dealt out in turn (batch tiles fastest, so that the tiles in flight share weights in L2);
 // the accumulator is double-buffered (2 x 256 TMEM columns), the epilogue of a tile runs under the products of the next.
-// The epilogue moves 32 columns at a time through a private staging area so that global accesses run along the weight rows.
+// Sixteen epilogue warps move 16 columns at a time through a private staging area so that global accesses run along the weight
+// rows (eight warps took 6.6 us per tile with the GELU epilogue, longer than the 4.1 us of a tile's products at K = 768).
+// A residual product with too few tiles for the chip is cut along K; its slices add into the residual stream.
 //
-// Roles (320 threads): warp 0 TMA, warp 1 MMA (in the pair's first CTA), warps 2..9 epilogue.  Barriers: `full` of the first
+// Roles (576 threads): warp 0 TMA, warp 1 MMA (in the pair's first CTA), warps 2..17 epilogue.  Barriers: `full` of the first
 // CTA counts the bytes of both CTAs' copies; `empty` and `acc_full` are arrived in both CTAs by one commit; `acc_empty` of the
-// first CTA collects the sixteen epilogue warps of the pair.  Every wait is bounded (error code 7).
+// first CTA collects the epilogue warps of both.  Every wait is bounded (error code 7).
 #pragma once
 #include "stream_gemm.cuh"
 
 namespace esp {
 
-constexpr int kPgThreads = 320;
-constexpr int kPgEpiWarps = 8;
+constexpr int kPgThreads = 576;
+constexpr int kPgEpiWarps = 16;
 constexpr int kPgRows = 256;         // batch rows of a tile (128 per CTA)
 constexpr int kPgStages = 5;
 constexpr int kPgXBytes = 128 * kTcBlockK * 2, kPgWBytes = 128 * kTcBlockK * 2;
 constexpr int kPgStageBytes = kPgXBytes + kPgWBytes;
-constexpr int kPgStageStride = 36;   // floats per staged row of 32 columns: 16-byte aligned, conflict-free
+constexpr int kPgStageStride = 20;   // floats per staged row of 16 columns: 16-byte aligned, conflict-free
 constexpr int kPgEpiBytes = kPgEpiWarps * 32 * kPgStageStride * 4;
 constexpr size_t kPgSmemBytes = (size_t)kPgStages * kPgStageBytes + kPgEpiBytes + 1024;
 
-enum PgEpilogue { PG_STORE = 0, PG_RESIDUAL = 1, PG_GELU = 2, PG_SWIGLU = 3 };
+enum PgEpilogue { PG_STORE = 0, PG_RESIDUAL = 1, PG_QKV = 2, PG_GELU = 3, PG_SWIGLU = 4 };
 
 struct PgGroup {
     int M;              // weight rows (a multiple of 4)
     int half0;          // index of its first 128-row half
-    float* out;         // PG_STORE / PG_RESIDUAL: [n][ldo] fp32
+    float* out;         // PG_STORE / PG_RESIDUAL / q of PG_QKV: [n][ldo] fp32
     int ldo;
     const float* bias;  // [M] or null
 };
@@ -44,21 +46,25 @@ struct PgArgs {
     int epilogue, bf16;
     uint16_t* out16;       // PG_GELU / PG_SWIGLU: [n][ld16]
     int ld16;
+    int splits, kb_per_split;  // K slices (PG_RESIDUAL only; else 1)
     const int* active;     // [rows]: rows with 0 are not written
-    float* debug;          // optional capture of batch row 0 (PG_GELU / PG_SWIGLU)
+    float* debug;          // optional capture of batch row 0 (PG_QKV / PG_GELU / PG_SWIGLU)
+    // PG_QKV: groups q, k, v
+    ModelDims m;
+    RowState rs;           // pos, seq
+    KvLayout kv;
+    const float2* rope;    // null for GPT-2
+    int layer;
     int* error;
 };
 
 template <>
-__device__ __forceinline__ void tmem_ld_cols<32>(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, "
-        "%24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-          "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
-          "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
+__device__ __forceinline__ void tmem_ld_cols<16>(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                   "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr)
+                 : "memory");
 }
 
 // A copy into this CTA's shared memory that completes on the pair's first CTA's barrier (same offset, rank bit cleared).
@@ -83,74 +89,129 @@ __device__ __forceinline__ void arrive_first_cta(uint64_t* bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(smem_u32(bar), 0)) : "memory");
 }
 
-// The 32 x 32 block in a warp's staging rows (batch rows nrow0.., weight rows m0..) to memory: eight lanes x four columns per
-// batch row, four rows per step; live = the rows to write.  Whole blocks take the branch-free form: all reads of the staging
-// rows and of the residual are in flight before the first store.
-template <int EPI, bool WHOLE>
-__device__ __forceinline__ void pg_store_rows(const PgArgs& a, const float* stg, int rr, int c, int nrow0, unsigned live, float* out, size_t step, int m, const float4& b) {
-    float4 res[8];
-    if constexpr (EPI == PG_RESIDUAL) {
+// What a warp's epilogue works on: 32 batch rows (TMEM lanes) from nrow0, of which `live` are written.
+struct PgWarp {
+    float* stg;        // private staging rows
+    uint32_t base;     // accumulator, this warp's lanes
+    int lane, sub, nrow0;
+    unsigned live;
+    bool first_slice;
+    size_t kv_row;     // PG_QKV: this lane's row: (sequence, position) part of its cache offset
+    int pos;
+};
+
+// The 32 x 16 block in the staging rows (weight rows m0.. of matrix gi) to memory: four lanes x four columns per batch row,
+// eight rows per step.
+template <int EPI>
+__device__ __forceinline__ void pg_store_block(const PgArgs& a, const PgWarp& w, int gi, int m0) {
+#define ESP_PG_G(field) (gi == 0 ? a.g[0].field : gi == 1 ? a.g[1].field : a.g[2].field)
+    const int c = (w.lane & 3) * 4, rr = w.lane >> 2, m = m0 + c;
+    const bool ok = m < ESP_PG_G(M);
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (const float* bias = ESP_PG_G(bias))
+        if (ok && w.first_slice) b = __ldg(reinterpret_cast<const float4*>(bias + m));
+    const bool to_cache = EPI == PG_QKV && gi > 0;
+    const int ldo = EPI >= PG_GELU ? a.ld16 : ESP_PG_G(ldo);
+    float* const out = EPI >= PG_GELU || to_cache ? nullptr : ESP_PG_G(out) + (size_t)(w.nrow0 + rr) * ldo + m;
+#undef ESP_PG_G
+    float4 res[4];
+    const bool add = EPI == PG_RESIDUAL && a.splits == 1;
+    if (add) {
 #pragma unroll
-        for (int i = 0; i < 8; i++)
-            if (WHOLE || ((live >> (4 * i + rr)) & 1u)) res[i] = *reinterpret_cast<const float4*>(out + i * step);
+        for (int i = 0; i < 4; i++)
+            if (ok && ((w.live >> (8 * i + rr)) & 1u)) res[i] = *reinterpret_cast<const float4*>(out + (size_t)(8 * i) * ldo);
     }
-    float4 v[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = *reinterpret_cast<const float4*>(stg + (4 * i + rr) * kPgStageStride + c);
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int r = 4 * i + rr;
-        if (!WHOLE && !((live >> r) & 1u)) continue;
-        v[i].x += b.x; v[i].y += b.y; v[i].z += b.z; v[i].w += b.w;
-        if constexpr (EPI == PG_RESIDUAL) { v[i].x += res[i].x; v[i].y += res[i].y; v[i].z += res[i].z; v[i].w += res[i].w; }
-        if constexpr (EPI == PG_STORE || EPI == PG_RESIDUAL) {
-            *reinterpret_cast<float4*>(out + i * step) = v[i];
+    for (int i = 0; i < 4; i++) {
+        const int r = 8 * i + rr;
+        float4 v = *reinterpret_cast<const float4*>(w.stg + r * kPgStageStride + c);
+        size_t at = 0;
+        if (EPI == PG_QKV) at = __shfl_sync(0xffffffffu, w.kv_row, r);
+        if (!ok || !((w.live >> r) & 1u)) continue;
+        v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+        if (EPI == PG_RESIDUAL) {
+            if (add) {
+                v.x += res[i].x; v.y += res[i].y; v.z += res[i].z; v.w += res[i].w;
+                *reinterpret_cast<float4*>(out + (size_t)(8 * i) * ldo) = v;
+            } else {
+                red_add_v4(out + (size_t)(8 * i) * ldo, v.x, v.y, v.z, v.w);
+            }
+        } else if (EPI == PG_STORE || (EPI == PG_QKV && !to_cache)) {
+            *reinterpret_cast<float4*>(out + (size_t)(8 * i) * ldo) = v;
+            if (EPI == PG_QKV && a.debug && w.nrow0 + r == 0) *reinterpret_cast<float4*>(a.debug + m) = v;
+        } else if (EPI == PG_QKV) {
+            const int head = m / a.m.head_dim;
+            const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
+            __half* dst = (gi == 1 ? a.kv.k : a.kv.v) + at + (size_t)head * a.m.max_seq * a.m.head_dim + (m & (a.m.head_dim - 1));
+            *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+            if (a.debug && w.nrow0 + r == 0) {
+                const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+                *reinterpret_cast<float4*>(a.debug + a.m.q_dim + (gi == 2 ? a.m.kv_dim : 0) + m) = make_float4(f0.x, f0.y, f1.x, f1.y);
+            }
         } else {
-            if constexpr (EPI == PG_GELU) v[i] = make_float4(gelu_fast(v[i].x), gelu_fast(v[i].y), gelu_fast(v[i].z), gelu_fast(v[i].w));
-            *reinterpret_cast<uint2*>(a.out16 + (size_t)(nrow0 + r) * a.ld16 + m) = make_uint2(pack16x2(v[i].x, v[i].y, a.bf16), pack16x2(v[i].z, v[i].w, a.bf16));
-            if (a.debug && nrow0 + r == 0) *reinterpret_cast<float4*>(a.debug + m) = v[i];
+            if (EPI == PG_GELU) v = make_float4(gelu_fast(v.x), gelu_fast(v.y), gelu_fast(v.z), gelu_fast(v.w));
+            *reinterpret_cast<uint2*>(a.out16 + (size_t)(w.nrow0 + r) * ldo + m) = make_uint2(pack16x2(v.x, v.y, a.bf16), pack16x2(v.z, v.w, a.bf16));
+            if (a.debug && w.nrow0 + r == 0) *reinterpret_cast<float4*>(a.debug + m) = v;
         }
     }
-}
-template <int EPI>
-__device__ __forceinline__ void pg_store_block(const PgArgs& a, const float* stg, int lane, int nrow0, unsigned live, int gi, int m0) {
-#define ESP_PG_G(field) (gi == 0 ? a.g[0].field : gi == 1 ? a.g[1].field : a.g[2].field)
-    const int c = (lane & 7) * 4, rr = lane >> 3, m = m0 + c;
-    if (m >= ESP_PG_G(M)) return;
-    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (const float* bias = ESP_PG_G(bias)) b = __ldg(reinterpret_cast<const float4*>(bias + m));
-    float* const out = EPI <= PG_RESIDUAL ? ESP_PG_G(out) + (size_t)(nrow0 + rr) * ESP_PG_G(ldo) + m : nullptr;
-    const size_t step = (size_t)4 * ESP_PG_G(ldo);
-#undef ESP_PG_G
-    if (live == 0xffffffffu) pg_store_rows<EPI, true>(a, stg, rr, c, nrow0, live, out, step, m, b);
-    else pg_store_rows<EPI, false>(a, stg, rr, c, nrow0, live, out, step, m, b);
 }
 
-// One accumulator (this warp's 32 batch rows x its columns of both halves) to memory.  half_of: see k_gemm_pair.
+__device__ __forceinline__ void pg_to_staging(const PgWarp& w, const uint32_t (&v)[16]) {
+    float* const mine = w.stg + w.lane * kPgStageStride;
+    __syncwarp();  // the block staged before has been read
+#pragma unroll
+    for (int i = 0; i < 4; i++) reinterpret_cast<uint4*>(mine)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    __syncwarp();
+}
+
+// One accumulator to memory: per half of 128 weight rows this warp takes two 16-column blocks, chosen so that with RoPE they
+// hold the two members of every rotation pair.  half_of: see k_gemm_pair.
 template <int EPI, class HalfOf>
-__device__ __forceinline__ void pg_epilogue(const PgArgs& a, float* stg, uint32_t base, int sub, int lane, int nrow0, unsigned live, int tile_w, HalfOf half_of) {
+__device__ __forceinline__ void pg_epilogue(const PgArgs& a, const PgWarp& w, int tile_w, HalfOf half_of) {
+    const bool rope = EPI == PG_QKV && a.rope;
+    const int apart = rope ? a.m.head_dim >> 5 : 1;  // blocks between the members of a pair
+    const int b0 = (w.sub / apart) * 2 * apart + w.sub % apart;
 #pragma unroll 1
-    for (int blk = 0; blk < (EPI == PG_SWIGLU ? 2 : 4); blk++) {  // 32 columns: half blk / 2, its columns sub * 64 + (blk & 1) * 32
-        const int h = blk >> 1, col = sub * 64 + (blk & 1) * 32;
-        uint32_t v[32];
-        tmem_ld_cols<32>(base + (uint32_t)(h * 128 + col), v);
-        if constexpr (EPI == PG_SWIGLU) {
-            uint32_t u[32];
-            tmem_ld_cols<32>(base + (uint32_t)(128 + col), u);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int i = 0; i < 32; i++) v[i] = __float_as_uint(silu_fast(__uint_as_float(v[i])) * __uint_as_float(u[i]));
-        } else {
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        }
-        float* const mine = stg + lane * kPgStageStride;
-#pragma unroll
-        for (int i = 0; i < 8; i++) reinterpret_cast<uint4*>(mine)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        __syncwarp();
+    for (int h = 0; h < (EPI == PG_SWIGLU ? 1 : 2); h++) {
         int gi, m0;
         half_of(tile_w, h, gi, m0);
-        pg_store_block<EPI>(a, stg, lane, nrow0, live, gi, m0 + col);
-        __syncwarp();
+        if (EPI == PG_SWIGLU) {
+#pragma unroll 1
+            for (int i = 0; i < 2; i++) {
+                uint32_t v[16], u[16];
+                tmem_ld_cols<16>(w.base + (uint32_t)((b0 + i) * 16), v);
+                tmem_ld_cols<16>(w.base + (uint32_t)(128 + (b0 + i) * 16), u);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] = __float_as_uint(silu_fast(__uint_as_float(v[j])) * __uint_as_float(u[j]));
+                pg_to_staging(w, v);
+                pg_store_block<EPI>(a, w, gi, m0 + (b0 + i) * 16);
+            }
+            continue;
+        }
+        uint32_t v[16], u[16];
+        tmem_ld_cols<16>(w.base + (uint32_t)(h * 128 + b0 * 16), v);
+        tmem_ld_cols<16>(w.base + (uint32_t)(h * 128 + (b0 + apart) * 16), u);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (EPI == PG_QKV && rope && gi < 2) {  // halves of a head: v is the first, u the second member of sixteen rotation pairs
+            const float4* cs = reinterpret_cast<const float4*>(a.rope + (size_t)w.pos * (a.m.head_dim >> 1) + ((b0 * 16) & ((a.m.head_dim >> 1) - 1)));
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float4 f = __ldg(cs + j);
+                const float v0 = __uint_as_float(v[2 * j]), u0 = __uint_as_float(u[2 * j]), v1 = __uint_as_float(v[2 * j + 1]), u1 = __uint_as_float(u[2 * j + 1]);
+                v[2 * j] = __float_as_uint(v0 * f.x - u0 * f.y); u[2 * j] = __float_as_uint(v0 * f.y + u0 * f.x);
+                v[2 * j + 1] = __float_as_uint(v1 * f.z - u1 * f.w); u[2 * j + 1] = __float_as_uint(v1 * f.w + u1 * f.z);
+            }
+        }
+#pragma unroll 1
+        for (int i = 0; i < 2; i++) {
+            if (i == 1) {
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] = u[j];
+            }
+            pg_to_staging(w, v);
+            pg_store_block<EPI>(a, w, gi, m0 + (b0 + i * apart) * 16);
+        }
     }
 }
 
@@ -165,7 +226,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
     float* const stage_area = reinterpret_cast<float*>(tiles + (size_t)kPgStages * kPgStageBytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x & 1, pair = (int)blockIdx.x >> 1, n_pairs = (int)gridDim.x >> 1;
-    const int n_tiles = a.tiles_n * a.tiles_w, num_kb = a.K / kTcBlockK;
+    const int n_tiles = a.tiles_n * a.tiles_w, n_units = n_tiles * a.splits, all_kb = a.K / kTcBlockK;  // a unit: one K slice of a tile, slices slowest
     // (matrix, first row) of a 128-row half; past the last matrix the rows load as zeros
     auto half_of = [&](int tile_w, int h, int& gi, int& m0) {
         if (a.epilogue == PG_SWIGLU) { gi = h; m0 = tile_w * 128; return; }  // half 0 gate, half 1 the same rows of the up matrix
@@ -198,7 +259,8 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
         int s = 0;
         uint32_t phase = 0;
         bool first_round = true, ok = true;
-        for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+        for (int unit = pair; unit < n_units && ok; unit += n_pairs) {
+            const int slice = unit / n_tiles, tile = unit - slice * n_tiles, kb0 = slice * a.kb_per_split, num_kb = min(a.kb_per_split, all_kb - kb0);
             const int tw = tile / a.tiles_n, n0 = (tile - tw * a.tiles_n) * kPgRows + rank * 128;
             int gi, m0;
             half_of(tw, rank, gi, m0);
@@ -208,8 +270,8 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
                 if (elect_one()) {
                     uint8_t* const sx = tiles + (size_t)s * kPgStageBytes;
                     if (rank == 0) mbar_expect_tx(s_full + s, 2 * kPgStageBytes);
-                    tma_load_pair(sx, &map_x, kb * kTcBlockK, n0, s_full + s);
-                    tma_load_pair(sx + kPgXBytes, map, kb * kTcBlockK, m0, s_full + s);
+                    tma_load_pair(sx, &map_x, (kb0 + kb) * kTcBlockK, n0, s_full + s);
+                    tma_load_pair(sx + kPgXBytes, map, (kb0 + kb) * kTcBlockK, m0, s_full + s);
                 }
                 __syncwarp();
                 if (++s == kPgStages) { s = 0; phase ^= 1u; first_round = false; }
@@ -224,7 +286,8 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
             uint32_t phase = 0;
             bool ok = true;
             int it = 0;
-            for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, it++) {
+            for (int unit = pair; unit < n_units && ok; unit += n_pairs, it++) {
+                const int num_kb = min(a.kb_per_split, all_kb - unit / n_tiles * a.kb_per_split);
                 const int buf = it & 1;
                 if (it >= 2 && !tc_wait(s_acc_empty + buf, ((it >> 1) - 1) & 1, a.error)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -256,21 +319,31 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
         }
     } else {
         // ---------------- epilogue: TMEM -> registers -> staging -> global ----------------
-        const int ew = warp - 2, quad = warp & 3, sub = ew >> 2;  // lanes 32 * quad.. of TMEM; which 64 columns of each half
-        float* const stg = stage_area + (size_t)ew * 32 * kPgStageStride;
+        const int ew = warp - 2, quad = warp & 3, sub = ew >> 2;  // lanes 32 * quad.. of TMEM; which quarter of the columns
+        PgWarp w{};
+        w.stg = stage_area + (size_t)ew * 32 * kPgStageStride;
+        w.lane = lane; w.sub = sub;
         int it = 0;
-        for (int tile = pair; tile < n_tiles; tile += n_pairs, it++) {
-            const int buf = it & 1;
-            const int tw = tile / a.tiles_n, nrow0 = (tile - tw * a.tiles_n) * kPgRows + rank * 128 + 32 * quad;
+        for (int unit = pair; unit < n_units; unit += n_pairs, it++) {
+            const int buf = it & 1, slice = unit / n_tiles, tile = unit - slice * n_tiles;
+            const int tw = tile / a.tiles_n;
+            w.nrow0 = (tile - tw * a.tiles_n) * kPgRows + rank * 128 + 32 * quad;
+            const int row = w.nrow0 + lane;
+            w.live = __ballot_sync(0xffffffffu, row < a.rows && (!a.active || __ldcg(a.active + row)));
+            w.first_slice = slice == 0;
+            if (a.epilogue == PG_QKV && row < a.rows) {
+                w.pos = __ldcg(a.rs.pos + row);
+                w.kv_row = a.kv.offset(a.m, a.layer, __ldcg(a.rs.seq + row), 0, w.pos);
+            }
             if (!tc_wait(s_acc_full + buf, (it >> 1) & 1, a.error)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned live = __ballot_sync(0xffffffffu, nrow0 + lane < a.rows && (!a.active || __ldcg(a.active + nrow0 + lane)));
-            const uint32_t base = tmem + (uint32_t)buf * 256u + ((uint32_t)(32 * quad) << 16);
-            if (live) {
-                if (a.epilogue == PG_STORE) pg_epilogue<PG_STORE>(a, stg, base, sub, lane, nrow0, live, tw, half_of);
-                else if (a.epilogue == PG_RESIDUAL) pg_epilogue<PG_RESIDUAL>(a, stg, base, sub, lane, nrow0, live, tw, half_of);
-                else if (a.epilogue == PG_GELU) pg_epilogue<PG_GELU>(a, stg, base, sub, lane, nrow0, live, tw, half_of);
-                else pg_epilogue<PG_SWIGLU>(a, stg, base, sub, lane, nrow0, live, tw, half_of);
+            w.base = tmem + (uint32_t)buf * 256u + ((uint32_t)(32 * quad) << 16);
+            if (w.live) {
+                if (a.epilogue == PG_STORE) pg_epilogue<PG_STORE>(a, w, tw, half_of);
+                else if (a.epilogue == PG_RESIDUAL) pg_epilogue<PG_RESIDUAL>(a, w, tw, half_of);
+                else if (a.epilogue == PG_QKV) pg_epilogue<PG_QKV>(a, w, tw, half_of);
+                else if (a.epilogue == PG_GELU) pg_epilogue<PG_GELU>(a, w, tw, half_of);
+                else pg_epilogue<PG_SWIGLU>(a, w, tw, half_of);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             if (lane == 0) arrive_first_cta(s_acc_empty + buf);

@@ -127,8 +127,21 @@ cudaError_t pg_launch(const CUtensorMap* const* mw, const CUtensorMap& mx, PgArg
     for (int g = 0; g < groups; g++) { a.g[g].half0 = halves; halves += (a.g[g].M + 127) / 128; }
     a.tiles_w = a.epilogue == PG_SWIGLU ? halves : (halves + 1) / 2;
     a.tiles_n = (a.rows + kPgRows - 1) / kPgRows;
+    // K slices of a residual product: the fewest k blocks on the busiest pair (about 0.27 us each), a unit's epilogue and its
+    // atomics counted as 8 blocks.  401 rows x 5632 x 2048: 16 tiles on 74 pairs, one slice 46 us.
+    const int tiles = a.tiles_n * a.tiles_w, kb = a.K / kTcBlockK, pairs = sms / 2;
+    a.splits = 1;
+    a.kb_per_split = kb;
+    if (a.epilogue == PG_RESIDUAL) {
+        int best = 1 << 30;
+        for (int want = 1; want <= 8; want++) {
+            const int per = (kb + want - 1) / want, n = (kb + per - 1) / per;
+            const int cost = (tiles * n + pairs - 1) / pairs * (per + (n > 1 ? 8 : 0));
+            if (cost < best) { best = cost; a.splits = n; a.kb_per_split = per; }
+        }
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * std::min(sms / 2, a.tiles_n * a.tiles_w));
+    cfg.gridDim = dim3(2 * std::min(pairs, tiles * a.splits));
     cfg.blockDim = dim3(kPgThreads);
     cfg.dynamicSmemBytes = kPgSmemBytes;
     cfg.stream = s;
