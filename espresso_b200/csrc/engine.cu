@@ -2137,16 +2137,17 @@ static size_t mega_arena_layout(const ModelDims& m, const MegaPlan& p, int np, M
     return o + kMegaLineWords;
 }
 
-template <int WT>
+template <int WT, bool GPT2>
 static const void* mega_kernel_of(int head_dim) {
-    if (head_dim == 64) return reinterpret_cast<const void*>(&k_decode_mega<64, WT>);
-    if (head_dim == 128) return reinterpret_cast<const void*>(&k_decode_mega<128, WT>);
-    return reinterpret_cast<const void*>(&k_decode_mega<32, WT>);
+    if (head_dim == 64) return reinterpret_cast<const void*>(&k_decode_mega<64, WT, GPT2>);
+    if (head_dim == 128) return reinterpret_cast<const void*>(&k_decode_mega<128, WT, GPT2>);
+    return reinterpret_cast<const void*>(&k_decode_mega<32, WT, GPT2>);
 }
-static const void* mega_kernel_for(int head_dim, int wt) {
-    if (wt == WT_Q8_0) return mega_kernel_of<WT_Q8_0>(head_dim);
-    if (wt == WT_Q4_0) return mega_kernel_of<WT_Q4_0>(head_dim);
-    return mega_kernel_of<WT_F16>(head_dim);
+static const void* mega_kernel_for(int head_dim, int wt, bool gpt2) {
+    if (gpt2) return mega_kernel_of<WT_F16, true>(head_dim);
+    if (wt == WT_Q8_0) return mega_kernel_of<WT_Q8_0, false>(head_dim);
+    if (wt == WT_Q4_0) return mega_kernel_of<WT_Q4_0, false>(head_dim);
+    return mega_kernel_of<WT_F16, false>(head_dim);
 }
 
 // Plans and packs the persistent decode kernel.  Every CTA owns a contiguous share of the rows of every matrix;
@@ -2154,7 +2155,8 @@ static const void* mega_kernel_for(int head_dim, int wt) {
 int32_t Engine::build_mega() {
     mega_ready_ = false;
     if ((cfg_.flags & ESP_CUDA_FLAG_NO_MEGAKERNEL) || tp_size_ > 1) return ESP_CUDA_OK;
-    if (m_.arch != ARCH_LLAMA || qk_norm_) return ESP_CUDA_OK;  // (the per-head q/k norm lives in the per-stage and batched kernels)
+    const bool gpt2 = m_.arch == ARCH_GPT2;
+    if (qk_norm_) return ESP_CUDA_OK;  // (the per-head q/k norm lives in the per-stage and batched kernels)
     if (m_.head_dim != 32 && m_.head_dim != 64 && m_.head_dim != 128) return ESP_CUDA_OK;
     if (m_.d_model % 32 || m_.hidden % 32 || m_.n_head > sm_count_ || m_.n_head > 255 || m_.vocab >= (1 << 24)) return ESP_CUDA_OK;
     // The layer matrices share one storage type (fp16, or GGUF Q8_0 / Q4_0 blocks, which travel through the ring as they
@@ -2162,12 +2164,12 @@ int32_t Engine::build_mega() {
     auto type_of = [&](const std::string& name) { return tensors_.at(name).type; };
     const int wt_layer = type_of("layers/0/wq");
     const int wt_head = type_of("lm_head");
-    if (wt_layer != ESP_CUDA_F16 && wt_layer != ESP_CUDA_Q8_0 && wt_layer != ESP_CUDA_Q4_0) return ESP_CUDA_OK;
+    if (wt_layer != ESP_CUDA_F16 && (gpt2 || (wt_layer != ESP_CUDA_Q8_0 && wt_layer != ESP_CUDA_Q4_0))) return ESP_CUDA_OK;
     if (wt_head != wt_layer && wt_head != ESP_CUDA_F16) return ESP_CUDA_OK;
     if (tensors_.at("embeddings/token").type != ESP_CUDA_F16) return ESP_CUDA_OK;
     for (int l = 0; l < m_.n_layer; l++)
         for (const char* n : {"wq", "wk", "wv", "wo", "w1", "w2", "w3"})
-            if (type_of("layers/" + std::to_string(l) + "/" + n) != wt_layer) return ESP_CUDA_OK;
+            if (!(gpt2 && n[1] == '3') && type_of("layers/" + std::to_string(l) + "/" + n) != wt_layer) return ESP_CUDA_OK;
     const bool quant = wt_layer != ESP_CUDA_F16 || wt_head != ESP_CUDA_F16;
     if (quant && (m_.d_model % 256 || m_.hidden % 256)) return ESP_CUDA_OK;  // chunk sizes must stay multiples of 16 bytes
     int coop = 0, smem_max = 0;
@@ -2206,7 +2208,8 @@ int32_t Engine::build_mega() {
     if (p.rpb % wo_rows) return ESP_CUDA_OK;
     p.s1_bytes = pad128((long long)2 * p.s1_max * p.row_bytes);
     p.s2_bytes = pad128((long long)p.rpb * p.wo_row_bytes);
-    p.s3a_bytes = pad128((long long)2 * p.hpc_max * p.row_bytes);
+    p.ffn_rows = gpt2 ? 1 : 2;
+    p.s3a_bytes = pad128((long long)p.ffn_rows * p.hpc_max * p.row_bytes);
     p.s3b_bytes = pad128((long long)p.dpc_max * p.down_row_bytes);
     p.layer_bytes = (long long)p.s1_bytes + p.s2_bytes + p.s3a_bytes + p.s3b_bytes;
     p.head_bytes = pad128((long long)p.vpc_max * p.head_row_bytes);
@@ -2216,20 +2219,23 @@ int32_t Engine::build_mega() {
     const int item_max = std::max(2 * p.row_bytes, p.down_row_bytes);
     p.slot_bytes = pad128(std::max(48 * 1024, item_max));
     p.s1_ipc = std::max(1, std::min(std::min(p.s1_max, kMegaChunkRows / 2), p.slot_bytes / (2 * p.row_bytes)));
-    p.s3a_ipc = std::max(1, std::min(std::min(p.hpc_max, kMegaChunkRows / 2), p.slot_bytes / (2 * p.row_bytes)));
+    p.s3a_ipc = std::max(1, std::min(std::min(p.hpc_max, kMegaChunkRows / p.ffn_rows), p.slot_bytes / (p.ffn_rows * p.row_bytes)));
     p.s3b_rpc = std::max(1, std::min(std::min(p.dpc_max, kMegaChunkRows), p.slot_bytes / p.down_row_bytes));
     p.head_rpc = std::max(1, std::min(std::min(p.vpc_max, kMegaChunkRows), p.slot_bytes / p.head_row_bytes));
     p.s2_rpc = std::max(1, std::min(std::min(p.rpb, kMegaChunkRows), p.slot_bytes / p.wo_row_bytes));
     p.s2_rpc = std::max(wo_rows, p.s2_rpc / wo_rows * wo_rows);
+    // As many ring slots as fit; then the largest group of chunks per CTA barrier whose partial sums do not cost a slot.
     p.n_slots = 0;
-    for (int ns = 8; ns >= 2; ns--) {
-        MegaPlan probe = p;
-        probe.n_slots = ns;
-        mega_layout(m_, probe);
-        if (probe.smem_bytes <= smem_max) { p = probe; break; }
-    }
+    for (int ns = 8; ns >= 2 && p.n_slots == 0; ns--)
+        for (int group : {4, 2, 1}) {
+            MegaPlan probe = p;
+            probe.n_slots = ns;
+            probe.group = group;
+            mega_layout(m_, probe);
+            if (probe.smem_bytes <= smem_max) { p = probe; break; }
+        }
     if (p.n_slots == 0) return ESP_CUDA_OK;  // does not fit: the per-stage kernels serve this model
-    const void* kern = mega_kernel_for(m_.head_dim, wt_layer);
+    const void* kern = mega_kernel_for(m_.head_dim, wt_layer, gpt2);
     ESP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem_bytes));
     int occ = 0;
     ESP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kMegaThreads, p.smem_bytes));
@@ -2250,6 +2256,7 @@ int32_t Engine::build_mega() {
     const char* names[7] = {"wq", "wk", "wv", "wo", "w1", "w2", "w3"};
     for (int k = 0; k < 7; k++)
         for (int l = 0; l < m_.n_layer; l++) {
+            if (gpt2 && k == 6) continue;
             const DeviceTensor& t = tensors_.at("layers/" + std::to_string(l) + "/" + names[k]);
             mats[(size_t)k * m_.n_layer + l] = PackMatrix{t.data, t.scales};
         }
@@ -2267,17 +2274,43 @@ int32_t Engine::build_mega() {
     }
     for (int l = 0; l < m_.n_layer && e == cudaSuccess; l++) {
         std::string pre = "layers/" + std::to_string(l) + "/";
-        e = cudaMemcpyAsync(d_norms_ + (size_t)(2 * l) * m_.d_model, tensors_.at(pre + "rms_att").f32, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_);
+        e = cudaMemcpyAsync(d_norms_ + (size_t)(2 * l) * m_.d_model, tensors_.at(pre + (gpt2 ? "ln_1_gamma" : "rms_att")).f32, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(d_norms_ + (size_t)(2 * l + 1) * m_.d_model, tensors_.at(pre + "rms_ffn").f32, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_);
+            e = cudaMemcpyAsync(d_norms_ + (size_t)(2 * l + 1) * m_.d_model, tensors_.at(pre + (gpt2 ? "ln_2_gamma" : "rms_ffn")).f32, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_);
     }
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_norms_ + (size_t)(2 * m_.n_layer) * m_.d_model, tensors_.at("rms_final").f32, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_);
+        e = cudaMemcpyAsync(d_norms_ + (size_t)(2 * m_.n_layer) * m_.d_model, tensors_.at(gpt2 ? "final_norm_gamma" : "rms_final").f32, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_);
+    if (e == cudaSuccess && gpt2 && (rc = build_mega_gpt2())) { cudaFree(d_mats); return rc; }
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
     cudaFree(d_mats);
     ESP_CUDA_TRY(e);
     mega_plan_ = p;
     mega_ready_ = true;
+    return ESP_CUDA_OK;
+}
+
+// GPT-2: the folded LayerNorm constants of every row and the biases of the two residual products.
+int32_t Engine::build_mega_gpt2() {
+    const int d = m_.d_model, q = m_.q_dim, kv = m_.kv_dim, h = m_.hidden, per = q + 2 * kv + h;
+    int32_t rc;
+    if ((rc = dev_alloc(owned_, &d_mega_ln_, (size_t)m_.n_layer * per + m_.vocab, false))) return rc;
+    if ((rc = dev_alloc(owned_, &d_mega_bias_, (size_t)m_.n_layer * 2 * d, false))) return rc;
+    auto fold = [&](const DeviceTensor& w, const float* g, const float* b, const float* bias, float2* out) {
+        k_fold_norm<<<(w.rows + 7) / 8, 256, 0, stream_>>>(static_cast<const uint16_t*>(w.data), w.rows, d, g, b, bias, out);
+    };
+    for (int l = 0; l < m_.n_layer; l++) {
+        const std::string pre = "layers/" + std::to_string(l) + "/";
+        const LayerWeights lw = layer_weights(l);
+        float2* out = d_mega_ln_ + (size_t)l * per;
+        fold(tensors_.at(pre + "wq"), lw.norm1_g, lw.norm1_b, lw.bq, out);
+        fold(tensors_.at(pre + "wk"), lw.norm1_g, lw.norm1_b, lw.bk, out + q);
+        fold(tensors_.at(pre + "wv"), lw.norm1_g, lw.norm1_b, lw.bv, out + q + kv);
+        fold(tensors_.at(pre + "w1"), lw.norm2_g, lw.norm2_b, lw.b1, out + q + 2 * kv);
+        ESP_CUDA_TRY(cudaMemcpyAsync(d_mega_bias_ + (size_t)(2 * l) * d, lw.bo, sizeof(float) * d, cudaMemcpyDeviceToDevice, stream_));
+        ESP_CUDA_TRY(cudaMemcpyAsync(d_mega_bias_ + (size_t)(2 * l + 1) * d, lw.b2, sizeof(float) * d, cudaMemcpyDeviceToDevice, stream_));
+    }
+    fold(tensors_.at("lm_head"), tensors_.at("final_norm_gamma").f32, tensors_.at("final_norm_beta").f32, nullptr, d_mega_ln_ + (size_t)m_.n_layer * per);
+    ESP_CUDA_TRY(cudaGetLastError());
     return ESP_CUDA_OK;
 }
 
@@ -2289,6 +2322,11 @@ int32_t Engine::launch_mega(int n_steps, const uint32_t* feed, bool times) {
     const MegaPlan& p = mega_plan_;
     a.m = m_; a.plan = p; a.pack = d_pack_; a.norms = d_norms_;
     a.tok_emb = static_cast<const uint16_t*>(tensors_.at("embeddings/token").data);
+    if (m_.arch == ARCH_GPT2) {
+        a.pos_emb = static_cast<const uint16_t*>(tensors_.at("embeddings/position").data);
+        a.ln = d_mega_ln_;
+        a.out_bias = d_mega_bias_;
+    }
     a.rope = d_rope_; a.kv = kv_; a.hidden_io = act_.hidden;
     a.x_words = d_mega_arena_;
     mega_arena_layout(m_, p, 1, &a);
@@ -2319,7 +2357,7 @@ int32_t Engine::launch_mega(int n_steps, const uint32_t* feed, bool times) {
     if (!ev_begin_) { ESP_CUDA_TRY(cudaEventCreate(&ev_begin_)); ESP_CUDA_TRY(cudaEventCreate(&ev_end_)); }
     if (times) ESP_CUDA_TRY(cudaEventRecord(ev_begin_, stream_));
     void* args[] = {&a};
-    ESP_CUDA_TRY(cudaLaunchCooperativeKernel(mega_kernel_for(m_.head_dim, p.wt_layer), dim3(p.n_cta), dim3(kMegaThreads), args, (size_t)p.smem_bytes, stream_));
+    ESP_CUDA_TRY(cudaLaunchCooperativeKernel(mega_kernel_for(m_.head_dim, p.wt_layer, m_.arch == ARCH_GPT2), dim3(p.n_cta), dim3(kMegaThreads), args, (size_t)p.smem_bytes, stream_));
     if (times) ESP_CUDA_TRY(cudaEventRecord(ev_end_, stream_));
     ESP_CUDA_TRY(cudaMemcpyAsync(h_mega_ctl_, d_mega_ctl_, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream_));
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
@@ -2332,7 +2370,7 @@ int32_t Engine::launch_mega(int n_steps, const uint32_t* feed, bool times) {
            << ": 3 = weight chunk, 4 = ring slot, 5/9 = layer output words, 6 = q/k/v words, 7 = attention sums, 8 = activation words, 10 = arg-max words)";
         return fail(ESP_CUDA_ERR_TIMEOUT, os.str());
     }
-    mega_cand_ = (a.cand0 + (unsigned)a.first + (unsigned)(h_mega_ctl_[5] & 0xffffffffull)) % 255u;  // right behind the last step that ran
+    mega_cand_ = (a.cand0 + (unsigned)a.first + (unsigned)(h_mega_ctl_[5] & 0xffffffffull) + 1u) % 255u;  // behind the last step that ran (GPT-2's last one may emit nothing)
     mega_dirty_ = false;
     return ESP_CUDA_OK;
 }
@@ -2343,20 +2381,20 @@ int32_t Engine::run_mega(int n_steps, int* emitted, float* device_ms, double* fi
     int32_t rc = launch_mega(n_steps, nullptr, true);
     if (rc) return rc;
     const int n = (int)(h_mega_ctl_[5] & 0xffffffffull);
-    if (n < 1 || n > n_steps) return fail(ESP_CUDA_ERR_CUDA, "persistent decode kernel reported an impossible token count");
+    if (n < (m_.arch == ARCH_GPT2 ? 0 : 1) || n > n_steps) return fail(ESP_CUDA_ERR_CUDA, "persistent decode kernel reported an impossible token count");
     if (emitted) *emitted = n;
     const bool have_times = n_steps <= m_.max_seq + 1;
     token_times_n_ = have_times ? n : 0;
     if (device_ms) ESP_CUDA_TRY(cudaEventElapsedTime(device_ms, ev_begin_, ev_end_));
-    if (first_token_ms) *first_token_ms = (double)(h_mega_ctl_[4] - h_mega_ctl_[3]) / 1e6;
+    if (first_token_ms) *first_token_ms = n > 0 ? (double)(h_mega_ctl_[4] - h_mega_ctl_[3]) / 1e6 : 0.0;
     latencies_ms_.clear();
-    if (have_times) {
+    if (have_times && n > 0) {
         std::vector<unsigned long long> tt((size_t)n);
         ESP_CUDA_TRY(cudaMemcpy(tt.data(), d_token_times_, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost));
         unsigned long long prev = h_mega_ctl_[3];  // kernel start
         for (int i = 0; i < n; i++) { latencies_ms_.push_back((float)((double)(tt[i] - prev) / 1e6)); prev = tt[i]; }
     }
-    h_visible_[0] += n - 1;
+    h_visible_[0] = (int)h_mega_ctl_[6];
     return ESP_CUDA_OK;
 }
 
@@ -2384,6 +2422,7 @@ int32_t Engine::ensure_norms2() {
 // The two-token kernel serves a target and a draft that are both fp16 Llama models on the persistent-kernel path, on one
 // device, with the same widths: they then share one plan (chunk sizes, work shares, ring) and differ in depth only.
 bool Engine::spec_compatible(const Engine& draft) const {
+    if (m_.arch != ARCH_LLAMA || draft.m_.arch != ARCH_LLAMA) return false;
     if (!mega_ready_ || !draft.mega_ready_ || tp_size_ > 1 || draft.tp_size_ > 1) return false;
     if ((cfg_.flags | draft.cfg_.flags) & (ESP_CUDA_FLAG_NO_MEGAKERNEL | ESP_CUDA_FLAG_NO_GRAPH)) return false;
     if (debug_layer_ >= 0 || draft.debug_layer_ >= 0 || cfg_.device != draft.cfg_.device) return false;
@@ -2427,6 +2466,7 @@ int32_t Engine::spec_prepare() {
 }
 
 bool Engine::spec_verify_ok() const {
+    if (m_.arch != ARCH_LLAMA) return false;
     if (!mega_ready_ || tp_size_ > 1 || debug_layer_ >= 0) return false;
     if (cfg_.flags & (ESP_CUDA_FLAG_NO_MEGAKERNEL | ESP_CUDA_FLAG_NO_GRAPH | ESP_CUDA_FLAG_KEEP_LOGITS)) return false;
     return mega_plan_.wt_layer == ESP_CUDA_F16 && mega_plan_.wt_head == ESP_CUDA_F16;

@@ -130,6 +130,7 @@ private:
     LayerWeights layer_weights(int l) const;
     size_t gemv_smem(int type, int K, bool with_tmp) const;
     int32_t build_mega();   // packs the weights for the persistent decode kernel when the model qualifies
+    int32_t build_mega_gpt2();
     int32_t launch_mega(int n_steps, const uint32_t* feed, bool times);
     bool mega_usable() const;
     int32_t run_mega(int n_steps, int* emitted, float* device_ms, double* first_token_ms);
@@ -220,6 +221,8 @@ private:
     MegaPlan mega_plan_{};
     uint8_t* d_pack_ = nullptr;
     float* d_norms_ = nullptr;
+    float2* d_mega_ln_ = nullptr;   // GPT-2: folded LayerNorm constants (MegaArgs::ln)
+    float* d_mega_bias_ = nullptr;  // GPT-2: biases of Wo and W2
     unsigned long long* d_mega_arena_ = nullptr;  // exchange words and counted sums of the persistent kernel
     size_t mega_arena_words_ = 0;
     unsigned mega_tag_ = 0, mega_cand_ = 0;       // numbering of the exchanges, continued from launch to launch

@@ -80,6 +80,8 @@ struct MegaPlan {
     int head_row_bytes;  // ... of d_model columns of the LM head
     int s1_bytes, s2_bytes, s3a_bytes, s3b_bytes;  // packed bytes of a stage per layer (multiples of 128, sized for the largest CTA share)
     // A stage whose slice is larger than a ring slot arrives in several chunks of whole items:
+    int group;        // chunks whose products share one CTA barrier (see group_products)
+    int ffn_rows;     // packed rows per FFN unit: (gate, up) pairs 2, GPT-2's single up projection 1
     int s1_ipc;       // S1 row pairs per chunk
     int s2_rpc;       // S2 projection rows per chunk (a multiple of the rows one pass of the CTA covers)
     int s3a_ipc;      // S3 (gate, up) pairs per chunk
@@ -105,6 +107,11 @@ struct MegaArgs {
     const uint8_t* pack;      // [n_cta][cta_bytes]
     const float* norms;       // [2*L + 1][d_model]: norm1(l), norm2(l), ..., final
     const uint16_t* tok_emb;  // fp16 [vocab][d_model]
+    // GPT-2 only.  LayerNorm is folded into the products: W.(x g) is accumulated while x arrives, and a row's result is
+    // inv (sum - mean W.g) + (W.b + bias); the two constants of every row are computed once.
+    const uint16_t* pos_emb;  // fp16 [max_seq][d_model]
+    const float2* ln;         // per layer [q_dim + 2 kv_dim + hidden], then [vocab] for the head: {W.g, W.b + bias}
+    const float* out_bias;    // per layer [bias of Wo, bias of W2], d_model each
     const float2* rope;       // [max_seq][head_dim/2]
     KvLayout kv;
     // exchange arena (zero before the first launch; tags keep launches apart, the counted sums are zeroed at the end)
@@ -115,7 +122,7 @@ struct MegaArgs {
     unsigned long long* cand_words; // [n_cta][kMegaCandStride] {logit bits, index, 8-bit tag} of each CTA's best row in word 0
     float* hidden_io;         // [d_model] last hidden state of the sequence (in and out)
     int* error;               // [1] 0 = ok
-    unsigned long long* stamps; // [3] globaltimer at kernel start and when the first token is known; {last token : 32}{number of tokens emitted : 32}
+    unsigned long long* stamps; // [4] globaltimer at kernel start and when the first token is known; {last token : 32}{number of tokens emitted : 32}; visible tokens
     unsigned long long* token_times; // optional [n_steps] globaltimer (ns) at which each token became known, or null
     long long* trace;         // optional [kMegaTraceLayer*L + kMegaTraceHead] SM clock stamps of the last step taken by CTA `trace_cta`, or null
     int trace_cta;
@@ -257,7 +264,7 @@ struct MegaShared {
     __half* vn;    // [head_dim]
     float* part;   // [warps][head_dim]
     float* red;    // [64]
-    float* partial;  // [2][kMegaChunkRows] partial row sums of a chunk (alternating halves)
+    float* partial;  // [2][group][kMegaChunkRows] partial row sums of a group of chunks (alternating halves)
     unsigned long long* key;   // [32] arg-max keys
     struct MegaShare* share;  // this CTA's work shares, computed once
     int* hbeg;     // [n_cta + 1] first FFN unit (= element of the activation vector) of every CTA
@@ -312,7 +319,7 @@ inline void mega_layout(const ModelDims& m, MegaPlan& p) {
     p.off_vn = take(sizeof(__half) * (size_t)m.head_dim);
     p.off_part = take(sizeof(float) * (size_t)kMegaConsumerWarps * m.head_dim);
     p.off_red = take(sizeof(float) * 64);
-    p.off_outv = take(sizeof(float) * 2 * kMegaChunkRows);
+    p.off_outv = take(sizeof(float) * 2 * p.group * kMegaChunkRows);
     p.off_flags = take(16);
     p.off_share = take(sizeof(MegaShare));
     p.off_beg = take(sizeof(int) * ((size_t)p.n_cta + 1));
@@ -388,7 +395,7 @@ __device__ __forceinline__ void mega_release(const MegaArgs& a, const MegaShared
     if ((threadIdx.x & 31) == 0) mbar_arrive(s.empty + c.slot);
     c.next((unsigned)a.plan.n_slots);
 }
-// Hands back `n` consecutive slots starting at `from` whose release was put off (see the kernel's chunk_products).
+// Hands back `n` consecutive slots starting at `from` whose release was put off (see the kernel's group_products).
 __device__ __forceinline__ void mega_release_deferred(const MegaArgs& a, const MegaShared& s, MegaCursor from, int n) {
     __syncwarp();
     for (int i = 0; i < n; i++) {
@@ -562,6 +569,22 @@ __device__ __forceinline__ float mega_block_sum(float v, float* red) {
     const float4 a = r4[0], b = r4[1], c = r4[2], e = r4[3];
     static_assert(kMegaConsumerWarps == 16, "mega_block_sum reads sixteen partial sums");
     return (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) + (((c.x + c.y) + (c.z + c.w)) + ((e.x + e.y) + (e.z + e.w)));
+}
+
+// The same for two floats (GPT-2: sum and sum of squares).
+__device__ __forceinline__ float2 mega_block_sum2(float v0, float v1, float* red) {
+    v0 = warp_sum(v0);
+    v1 = warp_sum(v1);
+    if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = v0; red[kMegaConsumerWarps + (threadIdx.x >> 5)] = v1; }
+    consumer_sync();
+    const float4* r4 = reinterpret_cast<const float4*>(red);
+    float out[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const float4 a = r4[4 * q], b = r4[4 * q + 1], c = r4[4 * q + 2], e = r4[4 * q + 3];
+        out[q] = (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) + (((c.x + c.y) + (c.z + c.w)) + ((e.x + e.y) + (e.z + e.w)));
+    }
+    return make_float2(out[0], out[1]);
 }
 
 // ------------------------------------------------------------------------------------------------ products
@@ -768,12 +791,15 @@ __device__ __forceinline__ float2 mega_tile_dot(const uint8_t* chunk, int R, int
 // shifts (per chunk every scalar instruction of this set-up is on the critical path of the token).  Unit u = tile <<
 // lg | range stores its sixteen partial sums at partial[u * 16 ...] (position q: + q * kMegaChunkRows); returns lg.  The
 // caller synchronises before reading.
+// log2 of the column ranges of a chunk of R rows: the largest value with tiles << lg <= warps and 1 << lg <= n_kb.
+__device__ __forceinline__ int mega_chunk_lg(int R, int n_kb) {
+    const int n_tiles = (R + 15) >> 4;
+    const int lg_t = n_tiles > 1 ? 32 - __clz(n_tiles - 1) : 0;  // ceil(log2(tiles))
+    return max(0, min(4 - lg_t, 31 - __clz(n_kb)));
+}
 template <int WT, int NP = 1>
 __device__ __forceinline__ int mega_chunk_dots(const uint8_t* chunk, int R, int n_kb, const uint8_t* xa, float* partial, int warp, int lane) {
-    const int n_tiles = (R + 15) >> 4;
-    // lg = log2(column ranges): the largest value with tiles << lg <= warps and 1 << lg <= n_kb
-    const int lg_t = n_tiles > 1 ? 32 - __clz(n_tiles - 1) : 0;  // ceil(log2(tiles))
-    const int lg = max(0, min(4 - lg_t, 31 - __clz(n_kb)));
+    const int n_tiles = (R + 15) >> 4, lg = mega_chunk_lg(R, n_kb);
     const int per = (n_kb + (1 << lg) - 1) >> lg;
     for (int u = warp; u < (n_tiles << lg); u += kMegaConsumerWarps) {
         const int tile = u >> lg, part = u & ((1 << lg) - 1);
@@ -979,7 +1005,7 @@ __device__ __forceinline__ void mega_attention(const MegaArgs& a, const MegaShar
 
 // ------------------------------------------------------------------------------------------------ the kernel
 
-template <int HD, int WT>
+template <int HD, int WT, bool GPT2>
 __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs a) {
     extern __shared__ __align__(128) uint8_t mega_smem[];
     const MegaShared s = mega_carve(mega_smem, a);
@@ -1058,7 +1084,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                         off += p.s1_bytes;
                         if (w.in_group) issue_stage(off, p.rpb, p.s2_rpc, p.wo_row_bytes);
                         off += p.s2_bytes;
-                        issue_stage(off, w.h_n, p.s3a_ipc, 2 * p.row_bytes); off += p.s3a_bytes;
+                        issue_stage(off, w.h_n, p.s3a_ipc, (GPT2 ? 1 : 2) * p.row_bytes); off += p.s3a_bytes;
                         issue_stage(off, w.d_n, p.s3b_rpc, p.down_row_bytes);
                     }
                 }
@@ -1129,13 +1155,14 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
     // Stages values of the residual stream: raw copy, gained copy as the products' staged operand (fp16 hi/lo parts, or
     // int8 digits for the quantised types; `K` = length of the vector being staged), sum of squares.
     constexpr bool kQuant = WT == WT_Q8_0;  // int8 digit staging (Q4_0 widens its nibbles to fp16 and reads the fp16 staging)
-    auto stage_x = [&](float* raw, int K, bool digits, int k, float v, float g, float& ss) {  // one element per lane, consecutive k
+    auto stage_x = [&](float* raw, int K, bool digits, int k, float v, float g, float& ss, float& sm) {  // one element per lane, consecutive k
         raw[k] = v;
         if (kQuant && digits) qx_store_elem(s.xa, reinterpret_cast<float*>(s.xa + xa_bytes(K)), k, v * g);
         else xa_store(xa_h, k, v * g);
         ss = fmaf(v, v, ss);
+        if (GPT2) sm += v;
     };
-    auto stage_x2 = [&](float* raw, int K, bool digits, int k, float v0, float v1, float g0, float g1, float& ss) {  // a pair per lane
+    auto stage_x2 = [&](float* raw, int K, bool digits, int k, float v0, float v1, float g0, float g1, float& ss, float& sm) {  // a pair per lane
         raw[k] = v0; raw[k + 1] = v1;
         if (kQuant && digits) {
             qx_store_pair(s.xa, reinterpret_cast<float*>(s.xa + xa_bytes(K)), k, v0 * g0, v1 * g1);
@@ -1144,10 +1171,21 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
             xa_store(xa_h, k + 1, v1 * g1);
         }
         ss = fmaf(v0, v0, fmaf(v1, v1, ss));
+        if (GPT2) sm += v0 + v1;
     };
+    // Norm scale (and mean) from the staged vector's sums; one CTA barrier.
+    float mean = 0.f;
+    auto norm_scale = [&](float ss, float sm) {
+        if constexpr (GPT2) {
+            const float2 t = mega_block_sum2(sm, ss, s.red);
+            mean = t.x * inv_d;
+            return rsqrtf(fmaxf(fmaf(-mean, mean, t.y * inv_d), 0.f) + m.eps);
+        } else {
+            return rsqrtf(mega_block_sum(ss, s.red) * inv_d + m.eps);  // (a correctly rounded division and square root cost ~200 cycles here)
+        }
+    };
+    const int ln_rows = m.q_dim + 2 * m.kv_dim + m.hidden;  // rows of a layer whose input is normalised
     const bool head_digits = kQuant && p.wt_head != WT_F16;  // an fp16 head on quantised layers reads the fp16 staging
-    // One chunk of a stage: acquire, all products, release, CTA barrier; returns where the sums are.
-    int lg_parts = 0;    // log2 of the column ranges of the chunk whose sums are being read
     // A freed slot makes the producer request the chunk that is n_slots ahead at once: megabytes of reads over all
     // CTAs, which would travel through L2 together with the words of the exchange that follows the stage and delay
     // them by microseconds.  The last chunk of a stage is therefore handed back only after that exchange (the chunk it
@@ -1158,30 +1196,45 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         if (n_pend) mega_release_deferred(a, s, pend_from, n_pend);
         n_pend = 0;
     };
-    auto chunk_products = [&](int rows, int n_kb, const uint8_t* xa, bool defer, bool is_head = false) {
-        const uint8_t* ch = mega_acquire(a, s, c, n_chunk++);
-        FINE();
-        float* partial = s.partial + par * kMegaChunkRows;
+    // The products of up to p.group chunks (`rows` rows, `per` per chunk): every warp goes from chunk to chunk on its own, one
+    // CTA barrier at the end; returns where the sums are.  (A barrier and an epilogue per chunk cost 0.7 us each, five times
+    // per layer on the 22-layer d2048 model.)  The last `keep` chunks of the rows still to come (`left`) are handed back later.
+    auto group_products = [&](int rows, int per, int n_kb, const uint8_t* xa, int left, int keep, bool is_head = false) {
+        float* const base = s.partial + par * p.group * kMegaChunkRows;
         par ^= 1;
-        if (WT != WT_F16 && is_head && p.wt_head == WT_F16) lg_parts = mega_chunk_dots<WT_F16>(ch, rows, n_kb, xa, partial, warp, lane);  // an fp16 head on quantised layers
-        else lg_parts = mega_chunk_dots<WT>(ch, rows, n_kb, xa, partial, warp, lane);
-        FINE();
-        if (defer) {
-            if (n_pend == 0) pend_from = c;
-            n_pend++;
-            c.next((unsigned)p.n_slots);
-        } else {
-            mega_release(a, s, c);
+        float* partial = base;
+#pragma unroll 1
+        for (int r0 = 0; r0 < rows; r0 += per) {
+            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++);
+            FINE();
+            const int n = min(per, rows - r0);
+            if (WT != WT_F16 && is_head && p.wt_head == WT_F16) mega_chunk_dots<WT_F16>(ch, n, n_kb, xa, partial, warp, lane);  // an fp16 head on quantised layers
+            else mega_chunk_dots<WT>(ch, n, n_kb, xa, partial, warp, lane);
+            FINE();
+            partial += kMegaChunkRows;
+            if (left - r0 <= keep * per) {
+                if (n_pend == 0) pend_from = c;
+                n_pend++;
+                c.next((unsigned)p.n_slots);
+            } else {
+                mega_release(a, s, c);
+            }
         }
         consumer_sync();
         FINE();
-        return partial;
+        return base;
+    };
+    // The sum of row r of a group.
+    auto row_sum = [&](const float* base, int rows, int per, int n_kb, int r) {
+        int i = 0;
+        while (r >= per) { r -= per; rows -= per; i++; }  // (at most three times)
+        return mega_take_sum(base + i * kMegaChunkRows, mega_chunk_lg(min(per, rows), n_kb), r);
     };
 
     for (int step = a.first; step < a.first + a.n_steps; step++) {
         if (step > 0) {
             const uint16_t* emb_row = a.tok_emb + (size_t)tok * d;
-            if (tid < half) s.rope[tid] = a.rope[(size_t)pos * half + tid];  // published by the barrier of the first norm
+            if (!GPT2 && tid < half) s.rope[tid] = a.rope[(size_t)pos * half + tid];  // published by the barrier of the first norm
             for (int l = 0; l < L; l++) {
                 const unsigned seq = a.tag0 + (unsigned)((step - 1) * L + l + 1);  // tag of everything this layer publishes
                 float inv = 0.f;
@@ -1193,41 +1246,59 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                     // ---- S1: x of this layer.  x_words is re-written by the W2 stage of this layer, which starts only
                     // after every CTA has published its activation, i.e. after every group CTA has read x here.
                     const float* gain = a.norms + (size_t)(2 * l) * d;
-                    float ss = 0.f;
+                    float ss = 0.f, sm = 0.f;
                     if (l == 0) {
-                        for (int k = tid; k < d; k += kMegaConsumers) stage_x(s.xraw, d, true, k, __half2float(__ushort_as_half(emb_row[k])), __ldg(gain + k), ss);
+                        for (int k = tid; k < d; k += kMegaConsumers) {
+                            float v = __half2float(__ushort_as_half(emb_row[k]));
+                            if (GPT2) v += __half2float(__ushort_as_half(__ldg(a.pos_emb + (size_t)pos * d + k)));
+                            stage_x(s.xraw, d, true, k, v, __ldg(gain + k), ss, sm);
+                        }
                     } else {
-                        mega_read_words(a, s, a.x_words, d, seq - 1, 5, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, true, k, v0, v1, g0, g1, ss); });
+                        mega_read_words(a, s, a.x_words, d, seq - 1, 5, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, true, k, v0, v1, g0, g1, ss, sm); });
                     }
                     FINE();
                     release_pending();  // the W2 chunk of the previous layer
-                    ss = mega_block_sum(ss, s.red);
-                    inv = rsqrtf(ss * inv_d + m.eps);  // (a correctly rounded division and square root cost ~200 cycles here)
+                    inv = norm_scale(ss, sm);
                     FINE();
                     stamp(step);
                     // q/k/v row pairs of this CTA, RoPE, words for the CTAs that share the KV head, KV-cache append.
                     // qkv_words is re-written one layer later, after x_words of this layer is complete, which needs every
                     // CTA's W2 rows, hence the whole activation vector, hence every group CTA past its S2 of this layer.
-                    for (int i0 = 0; i0 < w.s1_n; i0 += p.s1_ipc) {
-                        const int n_items = min(p.s1_ipc, w.s1_n - i0);
-                        // A chunk holds at most 128 row pairs: one per thread.  Where the pair goes (matrix, RoPE entry,
+                    const int s1_step = p.group * p.s1_ipc;
+                    for (int i0 = 0; i0 < w.s1_n; i0 += s1_step) {
+                        const int n_items = min(s1_step, w.s1_n - i0);
+                        // A group holds at most 512 row pairs: one per thread.  Where the pair goes (matrix, RoPE entry,
                         // exchange words, cache rows) does not depend on the products: worked out before them, it is off
                         // the path between the last product and the words the other CTAs are waiting for.
                         int kind = 0, row0 = 0, row1 = 0, idx = 0;
-                        float2 cs = make_float2(1.f, 0.f);
+                        float2 cs = make_float2(1.f, 0.f), n0 = cs, n1 = cs;
                         unsigned long long* dst = my_qkv;
                         __half* kv_row = nullptr;
                         if (tid < n_items) {
                             mega_s1_rows(m, p, w.kvh, w.s1_begin + i0 + tid, kind, row0, row1, idx);
-                            if (kind < 2) cs = s.rope[idx];
+                            if (!GPT2 && kind < 2) cs = s.rope[idx];
+                            if (GPT2) {
+                                const float2* ln = a.ln + (size_t)l * ln_rows + (kind == 0 ? 0 : kind == 1 ? m.q_dim : m.q_dim + m.kv_dim);
+                                n0 = __ldg(ln + row0);
+                                n1 = __ldg(ln + row1);
+                            }
                             dst = my_qkv + 2 * (w.s1_begin + i0 + tid);
                             if (kind > 0) kv_row = (kind == 1 ? a.kv.k : a.kv.v) + a.kv.offset(m, l, 0, w.kvh, pos) - w.kvh * HD;
                         }
-                        float* sums = chunk_products(2 * n_items, d >> 5, s.xa, i0 + p.s1_ipc >= w.s1_n);
+                        const float* sums = group_products(2 * n_items, 2 * p.s1_ipc, d >> 5, s.xa, 2 * (w.s1_n - i0), 1);
                         if (tid < n_items) {
-                            float v0 = mega_take_sum(sums, lg_parts, 2 * tid) * inv;
-                            float v1 = mega_take_sum(sums, lg_parts, 2 * tid + 1) * inv;
-                            const float r0 = v0 * cs.x - v1 * cs.y, r1 = v0 * cs.y + v1 * cs.x;  // (cos, sin) = (1, 0) for a value pair
+                            float v0 = row_sum(sums, 2 * n_items, 2 * p.s1_ipc, d >> 5, 2 * tid);
+                            float v1 = row_sum(sums, 2 * n_items, 2 * p.s1_ipc, d >> 5, 2 * tid + 1);
+                            float r0, r1;
+                            if (GPT2) {
+                                r0 = fmaf(fmaf(-mean, n0.x, v0), inv, n0.y);
+                                r1 = fmaf(fmaf(-mean, n1.x, v1), inv, n1.y);
+                            } else {
+                                v0 *= inv;
+                                v1 *= inv;
+                                r0 = v0 * cs.x - v1 * cs.y;  // (cos, sin) = (1, 0) for a value pair
+                                r1 = v0 * cs.y + v1 * cs.x;
+                            }
                             st_word(dst, tagged(r0, seq));
                             st_word(dst + 1, tagged(r1, seq));
                             if (kind > 0) {
@@ -1269,14 +1340,14 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                     stamp(step);
                     // ---- rows [blk*rpb, ...) of Wo restricted to this head's columns: every row's partial sum is one
                     // contribution to the counted sum of that row (head 0 also carries the residual)
-                    for (int r0 = 0; r0 < p.rpb; r0 += p.s2_rpc) {
-                        const int nr = min(p.s2_rpc, p.rpb - r0);
-                        float* sums = chunk_products(nr, HD >> 5, reinterpret_cast<const uint8_t*>(s.ctx), r0 + p.s2_rpc >= p.rpb);
+                    for (int r0 = 0; r0 < p.rpb; r0 += p.group * p.s2_rpc) {
+                        const int nr = min(p.group * p.s2_rpc, p.rpb - r0);
+                        const float* sums = group_products(nr, p.s2_rpc, HD >> 5, reinterpret_cast<const uint8_t*>(s.ctx), p.rpb - r0, 1);
                         for (int r = tid; r < nr; r += kMegaConsumers) {
                             const int orow = w.blk * p.rpb + r0 + r;
-                            float v = mega_take_sum(sums, lg_parts, r);
+                            float v = row_sum(sums, nr, p.s2_rpc, HD >> 5, r);
                             if (orow < d) {
-                                if (w.head == 0) v += s.xraw[orow];
+                                if (w.head == 0) v += s.xraw[orow] + (GPT2 ? __ldg(a.out_bias + (size_t)2 * l * d + orow) : 0.f);
                                 red_add_u64(a.mid_sums + orow, counted(v));
                             }
                         }
@@ -1293,28 +1364,41 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                     // token exchange does not start with a round trip to memory.
                     if (tid < p.n_cta) { unsigned long long keep; asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(keep) : "l"(a.cand_words + (size_t)tid * kMegaCandStride) : "memory"); }
                     const float* gain = a.norms + (size_t)(2 * l + 1) * d;
-                    float ss = 0.f;
+                    float ss = 0.f, sm = 0.f;
                     FINE();
-                    mega_read_sums(a, s, a.mid_sums, d, m.n_head, 7, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xmid, d, true, k, v0, v1, g0, g1, ss); });
+                    mega_read_sums(a, s, a.mid_sums, d, m.n_head, 7, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xmid, d, true, k, v0, v1, g0, g1, ss, sm); });
                     FINE();
                     release_pending();  // the Wo chunk (CTAs outside the head groups: the W2 chunk of the previous layer)
-                    ss = mega_block_sum(ss, s.red);
-                    inv = rsqrtf(ss * inv_d + m.eps);  // (a correctly rounded division and square root cost ~200 cycles here)
+                    inv = norm_scale(ss, sm);
                 }
                 stamp(step);
                 // (gate, up) row pairs of this CTA's hidden units, SiLU(gate) * up.  act_words is re-written one layer later,
                 // after mid_sums of that layer is complete, which needs every group CTA past x_words of this layer, i.e.
                 // every CTA past its W2 rows and so past this activation vector.
-                for (int j0 = 0; j0 < w.h_n; j0 += p.s3a_ipc) {
-                    const int n_items = min(p.s3a_ipc, w.h_n - j0);
-                    // (one item per thread; its word's address is known before the products)
-                    unsigned long long* const dst = a.act_words + (p.act_wpc ? (size_t)blockIdx.x * p.act_wpc : (size_t)w.h_begin) + j0 + tid;
-                    float* sums = chunk_products(2 * n_items, d >> 5, s.xa, j0 + p.s3a_ipc >= w.h_n);
-                    if (tid < n_items) {
-                        const float g = mega_take_sum(sums, lg_parts, 2 * tid) * inv;
-                        const float u = mega_take_sum(sums, lg_parts, 2 * tid + 1) * inv;
-                        // silu(g) = g * sigmoid(g) = 0.5 g (1 + tanh(g / 2))
-                        st_word(dst, tagged(__fdividef(g, 1.0f + __expf(-g)) * u, seq));
+                constexpr int kFfn = GPT2 ? 1 : 2;  // packed rows per unit
+                for (int j0 = 0; j0 < w.h_n; j0 += p.group * p.s3a_ipc) {
+                    const int n_items = min(p.group * p.s3a_ipc, w.h_n - j0), n_rows = kFfn * n_items, per = kFfn * p.s3a_ipc;
+                    // (the first item of a thread: its word's address and constants are known before the products)
+                    unsigned long long* const dst = a.act_words + (p.act_wpc ? (size_t)blockIdx.x * p.act_wpc : (size_t)w.h_begin) + j0;
+                    const float2* ln = GPT2 ? a.ln + (size_t)l * ln_rows + m.q_dim + 2 * m.kv_dim + w.h_begin + j0 : nullptr;
+                    float2 n0 = make_float2(0.f, 0.f);
+                    if (GPT2 && tid < n_items) n0 = __ldg(ln + tid);
+                    const float* sums = group_products(n_rows, per, d >> 5, s.xa, kFfn * (w.h_n - j0), 1);
+                    for (int j = tid; j < n_items; j += kMegaConsumers) {
+                        float v;
+                        if (GPT2) {
+                            if (j >= kMegaConsumers) n0 = __ldg(ln + j);
+                            const float x = fmaf(fmaf(-mean, n0.x, row_sum(sums, n_rows, per, d >> 5, j)), inv, n0.y);
+                            // gelu(x) = 0.5 x (1 + tanh(u)), tanh(u) = 1 - 2 / (1 + exp(2 u))
+                            const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
+                            v = 0.5f * x * (2.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * u)));
+                        } else {
+                            const float g = row_sum(sums, n_rows, per, d >> 5, 2 * j) * inv;
+                            const float u = row_sum(sums, n_rows, per, d >> 5, 2 * j + 1) * inv;
+                            // silu(g) = g * sigmoid(g) = 0.5 g (1 + tanh(g / 2))
+                            v = __fdividef(g, 1.0f + __expf(-g)) * u;
+                        }
+                        st_word(dst + j, tagged(v, seq));
                     }
                 }
                 stamp(step);
@@ -1337,13 +1421,17 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                 consumer_sync();
                 FINE();
                 stamp(step);
-                for (int r0 = 0; r0 < w.d_n; r0 += p.s3b_rpc) {
-                    const int nr = min(p.s3b_rpc, w.d_n - r0);
-                    // (at most 256 rows per chunk: one per thread; residual and address are fetched before the products)
-                    const float res = tid < nr ? s.xmid[w.d_begin + r0 + tid] : 0.f;
-                    unsigned long long* const dst = a.x_words + w.d_begin + r0 + tid;
-                    float* sums = chunk_products(nr, m.hidden >> 5, s.xa, r0 + p.s3b_rpc >= w.d_n);
-                    if (tid < nr) st_word(dst, tagged(mega_take_sum(sums, lg_parts, tid) + res, seq));
+                for (int r0 = 0; r0 < w.d_n; r0 += p.group * p.s3b_rpc) {
+                    const int nr = min(p.group * p.s3b_rpc, w.d_n - r0);
+                    // (residual and address of a thread's first row are fetched before the products)
+                    float res = 0.f;
+                    if (tid < nr) res = s.xmid[w.d_begin + r0 + tid] + (GPT2 ? __ldg(a.out_bias + (size_t)(2 * l + 1) * d + w.d_begin + r0 + tid) : 0.f);
+                    unsigned long long* const dst = a.x_words + w.d_begin + r0;
+                    const float* sums = group_products(nr, p.s3b_rpc, m.hidden >> 5, s.xa, w.d_n - r0, 1);
+                    for (int r = tid; r < nr; r += kMegaConsumers) {
+                        if (r >= kMegaConsumers) res = s.xmid[w.d_begin + r0 + r] + (GPT2 ? __ldg(a.out_bias + (size_t)(2 * l + 1) * d + w.d_begin + r0 + r) : 0.f);
+                        st_word(dst + r, tagged(row_sum(sums, nr, p.s3b_rpc, m.hidden >> 5, r) + res, seq));
+                    }
                 }
                 stamp(step);
             }
@@ -1358,27 +1446,36 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         // them before this thread) is made visible before the candidate words that thread 0 publishes at the end of the
         // head.  Issued here, the fence overlaps the wait for the last layer's output.
         if (tid == 0) __threadfence();
+        float head_inv = 1.f;
         {
-            float ss = 0.f;
+            float ss = 0.f, sm = 0.f;
             if (step == 0) {
-                for (int k = tid; k < d; k += kMegaConsumers) stage_x(s.xraw, d, head_digits, k, __ldcg(a.hidden_io + k), __ldg(fin_gain + k), ss);
+                for (int k = tid; k < d; k += kMegaConsumers) stage_x(s.xraw, d, head_digits, k, __ldcg(a.hidden_io + k), __ldg(fin_gain + k), ss, sm);
             } else {
-                mega_read_words(a, s, a.x_words, d, a.tag0 + (unsigned)(step * L), 9, fin_gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, head_digits, k, v0, v1, g0, g1, ss); });
+                mega_read_words(a, s, a.x_words, d, a.tag0 + (unsigned)(step * L), 9, fin_gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, head_digits, k, v0, v1, g0, g1, ss, sm); });
             }
             release_pending();  // the W2 chunk of the last layer
-            consumer_sync();  // the RMSNorm scale is positive: the arg-max does not need it
+            if (GPT2) head_inv = norm_scale(ss, sm);
+            else consumer_sync();  // the RMSNorm scale is positive: the arg-max does not need it
         }
         stamp(step);
         float best_v = -INFINITY;
         int best_i = 0x7fffffff;
-        for (int r0 = 0; r0 < w.v_n; r0 += p.head_rpc) {
-            const int nrows = min(p.head_rpc, w.v_n - r0);
+        const float2* head_ln = GPT2 ? a.ln + (size_t)L * ln_rows + w.v_begin : nullptr;
+        for (int r0 = 0; r0 < w.v_n; r0 += p.group * p.head_rpc) {
+            const int nrows = min(p.group * p.head_rpc, w.v_n - r0);
             FINE();
-            float* sums = chunk_products(nrows, d >> 5, s.xa, r0 + 2 * p.head_rpc >= w.v_n, true);
-            // thread r keeps the best of rows r0 + r over the chunks (ascending rows: '>' keeps the first maximum)
-            if (tid < nrows) {
-                const float v = mega_take_sum(sums, lg_parts, tid);
-                if (v > best_v) { best_v = v; best_i = w.v_begin + r0 + tid; }
+            float2 n0 = make_float2(0.f, 0.f);
+            if (GPT2 && tid < nrows) n0 = __ldg(head_ln + r0 + tid);
+            const float* sums = group_products(nrows, p.head_rpc, d >> 5, s.xa, w.v_n - r0, 2, true);
+            // a thread keeps the best of its rows (ascending: '>' keeps the first maximum)
+            for (int r = tid; r < nrows; r += kMegaConsumers) {
+                float v = row_sum(sums, nrows, p.head_rpc, d >> 5, r);
+                if (GPT2) {
+                    if (r >= kMegaConsumers) n0 = __ldg(head_ln + r0 + r);
+                    v = fmaf(fmaf(-mean, n0.x, v), head_inv, n0.y);
+                }
+                if (v > best_v) { best_v = v; best_i = w.v_begin + r0 + r; }
             }
         }
 #ifdef MEGA_FINE_TRACE
@@ -1434,8 +1531,9 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
 #ifdef MEGA_FINE_TRACE
         if (a.trace && tid == 0 && step == a.n_steps - 1) { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); a.trace[800 + blockIdx.x] = (long long)t; }
 #endif
-        emitted = step - a.first + 1;
-        if (blockIdx.x == 0 && tid == 0) {
+        const bool gpt2_stop = GPT2 && tok == GPT2_EOS;  // GPT-2 rule: the stop token ends the loop without being emitted
+        if (!gpt2_stop) emitted++;
+        if (blockIdx.x == 0 && tid == 0 && !gpt2_stop) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             if (emitted == 1) a.stamps[1] = t;
@@ -1443,7 +1541,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
             if (a.token_times) a.token_times[emitted - 1] = t;
         }
         // Llama rule: the end-of-sequence token is emitted, then the loop stops (every CTA sees the same token)
-        const bool eos = m.eos_token >= 0 && tok == (uint32_t)m.eos_token;
+        const bool eos = GPT2 ? gpt2_stop : m.eos_token >= 0 && tok == (uint32_t)m.eos_token;
         if (eos || s.red[63] != 0.f) {
             if (tid == 0) *reinterpret_cast<volatile int*>(s.stop) = 1;
             break;
@@ -1458,6 +1556,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
             a.rs.next[0] = tok;
             a.rs.n_out[0] = emitted;
             a.stamps[2] = (unsigned long long)emitted | ((unsigned long long)tok << 32);
+            a.stamps[3] = (unsigned long long)pos;
         }
     }
     // The counted sums go back to zero for the next launch: the token exchange above proves that every contribution has
@@ -1581,9 +1680,9 @@ __global__ void k_build_pack(PackSources src, MegaPlan p, ModelDims m, uint8_t* 
         base += p.s2_bytes;
         // S3: (gate_j, up_j) row pairs
         for (int j0 = 0; j0 < w.h_n; j0 += p.s3a_ipc) {
-            const int n = min(p.s3a_ipc, w.h_n - j0);
-            pack_tiled(wt, base + (size_t)j0 * 2 * p.row_bytes, 2 * n, d, [&](int r) {
-                return pack_row(wt, (r & 1) ? src.w3[l] : src.w1[l], d, (size_t)(w.h_begin + j0 + (r >> 1)), 0);
+            const int n = min(p.s3a_ipc, w.h_n - j0), fr = p.ffn_rows;
+            pack_tiled(wt, base + (size_t)j0 * fr * p.row_bytes, fr * n, d, [&](int r) {
+                return pack_row(wt, fr == 2 && (r & 1) ? src.w3[l] : src.w1[l], d, (size_t)(w.h_begin + j0 + (fr == 2 ? r >> 1 : r)), 0);
             });
         }
         base += p.s3a_bytes;
@@ -1598,6 +1697,21 @@ __global__ void k_build_pack(PackSources src, MegaPlan p, ModelDims m, uint8_t* 
         const int n = min(p.head_rpc, w.v_n - r0);
         pack_tiled(p.wt_head, hb + (size_t)r0 * p.head_row_bytes, n, d, [&](int r) { return pack_row(p.wt_head, src.lm_head, d, (size_t)(w.v_begin + r0 + r), 0); });
     }
+}
+
+// GPT-2: {W.g, W.b + bias} of every row of a matrix [rows][K] (see MegaArgs::ln).  One warp per row.
+__global__ void k_fold_norm(const uint16_t* w, int rows, int K, const float* g, const float* b, const float* bias, float2* out) {
+    const int r = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (r >= rows) return;
+    float sg = 0.f, sb = 0.f;
+    for (int k = lane; k < K; k += 32) {
+        const float v = __half2float(__ushort_as_half(w[(size_t)r * K + k]));
+        sg = fmaf(v, g[k], sg);
+        sb = fmaf(v, b[k], sb);
+    }
+    sg = warp_sum(sg);
+    sb = warp_sum(sb);
+    if (lane == 0) out[r] = make_float2(sg, sb + (bias ? bias[r] : 0.f));
 }
 
 }  // namespace esp
