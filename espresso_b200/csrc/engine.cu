@@ -2224,10 +2224,28 @@ int32_t Engine::build_mega() {
     p.head_rpc = std::max(1, std::min(std::min(p.vpc_max, kMegaChunkRows), p.slot_bytes / p.head_row_bytes));
     p.s2_rpc = std::max(1, std::min(std::min(p.rpb, kMegaChunkRows), p.slot_bytes / p.wo_row_bytes));
     p.s2_rpc = std::max(wo_rows, p.s2_rpc / wo_rows * wo_rows);
+    p.s3b_kpc = 0;
+    if (wt_layer != ESP_CUDA_F16) {
+        // The products of a chunk are spread over the warps as 16-row tiles times a power of two of column ranges: where a stage
+        // takes several chunks, a chunk is 16, 32, 64, ... rows (22 of 32 rows busy, or 12 of 16 warps, cost 20 to 30 %).
+        auto whole_tiles = [](int rows, int all) {
+            if (rows >= all || rows < 16) return rows;
+            int r = 16;
+            while (2 * r <= rows) r *= 2;
+            return r;
+        };
+        p.s3a_ipc = std::max(1, whole_tiles(2 * p.s3a_ipc, 2 * p.hpc_max) / 2);
+        p.head_rpc = whole_tiles(p.head_rpc, p.vpc_max);
+        const int n_kb = m_.hidden / 32;
+        if (p.dpc_max > kMegaChunkRows) return ESP_CUDA_OK;
+        const int fit = p.slot_bytes / (p.dpc_max * mega_row_bytes(wt_layer, 32)) / 8 * 8, chunks = fit ? (n_kb + fit - 1) / fit : 0;
+        if (!chunks) return ESP_CUDA_OK;
+        p.s3b_kpc = std::min(fit, ((n_kb + chunks - 1) / chunks + 7) / 8 * 8);  // equal shares, in steps of 8 blocks (16-byte chunks)
+    }
     // As many ring slots as fit; then the largest group of chunks per CTA barrier whose partial sums do not cost a slot.
     p.n_slots = 0;
     for (int ns = 8; ns >= 2 && p.n_slots == 0; ns--)
-        for (int group : {4, 2, 1}) {
+        for (int group : {wt_layer == ESP_CUDA_F16 ? 1 : 4, wt_layer == ESP_CUDA_F16 ? 1 : 2, 1}) {
             MegaPlan probe = p;
             probe.n_slots = ns;
             probe.group = group;

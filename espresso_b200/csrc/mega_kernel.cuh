@@ -85,7 +85,8 @@ struct MegaPlan {
     int s1_ipc;       // S1 row pairs per chunk
     int s2_rpc;       // S2 projection rows per chunk (a multiple of the rows one pass of the CTA covers)
     int s3a_ipc;      // S3 (gate, up) pairs per chunk
-    int s3b_rpc;      // S3 down-projection rows per chunk
+    int s3b_rpc;      // S3 down-projection rows per chunk (fp16)
+    int s3b_kpc;      // quantised types: blocks of 32 columns per chunk, all of the CTA's rows (a multiple of 8)
     int head_rpc;     // LM-head rows per chunk
     int slot_bytes, n_slots;
     long long layer_bytes, head_bytes, cta_bytes;  // packed bytes per CTA: one layer, the head, everything
@@ -708,14 +709,13 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, ui
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 // Q8_0 chunk: [block][row][piece t: the int8 of columns 4t..4t+3 and 16+4t..16+4t+3], then the scales [block][row] fp16.
-__device__ __forceinline__ float2 mega_tile_dot_q8(const uint8_t* chunk, int R, int n_kb, int tile, int kb0, int kb1, const uint8_t* xq, int lane) {
+__device__ __forceinline__ float2 mega_tile_dot_q8(const uint8_t* chunk, int R, int n_kb, int tile, int kb0, int kb1, const uint8_t* xq, const float* qs, int lane) {
     const int g = lane >> 2, t = lane & 3;
     const int row = tile * 16 + g;
     const uint8_t* wp = chunk + ((size_t)row * 32 + t * 8);
     const size_t kstride = (size_t)R * 32;
     const __half* sp = reinterpret_cast<const __half*>(chunk + (size_t)R * n_kb * 32) + row;
     const uint8_t* xp = xq + (g < 3 ? g * 32 + t * 8 : 0);
-    const float* qs = reinterpret_cast<const float*>(xq + (size_t)n_kb * 128);
     // what this lane's two result columns mean: t = 0 holds digits 0 and 1, t = 1 digit 2, the others nothing
     const float k0 = t == 0 ? 1.0f : t == 1 ? (1.0f / 16384.0f) : 0.f, k1 = t == 0 ? (1.0f / 128.0f) : 0.f;
     float a0 = 0.f, a8 = 0.f;
@@ -780,8 +780,8 @@ __device__ __forceinline__ float2 mega_tile_dot_q4(const uint8_t* chunk, int R, 
 }
 
 template <int WT, int NP>
-__device__ __forceinline__ float2 mega_tile_dot(const uint8_t* chunk, int R, int n_kb, int tile, int kb0, int kb1, const uint8_t* xa, int lane) {
-    if constexpr (WT == WT_Q8_0) return mega_tile_dot_q8(chunk, R, n_kb, tile, kb0, kb1, xa, lane);
+__device__ __forceinline__ float2 mega_tile_dot(const uint8_t* chunk, int R, int n_kb, int tile, int kb0, int kb1, const uint8_t* xa, const float* qs, int lane) {
+    if constexpr (WT == WT_Q8_0) return mega_tile_dot_q8(chunk, R, n_kb, tile, kb0, kb1, xa, qs, lane);
     else if constexpr (WT == WT_Q4_0) return mega_tile_dot_q4<NP>(chunk, R, n_kb, tile, kb0, kb1, xa, lane);
     else return mega_tile_dot_f16<NP>(chunk, R, n_kb, tile, kb0, kb1, xa, lane);
 }
@@ -798,12 +798,13 @@ __device__ __forceinline__ int mega_chunk_lg(int R, int n_kb) {
     return max(0, min(4 - lg_t, 31 - __clz(n_kb)));
 }
 template <int WT, int NP = 1>
-__device__ __forceinline__ int mega_chunk_dots(const uint8_t* chunk, int R, int n_kb, const uint8_t* xa, float* partial, int warp, int lane) {
+__device__ __forceinline__ int mega_chunk_dots(const uint8_t* chunk, int R, int n_kb, const uint8_t* xa, float* partial, int warp, int lane, const float* qs = nullptr) {
+    if (WT == WT_Q8_0 && !qs) qs = reinterpret_cast<const float*>(xa + (size_t)n_kb * 128);  // block scales behind the staged vector
     const int n_tiles = (R + 15) >> 4, lg = mega_chunk_lg(R, n_kb);
     const int per = (n_kb + (1 << lg) - 1) >> lg;
     for (int u = warp; u < (n_tiles << lg); u += kMegaConsumerWarps) {
         const int tile = u >> lg, part = u & ((1 << lg) - 1);
-        const float2 y = mega_tile_dot<WT, NP>(chunk, R, n_kb, tile, part * per, min(n_kb, (part + 1) * per), xa, lane);
+        const float2 y = mega_tile_dot<WT, NP>(chunk, R, n_kb, tile, part * per, min(n_kb, (part + 1) * per), xa, qs, lane);
         if ((lane & 3) < NP) {
             float* dst = partial + (NP > 1 ? (lane & 3) * kMegaChunkRows : 0) + u * 16 + (lane >> 2);
             dst[0] = y.x;
@@ -1085,7 +1086,16 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                         if (w.in_group) issue_stage(off, p.rpb, p.s2_rpc, p.wo_row_bytes);
                         off += p.s2_bytes;
                         issue_stage(off, w.h_n, p.s3a_ipc, (GPT2 ? 1 : 2) * p.row_bytes); off += p.s3a_bytes;
-                        issue_stage(off, w.d_n, p.s3b_rpc, p.down_row_bytes);
+                        if (WT == WT_F16) {
+                            issue_stage(off, w.d_n, p.s3b_rpc, p.down_row_bytes);
+                        } else {
+                            const int n_kb = m.hidden >> 5;
+                            for (int k = 0; k < n_kb; k += p.s3b_kpc) {
+                                const int bytes = w.d_n * mega_row_bytes(WT, 32 * min(p.s3b_kpc, n_kb - k));
+                                issue(off, bytes);
+                                off += bytes;
+                            }
+                        }
                     }
                 }
                 issue_stage(head_off, w.v_n, p.head_rpc, p.head_row_bytes);
@@ -1105,7 +1115,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         // ---------------- watcher: follows the chunks in order and counts the ones whose bytes have arrived ----------------
         if (lane == 0) {
             auto chunks_of = [](int items, int per_chunk) { return (items + per_chunk - 1) / per_chunk; };
-            const unsigned per_layer = (w.in_group ? chunks_of(w.s1_n, p.s1_ipc) + chunks_of(p.rpb, p.s2_rpc) : 0) + chunks_of(w.h_n, p.s3a_ipc) + chunks_of(w.d_n, p.s3b_rpc);
+            const unsigned per_layer = (w.in_group ? chunks_of(w.s1_n, p.s1_ipc) + chunks_of(p.rpb, p.s2_rpc) : 0) + chunks_of(w.h_n, p.s3a_ipc) +
+                                       (WT == WT_F16 ? chunks_of(w.d_n, p.s3b_rpc) : chunks_of(m.hidden >> 5, p.s3b_kpc));
             const unsigned total = (unsigned)a.n_steps * chunks_of(w.v_n, p.head_rpc) + (unsigned)(a.n_steps - 1 + a.first) * L * per_layer;
             MegaCursor k;
             for (unsigned i = 0; i < total; i++) {
@@ -1196,29 +1207,42 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         if (n_pend) mega_release_deferred(a, s, pend_from, n_pend);
         n_pend = 0;
     };
-    // The products of up to p.group chunks (`rows` rows, `per` per chunk): every warp goes from chunk to chunk on its own, one
-    // CTA barrier at the end; returns where the sums are.  (A barrier and an epilogue per chunk cost 0.7 us each, five times
-    // per layer on the 22-layer d2048 model.)  The last `keep` chunks of the rows still to come (`left`) are handed back later.
+    // Quantised models: a stage's slice is several chunks, and a barrier plus an epilogue per chunk cost 0.7 us each.  The
+    // products of up to p.group chunks (`rows` rows, `per` per chunk) share one CTA barrier; a warp goes from chunk to chunk on
+    // its own.  fp16 models: one chunk at a time (their stages are one chunk, and the short way is 4 us per token faster).
+    // The last `keep` chunks of the rows still to come (`left`) are handed back later.  Returns where the sums are.
+    constexpr bool kGrouped = WT != WT_F16;
+    const int group = kGrouped ? p.group : 1;
+    int lg_parts = 0;    // fp16: log2 of the column ranges of the chunk whose sums are being read
+    auto hand_back = [&](bool later) {
+        if (later) {
+            if (n_pend == 0) pend_from = c;
+            n_pend++;
+            c.next((unsigned)p.n_slots);
+        } else {
+            mega_release(a, s, c);
+        }
+    };
     auto group_products = [&](int rows, int per, int n_kb, const uint8_t* xa, int left, int keep, bool is_head = false) {
-        float* const base = s.partial + par * p.group * kMegaChunkRows;
+        float* const base = s.partial + par * group * kMegaChunkRows;
         par ^= 1;
-        float* partial = base;
+        if constexpr (kGrouped) {
+            float* partial = base;
 #pragma unroll 1
-        for (int r0 = 0; r0 < rows; r0 += per) {
+            for (int r0 = 0; r0 < rows; r0 += per) {
+                const uint8_t* ch = mega_acquire(a, s, c, n_chunk++);
+                const int n = min(per, rows - r0);
+                if (is_head && p.wt_head == WT_F16) mega_chunk_dots<WT_F16>(ch, n, n_kb, xa, partial, warp, lane);  // an fp16 head on quantised layers
+                else mega_chunk_dots<WT>(ch, n, n_kb, xa, partial, warp, lane);
+                partial += kMegaChunkRows;
+                hand_back(left - r0 <= keep * per);
+            }
+        } else {
             const uint8_t* ch = mega_acquire(a, s, c, n_chunk++);
             FINE();
-            const int n = min(per, rows - r0);
-            if (WT != WT_F16 && is_head && p.wt_head == WT_F16) mega_chunk_dots<WT_F16>(ch, n, n_kb, xa, partial, warp, lane);  // an fp16 head on quantised layers
-            else mega_chunk_dots<WT>(ch, n, n_kb, xa, partial, warp, lane);
+            lg_parts = mega_chunk_dots<WT>(ch, rows, n_kb, xa, base, warp, lane);
             FINE();
-            partial += kMegaChunkRows;
-            if (left - r0 <= keep * per) {
-                if (n_pend == 0) pend_from = c;
-                n_pend++;
-                c.next((unsigned)p.n_slots);
-            } else {
-                mega_release(a, s, c);
-            }
+            hand_back(left <= keep * per);
         }
         consumer_sync();
         FINE();
@@ -1226,9 +1250,18 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
     };
     // The sum of row r of a group.
     auto row_sum = [&](const float* base, int rows, int per, int n_kb, int r) {
+        if constexpr (!kGrouped) return mega_take_sum(base, lg_parts, r);
         int i = 0;
         while (r >= per) { r -= per; rows -= per; i++; }  // (at most three times)
         return mega_take_sum(base + i * kMegaChunkRows, mega_chunk_lg(min(per, rows), n_kb), r);
+    };
+    // f(i) for every i < n this thread owns (an fp16 chunk has at most 256 rows: at most one per thread)
+    auto each = [&](int n, auto f) {
+        if constexpr (kGrouped) {
+            for (int i = tid; i < n; i += kMegaConsumers) f(i);
+        } else {
+            if (tid < n) f(tid);
+        }
     };
 
     for (int step = a.first; step < a.first + a.n_steps; step++) {
@@ -1264,7 +1297,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                     // q/k/v row pairs of this CTA, RoPE, words for the CTAs that share the KV head, KV-cache append.
                     // qkv_words is re-written one layer later, after x_words of this layer is complete, which needs every
                     // CTA's W2 rows, hence the whole activation vector, hence every group CTA past its S2 of this layer.
-                    const int s1_step = p.group * p.s1_ipc;
+                    const int s1_step = group * p.s1_ipc;
                     for (int i0 = 0; i0 < w.s1_n; i0 += s1_step) {
                         const int n_items = min(s1_step, w.s1_n - i0);
                         // A group holds at most 512 row pairs: one per thread.  Where the pair goes (matrix, RoPE entry,
@@ -1340,17 +1373,17 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                     stamp(step);
                     // ---- rows [blk*rpb, ...) of Wo restricted to this head's columns: every row's partial sum is one
                     // contribution to the counted sum of that row (head 0 also carries the residual)
-                    for (int r0 = 0; r0 < p.rpb; r0 += p.group * p.s2_rpc) {
-                        const int nr = min(p.group * p.s2_rpc, p.rpb - r0);
+                    for (int r0 = 0; r0 < p.rpb; r0 += group * p.s2_rpc) {
+                        const int nr = min(group * p.s2_rpc, p.rpb - r0);
                         const float* sums = group_products(nr, p.s2_rpc, HD >> 5, reinterpret_cast<const uint8_t*>(s.ctx), p.rpb - r0, 1);
-                        for (int r = tid; r < nr; r += kMegaConsumers) {
+                        each(nr, [&](int r) {
                             const int orow = w.blk * p.rpb + r0 + r;
                             float v = row_sum(sums, nr, p.s2_rpc, HD >> 5, r);
                             if (orow < d) {
                                 if (w.head == 0) v += s.xraw[orow] + (GPT2 ? __ldg(a.out_bias + (size_t)2 * l * d + orow) : 0.f);
                                 red_add_u64(a.mid_sums + orow, counted(v));
                             }
-                        }
+                        });
                     }
                     stamp(step);
                 } else {
@@ -1376,15 +1409,15 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                 // after mid_sums of that layer is complete, which needs every group CTA past x_words of this layer, i.e.
                 // every CTA past its W2 rows and so past this activation vector.
                 constexpr int kFfn = GPT2 ? 1 : 2;  // packed rows per unit
-                for (int j0 = 0; j0 < w.h_n; j0 += p.group * p.s3a_ipc) {
-                    const int n_items = min(p.group * p.s3a_ipc, w.h_n - j0), n_rows = kFfn * n_items, per = kFfn * p.s3a_ipc;
+                for (int j0 = 0; j0 < w.h_n; j0 += group * p.s3a_ipc) {
+                    const int n_items = min(group * p.s3a_ipc, w.h_n - j0), n_rows = kFfn * n_items, per = kFfn * p.s3a_ipc;
                     // (the first item of a thread: its word's address and constants are known before the products)
                     unsigned long long* const dst = a.act_words + (p.act_wpc ? (size_t)blockIdx.x * p.act_wpc : (size_t)w.h_begin) + j0;
                     const float2* ln = GPT2 ? a.ln + (size_t)l * ln_rows + m.q_dim + 2 * m.kv_dim + w.h_begin + j0 : nullptr;
                     float2 n0 = make_float2(0.f, 0.f);
                     if (GPT2 && tid < n_items) n0 = __ldg(ln + tid);
                     const float* sums = group_products(n_rows, per, d >> 5, s.xa, kFfn * (w.h_n - j0), 1);
-                    for (int j = tid; j < n_items; j += kMegaConsumers) {
+                    each(n_items, [&](int j) {
                         float v;
                         if (GPT2) {
                             if (j >= kMegaConsumers) n0 = __ldg(ln + j);
@@ -1399,7 +1432,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                             v = __fdividef(g, 1.0f + __expf(-g)) * u;
                         }
                         st_word(dst + j, tagged(v, seq));
-                    }
+                    });
                 }
                 stamp(step);
                 // ---- the whole activation vector, then this CTA's rows of W2 (+ residual) = the next layer's x
@@ -1421,16 +1454,43 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                 consumer_sync();
                 FINE();
                 stamp(step);
-                for (int r0 = 0; r0 < w.d_n; r0 += p.group * p.s3b_rpc) {
-                    const int nr = min(p.group * p.s3b_rpc, w.d_n - r0);
-                    // (residual and address of a thread's first row are fetched before the products)
-                    float res = 0.f;
-                    if (tid < nr) res = s.xmid[w.d_begin + r0 + tid] + (GPT2 ? __ldg(a.out_bias + (size_t)(2 * l + 1) * d + w.d_begin + r0 + tid) : 0.f);
-                    unsigned long long* const dst = a.x_words + w.d_begin + r0;
-                    const float* sums = group_products(nr, p.s3b_rpc, m.hidden >> 5, s.xa, w.d_n - r0, 1);
-                    for (int r = tid; r < nr; r += kMegaConsumers) {
-                        if (r >= kMegaConsumers) res = s.xmid[w.d_begin + r0 + r] + (GPT2 ? __ldg(a.out_bias + (size_t)(2 * l + 1) * d + w.d_begin + r0 + r) : 0.f);
-                        st_word(dst + r, tagged(row_sum(sums, nr, p.s3b_rpc, m.hidden >> 5, r) + res, seq));
+                if constexpr (kGrouped) {
+                    // all rows of the CTA (at most 256), the chunks cut along the columns: a 16-row tile of the products is
+                    // then nearly full, and two chunks of eight rows would each cost as much as one of sixteen
+                    const int n_kb = m.hidden >> 5;
+                    float sum = tid < w.d_n ? s.xmid[w.d_begin + tid] : 0.f;
+                    const float* const qs = reinterpret_cast<const float*>(s.xa + xa_bytes(m.hidden));
+                    for (int k0 = 0; k0 < n_kb; k0 += group * p.s3b_kpc) {
+                        float* const base = s.partial + par * group * kMegaChunkRows;
+                        par ^= 1;
+                        const int k1 = min(n_kb, k0 + group * p.s3b_kpc);
+                        float* partial = base;
+#pragma unroll 1
+                        for (int k = k0; k < k1; k += p.s3b_kpc) {
+                            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++);
+                            mega_chunk_dots<WT>(ch, w.d_n, min(p.s3b_kpc, k1 - k), s.xa + (size_t)k * 128, partial, warp, lane, qs + k);
+                            partial += kMegaChunkRows;
+                            hand_back(k + p.s3b_kpc >= n_kb);
+                        }
+                        consumer_sync();
+                        if (tid < w.d_n) {
+                            partial = base;
+                            for (int k = k0; k < k1; k += p.s3b_kpc) {
+                                sum += mega_take_sum(partial, mega_chunk_lg(w.d_n, min(p.s3b_kpc, k1 - k)), tid);
+                                partial += kMegaChunkRows;
+                            }
+                        }
+                    }
+                    if (tid < w.d_n) st_word(a.x_words + w.d_begin + tid, tagged(sum, seq));
+                } else {
+                    for (int r0 = 0; r0 < w.d_n; r0 += p.s3b_rpc) {
+                        const int nr = min(p.s3b_rpc, w.d_n - r0);
+                        // (residual and address are fetched before the products)
+                        float res = 0.f;
+                        if (tid < nr) res = s.xmid[w.d_begin + r0 + tid] + (GPT2 ? __ldg(a.out_bias + (size_t)(2 * l + 1) * d + w.d_begin + r0 + tid) : 0.f);
+                        unsigned long long* const dst = a.x_words + w.d_begin + r0 + tid;
+                        const float* sums = group_products(nr, p.s3b_rpc, m.hidden >> 5, s.xa, w.d_n - r0, 1);
+                        if (tid < nr) st_word(dst, tagged(row_sum(sums, nr, p.s3b_rpc, m.hidden >> 5, tid) + res, seq));
                     }
                 }
                 stamp(step);
@@ -1462,21 +1522,21 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         float best_v = -INFINITY;
         int best_i = 0x7fffffff;
         const float2* head_ln = GPT2 ? a.ln + (size_t)L * ln_rows + w.v_begin : nullptr;
-        for (int r0 = 0; r0 < w.v_n; r0 += p.group * p.head_rpc) {
-            const int nrows = min(p.group * p.head_rpc, w.v_n - r0);
+        for (int r0 = 0; r0 < w.v_n; r0 += group * p.head_rpc) {
+            const int nrows = min(group * p.head_rpc, w.v_n - r0);
             FINE();
             float2 n0 = make_float2(0.f, 0.f);
             if (GPT2 && tid < nrows) n0 = __ldg(head_ln + r0 + tid);
             const float* sums = group_products(nrows, p.head_rpc, d >> 5, s.xa, w.v_n - r0, 2, true);
             // a thread keeps the best of its rows (ascending: '>' keeps the first maximum)
-            for (int r = tid; r < nrows; r += kMegaConsumers) {
+            each(nrows, [&](int r) {
                 float v = row_sum(sums, nrows, p.head_rpc, d >> 5, r);
                 if (GPT2) {
                     if (r >= kMegaConsumers) n0 = __ldg(head_ln + r0 + r);
                     v = fmaf(fmaf(-mean, n0.x, v), head_inv, n0.y);
                 }
                 if (v > best_v) { best_v = v; best_i = w.v_begin + r0 + r; }
-            }
+            });
         }
 #ifdef MEGA_FINE_TRACE
         if (a.trace && tid == 0 && step == a.n_steps - 1) { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); a.trace[600 + blockIdx.x] = (long long)t; }
@@ -1687,6 +1747,15 @@ __global__ void k_build_pack(PackSources src, MegaPlan p, ModelDims m, uint8_t* 
         }
         base += p.s3a_bytes;
         // S3: this CTA's rows of W2
+        if (wt != WT_F16) {
+            size_t at = 0;
+            for (int k = 0; k < m.hidden >> 5; k += p.s3b_kpc) {
+                const int cols = 32 * min(p.s3b_kpc, (m.hidden >> 5) - k);
+                pack_tiled(wt, base + at, w.d_n, cols, [&](int r) { return pack_row(wt, src.w2[l], m.hidden, (size_t)(w.d_begin + r), 32 * k); });
+                at += (size_t)w.d_n * mega_row_bytes(wt, cols);
+            }
+            continue;
+        }
         for (int r0 = 0; r0 < w.d_n; r0 += p.s3b_rpc) {
             const int n = min(p.s3b_rpc, w.d_n - r0);
             pack_tiled(wt, base + (size_t)r0 * p.down_row_bytes, n, m.hidden, [&](int r) { return pack_row(wt, src.w2[l], m.hidden, (size_t)(w.d_begin + r0 + r), 0); });
