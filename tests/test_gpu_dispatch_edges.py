@@ -1,0 +1,118 @@
+"""GPU parity at the edges of the kernels' tiles and of the rules that choose between them.
+
+Every case compares with the CPU oracle on the same seeded weights (or with an fp64 product), at the sizes where a
+kernel hands over to another one or a tile, a slice or a chunk is only partly filled.
+"""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from helpers import BF16_ABS_TOL, assert_logits_close, compare_greedy_stream, dense_pair, quantised_pair, to_bf16_bits, upload_all
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rt():
+    from espresso_b200 import runtime
+
+    runtime.load_library()
+    return runtime
+
+
+def _model(name, n_layer, n_head, n_kv, d, head_dim, hidden, vocab, max_seq):
+    from espresso_b200.model_config import MultiModelConfig
+
+    return MultiModelConfig(name, n_layer, n_head, n_kv, d, head_dim, hidden, vocab, max_seq, 1e-5, 10000.0, None, "llama")
+
+
+@pytest.mark.parametrize("kind", ["f16", "bf16"])
+@pytest.mark.parametrize("shape", [(128, 64, 1), (129, 128, 8), (127, 2048, 9), (300, 4096, 16), (640, 1024, 17), (2049, 768, 64), (1000, 704, 65), (257, 2048, 255)])
+def test_streamed_product(rt, kind, shape):
+    """Rows around the tile widths, ragged output columns, one K block up to many K slices."""
+    M, K, N = shape
+    rng = np.random.default_rng(M + K + N)
+    w = (rng.standard_normal((M, K)) * 0.05).astype(np.float32)
+    x = rng.standard_normal((N, K)).astype(np.float32)
+    if kind == "f16":
+        stored, wr, xr = w.astype(np.float16), w.astype(np.float16).astype(np.float64), x.astype(np.float16).astype(np.float64)
+    else:
+        stored = to_bf16_bits(w)
+        wr, xr = ((b.astype(np.uint32) << np.uint32(16)).view(np.float32).astype(np.float64) for b in (stored, to_bf16_bits(x)))
+    y, _ = rt.gemm_tc_bench(kind, stored, M, K, x, warmup=1, iterations=1)
+    np.testing.assert_allclose(y, xr @ wr.T, atol=2e-4, rtol=2e-4)
+
+
+@pytest.mark.parametrize("kind", ["f16", "bf16"])
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 65, 320, 321, 512, 515])
+def test_prompt_rows(rt, oracle_lib, kind, rows):
+    """A prompt of 320 rows is the last one of the streamed products at this width, 321 the first of the paired tiles (256 rows
+    each); hidden 1056 leaves a partial column tile in every product."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-rows", 2, 6, 2, 384, 64, 1056, 520, 640)
+    eng, model = dense_pair(rt, oracle_lib, cfg, kind)
+    prompt = synthetic_prompt(cfg.vocab, rows)
+    eng.prefill(prompt)
+    ora = oracle_lib.Runtime(model)
+    assert ora.prefill(prompt) == 0
+    tol = {} if kind == "f16" else {"abs_tol": BF16_ABS_TOL}
+    assert_logits_close(eng.logits(), ora.logits(), f"{kind} {rows} rows", **tol)
+    tok = eng.select_greedy_token()
+    eng.decode_step(tok)
+    assert ora.advance(tok) == 0
+    assert_logits_close(eng.logits(), ora.logits(), f"{kind} {rows} rows, one step on", **tol)
+    eng.close()
+
+
+@pytest.mark.parametrize("n_head,n_kv,head_dim", [(16, 1, 32), (12, 12, 64), (20, 2, 64), (4, 2, 128), (9, 1, 128)])
+@pytest.mark.parametrize("length", [14, 126])
+def test_decode_attention_edges(rt, oracle_lib, n_head, n_kv, head_dim, length):
+    """Three sequences, contexts that pass a multiple of 16 and of 128 positions; 1 to 16 query heads per KV head."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-attn", 1, n_head, n_kv, n_head * head_dim, head_dim, 512, 320, 160)
+    eng, model = dense_pair(rt, oracle_lib, cfg, "f16", 3)
+    prompts = np.stack([synthetic_prompt(cfg.vocab, length, stream=s) for s in range(3)])
+    streams, _ = eng.generate_batch(prompts, 5)
+    for s in range(3):
+        compare_greedy_stream(oracle_lib.Runtime(model), prompts[s], streams[s])
+    eng.close()
+
+
+@pytest.mark.parametrize("n_head,head_dim,hidden", [(4, 32, 512), (12, 64, 3072), (3, 128, 1536)])
+def test_gpt2_in_the_persistent_kernel(rt, oracle_lib, tmp_models, n_head, head_dim, hidden):
+    """One launch for the whole loop, the stream and the state after it equal to the per-stage kernels' and the oracle's."""
+    from espresso_b200.model_config import tiny_gpt2
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = dataclasses.replace(tiny_gpt2(vocab=515, max_seq=96), nHead=n_head, nKVHead=n_head, headDim=head_dim, dModel=n_head * head_dim, hiddenDim=hidden)
+    d = tmp_models(cfg)
+    prompt = synthetic_prompt(cfg.vocab, 9)
+    ora = oracle_lib.Runtime(oracle_lib.Model.from_dir(d))
+    for flags in (0, rt.FLAG_NO_MEGAKERNEL):
+        eng = rt.DecodeEngine.build(d, flags=flags)
+        eng.prefill(prompt)
+        toks, _ = eng.decode(40)
+        assert (eng.timings()["kernel_launches"] == 1) == (flags == 0)
+        compare_greedy_stream(ora, prompt, toks[0])
+        assert ora.prefill(list(prompt) + [int(t) for t in toks[0][:-1]]) == 0
+        assert_logits_close(eng.logits(), ora.logits(), f"flags {flags}")
+        eng.close()
+
+
+@pytest.mark.parametrize("kind,n_head,hidden", [("q8_0", 4, 256), ("q8_0", 4, 14592), ("q4_0", 6, 14592)])
+def test_quantised_down_projection_in_column_chunks(rt, oracle_lib, kind, n_head, hidden):
+    """W2 of the persistent kernel arrives cut along its columns: one short chunk, and chunks with a shorter last one."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-w2", 1, n_head, 2, 128 * n_head, 128, hidden, 300, 48)
+    model, uploads = quantised_pair(oracle_lib, cfg, kind)
+    eng = rt.DecodeEngine.empty(cfg)
+    upload_all(eng, uploads)
+    prompt = synthetic_prompt(cfg.vocab, 7)
+    res = eng.generate(prompt, 12)
+    assert eng.timings()["kernel_launches"] == 1
+    compare_greedy_stream(oracle_lib.Runtime(model), prompt, res.tokens)
+    eng.close()
