@@ -380,15 +380,16 @@ __device__ __forceinline__ unsigned ld_acquire_cta_shared(const unsigned* p) {
 __device__ __forceinline__ void st_release_cta_shared(unsigned* p, unsigned v) {
     asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
 }
-__device__ __forceinline__ const uint8_t* mega_acquire(const MegaArgs& a, const MegaShared& s, const MegaCursor& c, unsigned index) {
-    // one lane per warp polls; the warp barrier that follows orders the other lanes' reads of the chunk after it
-    if ((threadIdx.x & 31) == 0 && !mega_aborting(s)) {
+// `landed` is the count the thread read last: the ring runs ahead, so most chunks are known to be there without a read
+// (the read and the warp barrier behind it took 3 % of the token time of the quantised models).
+__device__ __forceinline__ const uint8_t* mega_acquire(const MegaArgs& a, const MegaShared& s, const MegaCursor& c, unsigned index, unsigned& landed) {
+    if ((int)(landed - index) <= 0) {
         unsigned spins = 0;
-        while ((int)(ld_acquire_cta_shared(s.landed) - index) <= 0) {
-            if (mega_spin_out(a, s, spins, 3)) break;
+        while ((int)((landed = ld_acquire_cta_shared(s.landed)) - index) <= 0) {
+            if (mega_aborting(s) || mega_spin_out(a, s, spins, 3)) break;
         }
+        __syncwarp();
     }
-    __syncwarp();
     return s.slots + (size_t)c.slot * a.plan.slot_bytes;
 }
 __device__ __forceinline__ void mega_release(const MegaArgs& a, const MegaShared& s, MegaCursor& c) {
@@ -1151,7 +1152,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         if (a.trace && (int)blockIdx.x == a.trace_cta && tid == 0 && step == a.first + a.n_steps - 1) a.trace[n_stamp++] = clock64();
     };
     MegaCursor c;        // ring position, advances in lock step with the producer's
-    unsigned n_chunk = 0;  // chunks consumed so far
+    unsigned n_chunk = 0, landed = 0;  // chunks consumed so far; chunks known to have arrived
     int pos = a.pos0;    // visible tokens
     uint32_t tok = a.tok0;
     int emitted = 0;
@@ -1230,7 +1231,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
             float* partial = base;
 #pragma unroll 1
             for (int r0 = 0; r0 < rows; r0 += per) {
-                const uint8_t* ch = mega_acquire(a, s, c, n_chunk++);
+                const uint8_t* ch = mega_acquire(a, s, c, n_chunk++, landed);
                 const int n = min(per, rows - r0);
                 if (is_head && p.wt_head == WT_F16) mega_chunk_dots<WT_F16>(ch, n, n_kb, xa, partial, warp, lane);  // an fp16 head on quantised layers
                 else mega_chunk_dots<WT>(ch, n, n_kb, xa, partial, warp, lane);
@@ -1238,7 +1239,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                 hand_back(left - r0 <= keep * per);
             }
         } else {
-            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++);
+            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++, landed);
             FINE();
             lg_parts = mega_chunk_dots<WT>(ch, rows, n_kb, xa, base, warp, lane);
             FINE();
@@ -1467,7 +1468,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                         float* partial = base;
 #pragma unroll 1
                         for (int k = k0; k < k1; k += p.s3b_kpc) {
-                            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++);
+                            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++, landed);
                             mega_chunk_dots<WT>(ch, w.d_n, min(p.s3b_kpc, k1 - k), s.xa + (size_t)k * 128, partial, warp, lane, qs + k);
                             partial += kMegaChunkRows;
                             hand_back(k + p.s3b_kpc >= n_kb);

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_spec_mega(const SpecArgs sa
 
     // ---------------- consumers ----------------
     MegaCursor c;          // ring position, advances in lock step with the producer's
-    unsigned n_chunk = 0;  // chunks consumed so far
+    unsigned n_chunk = 0, landed = 0;  // chunks consumed so far; chunks known to have arrived
     int par = 0;           // which half of s.partial the next chunk's sums go to
     unsigned seq = 0;      // tag of everything the current layer publishes: layers are numbered through both models
     unsigned n_heads = 0;  // heads run so far (tag of the arg-max words)
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_spec_mega(const SpecArgs sa
     // One chunk of a stage: acquire, all products of both positions, release (or defer it past the next exchange), CTA
     // barrier; returns where the sums are (position q at + q * kMegaChunkRows).
     auto chunk_products = [&](int rows, int n_kb, const uint8_t* xa, bool defer) {
-        const uint8_t* ch = mega_acquire(a, s, c, n_chunk++);
+        const uint8_t* ch = mega_acquire(a, s, c, n_chunk++, landed);
         float* partial = s.partial + par * (NP * kMegaChunkRows);
         par ^= 1;
         lg_parts = mega_chunk_dots<WT, NP>(ch, rows, n_kb, xa, partial, warp, lane);
