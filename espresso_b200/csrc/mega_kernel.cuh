@@ -662,12 +662,10 @@ __device__ __forceinline__ float2 mega_tile_dot_f16(const uint8_t* chunk, int R,
 // registers of lane (g = c, t); the block scales q sit behind the vector (qx_scale_bytes).
 __device__ __forceinline__ int qx_byte(int kb, int c, int e) { return kb * 128 + c * 32 + (((e & 15) >> 2) << 3) + ((e >> 4) << 2) + (e & 3); }
 
-// Rounding and integer <-> float conversion without conversion instructions (they issue at a quarter of the rate of an
-// addition, and this code runs once per staged element and four times per product block): adding 1.5 * 2^23 to a float
-// of magnitude below 2^22 rounds it to the nearest integer and leaves that integer in the low mantissa bits.
-constexpr float kRoundMagic = 12582912.0f;          // 1.5 * 2^23 = 0x4B400000
-constexpr int kRoundMagicBits = 0x4B400000;
-__device__ __forceinline__ float int_to_float_small(int v) { return __int_as_float(kRoundMagicBits + v) - kRoundMagic; }  // |v| < 2^22
+// Rounding without conversion instructions (they issue at a quarter of the rate of an addition, and this runs three times per
+// staged element): adding 1.5 * 2^23 to a float of magnitude below 2^22 rounds it to the nearest integer and leaves that
+// integer in the low mantissa bits.
+constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23
 
 // The three int8 digits of v * inv (|v * inv| <= 127); dg[c] carries digit c in its low 8 bits (two's complement).
 __device__ __forceinline__ void qx_digits(float v, float inv, int (&dg)[3]) {
@@ -717,8 +715,8 @@ __device__ __forceinline__ float2 mega_tile_dot_q8(const uint8_t* chunk, int R, 
     const size_t kstride = (size_t)R * 32;
     const __half* sp = reinterpret_cast<const __half*>(chunk + (size_t)R * n_kb * 32) + row;
     const uint8_t* xp = xq + (g < 3 ? g * 32 + t * 8 : 0);
-    // what this lane's two result columns mean: t = 0 holds digits 0 and 1, t = 1 digit 2, the others nothing
-    const float k0 = t == 0 ? 1.0f : t == 1 ? (1.0f / 16384.0f) : 0.f, k1 = t == 0 ? (1.0f / 128.0f) : 0.f;
+    // a lane's two result columns are one number, 128 c[0] + c[1] (below 2^27: exact as an integer), in units of 1 / 128 for
+    // t = 0 (digits 0 and 1) and of 1 / 2^21 for t = 1 (digit 2; the next column is zero, like all of the other lanes')
     float a0 = 0.f, a8 = 0.f;
 #pragma unroll 4
     for (int kb = kb0; kb < kb1; kb++) {
@@ -730,9 +728,12 @@ __device__ __forceinline__ float2 mega_tile_dot_q8(const uint8_t* chunk, int R, 
         const uint2 w8 = *reinterpret_cast<const uint2*>(wp + kb * kstride + 8 * 32);
         int c[4] = {0, 0, 0, 0};
         mma_s8(c, w0.x, w8.x, w0.y, w8.y, b.x, b.y);
-        a0 = fmaf(s0 * q, fmaf(int_to_float_small(c[1]), k1, int_to_float_small(c[0]) * k0), a0);
-        a8 = fmaf(s8 * q, fmaf(int_to_float_small(c[3]), k1, int_to_float_small(c[2]) * k0), a8);
+        a0 = fmaf(s0 * q, (float)(c[0] * 128 + c[1]), a0);
+        a8 = fmaf(s8 * q, (float)(c[2] * 128 + c[3]), a8);
     }
+    const float unit = t == 0 ? 1.0f / 128.0f : 1.0f / 2097152.0f;
+    a0 *= unit;
+    a8 *= unit;
     // lanes t = 0 and t = 1 hold the two parts of every row's sum
     a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
     a8 += __shfl_xor_sync(0xffffffffu, a8, 1);
