@@ -2055,6 +2055,13 @@ int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
         if (dbg) { k_copy_debug<<<(n + 255) / 256, 256, 0, s>>>(src, dbg + offset, n); launches++; }
     };
     const bool att_ok_hd = hd == 32 || hd == 64 || hd == 128;
+    // q/k/v cannot be cut along K on the pairs (its epilogue needs whole sums).  Where its 256 x 256 tiles occupy less than half
+    // of the pairs and the streamed product's 128 x 64 tiles fit the chip at once (two per SM, some room left), the streamed
+    // product takes it: prompt passes at d2048 330 rows 2390 -> 2190 us, 401 2385 -> 2260, 768 2855 -> 2690.  With 288 tiles
+    // (1000 rows, 2304 x 768) it lost up to 6 %.
+    const int pair_tiles = (rows + kPgRows - 1) / kPgRows * ((q + 2 * kv + 255) / 256);
+    const int stream_tiles = (rows + kSgMaxCols - 1) / kSgMaxCols * ((q + 2 * kv + kSgRows - 1) / kSgRows);
+    const bool stream_qkv = q % kSgHalf == 0 && kv % kSgHalf == 0 && 4 * pair_tiles <= sm_count_ && 4 * stream_tiles <= 7 * sm_count_;
     int32_t rc;
     if (mode & STEP_FORWARD) {
         if ((rc = launch_embed(rows, nullptr, s))) return rc;
@@ -2065,9 +2072,24 @@ int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
             const bool cap = dbg && l == debug_layer_;
             if ((rc = prep(act_.hidden, d, gpt2 ? NORM_LAYER : NORM_RMS, lw.norm1_g, lw.norm1_b, xh_d_))) return rc;
             const bool fuse_qkv = !qk_norm_ && att_ok_hd;  // (head_dim 32, 64 or 128: whole heads per 128-row half)
-            if ((rc = gemm({{t.wq, act_.q, q, lw.bq}, {t.wk, kraw_, kv, lw.bk}, {t.wv, vraw_, kv, lw.bv}}, xh_d_, fuse_qkv ? PG_QKV : PG_STORE, nullptr, 0,
-                           cap && fuse_qkv ? dbg : nullptr, false, l)))
+            if (fuse_qkv && stream_qkv) {
+                SgArgs a{};
+                const DeviceTensor* w[3] = {t.wq, t.wk, t.wv};
+                const CUtensorMap* maps[3] = {&t.wq->map64, &t.wk->map64, &t.wv->map64};
+                float* const out[3] = {act_.q, kraw_, vraw_};
+                const float* const bias[3] = {lw.bq, lw.bk, lw.bv};
+                for (int g = 0; g < 3; g++) { a.g[g].M = w[g]->rows; a.g[g].out = out[g]; a.g[g].ldo = g ? kv : q; a.g[g].bias = bias[g]; }
+                a.n_groups = 3; a.K = d; a.rows = rows; a.bf16 = tc_bf16_; a.error = d_tc_error_; a.m = m_; a.rs = rs_; a.kv = kv_; a.eps = m_.eps;
+                a.rope = gpt2 ? nullptr : d_rope_; a.layer = l; a.debug = cap ? dbg : nullptr;
+                const SgPlan plan = sg_plan((q / kSgHalf + 2 * (kv / kSgHalf) + 1) / 2, rows, d / kTcBlockK, 1, true, sm_count_);
+                const CUtensorMap* mx = activation_map(xh_d_, d, plan.n_cols);
+                if (!mx) return fail(ESP_CUDA_ERR_CUDA, "tensor map missing for the batched path");
+                ESP_CUDA_TRY(sg_launch(plan, SG_QKV, maps, *mx, a, s));
+                launches++;
+            } else if ((rc = gemm({{t.wq, act_.q, q, lw.bq}, {t.wk, kraw_, kv, lw.bk}, {t.wv, vraw_, kv, lw.bv}}, xh_d_, fuse_qkv ? PG_QKV : PG_STORE, nullptr, 0,
+                                  cap && fuse_qkv ? dbg : nullptr, false, l))) {
                 return rc;
+            }
             if (!fuse_qkv) {
                 RopeArgs ra{};
                 ra.m = m_; ra.rs = rs_; ra.kv = kv_; ra.q = act_.q; ra.k_raw = kraw_; ra.v_raw = vraw_; ra.rope = gpt2 ? nullptr : d_rope_; ra.layer = l;

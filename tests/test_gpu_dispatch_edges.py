@@ -66,6 +66,21 @@ def test_prompt_rows(rt, oracle_lib, kind, rows):
     eng.close()
 
 
+@pytest.mark.parametrize("rows", [768, 832])
+def test_query_key_value_product_of_a_prompt(rt, oracle_lib, rows):
+    """At 2560 rows of weights 768 is the last prompt whose q/k/v go through the streamed product, 832 the first on the pairs."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-qkv", 1, 20, 10, 1280, 64, 512, 320, 840)
+    eng, model = dense_pair(rt, oracle_lib, cfg)
+    prompt = synthetic_prompt(cfg.vocab, rows)
+    eng.prefill(prompt)
+    ora = oracle_lib.Runtime(model)
+    assert ora.prefill(prompt) == 0
+    assert_logits_close(eng.logits(), ora.logits(), f"{rows} rows")
+    eng.close()
+
+
 @pytest.mark.parametrize("n_head,n_kv,head_dim", [(16, 1, 32), (12, 12, 64), (20, 2, 64), (4, 2, 128), (9, 1, 128)])
 @pytest.mark.parametrize("length", [14, 126])
 def test_decode_attention_edges(rt, oracle_lib, n_head, n_kv, head_dim, length):
