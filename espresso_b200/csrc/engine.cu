@@ -1998,7 +1998,7 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
 }
 
 int32_t Engine::launch_attention_prefill(const PrefillAttArgs& pa, cudaStream_t s) {
-    const dim3 grid(n_runs_, m_.n_head);
+    const dim3 grid(m_.n_head, n_runs_);
     if (m_.head_dim == 32) ESP_CUDA_TRY(launch_pdl(k_attention_prefill<32>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<32>(), s, pa));
     else if (m_.head_dim == 64) ESP_CUDA_TRY(launch_pdl(k_attention_prefill<64>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<64>(), s, pa));
     else ESP_CUDA_TRY(launch_pdl(k_attention_prefill<128>, grid, dim3(kPfThreads), (size_t)pf_smem_bytes<128>(), s, pa));

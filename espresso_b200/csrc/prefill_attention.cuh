@@ -9,6 +9,11 @@
 // registers.  One warp = 16 query rows; scores never leave the registers: the accumulator layout of QK^T is the A
 // operand layout of PV.
 //
+// Bound: issue slots, shared memory and the tensor pipe about equally (2000 cycles each per round of sixteen warps), so the
+// inner loop carries no address arithmetic and no mask off the diagonal, and the runs that take longest are launched first.
+// 1531 positions, 32 heads of 64: 70 us per launch before the three, 45 after.  Two 16-row tiles per warp, which halve the
+// shared-memory reads, were slower (245 registers: two warps per scheduler).
+//
 // Shared-memory tiles are [row][HD] halves with the 16-byte chunks of a row XOR-swizzled by the row index, which makes
 // both the cp.async stores and the ldmatrix loads conflict-free.
 #pragma once
@@ -62,7 +67,13 @@ __device__ __forceinline__ uint32_t pf_pack(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// grid = (runs, query heads): a run is a row tile that belongs to one sequence and sits at consecutive positions; the host
+__device__ __forceinline__ float pf_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// grid = (query heads, runs), the last run first: runs at later positions take longest.  A run is a row tile that belongs to one sequence and sits at consecutive positions; the host
 // cuts a pass into runs wherever its sequences begin, so prompts of any length take this kernel (Engine::enqueue_pass).
 template <int HD>
 __global__ void __launch_bounds__(kPfThreads) k_attention_prefill(const PrefillAttArgs p) {
@@ -70,7 +81,7 @@ __global__ void __launch_bounds__(kPfThreads) k_attention_prefill(const PrefillA
     const ModelDims& m = p.m;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int head = blockIdx.y;
+    const int head = blockIdx.x;
     const int kvh = head / (m.n_head / m.n_kv_head);
     constexpr int kChunks = HD / 8;   // 16-byte chunks per row
     constexpr int kSteps = HD / 16;   // k-steps of QK^T
@@ -80,32 +91,52 @@ __global__ void __launch_bounds__(kPfThreads) k_attention_prefill(const PrefillA
     const uint32_t sV = sK + 2 * kPfCols * HD * 2;             // two stages
     pdl_launch_dependents();
     pdl_wait();
-    const int4 run = p.runs[blockIdx.x];
+    const int4 run = p.runs[gridDim.y - 1 - blockIdx.y];
     const int row0 = run.x, n_rows = run.y, seq = run.z, pos0 = run.w;
     const int last_pos = pos0 + n_rows - 1;                    // newest visible position of the tile
     const int n_tiles = last_pos / kPfCols + 1;
     const __half* Kbase = p.kv.k + p.kv.offset(m, p.layer, seq, kvh, 0);
     const __half* Vbase = p.kv.v + p.kv.offset(m, p.layer, seq, kvh, 0);
 
+    // A thread copies the same 16-byte column of every kPfThreads / kChunks-th row: one pair of pointers that advances with the
+    // tiles and constant offsets from them (the swizzle repeats every eight rows).
+    constexpr int kRowStep = kPfThreads / kChunks, kCopies = kPfCols / kRowStep;
+    static_assert(kRowStep % 8 == 0, "rows of one thread share the swizzle");
+    const int ld_row = tid / kChunks, ld_col = tid - ld_row * kChunks;
+    const __half* k_src = Kbase + (size_t)ld_row * HD + ld_col * 8;
+    const ptrdiff_t v_minus_k = Vbase - Kbase;
+    const uint32_t ld_off = pf_off<HD>(ld_row, ld_col);
     auto load_kv = [&](int tile, int stage) {
         const int n0 = tile * kPfCols;
-        for (int i = tid; i < kPfCols * kChunks; i += kPfThreads) {
-            const int r = i / kChunks, c = i - r * kChunks;
-            const uint32_t off = (uint32_t)(stage * kPfCols * HD * 2) + pf_off<HD>(r, c);
-            if (n0 + r <= last_pos) {
-                pf_cp_async16(sK + off, Kbase + (size_t)(n0 + r) * HD + c * 8);
-                pf_cp_async16(sV + off, Vbase + (size_t)(n0 + r) * HD + c * 8);
-            } else {  // beyond the visible range: zeros (their scores are masked, but 0 * NaN must not reach the output)
-                *reinterpret_cast<uint4*>(pf_smem + (sK - sQ) + off) = make_uint4(0, 0, 0, 0);
-                *reinterpret_cast<uint4*>(pf_smem + (sV - sQ) + off) = make_uint4(0, 0, 0, 0);
+        const uint32_t dst = sK + (uint32_t)(stage * kPfCols * HD * 2) + ld_off;
+        constexpr uint32_t kToV = 2 * kPfCols * HD * 2;
+        const __half* const v_src = k_src + v_minus_k;
+        if (n0 + kPfCols - 1 <= last_pos) {
+#pragma unroll
+            for (int i = 0; i < kCopies; i++) {
+                pf_cp_async16(dst + i * kRowStep * HD * 2, k_src + i * kRowStep * HD);
+                pf_cp_async16(dst + kToV + i * kRowStep * HD * 2, v_src + i * kRowStep * HD);
+            }
+        } else {  // beyond the visible range: zeros (their scores are masked, but 0 * NaN must not reach the output)
+#pragma unroll 1
+            for (int i = 0; i < kCopies; i++) {
+                const uint32_t at = dst + i * kRowStep * HD * 2;
+                if (n0 + ld_row + i * kRowStep <= last_pos) {
+                    pf_cp_async16(at, k_src + i * kRowStep * HD);
+                    pf_cp_async16(at + kToV, v_src + i * kRowStep * HD);
+                } else {
+                    *reinterpret_cast<uint4*>(pf_smem + (at - sQ)) = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4*>(pf_smem + (at + kToV - sQ)) = make_uint4(0, 0, 0, 0);
+                }
             }
         }
+        k_src += kPfCols * HD;  // tiles are loaded in order
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     load_kv(0, 0);
-    // the query tile, scaled by 1/sqrt(HD), as fp16
+    // the query tile, scaled by log2(e) / sqrt(HD) (the softmax works with powers of two), as fp16
     {
-        const float scale = 1.0f / sqrtf((float)HD);
+        const float scale = 1.4426950408889634f / sqrtf((float)HD);
         for (int i = tid; i < kPfRows * kChunks; i += kPfThreads) {
             const int r = i / kChunks, c = i - r * kChunks;
             uint4 v = make_uint4(0, 0, 0, 0);
@@ -164,15 +195,17 @@ __global__ void __launch_bounds__(kPfThreads) k_attention_prefill(const PrefillA
             // ---- causal mask (only tiles that reach past the row's position need it) and the online softmax
             const bool diag = n0 + kPfCols - 1 > pos0 + warp * 16;
             float mx[2] = {-INFINITY, -INFINITY};
+            if (diag) {
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
+                for (int j = 0; j < 8; j++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int col = n0 + j * 8 + 2 * t + (e & 1), rr = e >> 1;
-                    if (diag && col > my_pos[rr]) sc[j][e] = -INFINITY;
-                    mx[rr] = fmaxf(mx[rr], sc[j][e]);
-                }
+                    for (int e = 0; e < 4; e++)
+                        if (n0 + j * 8 + 2 * t + (e & 1) > my_pos[e >> 1]) sc[j][e] = -INFINITY;
             }
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) mx[e >> 1] = fmaxf(mx[e >> 1], sc[j][e]);
             float corr[2];
 #pragma unroll
             for (int rr = 0; rr < 2; rr++) {
@@ -180,15 +213,15 @@ __global__ void __launch_bounds__(kPfThreads) k_attention_prefill(const PrefillA
                 mx[rr] = fmaxf(mx[rr], __shfl_xor_sync(0xffffffffu, mx[rr], 2));
                 const float m_new = fmaxf(m_run[rr], mx[rr]);
                 // position 0 is visible to every row, so m_new is finite from the first tile on
-                corr[rr] = m_run[rr] == -INFINITY ? 0.f : __expf(m_run[rr] - m_new);
+                corr[rr] = m_run[rr] == -INFINITY ? 0.f : pf_exp2(m_run[rr] - m_new);
                 m_run[rr] = m_new;
             }
             float rs[2] = {0.f, 0.f};
             uint32_t pa[4][4];  // P as A fragments: k-step kk covers positions 16 kk .. 16 kk + 15
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const float p0 = __expf(sc[j][0] - m_run[0]), p1 = __expf(sc[j][1] - m_run[0]);
-                const float p2 = __expf(sc[j][2] - m_run[1]), p3 = __expf(sc[j][3] - m_run[1]);
+                const float p0 = pf_exp2(sc[j][0] - m_run[0]), p1 = pf_exp2(sc[j][1] - m_run[0]);
+                const float p2 = pf_exp2(sc[j][2] - m_run[1]), p3 = pf_exp2(sc[j][3] - m_run[1]);
                 rs[0] += p0 + p1;
                 rs[1] += p2 + p3;
                 pa[j >> 1][(j & 1) * 2] = pf_pack(p0, p1);
@@ -200,8 +233,10 @@ __global__ void __launch_bounds__(kPfThreads) k_attention_prefill(const PrefillA
                 rs[rr] += __shfl_xor_sync(0xffffffffu, rs[rr], 2);
                 l_run[rr] = l_run[rr] * corr[rr] + rs[rr];
             }
+            if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {  // (the maxima rarely move after the first tiles)
 #pragma unroll
-            for (int j = 0; j < kOut; j++) { o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1]; }
+                for (int j = 0; j < kOut; j++) { o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1]; }
+            }
             // ---- O += P V
 #pragma unroll
             for (int kk = 0; kk < 4; kk++) {
