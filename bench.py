@@ -10,8 +10,7 @@ decode, token download all inside the timed region).
     python bench.py --kernel gemv|gemm --rows R --cols C --type f16|bf16|q8_0|q4_0 [--batch N]   # one stand-alone kernel
 
 The second form times a single kernel on a matrix of the given shape and prints one JSON line (mean kernel
-milliseconds, GB/s over the algorithmic bytes, TFLOP/s for the GEMM); it launches nothing but that kernel (plus, for
-a K-sliced GEMM, the clearing of its output), which makes it the command the profiler summaries capture.
+milliseconds, GB/s over the algorithmic bytes, TFLOP/s for the GEMM); it launches nothing but that kernel, which makes it the command the profiler summaries capture.
 """
 from __future__ import annotations
 
@@ -542,7 +541,7 @@ def measure(args, wl: dict, rank: int, local_rank: int, world: int, steps: int, 
             sustained = float(peaks.get("bf16_tflops_sustained", 1400.0))
             out["prefill"] = {"tokens_per_s": toks / t, "ms": t * 1e3, "TFLOPs_per_gpu": tflops, "frac_of_bf16_sustained": tflops / sustained,
                               "peak_kind": "measured" if peaks else "fallback", "prompt_tokens": toks,
-                              "note": "prefill_batch(): host wall clock around the call incl. prompt upload; passes of up to 512 rows"}
+                              "note": "prefill_batch(): host wall clock around the call incl. prompt upload; passes of up to 2048 rows (4096 up to d_model 1024)"}
         if full and rank == 0 and draft is None and n_seq == 1:
             st = stage_trace_us(eng, cfg, prompts[0], n_decode, clocks.get("sm_mhz") or 1965.0)
             if st:

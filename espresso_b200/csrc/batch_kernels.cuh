@@ -1,7 +1,7 @@
-// Element-wise stages of the batched (tensor-core) decode path.  The matrix products run in k_gemm_tc; these
-// kernels prepare its 16-bit operand rows and apply what the GEMV path fuses into its epilogues:
-//   k_prep_rows    (embedding) -> RMSNorm / LayerNorm / none -> fp16 or bf16 operand rows
-//   k_rope_append  half-split RoPE on q (in place) and k, KV-cache append of k and v
+// Element-wise stages beside the products of many rows (stream_gemm.cuh, pair_gemm.cuh):
+//   k_prep_rows    RMSNorm / LayerNorm / none -> fp16 or bf16 operand rows, in one or more 16-bit parts
+//   k_rope_append  per-head q/k norm, half-split RoPE on q (in place) and k, KV-cache append of k and v: models whose q/k/v
+//                  product cannot do this in its epilogue
 //   k_head_done    turns the packed per-row maxima of the LM-head GEMM into tokens (head_finalize)
 // Every kernel here is launched with programmatic stream serialization: it lets its successor start early and
 // waits for its predecessor before it touches global memory.

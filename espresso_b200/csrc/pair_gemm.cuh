@@ -1,4 +1,4 @@
-// Products of wide prompt passes (more than kSgMaxRows rows): Y[n][m] = sum_k W[m][k] * X[n][k] on pairs of SMs.
+// Products of prompt passes with more rows than the streamed products take: Y[n][m] = sum_k W[m][k] * X[n][k] on pairs of SMs.
 //
 // Bound: the tensor pipe.  A single SM's 128 x 256 tile needs 48 KB of operands per 64-wide K block, 96 bytes per cycle at
 // the pipe's rate of 512 cycles per block, more than an SM can pull out of L2 (about 64): such a kernel stood at 0.6 of the
