@@ -61,10 +61,13 @@ __global__ void k_add_rows(float* dst, const float* src, int n4) {
 }
 SgPlan sg_plan(int w_tiles, int rows, int kb, int parts, bool may_split, int sms);
 cudaError_t sg_launch(const SgPlan& plan, int epilogue, const CUtensorMap* const* mw, const CUtensorMap& mx, SgArgs a, cudaStream_t s);
-// Rows of a pass that take the streamed products; wider passes take the products on SM pairs.  Measured crossings (prompt pass,
-// us, streamed / pairs): 1.1B 256 rows 2181 / 2602, 400 rows 3246 / 2930; GPT-2 400 rows 1056 / 1078; 8B (4 layers) 128 rows
-// 716 / 959, 192 rows 942 / 974, 256 rows 1188 / 992.
-constexpr int kSgMaxRows = 320, kSgMaxRowsWide = 192;  // d_model <= 2048 / above
+// Rows of a pass that take the streamed products; wider passes take the products on SM pairs.  Decode batches (one position per
+// sequence) up to kSgMaxRows.  Prompt passes, whose attention is the same tiled kernel either way, cross where a second or
+// third read of the weights by the 64-row tiles costs more than idle pairs: measured (us, streamed / pairs) 1.1B 160 rows 1500 /
+// 1590, 200 rows 1925 / 1657, 300 rows 2290 / 2110; 8 layers of 8B 100 rows 1310 / 1310, 144 rows 1675 / 1318; GPT-2 300 rows
+// 662 / 800, 512 rows 771 / 892, 700 rows 908 / 945, 768 rows 934 / 943.
+constexpr int kSgMaxRows = 320, kSgMaxRowsWide = 192;  // decode: d_model <= 2048 / above
+constexpr int sg_prompt_rows(int d_model) { return d_model <= 1024 ? 704 : d_model <= 2048 ? 192 : 128; }
 constexpr int kTcMinRows = 9;  // below this the row-batched GEMV stages are used
 // Rows of a prompt pass on the batched path.  Every pass streams all the weights once and is a chain of ~8 dependent
 // launches per layer, so few wide passes win: 256 GPT-2 prompts of 64 tokens took 32 passes of 512 rows at 0.74 ms, nearly
@@ -837,8 +840,8 @@ int32_t Engine::check_ready(const char* what) const {
 // row; STEP_HEAD runs final norm + LM head + argmax; STEP_FEEDBACK makes the head emit and feed back its token.
 int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
     if (tp_size_ > 1 && !tc_ready_) return fail(ESP_CUDA_ERR_STATE, "tensor parallelism needs 16-bit weights with 64-aligned shard sizes");
-    if (stream_path(rows)) return launch_step_stream(rows, mode, s, profile);
-    if (tc_ready_ && rows > sg_max_rows_) return launch_step_wide(rows, mode, s);
+    if (stream_path(rows, mode)) return launch_step_stream(rows, mode, s, profile);
+    if (tc_ready_ && rows > ((mode & STEP_TILED_ATT) ? sg_prompt_rows(m_.d_model) : sg_max_rows_)) return launch_step_wide(rows, mode, s);
     const bool gpt2 = m_.arch == ARCH_GPT2;
     const int cap = sm_count_ * 2;  // one wave: the stage kernels hold ~120 registers, two CTAs per SM
     int launches = 0;
@@ -934,7 +937,7 @@ int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
 
 int32_t Engine::submit(int rows, int mode) {
     if (force_failure_enabled()) return fail(ESP_CUDA_ERR_FORCED_FAILURE, "forced failure is enabled");
-    if (tc_ready_ && !tc_operands_ready_ && (stream_path(rows) || rows >= kTcMinRows)) {
+    if (tc_ready_ && !tc_operands_ready_ && (stream_path(rows, 0) || rows >= kTcMinRows)) {
         int32_t rc = tc_operands();  // before any capture: it allocates
         if (rc) return rc;
     }
@@ -1729,7 +1732,7 @@ int32_t Engine::build_tc() {
     if ((rc = dev_alloc(owned_, &kraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &vraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &d_tc_error_, 4))) return rc;
-    if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, sg_max_rows_) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
+    if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, std::max(sg_max_rows_, sg_prompt_rows(m_.d_model))) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
     if (tp_size_ > 1 && (rc = dev_alloc(owned_, &tp_partial_, (size_t)max_rows_ * m_.d_model))) return rc;
     ESP_CUDA_TRY(cudaDeviceSynchronize());
     tc_ready_ = true;
@@ -1803,10 +1806,10 @@ int32_t Engine::launch_attention_decode(const DecodeAttArgs& a, int rows, cudaSt
     return ESP_CUDA_OK;
 }
 
-bool Engine::stream_path(int rows) const {
+bool Engine::stream_path(int rows, int mode) const {
     // A quantised model's single rows stay on the kernels that read the GGUF blocks themselves (the persistent kernel and the
     // row-wise GEMVs): an engine that only ever decodes one sequence then never builds the fp16 expansion.
-    return tc_ready_ && rows <= sg_max_rows_ && !(tc_quant_ && rows == 1);
+    return tc_ready_ && rows <= ((mode & STEP_TILED_ATT) ? sg_prompt_rows(m_.d_model) : sg_max_rows_) && !(tc_quant_ && rows == 1);
 }
 
 int32_t Engine::launch_embed(int rows, float2* stat, cudaStream_t s) {
@@ -1861,7 +1864,7 @@ int32_t Engine::launch_head_stream(int rows, int mode, int parts, cudaStream_t s
     return ESP_CUDA_OK;
 }
 
-// One pass over the model for up to kSgMaxRows rows with the streamed products (stream_gemm.cuh): per layer q/k/v (norm,
+// One pass over the model for few rows (see stream_path) with the streamed products (stream_gemm.cuh): per layer q/k/v (norm,
 // bias, RoPE and cache append inside), attention, Wo + residual, FFN up (norm and activation inside), W2 + residual.
 int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool profile) {
     const bool gpt2 = m_.arch == ARCH_GPT2;
@@ -1931,6 +1934,10 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
         if (dbg) { k_copy_debug<<<(n + 255) / 256, 256, 0, s>>>(src, dbg + offset, n); launches++; }
     };
     const bool att_ok_hd = hd == 32 || hd == 64 || hd == 128;
+    // Prompt passes: the tiled attention reads a sequence's keys and values once per 64 rows and query head, the decode kernel once
+    // per row and KV head.  100 rows, 12 heads: 540 -> 520 us a pass, 300 rows 858 -> 662; 32 query heads on 4: 128 rows 1372 -> 1393,
+    // 160 rows 1524 -> 1500.
+    const bool tiled_att = (mode & STEP_TILED_ATT) && parts == 1 && rows >= (m_.n_head == m_.n_kv_head ? 80 : 144);
     const bool fuse_qkv = !qk_norm_ && att_ok_hd && kv % kSgHalf == 0;  // whole heads per 64-row half (a 128-wide head: per tile)
     int32_t rc;
     mark();
@@ -1957,7 +1964,13 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
                 launches++;
             }
             mark();
-            if (att_ok_hd) {
+            if (tiled_att) {
+                PrefillAttArgs pa{};
+                pa.m = m_; pa.rs = rs_; pa.kv = kv_; pa.q = act_.q; pa.ctx16 = xh_q_; pa.bf16 = tc_bf16_; pa.layer = l; pa.runs = d_runs_;
+                pa.debug = cap ? dbg + q + 2 * kv : nullptr;
+                if ((rc = launch_attention_prefill(pa, s))) return rc;
+                launches++;
+            } else if (att_ok_hd) {
                 DecodeAttArgs da{};
                 da.m = m_; da.rs = rs_; da.kv = kv_; da.q = act_.q; da.ctx16 = xh_q_; da.bf16 = tc_bf16_; da.parts = parts; da.layer = l;
                 da.debug = cap ? dbg + q + 2 * kv : nullptr;

@@ -116,8 +116,8 @@ private:
     int32_t launch_embed(int rows, float2* stat, cudaStream_t s);
     int32_t launch_prep(int rows, const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst, int parts, cudaStream_t s);
     int32_t launch_attention_prefill(const PrefillAttArgs& pa, cudaStream_t s);
-    int32_t launch_step_stream(int rows, int mode, cudaStream_t s, bool profile);  // up to kSgMaxRows rows: streamed products, fused stages
-    bool stream_path(int rows) const;
+    int32_t launch_step_stream(int rows, int mode, cudaStream_t s, bool profile);  // few rows: streamed products, fused stages
+    bool stream_path(int rows, int mode) const;
     int32_t launch_attention_decode(const DecodeAttArgs& a, int rows, cudaStream_t s);
     int32_t build_tc();
     int32_t tc_operands();  // weight maps (and a quantised model's fp16 expansion), built on first use of the batched path

@@ -45,13 +45,13 @@ def test_streamed_product(rt, kind, shape):
 
 
 @pytest.mark.parametrize("kind", ["f16", "bf16"])
-@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 65, 320, 321, 512, 515])
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 65, 143, 144, 512, 704, 705])
 def test_prompt_rows(rt, oracle_lib, kind, rows):
-    """A prompt of 320 rows is the last one of the streamed products at this width, 321 the first of the paired tiles (256 rows
-    each); hidden 1056 leaves a partial column tile in every product."""
+    """A prompt of 144 rows is the first with the tiled attention (three query heads per KV head), 704 rows the last of the
+    streamed products at this width, 705 the first of the paired tiles; hidden 1056 leaves a partial column tile in every product."""
     from espresso_b200.synthetic import synthetic_prompt
 
-    cfg = _model("edge-rows", 2, 6, 2, 384, 64, 1056, 520, 640)
+    cfg = _model("edge-rows", 2, 6, 2, 384, 64, 1056, 520, 768)
     eng, model = dense_pair(rt, oracle_lib, cfg, kind)
     prompt = synthetic_prompt(cfg.vocab, rows)
     eng.prefill(prompt)
