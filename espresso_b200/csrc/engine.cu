@@ -61,13 +61,6 @@ __global__ void k_add_rows(float* dst, const float* src, int n4) {
 }
 SgPlan sg_plan(int w_tiles, int rows, int kb, int parts, bool may_split, int sms);
 cudaError_t sg_launch(const SgPlan& plan, int epilogue, const CUtensorMap* const* mw, const CUtensorMap& mx, SgArgs a, cudaStream_t s);
-// Rows of a pass that take the streamed products; wider passes take the products on SM pairs.  Decode batches (one position per
-// sequence) up to kSgMaxRows.  Prompt passes, whose attention is the same tiled kernel either way, cross where a second or
-// third read of the weights by the 64-row tiles costs more than idle pairs: measured (us, streamed / pairs) 1.1B 160 rows 1500 /
-// 1590, 200 rows 1925 / 1657, 300 rows 2290 / 2110; 8 layers of 8B 100 rows 1310 / 1310, 144 rows 1675 / 1318; GPT-2 300 rows
-// 662 / 800, 512 rows 771 / 892, 700 rows 908 / 945, 768 rows 934 / 943.
-constexpr int kSgMaxRows = 320, kSgMaxRowsWide = 192;  // decode: d_model <= 2048 / above
-constexpr int sg_prompt_rows(int d_model) { return d_model <= 1024 ? 704 : d_model <= 2048 ? 192 : 128; }
 constexpr int kTcMinRows = 9;  // below this the row-batched GEMV stages are used
 // Rows of a prompt pass on the batched path.  Every pass streams all the weights once and is a chain of ~8 dependent
 // launches per layer, so few wide passes win: 256 GPT-2 prompts of 64 tokens took 32 passes of 512 rows at 0.74 ms, nearly
@@ -839,9 +832,12 @@ int32_t Engine::check_ready(const char* what) const {
 // One pass over the model for `rows` rows.  mode: STEP_FORWARD runs the layers on (tok, pos) of every active
 // row; STEP_HEAD runs final norm + LM head + argmax; STEP_FEEDBACK makes the head emit and feed back its token.
 int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
-    if (tp_size_ > 1 && !tc_ready_) return fail(ESP_CUDA_ERR_STATE, "tensor parallelism needs 16-bit weights with 64-aligned shard sizes");
-    if (stream_path(rows, mode)) return launch_step_stream(rows, mode, s, profile);
-    if (tc_ready_ && rows > ((mode & STEP_TILED_ATT) ? sg_prompt_rows(m_.d_model) : sg_max_rows_)) return launch_step_wide(rows, mode, s);
+    switch (path_of(rows, mode)) {
+        case PATH_REFUSED: return fail(ESP_CUDA_ERR_STATE, "tensor parallelism needs tensor-core operands: one storage type and 64-aligned shard sizes");
+        case PATH_STREAM: return launch_step_stream(rows, mode, s, profile);
+        case PATH_PAIRS: return launch_step_wide(rows, mode, s);
+        case PATH_ROWWISE: break;
+    }
     const bool gpt2 = m_.arch == ARCH_GPT2;
     const int cap = sm_count_ * 2;  // one wave: the stage kernels hold ~120 registers, two CTAs per SM
     int launches = 0;
@@ -937,7 +933,7 @@ int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
 
 int32_t Engine::submit(int rows, int mode) {
     if (force_failure_enabled()) return fail(ESP_CUDA_ERR_FORCED_FAILURE, "forced failure is enabled");
-    if (tc_ready_ && !tc_operands_ready_ && (stream_path(rows, 0) || rows >= kTcMinRows)) {
+    if (tc_ready_ && !tc_operands_ready_ && path_of(rows, mode) != PATH_ROWWISE) {
         int32_t rc = tc_operands();  // before any capture: it allocates
         if (rc) return rc;
     }
@@ -1714,7 +1710,6 @@ int32_t Engine::build_tc() {
     if (quantised && (cfg_.flags & ESP_CUDA_FLAG_NO_TC_SHADOW)) return ESP_CUDA_OK;
     tc_bf16_ = t0 == ESP_CUDA_BF16;
     tc_quant_ = quantised;
-    sg_max_rows_ = m_.d_model <= 2048 ? kSgMaxRows : kSgMaxRowsWide;
     tc_mats_ = mats;
     tc_operands_ready_ = false;
     // 16-bit matrices get their TMA maps now.  A quantised model's fp16 expansion (what batches and prefill chunks
@@ -1732,7 +1727,7 @@ int32_t Engine::build_tc() {
     if ((rc = dev_alloc(owned_, &kraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &vraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &d_tc_error_, 4))) return rc;
-    if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, std::max(sg_max_rows_, sg_prompt_rows(m_.d_model))) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
+    if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, std::max(sg_decode_rows(m_.d_model), sg_prompt_rows(m_.d_model))) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
     if (tp_size_ > 1 && (rc = dev_alloc(owned_, &tp_partial_, (size_t)max_rows_ * m_.d_model))) return rc;
     ESP_CUDA_TRY(cudaDeviceSynchronize());
     tc_ready_ = true;
@@ -1806,11 +1801,7 @@ int32_t Engine::launch_attention_decode(const DecodeAttArgs& a, int rows, cudaSt
     return ESP_CUDA_OK;
 }
 
-bool Engine::stream_path(int rows, int mode) const {
-    // A quantised model's single rows stay on the kernels that read the GGUF blocks themselves (the persistent kernel and the
-    // row-wise GEMVs): an engine that only ever decodes one sequence then never builds the fp16 expansion.
-    return tc_ready_ && rows <= ((mode & STEP_TILED_ATT) ? sg_prompt_rows(m_.d_model) : sg_max_rows_) && !(tc_quant_ && rows == 1);
-}
+StepPath Engine::path_of(int rows, int mode) const { return step_path(tc_ready_, tc_quant_, tp_size_, m_.d_model, rows, (mode & STEP_TILED_ATT) != 0); }
 
 int32_t Engine::launch_embed(int rows, float2* stat, cudaStream_t s) {
     const DeviceTensor& te = tensors_.at("embeddings/token");
@@ -1864,7 +1855,7 @@ int32_t Engine::launch_head_stream(int rows, int mode, int parts, cudaStream_t s
     return ESP_CUDA_OK;
 }
 
-// One pass over the model for few rows (see stream_path) with the streamed products (stream_gemm.cuh): per layer q/k/v (norm,
+// One pass over the model for few rows (see step_path) with the streamed products (stream_gemm.cuh): per layer q/k/v (norm,
 // bias, RoPE and cache append inside), attention, Wo + residual, FFN up (norm and activation inside), W2 + residual.
 int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool profile) {
     const bool gpt2 = m_.arch == ARCH_GPT2;

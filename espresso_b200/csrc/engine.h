@@ -13,6 +13,7 @@
 #include "../../include/espresso_cuda.h"
 #include "decode_kernels.cuh"
 #include "mega_kernel.cuh"
+#include "step_path.h"
 
 namespace esp {
 
@@ -117,7 +118,7 @@ private:
     int32_t launch_prep(int rows, const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst, int parts, cudaStream_t s);
     int32_t launch_attention_prefill(const PrefillAttArgs& pa, cudaStream_t s);
     int32_t launch_step_stream(int rows, int mode, cudaStream_t s, bool profile);  // few rows: streamed products, fused stages
-    bool stream_path(int rows, int mode) const;
+    StepPath path_of(int rows, int mode) const;
     int32_t launch_attention_decode(const DecodeAttArgs& a, int rows, cudaStream_t s);
     int32_t build_tc();
     int32_t tc_operands();  // weight maps (and a quantised model's fp16 expansion), built on first use of the batched path
@@ -205,7 +206,6 @@ private:
     bool tc_operands_ready_ = false;
     std::vector<std::string> tc_mats_;
     int tc_bf16_ = 0;
-    int sg_max_rows_ = 0;    // widest pass of the streamed products
     bool tc_quant_ = false;  // the operands are the fp16 expansion of a quantised model
     std::vector<LayerTensors> layer_tensors_;
     int tc_rows_alloc_ = 0;

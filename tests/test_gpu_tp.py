@@ -30,7 +30,7 @@ def test_tp_shard_shapes():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("case", ["small", "wide_bf16"])
+@pytest.mark.parametrize("case", ["small", "wide_bf16", "small_q8"])
 def test_tensor_parallel_two_gpus_matches_oracle(case):
     import torch
 

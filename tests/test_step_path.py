@@ -1,0 +1,50 @@
+"""The rule that picks the kernels of a pass (csrc/step_path.h, plain C++), compiled and evaluated on the host."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "espresso_b200", "csrc")
+MAIN = r"""
+#include <cstdio>
+#include "step_path.h"
+int main() {
+    int ready, quantised, tp, d, rows, tiled;
+    while (scanf("%d %d %d %d %d %d", &ready, &quantised, &tp, &d, &rows, &tiled) == 6) printf("%d\n", (int)esp::step_path(ready, quantised, tp, d, rows, tiled));
+}
+"""
+ROWWISE, STREAM, PAIRS, REFUSED = range(4)
+
+
+@pytest.fixture(scope="module")
+def path(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("no g++")
+    d = tmp_path_factory.mktemp("step_path")
+    (d / "main.cc").write_text(MAIN)
+    subprocess.run([gxx, "-std=c++17", "-I", CSRC, "-o", str(d / "main"), str(d / "main.cc")], check=True)
+
+    def ask(ready, quantised, tp, d_model, rows, tiled=0):
+        line = f"{ready} {quantised} {tp} {d_model} {rows} {tiled}\n"
+        return int(subprocess.run([str(d / "main")], input=line, capture_output=True, text=True, check=True).stdout)
+
+    return ask
+
+
+@pytest.mark.parametrize("quantised", [0, 1])
+@pytest.mark.parametrize("rows", [1, 2, 8, 9, 320, 321, 2048])
+def test_tensor_parallel_ranks_never_take_the_rowwise_kernels(path, quantised, rows):
+    """Only the batched paths add up the ranks' partial sums and know the vocabulary shard."""
+    for d_model in (256, 2048, 4096):
+        assert path(1, quantised, 2, d_model, rows) in (STREAM, PAIRS)
+        assert path(0, quantised, 2, d_model, rows) == REFUSED
+
+
+def test_single_device_rows(path):
+    assert path(1, 1, 1, 2048, 1) == ROWWISE and path(1, 1, 1, 2048, 2) == STREAM  # a quantised row reads the blocks
+    assert path(1, 0, 1, 2048, 1) == STREAM
+    assert path(0, 0, 1, 2048, 300) == ROWWISE
+    assert path(1, 0, 1, 2048, 320) == STREAM and path(1, 0, 1, 2048, 321) == PAIRS
+    assert path(1, 0, 1, 4096, 192) == STREAM and path(1, 0, 1, 4096, 193) == PAIRS

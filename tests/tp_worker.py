@@ -10,7 +10,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 sys.path.insert(0, ROOT)
 sys.path.insert(0, os.path.join(ROOT, "tests"))
 
-from espresso_b200 import runtime  # noqa: E402
+from espresso_b200 import gguf_quant, runtime  # noqa: E402
 from espresso_b200.model_config import MultiModelConfig  # noqa: E402
 from espresso_b200.sharding import tp_shard  # noqa: E402
 from espresso_b200.synthetic import synthetic_prompt, synthetic_tensors  # noqa: E402
@@ -30,10 +30,13 @@ def main() -> None:
     else:
         cfg = MultiModelConfig("tp-llama", 2, 8, 4, 256, 32, 512, 1024, 64, 1e-5, 10000.0, None, "llama")
         n_seq, n_prompt, n_decode = 6, 9, 14
-    bf16 = case == "wide_bf16"
+    bf16, quantised = case == "wide_bf16", case == "small_q8"
 
-    def stored(vals, wide):
+    def stored(vals, wide, matrix=False):
         """(array to upload, type name, the fp32 values the storage decodes to)"""
+        if quantised and matrix:
+            blocks = gguf_quant.quantize("q8_0", vals.astype(np.float32))
+            return blocks, "q8_0", gguf_quant.dequantize("q8_0", blocks).reshape(vals.shape)
         if bf16 and wide:
             u = np.ascontiguousarray(vals, np.float32).view(np.uint32)
             bits = ((u + np.uint32(0x7FFF) + ((u >> np.uint32(16)) & np.uint32(1))) >> np.uint32(16)).astype(np.uint16)
@@ -47,8 +50,9 @@ def main() -> None:
     eng = runtime.DecodeEngine.empty(cfg, max_batch=n_seq, device=rank, tp_rank=rank, tp_size=world)
     eng.tp_init(ids[0])
     for name, vals in synthetic_tensors(cfg):
-        arr, kind, _ = stored(vals, is_matrix(name) or name.startswith("embeddings/"))
-        eng.load_tensor(name, kind, np.ascontiguousarray(tp_shard(name, arr, rank, world)))
+        # (a rank's slice of every row is whole blocks of 32: quantising the slice gives the blocks of the whole matrix)
+        arr, kind, _ = stored(np.ascontiguousarray(tp_shard(name, vals, rank, world)), is_matrix(name) or name.startswith("embeddings/"), is_matrix(name))
+        eng.load_tensor(name, kind, arr)
     eng.finalize()
     toks, res = eng.generate_batch(prompts, n_decode)
     single = eng.generate(prompts[0], n_decode).tokens  # rows = 1 also runs tensor parallel
@@ -60,7 +64,7 @@ def main() -> None:
 
         model = oracle.Model(cfg.to_metadata())
         for name, vals in synthetic_tensors(cfg):
-            model.set_tensor(name, stored(vals, is_matrix(name) or name.startswith("embeddings/"))[2])
+            model.set_tensor(name, stored(vals, is_matrix(name) or name.startswith("embeddings/"), is_matrix(name))[2])
         for s in range(n_seq):
             assert len(toks[s]) == n_decode
             compare_greedy_stream(oracle.Runtime(model), prompts[s], toks[s], tol=tol)
