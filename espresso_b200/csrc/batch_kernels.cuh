@@ -41,6 +41,10 @@ __device__ __forceinline__ void store_parts4(uint16_t* buf, int ld, int r, int k
     }
 }
 
+// Row of the rotation table (max_seq rows) for a batch row at position `pos`.  A sequence that has filled its context stays in
+// the batch as an inactive row at pos = max_seq; the products read a row's rotation before they know whether it is active.
+__host__ __device__ __forceinline__ int rope_row(int pos, int max_seq) { return pos < max_seq ? pos : max_seq - 1; }
+
 struct PrepArgs {
     const int* active;
     const float* src;  // [rows][K] fp32

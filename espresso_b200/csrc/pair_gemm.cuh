@@ -194,7 +194,7 @@ __device__ __forceinline__ void pg_epilogue(const PgArgs& a, const PgWarp& w, in
         tmem_ld_cols<16>(w.base + (uint32_t)(h * 128 + (b0 + apart) * 16), u);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (EPI == PG_QKV && rope && gi < 2) {  // halves of a head: v is the first, u the second member of sixteen rotation pairs
-            const float4* cs = reinterpret_cast<const float4*>(a.rope + (size_t)w.pos * (a.m.head_dim >> 1) + ((b0 * 16) & ((a.m.head_dim >> 1) - 1)));
+            const float4* cs = reinterpret_cast<const float4*>(a.rope + (size_t)rope_row(w.pos, a.m.max_seq) * (a.m.head_dim >> 1) + ((b0 * 16) & ((a.m.head_dim >> 1) - 1)));
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 const float4 f = __ldg(cs + j);

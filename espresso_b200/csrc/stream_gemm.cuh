@@ -224,8 +224,8 @@ __device__ __forceinline__ SgRowPre sg_row_prefetch(const SgArgs& a, int row, in
         if (ok) p.x0 = __ldcg(reinterpret_cast<const float4*>(a.g[0].out + (size_t)row * a.g[0].ldo + m0));
     } else if (a.epilogue == SG_QKV) {
         if (a.rope && gi < 2) {
-            const int half = a.m.head_dim >> 1;
-            const float4* cs = reinterpret_cast<const float4*>(a.rope + (size_t)__ldcg(a.rs.pos + row) * half + (m0 & (half - 1)));
+            const int half = a.m.head_dim >> 1, pos = rope_row(__ldcg(a.rs.pos + row), a.m.max_seq);
+            const float4* cs = reinterpret_cast<const float4*>(a.rope + (size_t)pos * half + (m0 & (half - 1)));
             p.x0 = __ldg(cs);
             p.x1 = __ldg(cs + 1);
         }

@@ -131,3 +131,23 @@ def test_quantised_down_projection_in_column_chunks(rt, oracle_lib, kind, n_head
     assert eng.timings()["kernel_launches"] == 1
     compare_greedy_stream(oracle_lib.Runtime(model), prompt, res.tokens)
     eng.close()
+
+
+@pytest.mark.parametrize("n_seq", [3, 40, 330])
+def test_full_sequence_beside_unfinished_ones(rt, oracle_lib, n_seq):
+    """A sequence that has filled its context stays in the batch as an inactive row one position past the rotation table;
+    330 rows go through the products on SM pairs."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-full", 2, 4, 2, 256, 64, 512, 320, 24)
+    eng, model = dense_pair(rt, oracle_lib, cfg, "f16", n_seq)
+    prompts = np.stack([synthetic_prompt(cfg.vocab, 10, stream=s) for s in range(n_seq)])
+    eng.prefill_batch(prompts)
+    for i in range(cfg.maxSeq - 10):
+        eng.decode_step(i % cfg.vocab)  # sequence 0 only
+    toks, _ = eng.decode(6, n_seq)
+    assert eng.visible_token_count(0) == cfg.maxSeq and len(toks[0]) == 0
+    for s in (1, 2, n_seq - 1):
+        assert len(toks[s]) == 6
+        compare_greedy_stream(oracle_lib.Runtime(model), prompts[s], toks[s])
+    eng.close()
