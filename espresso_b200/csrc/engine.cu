@@ -1093,8 +1093,9 @@ int32_t Engine::decode_step(uint32_t token, uint32_t* next) {
     return ESP_CUDA_OK;
 }
 
-// One prompt pass over `rows` rows (seq[r], tok[r]), enqueued without waiting for it.  `last_of`: for every sequence that
-// ends in this pass its last row, or -1; that row's hidden state goes to d_last_hidden_[sequence].  The rows' control
+// One prompt pass over `rows` rows (seq[r], tok[r]), enqueued without waiting for it.  `ends`: (last row, sequence) of every
+// sequence that ends in this pass; that row's hidden state goes to d_last_hidden_[sequence].  h_visible_ counts the rows at
+// once; a caller whose prompt fails, here or in finish_passes, drops the whole prompt (drop_prompt).  The rows' control
 // words, the list of runs (at most kPfRows consecutive positions of one sequence: the tiles of the prompt attention)
 // and the list of last rows travel in a pinned slot; two slots alternate, so the host prepares a pass while the device
 // works on the one before it.
@@ -1113,7 +1114,6 @@ int32_t Engine::enqueue_pass(int rows, const int* seq, const uint32_t* tok, cons
             std::ostringstream os;
             if (full) os << "position " << pos << " exceeds context " << m_.max_seq;
             else os << "token " << tok[r] << " is outside vocab " << vocab_global_;
-            while (r-- > 0) h_visible_[seq[r]]--;
             return fail(ESP_CUDA_ERR_OUT_OF_RANGE, os.str());
         }
         h_visible_[s]++;
@@ -1138,6 +1138,13 @@ int32_t Engine::enqueue_pass(int rows, const int* seq, const uint32_t* tok, cons
     return ESP_CUDA_OK;
 }
 
+// A prompt that failed leaves nothing visible, as after reset(): whatever its passes wrote to the caches is not decoded from.
+int32_t Engine::drop_prompt(int32_t rc) {
+    cudaStreamSynchronize(stream_);
+    std::fill(h_visible_.begin(), h_visible_.end(), 0);
+    return rc;
+}
+
 // Waits for the passes enqueued so far and reports a device-side wait that gave up.
 int32_t Engine::finish_passes() {
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
@@ -1159,12 +1166,14 @@ int32_t Engine::prefill(const uint32_t* tokens, int32_t n) {
     const std::vector<int2> none;
     for (int i = 0; i < n; i += chunk) {
         const int c = std::min(chunk, n - i);
-        if ((rc = enqueue_pass(c, seq.data(), tokens + i, none))) { cudaStreamSynchronize(stream_); return rc; }
-        if (c > 1)  // the last row's hidden state is the sequence's lastHidden
-            ESP_CUDA_TRY(cudaMemcpyAsync(act_.hidden, act_.hidden + (size_t)(c - 1) * m_.d_model, sizeof(float) * m_.d_model,
-                                         cudaMemcpyDeviceToDevice, stream_));
+        if ((rc = enqueue_pass(c, seq.data(), tokens + i, none))) return drop_prompt(rc);
+        if (c > 1) {  // the last row's hidden state is the sequence's lastHidden
+            const cudaError_t e = cudaMemcpyAsync(act_.hidden, act_.hidden + (size_t)(c - 1) * m_.d_model, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_);
+            if (e != cudaSuccess) return drop_prompt(fail(ESP_CUDA_ERR_CUDA, cudaGetErrorString(e)));
+        }
     }
-    return finish_passes();
+    rc = finish_passes();
+    return rc ? drop_prompt(rc) : ESP_CUDA_OK;
 }
 
 int32_t Engine::select_greedy(uint32_t* token) {
@@ -1281,7 +1290,7 @@ int32_t Engine::prefill_batch(const uint32_t* tokens, int32_t n_seq, int32_t len
         for (int s = 0; s < n_seq; s++) seq[s] = s;
         for (int t = 0; t < len; t++) {
             for (int s = 0; s < n_seq; s++) tok[s] = tokens[(size_t)s * len + t];
-            if ((rc = feed_rows(n_seq, seq.data(), tok.data(), false, nullptr))) return rc;
+            if ((rc = feed_rows(n_seq, seq.data(), tok.data(), false, nullptr))) return drop_prompt(rc);
         }
         return ESP_CUDA_OK;
     }
@@ -1299,14 +1308,16 @@ int32_t Engine::prefill_batch(const uint32_t* tokens, int32_t n_seq, int32_t len
             t += take;
             if (t == len) ends.push_back(make_int2((int)seq.size() - 1, s));
             if ((int)seq.size() == prefill_rows_ || (s == n_seq - 1 && t == len)) {
-                if ((rc = enqueue_pass((int)seq.size(), seq.data(), tok.data(), ends))) { cudaStreamSynchronize(stream_); return rc; }
+                if ((rc = enqueue_pass((int)seq.size(), seq.data(), tok.data(), ends))) return drop_prompt(rc);
                 seq.clear(); tok.clear(); ends.clear();
             }
         }
     }
     // row s must hold the last hidden state of sequence s (decode passes have one row per sequence)
-    ESP_CUDA_TRY(cudaMemcpyAsync(act_.hidden, d_last_hidden_, sizeof(float) * (size_t)n_seq * m_.d_model, cudaMemcpyDeviceToDevice, stream_));
-    return finish_passes();
+    const cudaError_t e = cudaMemcpyAsync(act_.hidden, d_last_hidden_, sizeof(float) * (size_t)n_seq * m_.d_model, cudaMemcpyDeviceToDevice, stream_);
+    if (e != cudaSuccess) return drop_prompt(fail(ESP_CUDA_ERR_CUDA, cudaGetErrorString(e)));
+    rc = finish_passes();
+    return rc ? drop_prompt(rc) : ESP_CUDA_OK;
 }
 
 int32_t Engine::decode_step_batch(const uint32_t* tokens, int32_t n_seq, uint32_t* next) {

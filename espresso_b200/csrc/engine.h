@@ -126,6 +126,7 @@ private:
     const CUtensorMap* activation_map(const uint16_t* buf, int K, int tile);
     int32_t enqueue_pass(int rows, const int* seq, const uint32_t* tok, const std::vector<int2>& ends);  // one prompt pass, not waited for
     int32_t finish_passes();
+    int32_t drop_prompt(int32_t rc);
     int32_t feed_rows(int rows, const int* seq, const uint32_t* tok, bool with_head, uint32_t* next_out);
     Weight weight_of(const DeviceTensor& t) const;
     LayerWeights layer_weights(int l) const;

@@ -151,3 +151,38 @@ def test_full_sequence_beside_unfinished_ones(rt, oracle_lib, n_seq):
         assert len(toks[s]) == 6
         compare_greedy_stream(oracle_lib.Runtime(model), prompts[s], toks[s])
     eng.close()
+
+
+def test_failed_prompt_leaves_nothing_to_decode(rt, oracle_lib):
+    """A prompt that fails in a later pass: nothing is visible, decode is refused, and the next prompt is served as usual."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-fail", 1, 4, 2, 128, 32, 256, 320, 128)
+    n_seq, length = 64, 100  # 6400 rows: two passes
+    eng, model = dense_pair(rt, oracle_lib, cfg, "f16", n_seq)
+    prompts = np.stack([synthetic_prompt(cfg.vocab, length, stream=s) for s in range(n_seq)])
+    bad = prompts.copy()
+    bad[-1, -1] = cfg.vocab
+    with pytest.raises(rt.RealModelInferenceError):
+        eng.prefill_batch(bad)
+    assert [eng.visible_token_count(s) for s in range(n_seq)] == [0] * n_seq
+    with pytest.raises(rt.RealModelInferenceError):
+        eng.decode(2)
+    eng.prefill_batch(prompts)
+    toks, _ = eng.decode(4, n_seq)
+    compare_greedy_stream(oracle_lib.Runtime(model), prompts[-1], toks[-1])
+    eng.close()
+
+    model, uploads = quantised_pair(oracle_lib, cfg, "q8_0")
+    eng = rt.DecodeEngine.empty(cfg, flags=rt.FLAG_NO_TC_SHADOW)  # row-wise kernels: passes of eight positions
+    upload_all(eng, uploads)
+    bad = synthetic_prompt(cfg.vocab, 20)
+    bad[12] = cfg.vocab
+    with pytest.raises(rt.RealModelInferenceError):
+        eng.prefill(bad)
+    assert eng.visible_token_count() == 0
+    with pytest.raises(rt.RealModelInferenceError):
+        eng.decode(2)
+    prompt = synthetic_prompt(cfg.vocab, 20)
+    compare_greedy_stream(oracle_lib.Runtime(model), prompt, eng.generate(prompt, 6).tokens)
+    eng.close()
