@@ -2344,27 +2344,27 @@ int32_t Engine::build_mega() {
     return ESP_CUDA_OK;
 }
 
-// GPT-2: the folded LayerNorm constants of every row and the biases of the two residual products.
+// GPT-2: the constant of every row behind a LayerNorm and the biases of the two residual products.
 int32_t Engine::build_mega_gpt2() {
     const int d = m_.d_model, q = m_.q_dim, kv = m_.kv_dim, h = m_.hidden, per = q + 2 * kv + h;
     int32_t rc;
     if ((rc = dev_alloc(owned_, &d_mega_ln_, (size_t)m_.n_layer * per + m_.vocab, false))) return rc;
     if ((rc = dev_alloc(owned_, &d_mega_bias_, (size_t)m_.n_layer * 2 * d, false))) return rc;
-    auto fold = [&](const DeviceTensor& w, const float* g, const float* b, const float* bias, float2* out) {
-        k_fold_norm<<<(w.rows + 7) / 8, 256, 0, stream_>>>(static_cast<const uint16_t*>(w.data), w.rows, d, g, b, bias, out);
+    auto fold = [&](const DeviceTensor& w, const float* b, const float* bias, float* out) {
+        k_fold_norm<<<(w.rows + 7) / 8, 256, 0, stream_>>>(static_cast<const uint16_t*>(w.data), w.rows, d, b, bias, out);
     };
     for (int l = 0; l < m_.n_layer; l++) {
         const std::string pre = "layers/" + std::to_string(l) + "/";
         const LayerWeights lw = layer_weights(l);
-        float2* out = d_mega_ln_ + (size_t)l * per;
-        fold(tensors_.at(pre + "wq"), lw.norm1_g, lw.norm1_b, lw.bq, out);
-        fold(tensors_.at(pre + "wk"), lw.norm1_g, lw.norm1_b, lw.bk, out + q);
-        fold(tensors_.at(pre + "wv"), lw.norm1_g, lw.norm1_b, lw.bv, out + q + kv);
-        fold(tensors_.at(pre + "w1"), lw.norm2_g, lw.norm2_b, lw.b1, out + q + 2 * kv);
+        float* out = d_mega_ln_ + (size_t)l * per;
+        fold(tensors_.at(pre + "wq"), lw.norm1_b, lw.bq, out);
+        fold(tensors_.at(pre + "wk"), lw.norm1_b, lw.bk, out + q);
+        fold(tensors_.at(pre + "wv"), lw.norm1_b, lw.bv, out + q + kv);
+        fold(tensors_.at(pre + "w1"), lw.norm2_b, lw.b1, out + q + 2 * kv);
         ESP_CUDA_TRY(cudaMemcpyAsync(d_mega_bias_ + (size_t)(2 * l) * d, lw.bo, sizeof(float) * d, cudaMemcpyDeviceToDevice, stream_));
         ESP_CUDA_TRY(cudaMemcpyAsync(d_mega_bias_ + (size_t)(2 * l + 1) * d, lw.b2, sizeof(float) * d, cudaMemcpyDeviceToDevice, stream_));
     }
-    fold(tensors_.at("lm_head"), tensors_.at("final_norm_gamma").f32, tensors_.at("final_norm_beta").f32, nullptr, d_mega_ln_ + (size_t)m_.n_layer * per);
+    fold(tensors_.at("lm_head"), tensors_.at("final_norm_beta").f32, nullptr, d_mega_ln_ + (size_t)m_.n_layer * per);
     ESP_CUDA_TRY(cudaGetLastError());
     return ESP_CUDA_OK;
 }

@@ -222,7 +222,7 @@ private:
     MegaPlan mega_plan_{};
     uint8_t* d_pack_ = nullptr;
     float* d_norms_ = nullptr;
-    float2* d_mega_ln_ = nullptr;   // GPT-2: folded LayerNorm constants (MegaArgs::ln)
+    float* d_mega_ln_ = nullptr;    // GPT-2: constants of the rows behind a LayerNorm (MegaArgs::ln)
     float* d_mega_bias_ = nullptr;  // GPT-2: biases of Wo and W2
     unsigned long long* d_mega_arena_ = nullptr;  // exchange words and counted sums of the persistent kernel
     size_t mega_arena_words_ = 0;

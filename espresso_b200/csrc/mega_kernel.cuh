@@ -108,10 +108,10 @@ struct MegaArgs {
     const uint8_t* pack;      // [n_cta][cta_bytes]
     const float* norms;       // [2*L + 1][d_model]: norm1(l), norm2(l), ..., final
     const uint16_t* tok_emb;  // fp16 [vocab][d_model]
-    // GPT-2 only.  LayerNorm is folded into the products: W.(x g) is accumulated while x arrives, and a row's result is
-    // inv (sum - mean W.g) + (W.b + bias); the two constants of every row are computed once.
+    // GPT-2 only.  The products run on the centred rows (x - mean) g; a row's result is inv sum + (W.b + bias), and the
+    // constant of every row is computed once.
     const uint16_t* pos_emb;  // fp16 [max_seq][d_model]
-    const float2* ln;         // per layer [q_dim + 2 kv_dim + hidden], then [vocab] for the head: {W.g, W.b + bias}
+    const float* ln;          // per layer [q_dim + 2 kv_dim + hidden], then [vocab] for the head: W.b + bias
     const float* out_bias;    // per layer [bias of Wo, bias of W2], d_model each
     const float2* rope;       // [max_seq][head_dim/2]
     KvLayout kv;
@@ -573,20 +573,21 @@ __device__ __forceinline__ float mega_block_sum(float v, float* red) {
     return (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) + (((c.x + c.y) + (c.z + c.w)) + ((e.x + e.y) + (e.z + e.w)));
 }
 
-// The same for two floats (GPT-2: sum and sum of squares).
-__device__ __forceinline__ float2 mega_block_sum2(float v0, float v1, float* red) {
+// The sum of v0 and the maximum of v1 >= 0 (GPT-2).
+__device__ __forceinline__ float2 mega_block_sum_max(float v0, float v1, float* red) {
+    v1 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v1)));  // (non-negative floats order as their bits)
     v0 = warp_sum(v0);
-    v1 = warp_sum(v1);
     if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = v0; red[kMegaConsumerWarps + (threadIdx.x >> 5)] = v1; }
     consumer_sync();
     const float4* r4 = reinterpret_cast<const float4*>(red);
-    float out[2];
+    float2 t = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int q = 0; q < 2; q++) {
-        const float4 a = r4[4 * q], b = r4[4 * q + 1], c = r4[4 * q + 2], e = r4[4 * q + 3];
-        out[q] = (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) + (((c.x + c.y) + (c.z + c.w)) + ((e.x + e.y) + (e.z + e.w)));
+    for (int q = 0; q < kMegaConsumerWarps / 4; q++) {
+        const float4 x = r4[q], y = r4[kMegaConsumerWarps / 4 + q];
+        t.x += (x.x + x.y) + (x.z + x.w);
+        t.y = fmaxf(t.y, fmaxf(fmaxf(y.x, y.y), fmaxf(y.z, y.w)));
     }
-    return make_float2(out[0], out[1]);
+    return t;
 }
 
 // ------------------------------------------------------------------------------------------------ products
@@ -1168,14 +1169,13 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
     // Stages values of the residual stream: raw copy, gained copy as the products' staged operand (fp16 hi/lo parts, or
     // int8 digits for the quantised types; `K` = length of the vector being staged), sum of squares.
     constexpr bool kQuant = WT == WT_Q8_0;  // int8 digit staging (Q4_0 widens its nibbles to fp16 and reads the fp16 staging)
-    auto stage_x = [&](float* raw, int K, bool digits, int k, float v, float g, float& ss, float& sm) {  // one element per lane, consecutive k
+    auto stage_x = [&](float* raw, int K, bool digits, int k, float v, float g, float& ss) {  // one element per lane, consecutive k
         raw[k] = v;
         if (kQuant && digits) qx_store_elem(s.xa, reinterpret_cast<float*>(s.xa + xa_bytes(K)), k, v * g);
         else xa_store(xa_h, k, v * g);
         ss = fmaf(v, v, ss);
-        if (GPT2) sm += v;
     };
-    auto stage_x2 = [&](float* raw, int K, bool digits, int k, float v0, float v1, float g0, float g1, float& ss, float& sm) {  // a pair per lane
+    auto stage_x2 = [&](float* raw, int K, bool digits, int k, float v0, float v1, float g0, float g1, float& ss) {  // a pair per lane
         raw[k] = v0; raw[k + 1] = v1;
         if (kQuant && digits) {
             qx_store_pair(s.xa, reinterpret_cast<float*>(s.xa + xa_bytes(K)), k, v0 * g0, v1 * g1);
@@ -1184,18 +1184,52 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
             xa_store(xa_h, k + 1, v1 * g1);
         }
         ss = fmaf(v0, v0, fmaf(v1, v1, ss));
-        if (GPT2) sm += v0 + v1;
     };
-    // Norm scale (and mean) from the staged vector's sums; one CTA barrier.
-    float mean = 0.f;
-    auto norm_scale = [&](float ss, float sm) {
-        if constexpr (GPT2) {
-            const float2 t = mega_block_sum2(sm, ss, s.red);
-            mean = t.x * inv_d;
-            return rsqrtf(fmaxf(fmaf(-mean, mean, t.y * inv_d), 0.f) + m.eps);
-        } else {
-            return rsqrtf(mega_block_sum(ss, s.red) * inv_d + m.eps);  // (a correctly rounded division and square root cost ~200 cycles here)
+    auto rms_scale = [&](float ss) { return rsqrtf(mega_block_sum(ss, s.red) * inv_d + m.eps); };  // (a correctly rounded division and square root cost ~200 cycles here)
+    // GPT-2's LayerNorm.  The values are staged only when the mean is known: with a mean far from zero both E[x^2] - mean^2 and
+    // W.(x g) - mean W.g cancel (one barrier less, but a stream of mean 32 and deviation 0.05 had no correct digit left).  The
+    // centred values carry a power of two that puts the largest of them near 32: the fp16 parts then neither saturate on a large
+    // residual stream nor lose their low half to subnormals on a small one.  Every thread normalises the pairs that it received.
+    // GPT-2 117M, 64 tokens: 10.88 ms with one pass over the values, 11.37 with two (25 barriers per token).
+    constexpr int kLnAhead = 2;  // gain pairs of a thread requested before the values arrive (d_model <= 2048: all)
+    struct LnGains { float2 g[kLnAhead]; };
+    auto ln_gains = [&](const float* gain) {
+        LnGains p2;
+#pragma unroll
+        for (int i = 0; i < kLnAhead; i++) {
+            const int k = 2 * (tid + i * kMegaConsumers);
+            p2.g[i] = k < d ? __ldg(reinterpret_cast<const float2*>(gain + k)) : make_float2(0.f, 0.f);
         }
+        return p2;
+    };
+    float ln_sum = 0.f, ln_top = 0.f;
+    auto ln_take = [&](float* raw, int k, float v0, float v1) {
+        *reinterpret_cast<float2*>(raw + k) = make_float2(v0, v1);
+        ln_sum += v0 + v1;
+        ln_top = fmaxf(ln_top, fmaxf(fabsf(v0), fabsf(v1)));
+    };
+    auto layer_norm = [&](const float* raw, const float* gain, const LnGains& ahead) {  // stages the vector, returns the factor of the products' sums
+        const float2 t = mega_block_sum_max(ln_sum, ln_top, s.red);
+        ln_sum = ln_top = 0.f;
+        const float mean = t.x * inv_d;
+        const unsigned e = min(__float_as_uint(t.y + fabsf(mean)) >> 23, 254u), f = min(258u - e, 253u);
+        const float up = __uint_as_float(f << 23);
+        float ss = 0.f;
+        auto pair = [&](int k, float2 g) {
+            const float2 x = *reinterpret_cast<const float2*>(raw + k);
+            const float v0 = x.x - mean, v1 = x.y - mean;
+            ss = fmaf(v0, v0, fmaf(v1, v1, ss));
+            xa_store(xa_h, k, v0 * up * g.x);
+            xa_store(xa_h, k + 1, v1 * up * g.y);
+        };
+#pragma unroll
+        for (int i = 0; i < kLnAhead; i++)
+            if (2 * (tid + i * kMegaConsumers) < d) pair(2 * (tid + i * kMegaConsumers), ahead.g[i]);
+        for (int k = 2 * (tid + kLnAhead * kMegaConsumers); k < d; k += 2 * kMegaConsumers) pair(k, __ldg(reinterpret_cast<const float2*>(gain + k)));
+        const float var = fmaf(mega_block_sum(ss, s.red + 2 * kMegaConsumerWarps), inv_d, m.eps);  // (its barrier also publishes the staged vector)
+        float r = rsqrtf(var);
+        r *= fmaf(-0.5f * var * r, r, 1.5f);  // one Newton step: rounding error only
+        return r * __uint_as_float((254u - f) << 23);
     };
     const int ln_rows = m.q_dim + 2 * m.kv_dim + m.hidden;  // rows of a layer whose input is normalised
     const bool head_digits = kQuant && p.wt_head != WT_F16;  // an fp16 head on quantised layers reads the fp16 staging
@@ -1281,19 +1315,25 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                     // ---- S1: x of this layer.  x_words is re-written by the W2 stage of this layer, which starts only
                     // after every CTA has published its activation, i.e. after every group CTA has read x here.
                     const float* gain = a.norms + (size_t)(2 * l) * d;
-                    float ss = 0.f, sm = 0.f;
-                    if (l == 0) {
-                        for (int k = tid; k < d; k += kMegaConsumers) {
-                            float v = __half2float(__ushort_as_half(emb_row[k]));
-                            if (GPT2) v += __half2float(__ushort_as_half(__ldg(a.pos_emb + (size_t)pos * d + k)));
-                            stage_x(s.xraw, d, true, k, v, __ldg(gain + k), ss, sm);
+                    float ss = 0.f;
+                    LnGains ahead;
+                    if (GPT2) ahead = ln_gains(gain);
+                    if (l == 0 && GPT2) {
+                        for (int k = 2 * tid; k < d; k += 2 * kMegaConsumers) {
+                            const __half2 te = *reinterpret_cast<const __half2*>(emb_row + k), pe = *reinterpret_cast<const __half2*>(a.pos_emb + (size_t)pos * d + k);
+                            ln_take(s.xraw, k, __low2float(te) + __low2float(pe), __high2float(te) + __high2float(pe));
                         }
+                    } else if (l == 0) {
+                        for (int k = tid; k < d; k += kMegaConsumers) stage_x(s.xraw, d, true, k, __half2float(__ushort_as_half(emb_row[k])), __ldg(gain + k), ss);
+                    } else if (GPT2) {
+                        mega_read_words(a, s, a.x_words, d, seq - 1, 5, nullptr, [&](int k, float v0, float v1, float, float) { ln_take(s.xraw, k, v0, v1); });
                     } else {
-                        mega_read_words(a, s, a.x_words, d, seq - 1, 5, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, true, k, v0, v1, g0, g1, ss, sm); });
+                        mega_read_words(a, s, a.x_words, d, seq - 1, 5, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, true, k, v0, v1, g0, g1, ss); });
                     }
                     FINE();
                     release_pending();  // the W2 chunk of the previous layer
-                    inv = norm_scale(ss, sm);
+                    if (GPT2) inv = layer_norm(s.xraw, gain, ahead);
+                    else inv = rms_scale(ss);
                     FINE();
                     stamp(step);
                     // q/k/v row pairs of this CTA, RoPE, words for the CTAs that share the KV head, KV-cache append.
@@ -1306,14 +1346,15 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                         // exchange words, cache rows) does not depend on the products: worked out before them, it is off
                         // the path between the last product and the words the other CTAs are waiting for.
                         int kind = 0, row0 = 0, row1 = 0, idx = 0;
-                        float2 cs = make_float2(1.f, 0.f), n0 = cs, n1 = cs;
+                        float2 cs = make_float2(1.f, 0.f);
+                        float n0 = 0.f, n1 = 0.f;
                         unsigned long long* dst = my_qkv;
                         __half* kv_row = nullptr;
                         if (tid < n_items) {
                             mega_s1_rows(m, p, w.kvh, w.s1_begin + i0 + tid, kind, row0, row1, idx);
                             if (!GPT2 && kind < 2) cs = s.rope[idx];
                             if (GPT2) {
-                                const float2* ln = a.ln + (size_t)l * ln_rows + (kind == 0 ? 0 : kind == 1 ? m.q_dim : m.q_dim + m.kv_dim);
+                                const float* ln = a.ln + (size_t)l * ln_rows + (kind == 0 ? 0 : kind == 1 ? m.q_dim : m.q_dim + m.kv_dim);
                                 n0 = __ldg(ln + row0);
                                 n1 = __ldg(ln + row1);
                             }
@@ -1326,8 +1367,8 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                             float v1 = row_sum(sums, 2 * n_items, 2 * p.s1_ipc, d >> 5, 2 * tid + 1);
                             float r0, r1;
                             if (GPT2) {
-                                r0 = fmaf(fmaf(-mean, n0.x, v0), inv, n0.y);
-                                r1 = fmaf(fmaf(-mean, n1.x, v1), inv, n1.y);
+                                r0 = fmaf(v0, inv, n0);
+                                r1 = fmaf(v1, inv, n1);
                             } else {
                                 v0 *= inv;
                                 v1 *= inv;
@@ -1399,12 +1440,19 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                     // token exchange does not start with a round trip to memory.
                     if (tid < p.n_cta) { unsigned long long keep; asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(keep) : "l"(a.cand_words + (size_t)tid * kMegaCandStride) : "memory"); }
                     const float* gain = a.norms + (size_t)(2 * l + 1) * d;
-                    float ss = 0.f, sm = 0.f;
+                    float ss = 0.f;
                     FINE();
-                    mega_read_sums(a, s, a.mid_sums, d, m.n_head, 7, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xmid, d, true, k, v0, v1, g0, g1, ss, sm); });
+                    LnGains ahead;
+                    if (GPT2) {
+                        ahead = ln_gains(gain);
+                        mega_read_sums(a, s, a.mid_sums, d, m.n_head, 7, nullptr, [&](int k, float v0, float v1, float, float) { ln_take(s.xmid, k, v0, v1); });
+                    } else {
+                        mega_read_sums(a, s, a.mid_sums, d, m.n_head, 7, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xmid, d, true, k, v0, v1, g0, g1, ss); });
+                    }
                     FINE();
                     release_pending();  // the Wo chunk (CTAs outside the head groups: the W2 chunk of the previous layer)
-                    inv = norm_scale(ss, sm);
+                    if (GPT2) inv = layer_norm(s.xmid, gain, ahead);
+                    else inv = rms_scale(ss);
                 }
                 stamp(step);
                 // (gate, up) row pairs of this CTA's hidden units, SiLU(gate) * up.  act_words is re-written one layer later,
@@ -1415,15 +1463,15 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                     const int n_items = min(group * p.s3a_ipc, w.h_n - j0), n_rows = kFfn * n_items, per = kFfn * p.s3a_ipc;
                     // (the first item of a thread: its word's address and constants are known before the products)
                     unsigned long long* const dst = a.act_words + (p.act_wpc ? (size_t)blockIdx.x * p.act_wpc : (size_t)w.h_begin) + j0;
-                    const float2* ln = GPT2 ? a.ln + (size_t)l * ln_rows + m.q_dim + 2 * m.kv_dim + w.h_begin + j0 : nullptr;
-                    float2 n0 = make_float2(0.f, 0.f);
+                    const float* ln = GPT2 ? a.ln + (size_t)l * ln_rows + m.q_dim + 2 * m.kv_dim + w.h_begin + j0 : nullptr;
+                    float n0 = 0.f;
                     if (GPT2 && tid < n_items) n0 = __ldg(ln + tid);
                     const float* sums = group_products(n_rows, per, d >> 5, s.xa, kFfn * (w.h_n - j0), 1);
                     each(n_items, [&](int j) {
                         float v;
                         if (GPT2) {
                             if (j >= kMegaConsumers) n0 = __ldg(ln + j);
-                            const float x = fmaf(fmaf(-mean, n0.x, row_sum(sums, n_rows, per, d >> 5, j)), inv, n0.y);
+                            const float x = fmaf(row_sum(sums, n_rows, per, d >> 5, j), inv, n0);
                             // gelu(x) = 0.5 x (1 + tanh(u)), tanh(u) = 1 - 2 / (1 + exp(2 u))
                             const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
                             v = 0.5f * x * (2.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * u)));
@@ -1510,24 +1558,33 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         if (tid == 0) __threadfence();
         float head_inv = 1.f;
         {
-            float ss = 0.f, sm = 0.f;
-            if (step == 0) {
-                for (int k = tid; k < d; k += kMegaConsumers) stage_x(s.xraw, d, head_digits, k, __ldcg(a.hidden_io + k), __ldg(fin_gain + k), ss, sm);
+            float ss = 0.f;
+            LnGains ahead;
+            if (GPT2) ahead = ln_gains(fin_gain);
+            if (step == 0 && GPT2) {
+                for (int k = 2 * tid; k < d; k += 2 * kMegaConsumers) {
+                    const float2 v = __ldcg(reinterpret_cast<const float2*>(a.hidden_io + k));
+                    ln_take(s.xraw, k, v.x, v.y);
+                }
+            } else if (step == 0) {
+                for (int k = tid; k < d; k += kMegaConsumers) stage_x(s.xraw, d, head_digits, k, __ldcg(a.hidden_io + k), __ldg(fin_gain + k), ss);
+            } else if (GPT2) {
+                mega_read_words(a, s, a.x_words, d, a.tag0 + (unsigned)(step * L), 9, nullptr, [&](int k, float v0, float v1, float, float) { ln_take(s.xraw, k, v0, v1); });
             } else {
-                mega_read_words(a, s, a.x_words, d, a.tag0 + (unsigned)(step * L), 9, fin_gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, head_digits, k, v0, v1, g0, g1, ss, sm); });
+                mega_read_words(a, s, a.x_words, d, a.tag0 + (unsigned)(step * L), 9, fin_gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, head_digits, k, v0, v1, g0, g1, ss); });
             }
             release_pending();  // the W2 chunk of the last layer
-            if (GPT2) head_inv = norm_scale(ss, sm);
+            if (GPT2) head_inv = layer_norm(s.xraw, fin_gain, ahead);
             else consumer_sync();  // the RMSNorm scale is positive: the arg-max does not need it
         }
         stamp(step);
         float best_v = -INFINITY;
         int best_i = 0x7fffffff;
-        const float2* head_ln = GPT2 ? a.ln + (size_t)L * ln_rows + w.v_begin : nullptr;
+        const float* head_ln = GPT2 ? a.ln + (size_t)L * ln_rows + w.v_begin : nullptr;
         for (int r0 = 0; r0 < w.v_n; r0 += group * p.head_rpc) {
             const int nrows = min(group * p.head_rpc, w.v_n - r0);
             FINE();
-            float2 n0 = make_float2(0.f, 0.f);
+            float n0 = 0.f;
             if (GPT2 && tid < nrows) n0 = __ldg(head_ln + r0 + tid);
             const float* sums = group_products(nrows, p.head_rpc, d >> 5, s.xa, w.v_n - r0, 2, true);
             // a thread keeps the best of its rows (ascending: '>' keeps the first maximum)
@@ -1535,7 +1592,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                 float v = row_sum(sums, nrows, p.head_rpc, d >> 5, r);
                 if (GPT2) {
                     if (r >= kMegaConsumers) n0 = __ldg(head_ln + r0 + r);
-                    v = fmaf(fmaf(-mean, n0.x, v), head_inv, n0.y);
+                    v = fmaf(v, head_inv, n0);
                 }
                 if (v > best_v) { best_v = v; best_i = w.v_begin + r0 + r; }
             });
@@ -1770,19 +1827,14 @@ __global__ void k_build_pack(PackSources src, MegaPlan p, ModelDims m, uint8_t* 
     }
 }
 
-// GPT-2: {W.g, W.b + bias} of every row of a matrix [rows][K] (see MegaArgs::ln).  One warp per row.
-__global__ void k_fold_norm(const uint16_t* w, int rows, int K, const float* g, const float* b, const float* bias, float2* out) {
+// GPT-2: W.b + bias of every row of a matrix [rows][K] (see MegaArgs::ln).  One warp per row.
+__global__ void k_fold_norm(const uint16_t* w, int rows, int K, const float* b, const float* bias, float* out) {
     const int r = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (r >= rows) return;
-    float sg = 0.f, sb = 0.f;
-    for (int k = lane; k < K; k += 32) {
-        const float v = __half2float(__ushort_as_half(w[(size_t)r * K + k]));
-        sg = fmaf(v, g[k], sg);
-        sb = fmaf(v, b[k], sb);
-    }
-    sg = warp_sum(sg);
+    float sb = 0.f;
+    for (int k = lane; k < K; k += 32) sb = fmaf(__half2float(__ushort_as_half(w[(size_t)r * K + k])), b[k], sb);
     sb = warp_sum(sb);
-    if (lane == 0) out[r] = make_float2(sg, sb + (bias ? bias[r] : 0.f));
+    if (lane == 0) out[r] = sb + (bias ? bias[r] : 0.f);
 }
 
 }  // namespace esp

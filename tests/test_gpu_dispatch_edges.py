@@ -186,3 +186,36 @@ def test_failed_prompt_leaves_nothing_to_decode(rt, oracle_lib):
     prompt = synthetic_prompt(cfg.vocab, 20)
     compare_greedy_stream(oracle_lib.Runtime(model), prompt, eng.generate(prompt, 6).tokens)
     eng.close()
+
+
+@pytest.mark.parametrize("d_head,offset,spike", [(64, 0.0, 0.0), (64, 32.0, 0.0), (64, 0.0, 30000.0), (1088, 32.0, 0.0)])
+def test_gpt2_stream_far_from_zero(rt, oracle_lib, d_head, offset, spike):
+    """GPT-2 in the persistent kernel on a residual stream whose mean is a thousand times its deviation, and on one whose largest
+    value times its gain is beyond fp16: the LayerNorm has to centre before it squares, and to scale before it rounds.  The stream
+    itself is fp32 on both sides: one rounding at 32 is 1e-4 of a deviation of 0.02, well inside the logit tolerances."""
+    from espresso_b200.model_config import tiny_gpt2
+    from espresso_b200.synthetic import synthetic_prompt, synthetic_tensor
+    from espresso_b200.weight_blob import tensor_shapes
+
+    n_head = 3 if d_head == 64 else 17  # 1088: some threads normalise two pairs
+    cfg = dataclasses.replace(tiny_gpt2(vocab=515, max_seq=48), nHead=n_head, nKVHead=n_head, headDim=64, dModel=64 * n_head, hiddenDim=256 * n_head)
+    eng, model = rt.DecodeEngine.empty(cfg), oracle_lib.Model(cfg.to_metadata())
+    for name, shape in tensor_shapes(cfg).items():
+        h = synthetic_tensor(cfg, name, shape, 1234).astype(np.float16)
+        if name == "embeddings/position":
+            h = (h.astype(np.float32) + offset).astype(np.float16)
+            h[:, 5] += np.float16(spike)
+        if spike and name.endswith("gamma"):
+            h[5] = 8.0
+        eng.load_tensor(name, "f16", h)
+        model.set_tensor(name, h.astype(np.float32))
+    eng.finalize()
+    prompt = synthetic_prompt(cfg.vocab, 9)
+    eng.prefill(prompt)
+    toks, _ = eng.decode(12)
+    assert eng.timings()["kernel_launches"] == 1
+    ora = oracle_lib.Runtime(model)
+    compare_greedy_stream(ora, prompt, toks[0])
+    assert ora.prefill(list(prompt) + [int(t) for t in toks[0][:-1]]) == 0
+    assert_logits_close(eng.logits(), ora.logits(), f"offset {offset} spike {spike}")
+    eng.close()
