@@ -1472,9 +1472,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
                         if (GPT2) {
                             if (j >= kMegaConsumers) n0 = __ldg(ln + j);
                             const float x = fmaf(row_sum(sums, n_rows, per, d >> 5, j), inv, n0);
-                            // gelu(x) = 0.5 x (1 + tanh(u)), tanh(u) = 1 - 2 / (1 + exp(2 u))
-                            const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-                            v = 0.5f * x * (2.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * u)));
+                            v = gelu_f(x);
                         } else {
                             const float g = row_sum(sums, n_rows, per, d >> 5, 2 * j) * inv;
                             const float u = row_sum(sums, n_rows, per, d >> 5, 2 * j + 1) * inv;

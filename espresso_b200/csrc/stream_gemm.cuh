@@ -233,6 +233,13 @@ __device__ __forceinline__ SgRowPre sg_row_prefetch(const SgArgs& a, int row, in
     return p;
 }
 
+// The activations of rows that are split into several 16-bit parts, as the single-row kernels compute them.  Not inlined: the
+// kernel's code size is a cost of its own (see k_gemm_stream), and these rows are few.
+__device__ __noinline__ float4 act_f4(float4 v, bool gelu) {
+    if (gelu) return make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
+    return make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
+}
+
 // What happens to complete sums: lane l of the calling warp holds v = four consecutive weight rows of batch row `row`
 // (lanes 0..15: half 0 of the tile, 16..31: half 1), first of them m0 of matrix gi; ok = false past the matrix' end (nothing is
 // stored; the warp's exchanges still take place).
@@ -280,14 +287,17 @@ __device__ __forceinline__ void sg_epilogue_row(const SgArgs& a, int row, float4
             }
         }
     } else if constexpr (EPI == SG_GELU) {
-        v = make_float4(gelu_fast(v.x), gelu_fast(v.y), gelu_fast(v.z), gelu_fast(v.w));
+        if (a.parts > 1) v = act_f4(v, true);
+        else v = make_float4(gelu_fast(v.x), gelu_fast(v.y), gelu_fast(v.z), gelu_fast(v.w));
         if (ok) store_parts4(a.out16, a.ld16, row, m0, v, a.parts, BF16);
         if (ok && dbg) *reinterpret_cast<float4*>(a.debug + m0) = v;
     } else if constexpr (EPI == SG_SWIGLU) {  // lanes 0..15 hold the gate values, 16..31 the up values of the same hidden units
         float4 u;
         u.x = __shfl_xor_sync(0xffffffffu, v.x, 16); u.y = __shfl_xor_sync(0xffffffffu, v.y, 16);
         u.z = __shfl_xor_sync(0xffffffffu, v.z, 16); u.w = __shfl_xor_sync(0xffffffffu, v.w, 16);
-        v = make_float4(silu_fast(v.x) * u.x, silu_fast(v.y) * u.y, silu_fast(v.z) * u.z, silu_fast(v.w) * u.w);
+        if (a.parts > 1) v = act_f4(v, false);
+        else v = make_float4(silu_fast(v.x), silu_fast(v.y), silu_fast(v.z), silu_fast(v.w));
+        v = make_float4(v.x * u.x, v.y * u.y, v.z * u.z, v.w * u.w);
         if (ok && lane < 16) {
             store_parts4(a.out16, a.ld16, row, m0, v, a.parts, BF16);
             if (dbg) *reinterpret_cast<float4*>(a.debug + m0) = v;

@@ -68,8 +68,9 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t 
         : "memory");
 }
 
-// Activations of the batched epilogue.  The results are rounded to 16 bits right away, so the exponential may be
-// the hardware approximation (relative error ~2^-21) instead of the exact tanhf of the single-row kernels.
+// Activations of epilogues whose results are rounded to one 16-bit part right away (2^-12 or 2^-9): the hardware
+// approximations of exponential and division may stand in for tanhf.  Error against 64 bits over [-3, 3], 2-norm relative:
+// silu 4.8e-8 and gelu 5.3e-8, with tanhf (silu_f, gelu_f) 3.8e-8 and 3.6e-8.  Rows of several parts take the latter.
 __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 __device__ __forceinline__ float gelu_fast(float x) {
     const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
