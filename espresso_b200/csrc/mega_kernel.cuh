@@ -380,15 +380,20 @@ __device__ __forceinline__ unsigned ld_acquire_cta_shared(const unsigned* p) {
 __device__ __forceinline__ void st_release_cta_shared(unsigned* p, unsigned v) {
     asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
 }
-// `landed` is the count the thread read last: the ring runs ahead, so most chunks are known to be there without a read
-// (the read and the warp barrier behind it took 3 % of the token time of the quantised models).
+// `landed` is the count the warp read last: the ring runs ahead, so most chunks are known to be there without a read
+// (the read and the warp barrier behind it took 3 % of the token time of the quantised models).  It is the same in every lane:
+// lane 0 polls and hands its count to the others, so that a wait which gives up leaves the warp together, whatever each
+// lane would have seen of the count and of the abort flag.  The shuffle and the barrier order the lanes' reads of the chunk.
 __device__ __forceinline__ const uint8_t* mega_acquire(const MegaArgs& a, const MegaShared& s, const MegaCursor& c, unsigned index, unsigned& landed) {
     if ((int)(landed - index) <= 0) {
-        unsigned spins = 0;
-        while ((int)((landed = ld_acquire_cta_shared(s.landed)) - index) <= 0) {
-            if (mega_aborting(s) || mega_spin_out(a, s, spins, 3)) break;
+        if ((threadIdx.x & 31) == 0) {
+            unsigned spins = 0;
+            while ((int)((landed = ld_acquire_cta_shared(s.landed)) - index) <= 0) {
+                if (mega_aborting(s) || mega_spin_out(a, s, spins, 3)) break;
+            }
         }
         __syncwarp();
+        landed = __shfl_sync(0xffffffffu, landed, 0);
     }
     return s.slots + (size_t)c.slot * a.plan.slot_bytes;
 }
