@@ -1459,9 +1459,13 @@ int32_t Engine::decode_loop(int32_t n_seq, int32_t count, uint32_t* out_tokens, 
         h_visible_[s] = h_rows_block_[max_rows_ + s];
         most = std::max(most, n);
     }
-    // one copy for all sequences: `most` tokens of each (what lies behind a sequence's own count is unspecified)
-    if (most > 0 && out_tokens)
-        ESP_CUDA_TRY(cudaMemcpy2D(out_tokens, sizeof(uint32_t) * out_stride, rs_.out, sizeof(uint32_t) * out_stride_, sizeof(uint32_t) * most, n_seq, cudaMemcpyDeviceToHost));
+    // One device copy for all sequences, `most` tokens of each; the caller's rows receive their own counts only.
+    if (most > 0 && out_tokens) {
+        std::vector<uint32_t> all((size_t)most * n_seq);
+        ESP_CUDA_TRY(cudaMemcpy2D(all.data(), sizeof(uint32_t) * most, rs_.out, sizeof(uint32_t) * out_stride_, sizeof(uint32_t) * most, n_seq, cudaMemcpyDeviceToHost));
+        for (int s = 0; s < n_seq; s++)
+            memcpy(out_tokens + (size_t)s * out_stride, all.data() + (size_t)s * most, sizeof(uint32_t) * std::max(0, std::min(h_rows_block_[4 * max_rows_ + s], lim[s])));
+    }
     return ESP_CUDA_OK;
 }
 

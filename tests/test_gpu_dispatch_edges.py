@@ -219,3 +219,28 @@ def test_gpt2_stream_far_from_zero(rt, oracle_lib, d_head, offset, spike):
     assert ora.prefill(list(prompt) + [int(t) for t in toks[0][:-1]]) == 0
     assert_logits_close(eng.logits(), ora.logits(), f"offset {offset} spike {spike}")
     eng.close()
+
+
+def test_token_rows_receive_their_own_counts(rt, oracle_lib):
+    """Behind a sequence's own tokens the caller's buffer keeps what it held, for a batch whose sequences stop at different steps."""
+    import ctypes as C
+
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-own", 1, 4, 2, 128, 32, 256, 320, 64)
+    prompts = np.stack([synthetic_prompt(cfg.vocab, 6, stream=s) for s in range(3)])
+    eng, _ = dense_pair(rt, oracle_lib, cfg, "f16", 3)
+    free, _ = eng.generate_batch(prompts, 12)
+    eng.close()
+    # a stop token that ends the sequences at different steps
+    at = lambda t: [list(s).index(t) + 1 if t in s else 12 for s in free]
+    stop = next(int(t) for t in free[0] if len(set(at(t))) > 1)
+    cfg = dataclasses.replace(cfg, eosToken=stop)
+    eng, _ = dense_pair(rt, oracle_lib, cfg, "f16", 3)
+    eng.prefill_batch(prompts)
+    out, n = np.full((3, 12), 0xABCDEF01, np.uint32), np.zeros(3, np.int32)
+    rc = eng._lib.esp_cuda_decode(eng._h, 3, 12, out.ctypes.data_as(C.POINTER(C.c_uint32)), n.ctypes.data_as(C.POINTER(C.c_int32)), None)
+    assert rc == 0 and list(n) == at(stop)
+    for s in range(3):
+        assert np.array_equal(out[s, : n[s]], free[s][: n[s]]) and np.all(out[s, n[s] :] == 0xABCDEF01)
+    eng.close()
