@@ -76,7 +76,8 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
     const __half* K = p.kv.k + p.kv.offset(m, p.layer, seq, kvh, 0);
     const __half* V = p.kv.v + p.kv.offset(m, p.layer, seq, kvh, 0);
 
-    // keys base + g and base + g + 8: this lane's 16-byte piece of every 32 dimensions
+    // keys base + g and base + g + 8: this lane's 16-byte piece of every 32 dimensions.  (Coherent loads: the product before this
+    // kernel appends to the cache while the kernel is already resident.)
     uint4 kr[2][KB];
     auto load_k = [&](int base) {
 #pragma unroll
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
 #pragma unroll
             for (int kb = 0; kb < KB; kb++) {
                 kr[i][kb] = make_uint4(0, 0, 0, 0);
-                if (key < visible) kr[i][kb] = __ldg(reinterpret_cast<const uint4*>(K + (size_t)key * HD + kb * 32 + t * 8));
+                if (key < visible) kr[i][kb] = __ldca(reinterpret_cast<const uint4*>(K + (size_t)key * HD + kb * 32 + t * 8));
             }
         }
     };
@@ -100,12 +101,12 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
             for (int w = 0; w < kVw; w++) vr[i][w] = 0u;
             if (key < visible) {
                 if constexpr (kVw == 2) {
-                    const uint2 x = __ldg(reinterpret_cast<const uint2*>(src));
+                    const uint2 x = __ldca(reinterpret_cast<const uint2*>(src));
                     vr[i][0] = x.x; vr[i][1] = x.y;
                 } else {
 #pragma unroll
                     for (int w = 0; w < kVw; w += 4) {
-                        const uint4 x = __ldg(reinterpret_cast<const uint4*>(src) + w / 4);
+                        const uint4 x = __ldca(reinterpret_cast<const uint4*>(src) + w / 4);
                         vr[i][w] = x.x; vr[i][w + 1] = x.y; vr[i][w + 2] = x.z; vr[i][w + 3] = x.w;
                     }
                 }
