@@ -13,8 +13,10 @@
 //
 // Roles (576 threads): warp 0 TMA, warp 1 MMA (in the pair's first CTA), warps 2..17 epilogue.  Barriers: `full` of the first
 // CTA counts the bytes of both CTAs' copies; `empty` and `acc_full` are arrived in both CTAs by one commit; `acc_empty` of the
-// first CTA collects the epilogue warps of both.  Every wait is bounded (error code 7).
+// first CTA collects the epilogue warps of both.  Every wait is bounded (error code 7); after one that ran out, nobody leaves
+// before the copies and MMAs in flight are done (`done` and `peer` barriers, pair_drain.h).
 #pragma once
+#include "pair_drain.h"
 #include "stream_gemm.cuh"
 
 namespace esp {
@@ -87,6 +89,23 @@ __device__ __forceinline__ void commit_pair(uint64_t* bar) {
 }
 __device__ __forceinline__ void arrive_first_cta(uint64_t* bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(smem_u32(bar), 0)) : "memory");
+}
+
+// Bounded wait that does not give up early because of a recorded error: what it waits for arrives within microseconds.
+__device__ __forceinline__ bool pg_wait_quiet(uint64_t* bar, unsigned parity) {
+    for (unsigned spins = 0; spins < (1u << 20); spins++) {
+        unsigned ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(smem_u32(bar)), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+        __nanosleep(100);
+    }
+    return false;
+}
+__device__ __forceinline__ void mbar_complete_tx(uint64_t* bar, unsigned bytes) {
+    asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
 // What a warp's epilogue works on: 32 batch rows (TMEM lanes) from nrow0, of which `live` are written.
@@ -220,8 +239,9 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
                                                              const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x,
                                                              const __grid_constant__ PgArgs a) {
     extern __shared__ __align__(1024) uint8_t pg_smem[];
-    __shared__ uint64_t s_full[kPgStages], s_empty[kPgStages], s_acc_full[2], s_acc_empty[2];
+    __shared__ uint64_t s_full[kPgStages], s_empty[kPgStages], s_acc_full[2], s_acc_empty[2], s_done, s_peer;
     __shared__ uint32_t s_tmem;
+    __shared__ int s_peer_fills, s_consumed;  // first CTA: fills its peer has issued, fills the MMAs have waited for
     uint8_t* const tiles = reinterpret_cast<uint8_t*>(((uintptr_t)pg_smem + 1023) & ~(uintptr_t)1023);
     float* const stage_area = reinterpret_cast<float*>(tiles + (size_t)kPgStages * kPgStageBytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -239,6 +259,8 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
     if (threadIdx.x == 0) {
         for (int s = 0; s < kPgStages; s++) { mbar_init(s_full + s, 1); mbar_init(s_empty + s, 1); }
         for (int i = 0; i < 2; i++) { mbar_init(s_acc_full + i, 1); mbar_init(s_acc_empty + i, 2 * kPgEpiWarps); }
+        mbar_init(&s_done, 1);
+        mbar_init(&s_peer, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {
@@ -259,6 +281,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
         int s = 0;
         uint32_t phase = 0;
         bool first_round = true, ok = true;
+        int fills = 0;
         for (int unit = pair; unit < n_units && ok; unit += n_pairs) {
             const int slice = unit / n_tiles, tile = unit - slice * n_tiles, kb0 = slice * a.kb_per_split, num_kb = min(a.kb_per_split, all_kb - kb0);
             const int tw = tile / a.tiles_n, n0 = (tile - tw * a.tiles_n) * kPgRows + rank * 128;
@@ -274,7 +297,29 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
                     tma_load_pair(sx + kPgXBytes, map, (kb0 + kb) * kTcBlockK, m0, s_full + s);
                 }
                 __syncwarp();
+                fills++;
                 if (++s == kPgStages) { s = 0; phase ^= 1u; first_round = false; }
+            }
+        }
+        __syncwarp();
+        if (rank == 1) {
+            if (lane == 0) {
+                asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(mapa(smem_u32(&s_peer_fills), 0)), "r"(fills) : "memory");
+                arrive_first_cta(&s_peer);
+            }
+        } else {
+            asm volatile("bar.sync 3, 64;" ::: "memory");  // the MMA warp has recorded what it consumed
+            if (lane == 0 && pg_wait_quiet(&s_peer, 0)) {
+                const int peer = s_peer_fills;
+                if (s_consumed < pg_drain_end(fills, peer)) {  // a wait gave up: copies may be in flight that nobody waited for
+#pragma unroll 1
+                    for (int f = pg_drain_begin(fills, peer, kPgStages); f < pg_drain_end(fills, peer); f++) {
+                        const PgDrainStep d = pg_drain_step(f, fills, peer, kPgStages, kPgStageBytes);
+                        if (d.expect) mbar_expect_tx(s_full + d.stage, d.expect);
+                        if (d.complete) mbar_complete_tx(s_full + d.stage, d.complete);
+                        pg_wait_quiet(s_full + d.stage, d.parity);
+                    }
+                }
             }
         }
     } else if (warp == 1) {
@@ -285,7 +330,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
             int s = 0;
             uint32_t phase = 0;
             bool ok = true;
-            int it = 0;
+            int it = 0, consumed = 0;
             for (int unit = pair; unit < n_units && ok; unit += n_pairs, it++) {
                 const int num_kb = min(a.kb_per_split, all_kb - unit / n_tiles * a.kb_per_split);
                 const int buf = it & 1;
@@ -310,13 +355,20 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
                     }
                     __syncwarp();
                     accumulate = 1;
+                    consumed++;
                     s = s_next;
                     phase = phase_next;
                 }
                 if (ok && elect_one()) commit_pair(s_acc_full + buf);
                 __syncwarp();
             }
+            __syncwarp();
+            if (lane == 0) s_consumed = consumed;
+            if (elect_one()) commit_pair(&s_done);
+            __syncwarp();
+            asm volatile("bar.sync 3, 64;" ::: "memory");
         }
+        if (lane == 0) pg_wait_quiet(&s_done, 0);  // every MMA of the pair has read its operands, every commit before has arrived
     } else {
         // ---------------- epilogue: TMEM -> registers -> staging -> global ----------------
         const int ew = warp - 2, quad = warp & 3, sub = ew >> 2;  // lanes 32 * quad.. of TMEM; which quarter of the columns
@@ -349,9 +401,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
             if (lane == 0) arrive_first_cta(s_acc_empty + buf);
         }
     }
-    // nobody leaves while the pair's copies, commits or arrivals may still reach this CTA (after a wait that gave up, copies
-    // may be in flight without anyone waiting for them: they land within microseconds)
-    if (__ldcg(a.error) != 0) __nanosleep(200000);
+    // nobody leaves while the pair's copies, commits or arrivals may still reach this CTA
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
