@@ -289,14 +289,19 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
             half_of(tw, rank, gi, m0);
             const CUtensorMap* const map = gi == 0 ? &map_w0 : gi == 1 ? &map_w1 : &map_w2;
             for (int kb = 0; kb < num_kb; kb++) {
-                if (!first_round && !tc_wait(s_empty + s, phase ^ 1u, a.error)) { ok = false; break; }
-                if (elect_one()) {
+                const bool gave_up = !first_round && !tc_wait(s_empty + s, phase ^ 1u, a.error);  // (per lane: the votes below end the loop for all)
+                const bool issued = elect_one() && !gave_up;
+                if (issued) {
                     uint8_t* const sx = tiles + (size_t)s * kPgStageBytes;
                     if (rank == 0) mbar_expect_tx(s_full + s, 2 * kPgStageBytes);
                     tma_load_pair(sx, &map_x, (kb0 + kb) * kTcBlockK, n0, s_full + s);
                     tma_load_pair(sx + kPgXBytes, map, (kb0 + kb) * kTcBlockK, m0, s_full + s);
                 }
-                __syncwarp();
+                if (__any_sync(0xffffffffu, gave_up)) {
+                    fills += __any_sync(0xffffffffu, issued) ? 1 : 0;
+                    ok = false;
+                    break;
+                }
                 fills++;
                 if (++s == kPgStages) { s = 0; phase ^= 1u; first_round = false; }
             }
@@ -334,26 +339,26 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
             for (int unit = pair; unit < n_units && ok; unit += n_pairs, it++) {
                 const int num_kb = min(a.kb_per_split, all_kb - unit / n_tiles * a.kb_per_split);
                 const int buf = it & 1;
-                if (it >= 2 && !tc_wait(s_acc_empty + buf, ((it >> 1) - 1) & 1, a.error)) break;
+                if (it >= 2 && !tc_wait_warp(s_acc_empty + buf, ((it >> 1) - 1) & 1, a.error)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem + (uint32_t)buf * 256u;
                 uint32_t accumulate = 0;
                 bool ready = mbar_try_wait(s_full + s, phase);
                 for (int kb = 0; kb < num_kb; kb++) {
-                    if (!ready && !tc_wait(s_full + s, phase, a.error)) { ok = false; break; }
+                    const bool gave_up = !ready && !tc_wait(s_full + s, phase, a.error);  // (per lane: the vote below ends the loop for all)
                     const bool wrap = s + 1 == kPgStages;
                     const int s_next = wrap ? 0 : s + 1;
                     const uint32_t phase_next = phase ^ (wrap ? 1u : 0u);
                     ready = kb + 1 < num_kb && mbar_try_wait(s_full + s_next, phase_next);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (elect_one()) {
+                    if (elect_one() && !gave_up) {
                         const uint64_t da = d_first + (uint64_t)(s * (kPgStageBytes >> 4)), db = da + (kPgXBytes >> 4);
                         umma_pair(acc, da, db, idesc, accumulate);
 #pragma unroll
                         for (int k = 1; k < kTcBlockK / 16; k++) umma_pair(acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, 1u);
                         commit_pair(s_empty + s);
                     }
-                    __syncwarp();
+                    if (__any_sync(0xffffffffu, gave_up)) { ok = false; break; }
                     accumulate = 1;
                     consumed++;
                     s = s_next;
@@ -387,7 +392,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
                 w.pos = __ldcg(a.rs.pos + row);
                 w.kv_row = a.kv.offset(a.m, a.layer, __ldcg(a.rs.seq + row), 0, w.pos);
             }
-            if (!tc_wait(s_acc_full + buf, (it >> 1) & 1, a.error)) break;
+            if (!tc_wait_warp(s_acc_full + buf, (it >> 1) & 1, a.error)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             w.base = tmem + (uint32_t)buf * 256u + ((uint32_t)(32 * quad) << 16);
             if (w.live) {

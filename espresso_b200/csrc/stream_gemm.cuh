@@ -535,19 +535,19 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
         uint64_t da = d_first;
         bool ready = mbar_test(full0, 0);
         for (int kb = 0; kb < num_kb; kb++) {
-            if (!ready && !tc_wait(s_full + s, phase, a.error)) break;
+            const bool gave_up = !ready && !tc_wait(s_full + s, phase, a.error);  // (per lane: the vote below ends the loop for all)
             const bool wrap = (int)s + 1 == stages;
             const uint32_t s_next = wrap ? 0 : s + 1, phase_next = phase ^ (wrap ? 1u : 0u);
             ready = kb + 1 < num_kb && mbar_test(full0 + 8 * s_next, phase_next);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (elect_one()) {
+            if (elect_one() && !gave_up) {
                 const uint64_t db = da + (kSgWBytes >> 4);
                 umma_f16(acc, da, db, idesc, accumulate);
 #pragma unroll
                 for (int k = 1; k < kTcBlockK / 16; k++) umma_f16(acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, 1u);
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty0 + 8 * s) : "memory");
             }
-            __syncwarp();
+            if (__any_sync(0xffffffffu, gave_up)) break;
             accumulate = 1;
             s = s_next;
             phase = phase_next;
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
                 phase ^= 1u;
                 if (kb >= stages) {
                     if (norm) sg_norm_gains(a, pre_x, k0, lane);
-                    if (!tc_wait(s_empty + xw, phase ^ 1u, a.error)) break;
+                    if (!tc_wait_warp(s_empty + xw, phase ^ 1u, a.error)) break;
                     if (elect_one()) load_w(kb, xw);
                 }
                 if (!norm) {

@@ -60,6 +60,10 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, unsigned parity, int* err
     return true;
 }
 
+// The same with one answer for a whole warp, for loops whose next instructions are warp-wide (elect, tcgen05.ld, warp barriers):
+// lanes that poll on their own can end apart when a wait runs out, and those still in the loop would wait for the others for good.
+__device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, unsigned parity, int* error) { return __all_sync(0xffffffffu, tc_wait(bar, parity, error)); }
+
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
