@@ -61,7 +61,7 @@ __global__ void k_add_rows(float* dst, const float* src, int n4) {
 }
 SgPlan sg_plan(int w_tiles, int rows, int kb, int parts, bool may_split, int sms);
 cudaError_t sg_launch(const SgPlan& plan, int epilogue, const CUtensorMap* const* mw, const CUtensorMap& mx, SgArgs a, cudaStream_t s);
-constexpr int kTcMinRows = 9;  // below this the row-batched GEMV stages are used
+constexpr int kTcMinRows = 9;  // a shorter prompt pass runs the decode attention
 // Rows of a prompt pass on the batched path.  Every pass streams all the weights once and is a chain of ~8 dependent
 // launches per layer, so few wide passes win: 256 GPT-2 prompts of 64 tokens took 32 passes of 512 rows at 0.74 ms, nearly
 // all of it launch latency; the wide models are bound by their products from 512 rows on and gain from fewer re-reads.
@@ -832,10 +832,10 @@ int32_t Engine::check_ready(const char* what) const {
 // One pass over the model for `rows` rows.  mode: STEP_FORWARD runs the layers on (tok, pos) of every active
 // row; STEP_HEAD runs final norm + LM head + argmax; STEP_FEEDBACK makes the head emit and feed back its token.
 int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
-    switch (path_of(rows, mode)) {
+    switch (path_of(rows)) {
         case PATH_REFUSED: return fail(ESP_CUDA_ERR_STATE, "tensor parallelism needs tensor-core operands: one storage type and 64-aligned shard sizes");
         case PATH_STREAM: return launch_step_stream(rows, mode, s, profile);
-        case PATH_PAIRS: return launch_step_wide(rows, mode, s);
+        case PATH_TILES: return launch_step_wide(rows, mode, s);
         case PATH_ROWWISE: break;
     }
     const bool gpt2 = m_.arch == ARCH_GPT2;
@@ -933,7 +933,7 @@ int32_t Engine::launch_step(int rows, int mode, cudaStream_t s, bool profile) {
 
 int32_t Engine::submit(int rows, int mode) {
     if (force_failure_enabled()) return fail(ESP_CUDA_ERR_FORCED_FAILURE, "forced failure is enabled");
-    if (tc_ready_ && !tc_operands_ready_ && path_of(rows, mode) != PATH_ROWWISE) {
+    if (tc_ready_ && !tc_operands_ready_ && path_of(rows) != PATH_ROWWISE) {
         int32_t rc = tc_operands();  // before any capture: it allocates
         if (rc) return rc;
     }
@@ -1727,9 +1727,9 @@ int32_t Engine::build_tc() {
     tc_quant_ = quantised;
     tc_mats_ = mats;
     tc_operands_ready_ = false;
-    // 16-bit matrices get their TMA maps now.  A quantised model's fp16 expansion (what batches and prefill chunks
-    // multiply by) is built by the first step that takes the batched path: an engine that only ever decodes one
-    // sequence through the persistent kernel, which streams the GGUF blocks themselves, never allocates it.
+    // 16-bit matrices get their TMA maps now.  A quantised model's fp16 expansion (what passes of two
+    // or more rows multiply by) is built by the first of them: an engine that is only ever fed and decoded token by token through the
+    // persistent kernel, which streams the GGUF blocks themselves, never allocates it.
     if (!quantised) {
         int32_t rc0 = tc_operands();
         if (rc0) return rc0;
@@ -1742,7 +1742,7 @@ int32_t Engine::build_tc() {
     if ((rc = dev_alloc(owned_, &kraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &vraw_, (size_t)max_rows_ * m_.kv_dim))) return rc;
     if ((rc = dev_alloc(owned_, &d_tc_error_, 4))) return rc;
-    if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, std::max(sg_decode_rows(m_.d_model), sg_prompt_rows(m_.d_model))) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
+    if ((rc = dev_alloc(owned_, &row_stat_, (size_t)std::min(max_rows_, sg_rows(m_.d_model)) * ((m_.d_model + kSgRows - 1) / kSgRows)))) return rc;
     if (tp_size_ > 1 && (rc = dev_alloc(owned_, &tp_partial_, (size_t)max_rows_ * m_.d_model))) return rc;
     ESP_CUDA_TRY(cudaDeviceSynchronize());
     tc_ready_ = true;
@@ -1816,7 +1816,7 @@ int32_t Engine::launch_attention_decode(const DecodeAttArgs& a, int rows, cudaSt
     return ESP_CUDA_OK;
 }
 
-StepPath Engine::path_of(int rows, int mode) const { return step_path(tc_ready_, tc_quant_, tp_size_, m_.d_model, rows, (mode & STEP_TILED_ATT) != 0); }
+StepPath Engine::path_of(int rows) const { return step_path(tc_ready_, tc_quant_, tp_size_, m_.d_model, rows); }
 
 int32_t Engine::launch_embed(int rows, float2* stat, cudaStream_t s) {
     const DeviceTensor& te = tensors_.at("embeddings/token");
@@ -2074,13 +2074,11 @@ int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
         if (dbg) { k_copy_debug<<<(n + 255) / 256, 256, 0, s>>>(src, dbg + offset, n); launches++; }
     };
     const bool att_ok_hd = hd == 32 || hd == 64 || hd == 128;
-    // q/k/v cannot be cut along K on the pairs (its epilogue needs whole sums).  Where its 256 x 256 tiles occupy less than half
-    // of the pairs and the streamed product's 128 x 64 tiles fit the chip at once (two per SM, some room left), the streamed
-    // product takes it: prompt passes at d2048 330 rows 2390 -> 2190 us, 401 2385 -> 2260, 768 2855 -> 2690.  With 288 tiles
-    // (1000 rows, 2304 x 768) it lost up to 6 %.
-    const int pair_tiles = (rows + kPgRows - 1) / kPgRows * ((q + 2 * kv + 255) / 256);
+    // q/k/v cannot be cut along K here (its epilogue needs whole sums) and has few tiles.  Where the streamed product's 128 x 64
+    // tiles fit the chip at once, two per SM, it is the faster one: us, streamed / tiles, 2560 x 2048: 300 rows 10.9 / 18.2, 832 rows
+    // (260 tiles) 14.2 / 18.4, 900 (300) 23.5 / 18.7; 6144 x 4096 384 rows (288) 25.0 / 29.6; 2304 x 768 1000 rows (288) 8.8 / 11.8.
     const int stream_tiles = (rows + kSgMaxCols - 1) / kSgMaxCols * ((q + 2 * kv + kSgRows - 1) / kSgRows);
-    const bool stream_qkv = q % kSgHalf == 0 && kv % kSgHalf == 0 && 4 * pair_tiles <= sm_count_ && 4 * stream_tiles <= 7 * sm_count_;
+    const bool stream_qkv = q % kSgHalf == 0 && kv % kSgHalf == 0 && stream_tiles <= 2 * sm_count_ - 8;
     int32_t rc;
     if (mode & STEP_FORWARD) {
         if ((rc = launch_embed(rows, nullptr, s))) return rc;

@@ -118,7 +118,7 @@ private:
     int32_t launch_prep(int rows, const float* src, int K, int norm, const float* g, const float* b, uint16_t* dst, int parts, cudaStream_t s);
     int32_t launch_attention_prefill(const PrefillAttArgs& pa, cudaStream_t s);
     int32_t launch_step_stream(int rows, int mode, cudaStream_t s, bool profile);  // few rows: streamed products, fused stages
-    StepPath path_of(int rows, int mode) const;
+    StepPath path_of(int rows) const;
     int32_t launch_attention_decode(const DecodeAttArgs& a, int rows, cudaStream_t s);
     int32_t build_tc();
     int32_t tc_operands();  // weight maps (and a quantised model's fp16 expansion), built on first use of the batched path
@@ -202,7 +202,7 @@ private:
     unsigned long long* tp_stats_ = nullptr;    // [4] local: count and device time of the peer-memory all-reduces
     int tp_parity_ = 0;                         // partial buffer of the next all-reduce (host side, fixed at graph capture)
 
-    // batched tensor-core path (rows >= kTcMinRows, 16-bit weights)
+    // batched tensor-core paths (16-bit weights, or the fp16 expansion of a quantised model from two rows on)
     bool tc_ready_ = false;
     bool tc_operands_ready_ = false;
     std::vector<std::string> tc_mats_;

@@ -1,9 +1,16 @@
-// Products of prompt passes with more rows than the streamed products take: Y[n][m] = sum_k W[m][k] * X[n][k] on pairs of SMs.
+// Products of passes with more rows than the streamed products take: Y[n][m] = sum_k W[m][k] * X[n][k] on pairs of SMs, or on
+// single SMs where a pair's tile would be half empty.
 //
-// Bound: the tensor pipe.  A single SM's 128 x 256 tile needs 48 KB of operands per 64-wide K block, 96 bytes per cycle at
-// the pipe's rate of 512 cycles per block, more than an SM can pull out of L2 (about 64): such a kernel stood at 0.6 of the
-// pipe.  tcgen05.mma.cta_group::2 multiplies a 256 x 256 tile with the operands of two SMs: each loads 128 batch rows and
+// Bound: the tensor pipe; below a few hundred rows HBM and what comes before the first and after the last K block of a tile.
+// A single SM's 128 x 256 tile needs 48 KB of operands per 64-wide K block, 96 bytes per cycle at the pipe's rate of 512 cycles
+// per block, more than an SM can pull out of L2 (about 64).  tcgen05.mma.cta_group::2 multiplies a 256 x 256 tile with the operands of two SMs: each loads 128 batch rows and
 // 128 weight rows per block, 64 bytes per cycle, and accumulates its 128 batch rows x 256 weight rows.
+// A pair's tile has 256 batch rows: with 257 to 384 the second one is mostly empty and costs as much as the first.  The same
+// kernel on a single SM (cta_group::1, 128 batch rows, both weight halves) pays 1.28 times per K block and row, and wins wherever
+// it saves a wave; which one is the host's choice per product (pg_shape).  300 rows, us, pairs / single: gate/up 2 x 5632 x 2048
+// 27.6 / 19.7, 2 x 14336 x 4096 91.0 / 85.4, 4096 x 14336 46.9 / 41.4; 224 rows of the second 57.9 / 64.1.  A single SM also requests
+// the weights of its first stages before it waits for the previous kernel (0.3 us); on pairs the test for that in the copy loop
+// costs more than it saves (27.6 -> 29.2 us).
 //
 // Persistent: one CTA per SM, tiles dealt out in turn (batch tiles fastest, so that the tiles in flight share weights in L2);
 // the accumulator is double-buffered (2 x 256 TMEM columns), the epilogue of a tile runs under the products of the next.
@@ -23,13 +30,16 @@ namespace esp {
 
 constexpr int kPgThreads = 576;
 constexpr int kPgEpiWarps = 16;
-constexpr int kPgRows = 256;         // batch rows of a tile (128 per CTA)
-constexpr int kPgStages = 5;
 constexpr int kPgXBytes = 128 * kTcBlockK * 2, kPgWBytes = 128 * kTcBlockK * 2;
-constexpr int kPgStageBytes = kPgXBytes + kPgWBytes;
-constexpr int kPgStageStride = 20;   // floats per staged row of 16 columns: 16-byte aligned, conflict-free
-constexpr int kPgEpiBytes = kPgEpiWarps * 32 * kPgStageStride * 4;
-constexpr size_t kPgSmemBytes = (size_t)kPgStages * kPgStageBytes + kPgEpiBytes + 1024;
+constexpr int kPgEpiBytes = kPgEpiWarps * 32 * 16 * 4;  // 16 columns per staged row
+// Tile of a pair (256 batch rows, 128 per CTA, a weight half per CTA) or of a single SM (128 batch rows, both weight halves)
+template <bool PAIR>
+struct PgTile {
+    static constexpr int kRows = PAIR ? 256 : 128;
+    static constexpr int kStages = PAIR ? 5 : 4;
+    static constexpr int kStageBytes = kPgXBytes + (PAIR ? 1 : 2) * kPgWBytes;  // of one CTA
+    static constexpr int kSmemBytes = kStages * kStageBytes + kPgEpiBytes + 1024;
+};
 
 enum PgEpilogue { PG_STORE = 0, PG_RESIDUAL = 1, PG_QKV = 2, PG_GELU = 3, PG_SWIGLU = 4 };
 
@@ -44,7 +54,7 @@ struct PgArgs {
     PgGroup g[3];
     int n_groups;
     int K, rows;
-    int tiles_n, tiles_w;  // batch tiles of 256 rows, weight tiles of two halves
+    int tiles_n, tiles_w;  // batch tiles of 256 (pair) or 128 rows, weight tiles of two halves
     int epilogue, bf16;
     uint16_t* out16;       // PG_GELU / PG_SWIGLU: [n][ld16]
     int ld16;
@@ -87,6 +97,16 @@ __device__ __forceinline__ void commit_pair(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3)
                  : "memory");
 }
+template <bool PAIR>
+__device__ __forceinline__ void pg_mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (PAIR) umma_pair(tmem_d, da, db, idesc, accumulate);
+    else umma_f16(tmem_d, da, db, idesc, accumulate);
+}
+template <bool PAIR>
+__device__ __forceinline__ void pg_commit(uint64_t* bar) {
+    if constexpr (PAIR) commit_pair(bar);
+    else asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void arrive_first_cta(uint64_t* bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa(smem_u32(bar), 0)) : "memory");
 }
@@ -119,6 +139,10 @@ struct PgWarp {
     int pos;
 };
 
+// Staged rows are 64 bytes, two to a line of banks: XORing the 16-byte chunk with the row's line number makes both the row-wise
+// stores and the reads of four lanes per row conflict-free.
+__device__ __forceinline__ int pg_swizzle(int row) { return ((row >> 1) & 3) << 2; }
+
 // The 32 x 16 block in the staging rows (weight rows m0.. of matrix gi) to memory: four lanes x four columns per batch row,
 // eight rows per step.
 template <int EPI>
@@ -143,7 +167,7 @@ __device__ __forceinline__ void pg_store_block(const PgArgs& a, const PgWarp& w,
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int r = 8 * i + rr;
-        float4 v = *reinterpret_cast<const float4*>(w.stg + r * kPgStageStride + c);
+        float4 v = *reinterpret_cast<const float4*>(w.stg + r * 16 + (c ^ pg_swizzle(r)));
         size_t at = 0;
         if (EPI == PG_QKV) at = __shfl_sync(0xffffffffu, w.kv_row, r);
         if (!ok || !((w.live >> r) & 1u)) continue;
@@ -176,10 +200,11 @@ __device__ __forceinline__ void pg_store_block(const PgArgs& a, const PgWarp& w,
 }
 
 __device__ __forceinline__ void pg_to_staging(const PgWarp& w, const uint32_t (&v)[16]) {
-    float* const mine = w.stg + w.lane * kPgStageStride;
+    float* const mine = w.stg + w.lane * 16;
+    const int sw = pg_swizzle(w.lane);
     __syncwarp();  // the block staged before has been read
 #pragma unroll
-    for (int i = 0; i < 4; i++) reinterpret_cast<uint4*>(mine)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    for (int i = 0; i < 4; i++) *reinterpret_cast<uint4*>(mine + ((4 * i) ^ sw)) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
     __syncwarp();
 }
 
@@ -234,18 +259,21 @@ __device__ __forceinline__ void pg_epilogue(const PgArgs& a, const PgWarp& w, in
     }
 }
 
-// grid = up to one CTA per SM (an even number), cluster = 2.
+// grid = up to one CTA per SM; PAIR: an even number, cluster = 2.  Single SM: the CTA is the first and only one of its "pair".
+template <bool PAIR>
 __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                                                              const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x,
                                                              const __grid_constant__ PgArgs a) {
     extern __shared__ __align__(1024) uint8_t pg_smem[];
+    using T = PgTile<PAIR>;
+    constexpr int kPgStages = T::kStages, kPgStageBytes = T::kStageBytes, kPgRows = T::kRows;
     __shared__ uint64_t s_full[kPgStages], s_empty[kPgStages], s_acc_full[2], s_acc_empty[2], s_done, s_peer;
     __shared__ uint32_t s_tmem;
     __shared__ int s_peer_fills, s_consumed;  // first CTA: fills its peer has issued, fills the MMAs have waited for
     uint8_t* const tiles = reinterpret_cast<uint8_t*>(((uintptr_t)pg_smem + 1023) & ~(uintptr_t)1023);
     float* const stage_area = reinterpret_cast<float*>(tiles + (size_t)kPgStages * kPgStageBytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = (int)blockIdx.x & 1, pair = (int)blockIdx.x >> 1, n_pairs = (int)gridDim.x >> 1;
+    const int rank = PAIR ? (int)blockIdx.x & 1 : 0, pair = PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x, n_pairs = PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
     const int n_tiles = a.tiles_n * a.tiles_w, n_units = n_tiles * a.splits, all_kb = a.K / kTcBlockK;  // a unit: one K slice of a tile, slices slowest
     // (matrix, first row) of a 128-row half; past the last matrix the rows load as zeros
     auto half_of = [&](int tile_w, int h, int& gi, int& m0) {
@@ -258,26 +286,65 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
     };
     if (threadIdx.x == 0) {
         for (int s = 0; s < kPgStages; s++) { mbar_init(s_full + s, 1); mbar_init(s_empty + s, 1); }
-        for (int i = 0; i < 2; i++) { mbar_init(s_acc_full + i, 1); mbar_init(s_acc_empty + i, 2 * kPgEpiWarps); }
+        for (int i = 0; i < 2; i++) { mbar_init(s_acc_full + i, 1); mbar_init(s_acc_empty + i, (PAIR ? 2 : 1) * kPgEpiWarps); }
         mbar_init(&s_done, 1);
         mbar_init(&s_peer, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    cluster_arrive();  // both CTAs' barriers are initialised and their tensor memory is allocated before either is used
-    cluster_wait();
+    if constexpr (PAIR) {  // both CTAs' barriers are initialised and their tensor memory is allocated before either is used
+        cluster_arrive();
+        cluster_wait();
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // Weights do not depend on the previous kernel: those of the first stages are requested before the wait for it.
+    const CUtensorMap *map0 = &map_w0, *map1 = &map_w0;  // this CTA's weight halves of the unit being loaded (PAIR: the first only)
+    int m0 = 0, m1 = 0;
+    auto weights_of = [&](int tw) {
+        int gi;
+        half_of(tw, rank, gi, m0);
+        map0 = gi == 0 ? &map_w0 : gi == 1 ? &map_w1 : &map_w2;
+        if constexpr (!PAIR) {
+            half_of(tw, 1, gi, m1);
+            map1 = gi == 0 ? &map_w0 : gi == 1 ? &map_w1 : &map_w2;
+        }
+    };
+    auto load_weights = [&](int k, int s) {
+        uint8_t* const sw = tiles + (size_t)s * kPgStageBytes + kPgXBytes;
+        if (rank == 0) mbar_expect_tx(s_full + s, (PAIR ? 2 : 1) * kPgStageBytes);
+        if constexpr (PAIR) {
+            tma_load_pair(sw, map0, k, m0, s_full + s);
+        } else {
+            tma_load_2d(sw, map0, k, m0, s_full + s);
+            tma_load_2d(sw + kPgWBytes, map1, k, m1, s_full + s);
+        }
+    };
+    int ahead = 0;  // fills whose weights have been requested
+    if (!PAIR && warp == 0) {
+        const int slice = pair / n_tiles, kb0 = slice * a.kb_per_split;
+        weights_of((pair - slice * n_tiles) / a.tiles_n);
+        ahead = min(kPgStages, min(a.kb_per_split, all_kb - kb0));
+        for (int s = 0; s < ahead; s++) {
+            if (elect_one()) load_weights((kb0 + s) * kTcBlockK, s);
+            __syncwarp();
+        }
+    }
     pdl_launch_dependents();
     pdl_wait();
     const uint32_t tmem = s_tmem;
 
     if (warp == 0) {
-        // ---------------- TMA producer: this CTA's 128 batch rows and its weight half ----------------
+        // ---------------- TMA producer: this CTA's 128 batch rows and its weight halves ----------------
         int s = 0;
         uint32_t phase = 0;
         bool first_round = true, ok = true;
@@ -285,17 +352,15 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
         for (int unit = pair; unit < n_units && ok; unit += n_pairs) {
             const int slice = unit / n_tiles, tile = unit - slice * n_tiles, kb0 = slice * a.kb_per_split, num_kb = min(a.kb_per_split, all_kb - kb0);
             const int tw = tile / a.tiles_n, n0 = (tile - tw * a.tiles_n) * kPgRows + rank * 128;
-            int gi, m0;
-            half_of(tw, rank, gi, m0);
-            const CUtensorMap* const map = gi == 0 ? &map_w0 : gi == 1 ? &map_w1 : &map_w2;
+            weights_of(tw);
             for (int kb = 0; kb < num_kb; kb++) {
                 const bool gave_up = !first_round && !tc_wait(s_empty + s, phase ^ 1u, a.error);  // (per lane: the votes below end the loop for all)
                 const bool issued = elect_one() && !gave_up;
                 if (issued) {
-                    uint8_t* const sx = tiles + (size_t)s * kPgStageBytes;
-                    if (rank == 0) mbar_expect_tx(s_full + s, 2 * kPgStageBytes);
-                    tma_load_pair(sx, &map_x, (kb0 + kb) * kTcBlockK, n0, s_full + s);
-                    tma_load_pair(sx + kPgXBytes, map, (kb0 + kb) * kTcBlockK, m0, s_full + s);
+                    const int k = (kb0 + kb) * kTcBlockK;
+                    if (PAIR || fills >= ahead) load_weights(k, s);
+                    if constexpr (PAIR) tma_load_pair(tiles + (size_t)s * kPgStageBytes, &map_x, k, n0, s_full + s);
+                    else tma_load_2d(tiles + (size_t)s * kPgStageBytes, &map_x, k, n0, s_full + s);
                 }
                 if (__any_sync(0xffffffffu, gave_up)) {
                     fills += __any_sync(0xffffffffu, issued) ? 1 : 0;
@@ -314,8 +379,8 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
             }
         } else {
             asm volatile("bar.sync 3, 64;" ::: "memory");  // the MMA warp has recorded what it consumed
-            if (lane == 0 && pg_wait_quiet(&s_peer, 0)) {
-                const int peer = s_peer_fills;
+            if (lane == 0 && (!PAIR || pg_wait_quiet(&s_peer, 0))) {
+                const int peer = PAIR ? s_peer_fills : fills;
                 if (s_consumed < pg_drain_end(fills, peer)) {  // a wait gave up: copies may be in flight that nobody waited for
 #pragma unroll 1
                     for (int f = pg_drain_begin(fills, peer, kPgStages); f < pg_drain_end(fills, peer); f++) {
@@ -330,7 +395,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
     } else if (warp == 1) {
         // ---------------- MMA issuer of the pair ----------------
         if (rank == 0) {
-            const uint32_t idesc = umma_idesc_f16(256, 256, a.bf16);
+            const uint32_t idesc = umma_idesc_f16(T::kRows, 256, a.bf16);
             const uint64_t d_first = umma_smem_desc_sw128(tiles);
             int s = 0;
             uint32_t phase = 0;
@@ -353,10 +418,10 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (elect_one() && !gave_up) {
                         const uint64_t da = d_first + (uint64_t)(s * (kPgStageBytes >> 4)), db = da + (kPgXBytes >> 4);
-                        umma_pair(acc, da, db, idesc, accumulate);
+                        pg_mma<PAIR>(acc, da, db, idesc, accumulate);
 #pragma unroll
-                        for (int k = 1; k < kTcBlockK / 16; k++) umma_pair(acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, 1u);
-                        commit_pair(s_empty + s);
+                        for (int k = 1; k < kTcBlockK / 16; k++) pg_mma<PAIR>(acc, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, 1u);
+                        pg_commit<PAIR>(s_empty + s);
                     }
                     if (__any_sync(0xffffffffu, gave_up)) { ok = false; break; }
                     accumulate = 1;
@@ -364,12 +429,12 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
                     s = s_next;
                     phase = phase_next;
                 }
-                if (ok && elect_one()) commit_pair(s_acc_full + buf);
+                if (ok && elect_one()) pg_commit<PAIR>(s_acc_full + buf);
                 __syncwarp();
             }
             __syncwarp();
             if (lane == 0) s_consumed = consumed;
-            if (elect_one()) commit_pair(&s_done);
+            if (elect_one()) pg_commit<PAIR>(&s_done);
             __syncwarp();
             asm volatile("bar.sync 3, 64;" ::: "memory");
         }
@@ -378,7 +443,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
         // ---------------- epilogue: TMEM -> registers -> staging -> global ----------------
         const int ew = warp - 2, quad = warp & 3, sub = ew >> 2;  // lanes 32 * quad.. of TMEM; which quarter of the columns
         PgWarp w{};
-        w.stg = stage_area + (size_t)ew * 32 * kPgStageStride;
+        w.stg = stage_area + (size_t)ew * 32 * 16;
         w.lane = lane; w.sub = sub;
         int it = 0;
         for (int unit = pair; unit < n_units; unit += n_pairs, it++) {
@@ -403,18 +468,24 @@ __global__ void __launch_bounds__(kPgThreads, 1) k_gemm_pair(const __grid_consta
                 else pg_epilogue<PG_SWIGLU>(a, w, tw, half_of);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            if (lane == 0) arrive_first_cta(s_acc_empty + buf);
+            if (lane == 0) {
+                if constexpr (PAIR) arrive_first_cta(s_acc_empty + buf);
+                else mbar_arrive(s_acc_empty + buf);
+            }
         }
     }
     // nobody leaves while the pair's copies, commits or arrivals may still reach this CTA
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    cluster_arrive();
-    cluster_wait();
+    if constexpr (PAIR) {
+        cluster_arrive();
+        cluster_wait();
+    }
     if (warp == 2) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
 }
 

@@ -1,4 +1,4 @@
-// Products of up to 256 activation rows with a 16-bit weight matrix, for decode steps and short prompt passes:
+// Products of few activation rows (up to 704, see step_path.h) with a 16-bit weight matrix, for decode steps and short prompts:
 // Y[n][m] = sum_k W[m][k] * X[n][k] on tcgen05/TMEM, with everything the decode path does to a finished row of Y (bias,
 // RoPE and cache append, residual, activation, arg-max) in the epilogue.
 //

@@ -53,9 +53,11 @@ SgPlan sg_plan(int w_tiles, int rows, int kb, int parts, bool may_split, int sms
     p.n_cols = parts > 1 ? (parts == 2 ? 16 : 32) : std::min((rows + 15) / 16 * 16, kSgMaxCols);
     p.col_tiles = parts > 1 ? 1 : (rows + p.n_cols - 1) / p.n_cols;
     p.row_tiles = w_tiles;
-    // (several column tiles re-read the weights out of L2: 256 rows x 2304 x 768 takes 7.1 us in 144 CTAs, 7.7 in 216)
-    const int limit = p.col_tiles > 1 ? sms * 4 / 3 : sms * 9 / 5;
-    int want = may_split ? std::max(1, std::min(kSgMaxSplits, limit / std::max(1, w_tiles * p.col_tiles))) : 1;
+    const int tiles = std::max(1, w_tiles * p.col_tiles);
+    int want = may_split ? std::max(1, std::min(kSgMaxSplits, sms * 9 / 5 / tiles)) : 1;
+    // Pairs of CTAs find a place on nearly every SM, larger clusters do not: us per launch, with one slice less / this many: 20 x 6
+    // tiles in 2 slices (240 CTAs) 14.1 / 11.5, 16 x 4 in 4 (256) 9.6 / 9.4, 24 x 6 in 2 (288) 10.4 / 9.2, 16 x 6 in 3 (288) 11.7 / 16.7.
+    if (may_split && want == 1 && tiles <= sms - 4) want = 2;
     want = std::min(want, std::max(1, kb / 2));
     p.kb_per_split = (kb + want - 1) / want;
     p.splits = (kb + p.kb_per_split - 1) / p.kb_per_split;
@@ -107,6 +109,30 @@ cudaError_t sg_launch(const SgPlan& plan, int epilogue, const CUtensorMap* const
     return cudaLaunchKernelEx(&cfg, a.bf16 ? k_gemm_stream<true> : k_gemm_stream<false>, *mw[0], *mw[1], *mw[2], mx, a);
 }
 
+// Launch shape of a product on tiles: of SM pairs or of single SMs.
+struct PgShape { bool pair; int tiles_n, splits, kb_per_split, units; float cost; };
+// The work of the busiest SM or pair in K blocks of a pair (about 0.28 us); K slices of a residual product are the ones that make
+// it least, a sliced unit's epilogue and its atomics counted as 8 blocks.
+static PgShape pg_shape_of(bool pair, int rows, int tiles_w, int kb, bool may_split, int sms) {
+    PgShape p{};
+    p.pair = pair;
+    p.tiles_n = (rows + (pair ? 255 : 127)) / (pair ? 256 : 128);
+    const int tiles = p.tiles_n * tiles_w, lanes = pair ? sms / 2 : sms;
+    p.cost = 1e30f;
+    for (int want = 1; want <= (may_split ? 8 : 1); want++) {
+        const int per = (kb + want - 1) / want, n = (kb + per - 1) / per;
+        const float cost = (float)((tiles * n + lanes - 1) / lanes) * (float)(per + (n > 1 ? 8 : 0));
+        if (cost < p.cost) { p.cost = cost; p.splits = n; p.kb_per_split = per; p.units = tiles * n; }
+    }
+    return p;
+}
+static PgShape pg_shape(int rows, int tiles_w, int kb, bool may_split, int sms) {
+    const PgShape pair = pg_shape_of(true, rows, tiles_w, kb, may_split, sms), single = pg_shape_of(false, rows, tiles_w, kb, may_split, sms);
+    // Fitted to the times of twelve shapes at 33 to 2048 rows (2 x 14336 x 4096: pairs 22 + 17.8 us a wave, single SMs 18 + 23.1; 2 x
+    // 5632 x 2048: 10 + 9.3, 8 + 12): the better one of the two, or within 3 % of it, except for 4096 x 4096 at 1600 rows (12 %).
+    return single.cost * 1.28f < pair.cost + 7.f ? single : pair;
+}
+
 // mw: 128-row maps of the group's matrices (unused slots repeat slot 0); mx: map of the operand rows with 128-row boxes.
 cudaError_t pg_launch(const CUtensorMap* const* mw, const CUtensorMap& mx, PgArgs a, int sms, cudaStream_t s) {
     static std::mutex mu;
@@ -116,8 +142,10 @@ cudaError_t pg_launch(const CUtensorMap* const* mw, const CUtensorMap& mx, PgArg
     {
         std::lock_guard<std::mutex> lock(mu);
         if (dev >= 0 && dev < 64 && !configured[dev]) {
-            cudaError_t e = cudaFuncSetAttribute(k_gemm_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPgSmemBytes);
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_pair, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+            cudaError_t e = cudaFuncSetAttribute(k_gemm_pair<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PgTile<true>::kSmemBytes);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_pair<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PgTile<false>::kSmemBytes);
+            for (auto k : {k_gemm_pair<true>, k_gemm_pair<false>})
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
             if (e != cudaSuccess) return e;
             configured[dev] = true;
         }
@@ -126,24 +154,15 @@ cudaError_t pg_launch(const CUtensorMap* const* mw, const CUtensorMap& mx, PgArg
     const int groups = a.epilogue == PG_SWIGLU ? 1 : a.n_groups;
     for (int g = 0; g < groups; g++) { a.g[g].half0 = halves; halves += (a.g[g].M + 127) / 128; }
     a.tiles_w = a.epilogue == PG_SWIGLU ? halves : (halves + 1) / 2;
-    a.tiles_n = (a.rows + kPgRows - 1) / kPgRows;
-    // K slices of a residual product: the fewest k blocks on the busiest pair (about 0.27 us each), a unit's epilogue and its
-    // atomics counted as 8 blocks.  401 rows x 5632 x 2048: 16 tiles on 74 pairs, one slice 46 us.
-    const int tiles = a.tiles_n * a.tiles_w, kb = a.K / kTcBlockK, pairs = sms / 2;
-    a.splits = 1;
-    a.kb_per_split = kb;
-    if (a.epilogue == PG_RESIDUAL) {
-        int best = 1 << 30;
-        for (int want = 1; want <= 8; want++) {
-            const int per = (kb + want - 1) / want, n = (kb + per - 1) / per;
-            const int cost = (tiles * n + pairs - 1) / pairs * (per + (n > 1 ? 8 : 0));
-            if (cost < best) { best = cost; a.splits = n; a.kb_per_split = per; }
-        }
-    }
+    const int kb = a.K / kTcBlockK;
+    const PgShape shape = pg_shape(a.rows, a.tiles_w, kb, a.epilogue == PG_RESIDUAL, sms);
+    a.tiles_n = shape.tiles_n;
+    a.splits = shape.splits;
+    a.kb_per_split = shape.kb_per_split;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * std::min(pairs, tiles * a.splits));
+    cfg.gridDim = dim3(shape.pair ? 2 * std::min(sms / 2, shape.units) : std::min(sms, shape.units));
     cfg.blockDim = dim3(kPgThreads);
-    cfg.dynamicSmemBytes = kPgSmemBytes;
+    cfg.dynamicSmemBytes = shape.pair ? PgTile<true>::kSmemBytes : PgTile<false>::kSmemBytes;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -151,8 +170,8 @@ cudaError_t pg_launch(const CUtensorMap* const* mw, const CUtensorMap& mx, PgArg
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, k_gemm_pair, *mw[0], *mw[1], *mw[2], mx, a);
+    cfg.numAttrs = shape.pair ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, shape.pair ? k_gemm_pair<true> : k_gemm_pair<false>, *mw[0], *mw[1], *mw[2], mx, a);
 }
 
 __global__ void k_f32_to_16(const float* src, int64_t n, uint16_t* dst, int bf16) {

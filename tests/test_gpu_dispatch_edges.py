@@ -244,3 +244,37 @@ def test_token_rows_receive_their_own_counts(rt, oracle_lib):
     for s in range(3):
         assert np.array_equal(out[s, : n[s]], free[s][: n[s]]) and np.all(out[s, n[s] :] == 0xABCDEF01)
     eng.close()
+
+
+@pytest.mark.parametrize("kind", ["f16", "bf16"])
+@pytest.mark.parametrize("rows", [193, 256, 257, 300, 385, 641])
+def test_prompt_rows_of_a_wider_model(rt, oracle_lib, kind, rows):
+    """d_model 1280: products on 128- and 256-row tiles from 193 rows on, with an almost empty last tile at 257, 385 and 641 rows; the
+    residual products are cut along K; hidden 1088 leaves a partial weight tile."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-tiles", 1, 20, 4, 1280, 64, 1088, 320, 700)
+    eng, model = dense_pair(rt, oracle_lib, cfg, kind)
+    prompt = synthetic_prompt(cfg.vocab, rows)
+    eng.prefill(prompt)
+    ora = oracle_lib.Runtime(model)
+    assert ora.prefill(prompt) == 0
+    tol = {} if kind == "f16" else {"abs_tol": BF16_ABS_TOL}
+    assert_logits_close(eng.logits(), ora.logits(), f"{kind} {rows} rows", **tol)
+    eng.close()
+
+
+@pytest.mark.parametrize("n_head,head_dim", [(66, 32), (33, 64), (17, 128)])
+@pytest.mark.parametrize("rows", [321, 513])
+def test_query_key_value_product_on_tiles(rt, oracle_lib, n_head, head_dim, rows):
+    """q/k/v with more 128 x 64 tiles than the chip holds: on pairs at 321 rows, on single SMs at 513, RoPE across the columns of a tile."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-qkv-tiles", 1, n_head, n_head, n_head * head_dim, head_dim, 512, 320, 520)
+    eng, model = dense_pair(rt, oracle_lib, cfg)
+    prompt = synthetic_prompt(cfg.vocab, rows)
+    eng.prefill(prompt)
+    ora = oracle_lib.Runtime(model)
+    assert ora.prefill(prompt) == 0
+    assert_logits_close(eng.logits(), ora.logits(), f"head_dim {head_dim}, {rows} rows")
+    eng.close()
