@@ -484,7 +484,7 @@ int32_t Engine::init() {
     if ((rc = dev_alloc(owned_, &rs_.ticket, 4))) return rc;
     ESP_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&h_rows_block_), sizeof(int) * 6 * max_rows_));
     for (auto& slot : pass_slots_) {
-        ESP_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&slot.host), (sizeof(int) * 6 + sizeof(int4) * 2) * (size_t)max_rows_));
+        ESP_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&slot.host), sizeof(int) * slot_row_words(max_rows_) + sizeof(int4) * 2 * (size_t)max_rows_));
         ESP_CUDA_TRY(cudaEventCreateWithFlags(&slot.copied, cudaEventDisableTiming));
     }
     ESP_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&h_next_), sizeof(uint32_t) * max_rows_));
@@ -1104,7 +1104,7 @@ int32_t Engine::enqueue_pass(int rows, const int* seq, const uint32_t* tok, cons
     PassSlot& slot = pass_slots_[pass_slot_ ^= 1];
     ESP_CUDA_TRY(cudaEventSynchronize(slot.copied));
     int* h = slot.host;
-    int4* runs = reinterpret_cast<int4*>(h + (size_t)6 * max_rows_);
+    int4* runs = reinterpret_cast<int4*>(h + slot_row_words(max_rows_));
     int4* last = runs + max_rows_;
     int n_runs = 0;
     for (int r = 0; r < rows; r++) {

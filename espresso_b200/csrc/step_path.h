@@ -10,6 +10,10 @@ namespace esp {
 // 64 rows 478 / 545, 100 rows 663 / 552.
 constexpr int sg_rows(int d_model) { return d_model <= 1024 ? 704 : d_model <= 2048 ? 192 : 64; }
 
+// Words of a pinned pass slot in front of its int4 lists: six control words per row, rounded up to 16 bytes (an engine of an odd
+// number of sequences has an odd number of rows).
+constexpr unsigned long long slot_row_words(int max_rows) { return (6ull * (unsigned)max_rows + 3) / 4 * 4; }
+
 enum StepPath {
     PATH_ROWWISE,  // one kernel per stage on the stored weights, any row count
     PATH_STREAM,   // streamed products

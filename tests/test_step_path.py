@@ -10,6 +10,8 @@ MAIN = r"""
 #include <cstdio>
 #include "step_path.h"
 int main() {
+    for (int r = 1; r < 5000; r++)
+        if (esp::slot_row_words(r) % 4 || esp::slot_row_words(r) < 6ull * r) return 1;  // the lists behind it hold 16-byte elements
     int ready, quantised, tp, d, rows;
     while (scanf("%d %d %d %d %d", &ready, &quantised, &tp, &d, &rows) == 5) printf("%d\n", (int)esp::step_path(ready, quantised, tp, d, rows));
 }
