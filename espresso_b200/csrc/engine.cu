@@ -2209,89 +2209,13 @@ int32_t Engine::build_mega() {
     for (int l = 0; l < m_.n_layer; l++)
         for (const char* n : {"wq", "wk", "wv", "wo", "w1", "w2", "w3"})
             if (!(gpt2 && n[1] == '3') && type_of("layers/" + std::to_string(l) + "/" + n) != wt_layer) return ESP_CUDA_OK;
-    const bool quant = wt_layer != ESP_CUDA_F16 || wt_head != ESP_CUDA_F16;
-    if (quant && (m_.d_model % 256 || m_.hidden % 256)) return ESP_CUDA_OK;  // chunk sizes must stay multiples of 16 bytes
     int coop = 0, smem_max = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, cfg_.device);
     cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, cfg_.device);
     if (!coop) return ESP_CUDA_OK;
     MegaPlan p{};
-    // every CTA must own at least one FFN unit and one row of W2 (it then takes part in every all-to-all exchange)
-    const int P = std::min(sm_count_, std::min(m_.d_model, m_.hidden));
-    if (P < m_.n_head) return ESP_CUDA_OK;
-    p.n_cta = P;
-    p.qpk = m_.n_head / m_.n_kv_head;
-    p.group_items = (p.qpk + 2) * m_.head_dim / 2;
-    p.cph = std::max(1, std::min(std::min(P / m_.n_head, m_.d_model), p.group_items / p.qpk));
-    p.gsize = p.cph * p.qpk;
-    p.n_group_cta = p.cph * m_.n_head;
-    p.s1_max = (p.group_items + p.gsize - 1) / p.gsize;
-    p.rpb = (m_.d_model + p.cph - 1) / p.cph;
-    p.hpc_max = (m_.hidden + P - 1) / P;
-    p.dpc_max = (m_.d_model + P - 1) / P;
-    p.vpc_max = (m_.vocab + P - 1) / P;
-    // Exchange arrays: the activation vector gets cache lines per CTA when every reader can poll all of it in one round
-    // (four 16-byte loads per consumer thread); the layer output stays compact (see mega_kernel.cuh).
-    p.act_wpc = (p.hpc_max + kMegaLineWords - 1) / kMegaLineWords * kMegaLineWords;
-    if (P * ((p.hpc_max + 1) / 2) > 4 * kMegaConsumers) p.act_wpc = 0;
-    if (quant) p.act_wpc = 0;  // the int8 staging of Q8_0 works on whole blocks of consecutive elements (and the wide quantised models need two polling rounds anyway)
-    p.wt_layer = wt_layer;
-    p.wt_head = wt_head;
-    p.row_bytes = mega_row_bytes(wt_layer, m_.d_model);
-    p.down_row_bytes = mega_row_bytes(wt_layer, m_.hidden);
-    p.wo_row_bytes = mega_row_bytes(wt_layer, m_.head_dim);
-    p.head_row_bytes = mega_row_bytes(wt_head, m_.d_model);
-    // a quantised row of head_dim columns is 68 / 36 / ... bytes: chunks of the Wo stage must hold a multiple of `wo_rows`
-    // rows to stay multiples of 16 bytes
-    const int wo_rows = wt_layer == ESP_CUDA_F16 ? 1 : std::max(1, 8 / (m_.head_dim / 32));
-    if (p.rpb % wo_rows) return ESP_CUDA_OK;
-    p.s1_bytes = pad128((long long)2 * p.s1_max * p.row_bytes);
-    p.s2_bytes = pad128((long long)p.rpb * p.wo_row_bytes);
-    p.ffn_rows = gpt2 ? 1 : 2;
-    p.s3a_bytes = pad128((long long)p.ffn_rows * p.hpc_max * p.row_bytes);
-    p.s3b_bytes = pad128((long long)p.dpc_max * p.down_row_bytes);
-    p.layer_bytes = (long long)p.s1_bytes + p.s2_bytes + p.s3a_bytes + p.s3b_bytes;
-    p.head_bytes = pad128((long long)p.vpc_max * p.head_row_bytes);
-    p.cta_bytes = p.layer_bytes * m_.n_layer + p.head_bytes;
-    // ring slots of 48 KB (more when one item of a stage is larger); a stage slice travels as chunks of whole items,
-    // at most kMegaChunkRows rows each (the products of a chunk are spread over the warps as 8-row tiles)
-    const int item_max = std::max(2 * p.row_bytes, p.down_row_bytes);
-    p.slot_bytes = pad128(std::max(48 * 1024, item_max));
-    p.s1_ipc = std::max(1, std::min(std::min(p.s1_max, kMegaChunkRows / 2), p.slot_bytes / (2 * p.row_bytes)));
-    p.s3a_ipc = std::max(1, std::min(std::min(p.hpc_max, kMegaChunkRows / p.ffn_rows), p.slot_bytes / (p.ffn_rows * p.row_bytes)));
-    p.s3b_rpc = std::max(1, std::min(std::min(p.dpc_max, kMegaChunkRows), p.slot_bytes / p.down_row_bytes));
-    p.head_rpc = std::max(1, std::min(std::min(p.vpc_max, kMegaChunkRows), p.slot_bytes / p.head_row_bytes));
-    p.s2_rpc = std::max(1, std::min(std::min(p.rpb, kMegaChunkRows), p.slot_bytes / p.wo_row_bytes));
-    p.s2_rpc = std::max(wo_rows, p.s2_rpc / wo_rows * wo_rows);
-    p.s3b_kpc = 0;
-    if (wt_layer != ESP_CUDA_F16) {
-        // The products of a chunk are spread over the warps as 16-row tiles times a power of two of column ranges: where a stage
-        // takes several chunks, a chunk is 16, 32, 64, ... rows (22 of 32 rows busy, or 12 of 16 warps, cost 20 to 30 %).
-        auto whole_tiles = [](int rows, int all) {
-            if (rows >= all || rows < 16) return rows;
-            int r = 16;
-            while (2 * r <= rows) r *= 2;
-            return r;
-        };
-        p.s3a_ipc = std::max(1, whole_tiles(2 * p.s3a_ipc, 2 * p.hpc_max) / 2);
-        p.head_rpc = whole_tiles(p.head_rpc, p.vpc_max);
-        const int n_kb = m_.hidden / 32;
-        if (p.dpc_max > kMegaChunkRows) return ESP_CUDA_OK;
-        const int fit = p.slot_bytes / (p.dpc_max * mega_row_bytes(wt_layer, 32)) / 8 * 8, chunks = fit ? (n_kb + fit - 1) / fit : 0;
-        if (!chunks) return ESP_CUDA_OK;
-        p.s3b_kpc = std::min(fit, ((n_kb + chunks - 1) / chunks + 7) / 8 * 8);  // equal shares, in steps of 8 blocks (16-byte chunks)
-    }
-    // As many ring slots as fit; then the largest group of chunks per CTA barrier whose partial sums do not cost a slot.
-    p.n_slots = 0;
-    for (int ns = 8; ns >= 2 && p.n_slots == 0; ns--)
-        for (int group : {wt_layer == ESP_CUDA_F16 ? 1 : 4, wt_layer == ESP_CUDA_F16 ? 1 : 2, 1}) {
-            MegaPlan probe = p;
-            probe.n_slots = ns;
-            probe.group = group;
-            mega_layout(m_, probe);
-            if (probe.smem_bytes <= smem_max) { p = probe; break; }
-        }
-    if (p.n_slots == 0) return ESP_CUDA_OK;  // does not fit: the per-stage kernels serve this model
+    if (!mega_plan(m_, wt_layer, wt_head, sm_count_, smem_max, p)) return ESP_CUDA_OK;  // does not fit: the other kernels serve this model
+    const int P = p.n_cta;
     const void* kern = mega_kernel_for(m_.head_dim, wt_layer, gpt2);
     ESP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem_bytes));
     int occ = 0;
@@ -2305,7 +2229,7 @@ int32_t Engine::build_mega() {
     mega_arena_words_ = mega_arena_layout(m_, p, 1, nullptr);
     if ((rc = dev_alloc(owned_, &d_mega_arena_, mega_arena_words_))) return rc;
     if ((rc = dev_alloc(owned_, &d_mega_ctl_, 8))) return rc;
-    if ((rc = dev_alloc(owned_, &d_mega_trace_, (size_t)kMegaTraceLayer * m_.n_layer + kMegaTraceHead + 4 + 1024))) return rc;
+    if ((rc = dev_alloc(owned_, &d_mega_trace_, (size_t)kMegaTraceLayer * m_.n_layer + kMegaTraceHead))) return rc;
     if ((rc = dev_alloc(owned_, &d_token_times_, (size_t)m_.max_seq + 1))) return rc;
     ESP_CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&h_mega_ctl_), 8 * sizeof(unsigned long long)));
     // per-layer source matrices
@@ -2465,17 +2389,6 @@ static const void* spec_kernel_for(int head_dim) {
     return reinterpret_cast<const void*>(&k_spec_mega<32>);
 }
 
-int32_t Engine::ensure_norms2() {
-    if (d_norms2_) return ESP_CUDA_OK;
-    const size_t d = (size_t)m_.d_model, rows = (size_t)2 * m_.n_layer + 1;
-    int32_t rc;
-    if ((rc = dev_alloc(owned_, &d_norms2_, rows * 2 * d, false))) return rc;
-    for (int copy = 0; copy < 2; copy++)
-        ESP_CUDA_TRY(cudaMemcpy2DAsync(d_norms2_ + copy * d, 2 * d * sizeof(float), d_norms_, d * sizeof(float), d * sizeof(float), rows, cudaMemcpyDeviceToDevice, stream_));
-    ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
-    return ESP_CUDA_OK;
-}
-
 // The two-token kernel serves a target and a draft that are both fp16 Llama models on the persistent-kernel path, on one
 // device, with the same widths: they then share one plan (chunk sizes, work shares, ring) and differ in depth only.
 bool Engine::spec_compatible(const Engine& draft) const {
@@ -2489,8 +2402,9 @@ bool Engine::spec_compatible(const Engine& draft) const {
     if (x.d_model != y.d_model || x.n_head != y.n_head || x.n_kv_head != y.n_kv_head || x.head_dim != y.head_dim || x.hidden != y.hidden || x.vocab != y.vocab ||
         x.eps != y.eps || cfg_.rope_theta != draft.cfg_.rope_theta)
         return false;
-    return a.n_cta == b.n_cta && a.cph == b.cph && a.slot_bytes == b.slot_bytes && a.s1_ipc == b.s1_ipc && a.s2_rpc == b.s2_rpc && a.s3a_ipc == b.s3a_ipc &&
-           a.s3b_rpc == b.s3b_rpc && a.head_rpc == b.head_rpc && a.layer_bytes == b.layer_bytes;
+    for (int k = 0; k < 5; k++)
+        if (a.stage[k].group_rows != b.stage[k].group_rows || a.stage[k].chunk_units != b.stage[k].chunk_units) return false;
+    return a.n_cta == b.n_cta && a.cph == b.cph && a.slot_bytes == b.slot_bytes && a.layer_bytes == b.layer_bytes;
 }
 
 int32_t Engine::spec_prepare() {
@@ -2502,11 +2416,11 @@ int32_t Engine::spec_prepare() {
     for (int ns = mega_plan_.n_slots; ns >= 3; ns--) {  // a stage holds back one slot past its exchange: fewer than three would stall the ring
         MegaPlan probe = mega_plan_;
         probe.n_slots = ns;
-        spec_layout(m_, probe);
+        mega_layout(m_, probe, kSpecNP);
         if (probe.smem_bytes <= smem_max) { p = probe; break; }
     }
     if (p.n_slots == 0) return fail(ESP_CUDA_ERR_STATE, "two-token kernel: the model's working set does not fit shared memory");
-    if (kSpecNP * p.n_cta * ((p.hpc_max + 1) / 2) > 4 * kMegaConsumers) p.act_wpc = 0;  // two positions no longer fit one polling round
+    if (kSpecNP * m_.hidden > 4096) p.act_wpc = 0;  // two positions no longer fit one polling round
     const void* kern = spec_kernel_for(m_.head_dim);
     ESP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem_bytes));
     int occ = 0;
@@ -2534,7 +2448,6 @@ bool Engine::spec_verify_ok() const {
 int32_t Engine::run_spec_verify(uint32_t current, uint32_t proposed, uint32_t* exact_next, uint32_t* exact_future) {
     int32_t rc;
     if ((rc = spec_prepare())) return rc;
-    if ((rc = ensure_norms2())) return rc;
     const MegaPlan& p = spec_plan_;
     SpecArgs sa{};
     MegaArgs& a = sa.base;
@@ -2544,7 +2457,7 @@ int32_t Engine::run_spec_verify(uint32_t current, uint32_t proposed, uint32_t* e
     a.error = d_spec_result_ + 8;
     a.spin_limit = mega_spin_limit_;
     SpecModel& M = sa.model[1];
-    M.m = m_; M.pack = d_pack_; M.cta_bytes = mega_plan_.cta_bytes; M.norms2 = d_norms2_;
+    M.m = m_; M.pack = d_pack_; M.cta_bytes = mega_plan_.cta_bytes; M.norms = d_norms_;
     M.tok_emb = static_cast<const uint16_t*>(tensors_.at("embeddings/token").data);
     M.kv = kv_;
     sa.model[0] = M;
@@ -2579,8 +2492,6 @@ int32_t Engine::run_spec(Engine& draft, uint32_t prev, uint32_t current, int gen
     if (!spec_compatible(draft)) return fail(ESP_CUDA_ERR_STATE, "two-token kernel: draft and target do not share one plan");
     if (gen0 < 1 || eff <= gen0 || h_visible_[0] < 1 || h_visible_[0] + 1 >= max_seq) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "two-token kernel: nothing left to generate");
     if ((rc = spec_prepare())) return rc;
-    if ((rc = ensure_norms2())) return rc;
-    if ((rc = draft.ensure_norms2())) return rc;
     ESP_CUDA_TRY(cudaStreamSynchronize(draft.stream_));  // the draft's prefill ran on its own stream
     const MegaPlan& p = spec_plan_;
     SpecArgs sa{};
@@ -2596,7 +2507,7 @@ int32_t Engine::run_spec(Engine& draft, uint32_t prev, uint32_t current, int gen
         M.m = eng[i]->m_;
         M.pack = eng[i]->d_pack_;
         M.cta_bytes = eng[i]->mega_plan_.cta_bytes;
-        M.norms2 = eng[i]->d_norms2_;
+        M.norms = eng[i]->d_norms_;
         M.tok_emb = static_cast<const uint16_t*>(eng[i]->tensors_.at("embeddings/token").data);
         M.kv = eng[i]->kv_;
     }
@@ -2635,11 +2546,7 @@ int32_t Engine::stage_trace(int32_t cta, long long* out, int32_t capacity, int32
     if (!out || !n) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "stage_trace: null argument");
     *n = 0;
     if (!mega_ready_) return ESP_CUDA_OK;
-#ifdef MEGA_FINE_TRACE
-    const int count = 1000;
-#else
     const int count = kMegaTraceLayer * m_.n_layer + kMegaTraceHead;
-#endif
     if (capacity < count) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "stage_trace: capacity too small");
     ESP_CUDA_TRY(cudaSetDevice(cfg_.device));
     ESP_CUDA_TRY(cudaMemcpy(out, d_mega_trace_, sizeof(long long) * count, cudaMemcpyDeviceToHost));

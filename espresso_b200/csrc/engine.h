@@ -136,7 +136,6 @@ private:
     int32_t launch_mega(int n_steps, const uint32_t* feed, bool times);
     bool mega_usable() const;
     int32_t run_mega(int n_steps, int* emitted, float* device_ms, double* first_token_ms);
-    int32_t ensure_norms2();  // the gain vectors twice over, as the two-position kernel reads them
     int32_t spec_prepare();   // plan, arena and result block of the two-position kernel
     bool spec_verify_ok() const;  // verify2 can run as one launch of the two-position kernel
     int32_t run_spec_verify(uint32_t current, uint32_t proposed, uint32_t* exact_next, uint32_t* exact_future);
@@ -240,7 +239,6 @@ private:
     // two-token kernel (built on first use)
     bool spec_ready_ = false;
     MegaPlan spec_plan_{};
-    float* d_norms2_ = nullptr;
     unsigned long long* d_spec_arena_ = nullptr;
     size_t spec_arena_words_ = 0;
     uint32_t* d_spec_out_ = nullptr;   // [max_seq + 1] emitted tokens

@@ -2,7 +2,7 @@
 //
 // One cooperative launch runs an entire greedy decode loop: `n_steps` heads and up to `n_steps - 1` forward
 // passes.  The grid has one CTA per SM.  Inside a CTA one producer warp streams that CTA's weights from HBM into a
-// shared-memory ring with bulk async copies (cp.async.bulk + mbarrier), always running ahead of the sixteen
+// shared-memory ring with bulk async copies (cp.async.bulk + mbarrier), always running ahead of the eight
 // consumer warps (a watcher warp turns the copies' completions into a counter the consumers can read cheaply), so HBM keeps streaming while the consumers wait on the activation dependencies of the step.
 // Weights are re-laid out once ("pack") so that everything a CTA needs for one layer is contiguous.
 //
@@ -25,33 +25,38 @@
 //       vector -> this CTA's rows of W2 (+ residual) -> tagged words = the next layer's x
 // and the LM head streams the CTA's vocabulary rows through the same ring; every CTA publishes its best
 // (logit, index) as tagged words and every CTA reduces all of them, so the token is known everywhere at once.
+// Inside a CTA the columns of a stage's operand belong to the warps (MegaWorker): a warp awaits, stages and multiplies its own.
 // Products.  The fp16->fp32 conversion rate of the CUDA cores (measured: 20-26 weights per clock per SM from shared
 // memory) would make the row products the longest link of the chain, so they are issued as m16n8k16 tensor-core
 // instructions: sixteen weight rows are the A operand, and the fp32 activation vector, split exactly into two fp16
 // vectors (x = hi + lo, |error| <= 2^-22 |x|), occupies columns 0 and 1 of the B operand; the accumulators are fp32.  The
-// pack stores every chunk in the order the A fragments are read: for each block of 32 columns, for each row, 64 bytes.
+// pack stores every chunk in the order the A fragments are read.
 // GGUF Q8_0 / Q4_0 matrices travel through the ring as their blocks (32 or 16 bytes per row and block of 32 columns,
-// the fp16 scales behind them): 34/32 or 18/32 bytes per weight from HBM, never an fp16 copy.  A block of 32 columns
-// is exactly two m16n8k16 steps: the integers are widened to fp16 exactly in registers, the products of a block are
-// accumulated from zero and multiplied by the block's scale in fp32 (value = fp32(d) * q as in the GGUF definition).
-// Why single buffers suffice: each exchange is re-written only after an exchange of another kind that every
-// reader of the old contents must have passed (see the notes at each stage).
+// the fp16 scales behind them): 34/32 or 18/32 bytes per weight from HBM, never an fp16 copy; the activation becomes int8
+// digits (qx_store_quads) and a block one int8 m16n8k32 step, scaled in fp32 (value = fp32(d) * q as in the GGUF definition).
+// A warp's time per 16-row tile and block, weights in shared memory: 40 cycles per scheduler for Q8_0 and 56 for Q4_0 widened to
+// fp16, most of it shared-memory wavefronts (one per scale) and conversions.
+//
+// us per token (16 warps that staged and synchronised together, multiplying row tiles -> this): 6 layers d768 fp16 77.6 -> 64,
+// GPT-2 117M 169.5 -> 143, 22 layers d2048 Q8_0 482 -> 369, Q4_0 477 -> 388.
 // Every wait (mbarrier, tagged word, counted sum) is bounded: when a limit is hit the kernel records an error code,
 // stops waiting everywhere and runs to completion; the host reports a timeout.
 #pragma once
-#include <type_traits>
+#include <algorithm>
 
 #include "decode_kernels.cuh"
 
 namespace esp {
 
-constexpr int kMegaConsumerWarps = 16;
+constexpr int kMegaConsumerWarps = 8;
 constexpr int kMegaConsumers = kMegaConsumerWarps * 32;
 constexpr int kMegaThreads = kMegaConsumers + 64;  // + the producer warp and the watcher warp
 constexpr unsigned kMegaSpinLimit = 1u << 21;      // default attempts per wait before the kernel gives up (a few seconds)
 constexpr int kMegaTraceLayer = 10;                // stamps per layer
 constexpr int kMegaTraceHead = 4;                  // stamps of the head
-constexpr int kMegaChunkRows = 256;                // most rows of one chunk (16 tiles of 16 rows)
+constexpr int kMegaSlots = 4, kMegaSlotMax = 64 * 1024;  // ring slots and the most bytes of one (Q8_0, 22 layers of d2048: 4 slots of 44 KB 371 us per token, 5 of 35 KB 395, 7 of 25 KB 447)
+constexpr int kMegaRingMin = 96 * 1024;  // less than that is consumed faster than a refill takes to arrive
+constexpr int kMegaMaxTiles = 5;                   // 16-row tiles whose sums a warp keeps in registers
 // Which exchanges give every CTA cache lines of its own (see mega_read_lines) is the plan's choice (act_wpc > 0).
 // Measured on the 6-layer d768 model against compact arrays: arg-max candidates -4.6 us per token, activation vector
 // -1.4 us, layer output x +0.3 us (five words per CTA: three times as many lines to poll for little contention saved).
@@ -62,7 +67,16 @@ constexpr int kMegaCandStride = kMegaLineWords;  // 8-byte words between the arg
 constexpr float kMegaFix = 4294967296.0f;          // counted sums: fixed point with 32 fractional bits
 constexpr float kMegaUnfix = 2.3283064365386963e-10f;
 
+// Stages in the order a CTA takes them: q/k/v rows, rows of Wo (one head's columns), (gate, up) rows, rows of W2, vocabulary rows.
+enum MegaStageKind { MS_QKV = 0, MS_WO = 1, MS_UP = 2, MS_DOWN = 3, MS_HEAD = 4 };
+struct MegaStage {
+    int units;       // K units: 16 columns (fp16) or one block of 32 columns (quantised types)
+    int group_rows;  // rows of a chunk; except for Wo also the rows whose products run side by side (at most 16 kMegaMaxTiles)
+    int chunk_units; // consecutive units of a group's rows per chunk
+};
+
 struct MegaPlan {
+    float inv_d;      // 1 / d_model
     int n_cta;
     int cph;          // CTAs per query head (S2 row blocks of Wo)
     int qpk;          // query heads per KV head
@@ -74,29 +88,31 @@ struct MegaPlan {
     int hpc_max, dpc_max, vpc_max;  // largest number of FFN units / W2 rows / vocabulary rows of a CTA
     int act_wpc;  // exchange words reserved per CTA for its elements of the activation vector (whole cache lines); 0 = compact array
     int wt_layer, wt_head;  // storage type of the layer matrices and of the LM head: WT_F16, WT_Q8_0 or WT_Q4_0
-    int row_bytes;       // packed bytes of a row of d_model columns of a layer matrix
-    int down_row_bytes;  // ... of hidden columns (W2)
-    int wo_row_bytes;    // ... of head_dim columns (this head's part of a row of Wo)
-    int head_row_bytes;  // ... of d_model columns of the LM head
-    int s1_bytes, s2_bytes, s3a_bytes, s3b_bytes;  // packed bytes of a stage per layer (multiples of 128, sized for the largest CTA share)
-    // A stage whose slice is larger than a ring slot arrives in several chunks of whole items:
-    int group;        // chunks whose products share one CTA barrier (see group_products)
     int ffn_rows;     // packed rows per FFN unit: (gate, up) pairs 2, GPT-2's single up projection 1
-    int s1_ipc;       // S1 row pairs per chunk
-    int s2_rpc;       // S2 projection rows per chunk (a multiple of the rows one pass of the CTA covers)
-    int s3a_ipc;      // S3 (gate, up) pairs per chunk
-    int s3b_rpc;      // S3 down-projection rows per chunk (fp16)
-    int s3b_kpc;      // quantised types: blocks of 32 columns per chunk, all of the CTA's rows (a multiple of 8)
-    int head_rpc;     // LM-head rows per chunk
+    MegaStage stage[5];  // by MegaStageKind
+    int group_tiles;  // 16-row tiles of the largest group (partial sums are laid out for them)
+    int s1_bytes, s2_bytes, s3a_bytes, s3b_bytes;  // packed bytes of a stage per layer (multiples of 128, sized for the largest CTA share)
     int slot_bytes, n_slots;
     long long layer_bytes, head_bytes, cta_bytes;  // packed bytes per CTA: one layer, the head, everything
     int smem_bytes;
     // byte offsets of the shared-memory areas behind the ring (see MegaShared)
-    int off_bar, off_prev, off_key, off_xs, off_xraw, off_xmid, off_rope, off_qs, off_ctx, off_kn, off_vn, off_part, off_red, off_outv, off_flags, off_share, off_beg;
+    int off_bar, off_prev, off_key, off_xs, off_xq, off_xres, off_qs, off_ctx, off_kn, off_vn, off_part, off_red, off_ss, off_sums, off_flags, off_share, off_act, off_s1;
 };
 
-// Packed bytes of K columns of one row: fp16, or GGUF blocks of 32 (int8 / nibbles) with one fp16 scale each.
-__host__ __device__ inline int mega_row_bytes(int wt, int K) { return wt == WT_Q8_0 ? K + K / 16 : wt == WT_Q4_0 ? K / 2 + K / 16 : K * 2; }
+// K units of a storage type, and the packed bytes of one unit of `rows` rows: fp16 columns, or GGUF blocks (int8 / nibbles) and
+// one fp16 scale per row, the scales for whole tiles of sixteen rows.
+__host__ __device__ constexpr int mega_unit(int wt) { return wt == WT_F16 ? 16 : 32; }
+__host__ __device__ inline int mega_scale_bytes(int wt, int rows) { return wt == WT_F16 ? 0 : (rows + 15) / 16 * 32; }
+__host__ __device__ inline int mega_data_bytes(int wt, int rows) { return rows * (wt == WT_Q4_0 ? 16 : 32); }
+__host__ __device__ inline int mega_unit_bytes(int wt, int rows) { return mega_data_bytes(wt, rows) + mega_scale_bytes(wt, rows); }
+// Packed bytes of `rows` rows of a stage (every group but the last one is full).
+__host__ __device__ inline long long mega_stage_bytes(const MegaStage& st, int wt, int rows) {
+    const int full = rows / st.group_rows, rest = rows - full * st.group_rows;
+    return (long long)st.units * ((long long)full * mega_unit_bytes(wt, st.group_rows) + (rest ? mega_unit_bytes(wt, rest) : 0));
+}
+__host__ __device__ inline int mega_stage_chunks(const MegaStage& st, int rows) {
+    return (rows + st.group_rows - 1) / st.group_rows * ((st.units + st.chunk_units - 1) / st.chunk_units);
+}
 
 // Contiguous share [begin, end) of `n` items owned by part `i` of `parts` (every part gets floor or ceil of n/parts).
 // (n * parts stays far below 2^32 for every model size the plan accepts)
@@ -189,6 +205,9 @@ __device__ __forceinline__ ulonglong2 ld_words2(const unsigned long long* p) {
 __device__ __forceinline__ void st_word(unsigned long long* p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+__device__ __forceinline__ void st_words2(unsigned long long* p, unsigned long long v0, unsigned long long v1) {
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1,%2};" ::"l"(p), "l"(v0), "l"(v1) : "memory");
+}
 __device__ __forceinline__ void red_add_u64(unsigned long long* p, unsigned long long v) {
     asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -218,8 +237,8 @@ __host__ __device__ inline MegaShare mega_share(const ModelDims& m, const MegaPl
         w.s1_begin = mega_share_begin(p.group_items, p.gsize, w.member);
         w.s1_n = mega_share_begin(p.group_items, p.gsize, w.member + 1) - w.s1_begin;
     }
-    w.h_begin = mega_share_begin(m.hidden, p.n_cta, cta);
-    w.h_n = mega_share_begin(m.hidden, p.n_cta, cta + 1) - w.h_begin;
+    w.h_begin = 2 * mega_share_begin(m.hidden / 2, p.n_cta, cta);  // (whole pairs: a reader takes two words at a time)
+    w.h_n = 2 * mega_share_begin(m.hidden / 2, p.n_cta, cta + 1) - w.h_begin;
     w.d_begin = mega_share_begin(m.d_model, p.n_cta, cta);
     w.d_n = mega_share_begin(m.d_model, p.n_cta, cta + 1) - w.d_begin;
     w.v_begin = mega_share_begin(m.vocab, p.n_cta, cta);
@@ -243,10 +262,9 @@ __host__ __device__ inline void mega_s1_rows(const ModelDims& m, const MegaPlan&
     }
 }
 
-// Bytes of a staged vector of K values (hi and lo fp16 parts, see xa_index; or int8 digits, see qx_store_pair).
-__host__ __device__ inline int xa_bytes(int K) { return (K / 32) * 128; }
-// Bytes of the per-block scales that accompany a vector staged as int8 digits.
-__host__ __device__ inline int qx_scale_bytes(int K) { return (K / 32) * 4; }
+// Bytes of a staged vector of K values for np positions: fp16 hi and lo parts (xa_index), or int8 digits (qx_store_quads).
+__host__ __device__ constexpr int qx_digits(int wt) { return wt == WT_Q4_0 ? 4 : 3; }
+__host__ __device__ constexpr int xa_bytes(int wt, int K, int np) { return wt == WT_F16 ? K / 16 * 64 * np : K / 32 * 32 * qx_digits(wt); }
 
 // ------------------------------------------------------------------------------------------------ shared state
 
@@ -254,77 +272,189 @@ struct MegaShared {
     uint8_t* slots;
     uint64_t* full;
     uint64_t* empty;
-    uint8_t* xa;   // staged activation vector (x * gain, or the FFN activation) as the A operand: hi/lo fp16 (see xa_index)
-    float* xraw;   // [d_model] the residual stream entering the layer (also what the head reads)
-    float* xmid;   // [d_model] the residual stream after the attention block
-    float2* rope;  // [head_dim/2] (cos, sin) of the position being processed
-    unsigned long long* prev;  // [d_model] totals of the counted sums seen at the previous exchange
-    float* qs;     // [head_dim] query of this CTA's head
-    float* ctx;    // [head_dim] attention output of this CTA's head, staged like xa
-    __half* kn;    // [head_dim] the new token's key, rounded as the cache stores it
-    __half* vn;    // [head_dim]
+    uint8_t* xa;   // staged operand vector, every unit written and read by the warp that owns it
+    float* xq;     // quantised types: scale of every staged block
+    float* xres;   // [np][d_model] the residual stream: entering the layer, then after the attention block
+    unsigned long long* prev;  // [np][d_model] totals of the counted sums seen at the previous exchange
+    float* qs;     // [np][head_dim] query of this CTA's head
+    uint8_t* ctx;  // attention output of this CTA's head, staged like xa (block scales behind it)
+    __half* kn;    // [np][head_dim] the new token's key, rounded as the cache stores it
+    __half* vn;    // [np][head_dim]
     float* part;   // [warps][head_dim]
     float* red;    // [64]
-    float* partial;  // [2][group][kMegaChunkRows] partial row sums of a group of chunks (alternating halves)
+    float* ss;     // [2][np][warps] sums of squares of the warps' columns (alternating with the partial sums)
+    float* sums;   // [2][warps][np][16 group_tiles] partial row sums of a group
     unsigned long long* key;   // [32] arg-max keys
     struct MegaShare* share;  // this CTA's work shares, computed once
-    int* hbeg;     // [n_cta + 1] first FFN unit (= element of the activation vector) of every CTA
+    uint16_t* act;  // [hidden / 2] word of every pair of the activation vector (act_wpc > 0)
+    int4* s1;       // [s1_max] {kind, row, row, RoPE entry} of this CTA's S1 row pairs
     int* abort;    // [1] a wait gave up: no more waiting in this CTA
     int* stop;     // [1] the loop ended early (EOS): the producer stops issuing
-    unsigned* landed;  // [1] number of chunks whose bytes have arrived (written by the producer warp's watcher lane)
+    unsigned* landed;  // [1] number of chunks whose bytes have arrived (written by the watcher warp)
 };
 
 // The areas sit at offsets the host computed once (mega_layout): an address is the base plus a kernel-argument
 // constant, which costs no register to keep.
-__device__ __forceinline__ MegaShared mega_carve(uint8_t* base, const MegaArgs& a) {
+__device__ __forceinline__ MegaShared mega_carve(uint8_t* base, const MegaPlan& p) {
     MegaShared s;
-    const MegaPlan& p = a.plan;
     s.slots = base;
     s.full = reinterpret_cast<uint64_t*>(base + p.off_bar);
     s.empty = s.full + p.n_slots;
     s.prev = reinterpret_cast<unsigned long long*>(base + p.off_prev);
     s.key = reinterpret_cast<unsigned long long*>(base + p.off_key);
     s.xa = base + p.off_xs;
-    s.xraw = reinterpret_cast<float*>(base + p.off_xraw);
-    s.xmid = reinterpret_cast<float*>(base + p.off_xmid);
-    s.rope = reinterpret_cast<float2*>(base + p.off_rope);
+    s.xq = reinterpret_cast<float*>(base + p.off_xq);
+    s.xres = reinterpret_cast<float*>(base + p.off_xres);
     s.qs = reinterpret_cast<float*>(base + p.off_qs);
-    s.ctx = reinterpret_cast<float*>(base + p.off_ctx);
+    s.ctx = base + p.off_ctx;
     s.kn = reinterpret_cast<__half*>(base + p.off_kn);
     s.vn = reinterpret_cast<__half*>(base + p.off_vn);
     s.part = reinterpret_cast<float*>(base + p.off_part);
     s.red = reinterpret_cast<float*>(base + p.off_red);
-    s.partial = reinterpret_cast<float*>(base + p.off_outv);
+    s.ss = reinterpret_cast<float*>(base + p.off_ss);
+    s.sums = reinterpret_cast<float*>(base + p.off_sums);
     s.abort = reinterpret_cast<int*>(base + p.off_flags);
     s.stop = s.abort + 1;
     s.landed = reinterpret_cast<unsigned*>(s.abort + 2);
     s.share = reinterpret_cast<MegaShare*>(base + p.off_share);
-    s.hbeg = reinterpret_cast<int*>(base + p.off_beg);
+    s.act = reinterpret_cast<uint16_t*>(base + p.off_act);
+    s.s1 = reinterpret_cast<int4*>(base + p.off_s1);
     return s;
 }
 
-// Fills the offsets and the total size (host side; p.n_slots and p.slot_bytes must be set).
-inline void mega_layout(const ModelDims& m, MegaPlan& p) {
+// Fills the offsets and the total size for np token positions per pass (host side; p.n_slots and p.slot_bytes must be set).
+inline void mega_layout(const ModelDims& m, MegaPlan& p, int np) {
+    const int wide = m.d_model > m.hidden ? m.d_model : m.hidden;
     size_t o = (size_t)p.n_slots * p.slot_bytes;
     auto take = [&](size_t bytes) { size_t at = (o + 15) & ~(size_t)15; o = at + bytes; return (int)at; };
+    auto staged = [&](int K) { return (size_t)xa_bytes(p.wt_layer, K, np); };
+    const size_t xs = std::max(staged(wide), (size_t)xa_bytes(p.wt_head, m.d_model, np));
     p.off_bar = take(16 * (size_t)p.n_slots);
-    p.off_prev = take(8 * (size_t)m.d_model);
+    p.off_prev = take(8 * (size_t)np * m.d_model);
     p.off_key = take(8 * 32);
-    p.off_xs = take((size_t)xa_bytes(m.d_model > m.hidden ? m.d_model : m.hidden) + qx_scale_bytes(m.d_model > m.hidden ? m.d_model : m.hidden));
-    p.off_xraw = take(sizeof(float) * (size_t)m.d_model);
-    p.off_xmid = take(sizeof(float) * (size_t)m.d_model);
-    p.off_rope = take(sizeof(float2) * (size_t)(m.head_dim / 2));
-    p.off_qs = take(sizeof(float) * (size_t)m.head_dim);
-    p.off_ctx = take((size_t)xa_bytes(m.head_dim) + qx_scale_bytes(m.head_dim));
-    p.off_kn = take(sizeof(__half) * (size_t)m.head_dim);
-    p.off_vn = take(sizeof(__half) * (size_t)m.head_dim);
+    p.off_xs = take(xs);
+    p.off_xq = take(p.wt_layer == WT_F16 ? 0 : sizeof(float) * (size_t)(wide / 32));
+    p.off_xres = take(sizeof(float) * (size_t)np * m.d_model);
+    p.off_qs = take(sizeof(float) * (size_t)np * m.head_dim);
+    p.off_ctx = take(staged(m.head_dim) + sizeof(float) * (size_t)(m.head_dim / 32));
+    p.off_kn = take(sizeof(__half) * (size_t)np * m.head_dim);
+    p.off_vn = take(sizeof(__half) * (size_t)np * m.head_dim);
     p.off_part = take(sizeof(float) * (size_t)kMegaConsumerWarps * m.head_dim);
     p.off_red = take(sizeof(float) * 64);
-    p.off_outv = take(sizeof(float) * 2 * p.group * kMegaChunkRows);
+    p.off_ss = take(sizeof(float) * 2 * (size_t)np * kMegaConsumerWarps);
+    p.off_sums = take(sizeof(float) * 2 * (size_t)kMegaConsumerWarps * np * 16 * p.group_tiles);
     p.off_flags = take(16);
     p.off_share = take(sizeof(MegaShare));
-    p.off_beg = take(sizeof(int) * ((size_t)p.n_cta + 1));
+    p.off_act = take(p.act_wpc ? sizeof(uint16_t) * (size_t)(m.hidden / 2) : 0);
+    p.off_s1 = take(sizeof(int4) * (size_t)p.s1_max);
     p.smem_bytes = (int)((o + 127) & ~(size_t)127);
+}
+
+// Plans the persistent kernel for a model (host side): every CTA owns a contiguous share of the rows of every matrix.  False: the
+// model does not fit.
+inline bool mega_plan(const ModelDims& m, int wt_layer, int wt_head, int sms, int smem_max, MegaPlan& p) {
+    p = MegaPlan{};
+    const bool quant = wt_layer != WT_F16 || wt_head != WT_F16;
+    if (quant && (m.d_model % 256 || m.hidden % 256)) return false;
+    // every CTA must own at least one pair of FFN units and one row of W2 (it then takes part in every all-to-all exchange)
+    const int P = std::min(sms, std::min(m.d_model, m.hidden / 2));
+    if (P < m.n_head) return false;
+    auto pad128 = [](long long v) { return (int)((v + 127) / 128 * 128); };
+    auto ceil_div = [](int a, int b) { return (a + b - 1) / b; };
+    p.inv_d = 1.0f / (float)m.d_model;
+    p.n_cta = P;
+    p.qpk = m.n_head / m.n_kv_head;
+    p.group_items = (p.qpk + 2) * m.head_dim / 2;
+    p.cph = std::max(1, std::min(std::min(P / m.n_head, m.d_model), p.group_items / p.qpk));
+    p.gsize = p.cph * p.qpk;
+    p.n_group_cta = p.cph * m.n_head;
+    p.s1_max = ceil_div(p.group_items, p.gsize);
+    p.rpb = ceil_div(m.d_model, p.cph);
+    p.hpc_max = 2 * ceil_div(m.hidden / 2, P);
+    p.dpc_max = ceil_div(m.d_model, P);
+    p.vpc_max = ceil_div(m.vocab, P);
+    p.wt_layer = wt_layer;
+    p.wt_head = wt_head;
+    p.ffn_rows = m.arch == ARCH_GPT2 ? 1 : 2;
+    // Exchange arrays: the activation vector gets cache lines per CTA where a lane polls all of its pairs in one round (four
+    // 16-byte loads); the layer output stays compact (see kMegaLineWords).
+    p.act_wpc = !quant && m.hidden <= 4096 ? ceil_div(p.hpc_max, kMegaLineWords) * kMegaLineWords : 0;
+    // Row groups: as equal as whole tiles allow.
+    const int rows[5] = {2 * p.s1_max, p.rpb, p.ffn_rows * p.hpc_max, p.dpc_max, p.vpc_max};
+    for (int k = 0; k < 5; k++) {
+        MegaStage& st = p.stage[k];
+        st.units = (k == MS_WO ? m.head_dim : k == MS_DOWN ? m.hidden : m.d_model) / mega_unit(k == MS_HEAD ? wt_head : wt_layer);
+        st.chunk_units = st.units;
+        st.group_rows = rows[k];
+        if (k == MS_WO) continue;
+        const int groups = ceil_div(rows[k], 16 * kMegaMaxTiles);
+        if (groups > 1) st.group_rows = ceil_div(ceil_div(rows[k], groups), 16) * 16;
+        p.group_tiles = std::max(p.group_tiles, ceil_div(st.group_rows, 16));
+    }
+    // The ring: what the other areas leave, in kMegaSlots slots, and as many units of a group (for Wo: 16-row tiles) per chunk as
+    // fit one, in equal shares.
+    mega_layout(m, p, 1);
+    const int room = smem_max - p.smem_bytes - 512;
+    for (int ns = kMegaSlots; ns >= 2 && p.n_slots == 0; ns--) {
+        const int slot = std::min(room / ns / 128 * 128, kMegaSlotMax);
+        if (ns * slot < kMegaRingMin) continue;
+        bool fits = true;
+        for (int k = 0; k < 5; k++) {
+            MegaStage& st = p.stage[k];
+            const int wt = k == MS_HEAD ? wt_head : wt_layer;
+            if (k == MS_WO) {
+                int per = rows[k];
+                for (int n = 2; per > 16 && st.units * mega_unit_bytes(wt, per) > slot; n++) per = ceil_div(ceil_div(rows[k], n), 16) * 16;
+                st.group_rows = per;
+                fits = fits && st.units * mega_unit_bytes(wt, per) <= slot;
+            } else {
+                const int most = slot / mega_unit_bytes(wt, st.group_rows);
+                fits = fits && most >= 1;
+                if (most >= 1) st.chunk_units = ceil_div(st.units, ceil_div(st.units, most));
+            }
+        }
+        if (fits) { p.n_slots = ns; p.slot_bytes = slot; }
+    }
+    if (p.n_slots == 0) return false;
+    mega_layout(m, p, 1);
+    if (p.smem_bytes > smem_max) return false;
+    p.s1_bytes = pad128(mega_stage_bytes(p.stage[MS_QKV], wt_layer, rows[MS_QKV]));
+    p.s2_bytes = pad128(mega_stage_bytes(p.stage[MS_WO], wt_layer, rows[MS_WO]));
+    p.s3a_bytes = pad128(mega_stage_bytes(p.stage[MS_UP], wt_layer, rows[MS_UP]));
+    p.s3b_bytes = pad128(mega_stage_bytes(p.stage[MS_DOWN], wt_layer, rows[MS_DOWN]));
+    p.layer_bytes = (long long)p.s1_bytes + p.s2_bytes + p.s3a_bytes + p.s3b_bytes;
+    p.head_bytes = pad128(mega_stage_bytes(p.stage[MS_HEAD], wt_head, rows[MS_HEAD]));
+    p.cta_bytes = p.layer_bytes * m.n_layer + p.head_bytes;
+    return true;
+}
+
+// Shared state before the roles part (all threads of the CTA; the caller synchronises).
+__device__ __forceinline__ void mega_init(const MegaArgs& a, const MegaShared& s, int np) {
+    const ModelDims& m = a.m;
+    const MegaPlan& p = a.plan;
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        *s.share = mega_share(m, p, (int)blockIdx.x);
+        for (int i = 0; i < p.n_slots; i++) { mbar_init(s.full + i, 1); mbar_init(s.empty + i, kMegaConsumerWarps); }
+        *s.abort = 0;
+        *s.stop = 0;
+        *s.landed = 0u;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int k = tid; k < np * m.d_model; k += kMegaThreads) s.prev[k] = 0ull;  // the counted sums are zero at launch
+    if (p.act_wpc)
+        for (int c = tid; c < p.n_cta; c += kMegaThreads) {
+            const int b = mega_share_begin(m.hidden / 2, p.n_cta, c), e = mega_share_begin(m.hidden / 2, p.n_cta, c + 1);
+            for (int i = b; i < e; i++) s.act[i] = (uint16_t)(c * p.act_wpc + 2 * (i - b));
+        }
+    if ((int)blockIdx.x < p.n_group_cta) {
+        const MegaShare w = mega_share(m, p, (int)blockIdx.x);
+        for (int i = tid; i < w.s1_n; i += kMegaThreads) {
+            int4 e;
+            mega_s1_rows(m, p, w.kvh, w.s1_begin + i, e.x, e.y, e.z, e.w);
+            s.s1[i] = e;
+        }
+    }
 }
 
 __device__ __forceinline__ void mega_fail(const MegaArgs& a, const MegaShared& s, int code) {
@@ -411,208 +541,36 @@ __device__ __forceinline__ void mega_release_deferred(const MegaArgs& a, const M
     }
 }
 
-// ------------------------------------------------------------------------------------------------ exchanges
+// ------------------------------------------------------------------------------------------------ staged operands
 
-// Reads `n` tagged words (n even, 16-byte aligned base) and hands pairs (even index, two values, two gains) to `sink`
-// (when n is a multiple of 64 every warp reaches the sink with all its lanes, consecutive pairs in consecutive lanes).  A thread keeps up to
-// four 16-byte loads in flight; words that validated are not read again.  The gains (or 1 when `gain` is null) are
-// requested before the polling starts, so they cost nothing once the words arrive.
-template <class Sink>
-__device__ __forceinline__ void mega_read_words(const MegaArgs& a, const MegaShared& s, const unsigned long long* base, int n, unsigned tag, int code,
-                                                const float* gain, Sink sink) {
-    const int n_pairs = n >> 1;
-    for (int p0 = 0; p0 < n_pairs; p0 += 4 * kMegaConsumers) {
-        ulonglong2 w[4];
-        float2 g[4];
-        bool ok[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int p = p0 + j * kMegaConsumers + (int)threadIdx.x;
-            ok[j] = p >= n_pairs;
-            w[j] = make_ulonglong2(0, 0);
-            g[j] = (gain && !ok[j]) ? __ldg(reinterpret_cast<const float2*>(gain) + p) : make_float2(1.f, 1.f);
-        }
-        unsigned spins = 0;
-        if (!mega_aborting(s)) {
-            while (true) {
-                bool all = true;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    if (!ok[j]) {
-                        w[j] = ld_words2(base + 2 * (size_t)(p0 + j * kMegaConsumers + (int)threadIdx.x));
-                        ok[j] = (unsigned)(w[j].x >> 32) == tag && (unsigned)(w[j].y >> 32) == tag;
-                        all = all && ok[j];
-                    }
-                }
-                if (all) break;
-                if (mega_spin_out(a, s, spins, code)) break;
-                mega_backoff();
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int p = p0 + j * kMegaConsumers + (int)threadIdx.x;
-            if (p < n_pairs) sink(2 * p, __uint_as_float((unsigned)w[j].x), __uint_as_float((unsigned)w[j].y), g[j].x, g[j].y);
-        }
-    }
-}
-
-// Tagged words written line by line: the CTA that owns elements [beg[c], beg[c + 1]) of a vector writes them to the
-// first words of slot c (`wpc` words per slot: whole cache lines, at least the largest share).  Cache lines with a single
-// writer matter: a store to a line that every CTA is polling costs a round of invalidations, and the stores of several
-// writers to one line queue up behind one another (sixteen writers per line made the arg-max exchange take 6 us).
-// `lines` = positions x CTAs (position q's lines follow position q - 1's); the sink receives (q * n + element, value,
-// gain).  `ppl` = pairs of words to read per line = ceil(largest share / 2); every thread takes up to four pairs.
-template <class Sink>
-__device__ __forceinline__ void mega_read_lines(const MegaArgs& a, const MegaShared& s, const unsigned long long* base, int wpc, const int* beg, int n, int lines, int ppl,
-                                                unsigned tag, int code, const float* gain, Sink sink) {
-    const int n_cta = a.plan.n_cta;
-    const int slots = lines * ppl;
-    for (int s0 = 0; s0 < slots; s0 += 4 * kMegaConsumers) {
-        ulonglong2 w[4];
-        float2 g[4];
-        const unsigned long long* src[4];
-        int k0[4], cnt[4];
-        bool ok[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int slot = s0 + j * kMegaConsumers + (int)threadIdx.x;
-            w[j] = make_ulonglong2(0, 0);
-            g[j] = make_float2(1.f, 1.f);
-            cnt[j] = 0; k0[j] = 0; src[j] = base;
-            if (slot < slots) {
-                const int line = (int)((unsigned)slot / (unsigned)ppl), jj = slot - line * ppl;
-                const int q = line >= n_cta ? 1 : 0, cta = line - q * n_cta;  // at most two positions
-                const int first = beg[cta] + 2 * jj;
-                cnt[j] = max(0, min(2, beg[cta + 1] - first));
-                k0[j] = q * n + first;
-                src[j] = base + (size_t)line * wpc + 2 * jj;
-                if (gain && cnt[j] > 0) {
-                    g[j].x = __ldg(gain + k0[j]);
-                    if (cnt[j] > 1) g[j].y = __ldg(gain + k0[j] + 1);
-                }
-            }
-            ok[j] = cnt[j] == 0;
-        }
-        unsigned spins = 0;
-        if (!mega_aborting(s)) {
-            while (true) {
-                bool all = true;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    if (!ok[j]) {
-                        w[j] = ld_words2(src[j]);
-                        ok[j] = (unsigned)(w[j].x >> 32) == tag && (cnt[j] < 2 || (unsigned)(w[j].y >> 32) == tag);
-                        all = all && ok[j];
-                    }
-                }
-                if (all) break;
-                if (mega_spin_out(a, s, spins, code)) break;
-                mega_backoff();
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if (cnt[j] > 0) sink(k0[j], __uint_as_float((unsigned)w[j].x), g[j].x);
-            if (cnt[j] > 1) sink(k0[j] + 1, __uint_as_float((unsigned)w[j].y), g[j].y);
-        }
-    }
-}
-
-// Reads the counted sums once each has received `n_contrib` contributions since the previous exchange.
-template <class Sink>
-__device__ __forceinline__ void mega_read_sums(const MegaArgs& a, const MegaShared& s, const unsigned long long* base, int n, int n_contrib, int code,
-                                               const float* gain, Sink sink) {
-    const int n_pairs = n >> 1;
-    for (int p0 = 0; p0 < n_pairs; p0 += 2 * kMegaConsumers) {
-        ulonglong2 w[2], pv[2];
-        float2 g[2];
-        bool ok[2];
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int p = p0 + j * kMegaConsumers + (int)threadIdx.x;
-            ok[j] = p >= n_pairs;
-            w[j] = make_ulonglong2(0, 0);
-            pv[j] = ok[j] ? make_ulonglong2(0, 0) : *reinterpret_cast<const ulonglong2*>(s.prev + 2 * p);
-            g[j] = (gain && !ok[j]) ? __ldg(reinterpret_cast<const float2*>(gain) + p) : make_float2(1.f, 1.f);
-        }
-        unsigned spins = 0;
-        if (!mega_aborting(s)) {
-            while (true) {
-                bool all = true;
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    if (!ok[j]) {
-                        w[j] = ld_words2(base + 2 * (size_t)(p0 + j * kMegaConsumers + (int)threadIdx.x));
-                        ok[j] = ((w[j].x - pv[j].x) & 0xffull) == (unsigned long long)n_contrib && ((w[j].y - pv[j].y) & 0xffull) == (unsigned long long)n_contrib;
-                        all = all && ok[j];
-                    }
-                }
-                if (all) break;
-                if (mega_spin_out(a, s, spins, code)) break;
-                mega_backoff();
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int p = p0 + j * kMegaConsumers + (int)threadIdx.x;
-            if (p < n_pairs) {
-                *reinterpret_cast<ulonglong2*>(s.prev + 2 * p) = w[j];
-                const long long v0 = (long long)(w[j].x - pv[j].x - (unsigned long long)n_contrib) >> 8;
-                const long long v1 = (long long)(w[j].y - pv[j].y - (unsigned long long)n_contrib) >> 8;
-                sink(2 * p, (float)v0 * kMegaUnfix, (float)v1 * kMegaUnfix, g[j].x, g[j].y);
-            }
-        }
-    }
-}
-
-// Sum over the consumer threads of one float each; every thread receives the result.  One CTA barrier.
-__device__ __forceinline__ float mega_block_sum(float v, float* red) {
-    v = warp_sum(v);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    consumer_sync();
-    // sixteen partial sums: four 16-byte loads and a tree of additions instead of a chain of sixteen
-    const float4* r4 = reinterpret_cast<const float4*>(red);
-    const float4 a = r4[0], b = r4[1], c = r4[2], e = r4[3];
-    static_assert(kMegaConsumerWarps == 16, "mega_block_sum reads sixteen partial sums");
-    return (((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w))) + (((c.x + c.y) + (c.z + c.w)) + ((e.x + e.y) + (e.z + e.w)));
-}
-
-// The sum of v0 and the maximum of v1 >= 0 (GPT-2).
-__device__ __forceinline__ float2 mega_block_sum_max(float v0, float v1, float* red) {
-    v1 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v1)));  // (non-negative floats order as their bits)
-    v0 = warp_sum(v0);
-    if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = v0; red[kMegaConsumerWarps + (threadIdx.x >> 5)] = v1; }
-    consumer_sync();
-    const float4* r4 = reinterpret_cast<const float4*>(red);
-    float2 t = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < kMegaConsumerWarps / 4; q++) {
-        const float4 x = r4[q], y = r4[kMegaConsumerWarps / 4 + q];
-        t.x += (x.x + x.y) + (x.z + x.w);
-        t.y = fmaxf(t.y, fmaxf(fmaxf(y.x, y.y), fmaxf(y.z, y.w)));
-    }
-    return t;
-}
-
-// ------------------------------------------------------------------------------------------------ products
-
-// Where element k of a staged vector lives (in halves): block of 32 columns kb, column c of the B operand (position q's
-// hi part is column 2q, its lo part column 2q + 1; NP positions are staged side by side), piece t; the 16 bytes of a
-// piece are the B registers of the two m16n8k16 steps of the block.
-template <int NP = 1>
+// Where element k of a staged fp16 vector lives (in halves): unit of 16 columns, column c of the B operand (position q's
+// hi part is column 2q, its lo part column 2q + 1; NP positions are staged side by side), piece t; the 8 bytes of a piece
+// are the B registers of the unit's m16n8k16 step.
+template <int NP>
 __device__ __forceinline__ int xa_index(int k, int c) {
-    const int kb = k >> 5, kk = k & 31;
-    return (((kb * 2 * NP + c) * 4 + ((kk & 7) >> 1)) << 3) + ((kk >> 3) << 1) + (kk & 1);
+    return (((k >> 4) * 2 * NP + c) * 4 + ((k & 7) >> 1)) * 4 + ((k >> 3) & 1) * 2 + (k & 1);
 }
-
-// Stores v as hi + lo (both fp16, hi saturating) at element k of position q of a staged vector.
-template <int NP = 1>
-__device__ __forceinline__ void xa_store(__half* xa, int k, float v, int q = 0) {
-    __half hi;
-    asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(*reinterpret_cast<unsigned short*>(&hi)) : "f"(v));
-    xa[xa_index<NP>(k, 2 * q)] = hi;
-    xa[xa_index<NP>(k, 2 * q + 1)] = __float2half_rn(v - __half2float(hi));
+// hi saturates: it stays finite on any finite value
+__device__ __forceinline__ uint32_t xa_hi(float v) {
+    unsigned short h;
+    asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(h) : "f"(v));
+    return h;
+}
+// Stores elements k, k + 1 (k even) of position q as hi + lo fp16 parts.
+template <int NP>
+__device__ __forceinline__ void xa_store_pair(uint8_t* xa, int k, float v0, float v1, int q) {
+    const uint32_t h0 = xa_hi(v0), h1 = xa_hi(v1);
+    const __half2 lo = __floats2half2_rn(v0 - __half2float(__ushort_as_half((unsigned short)h0)), v1 - __half2float(__ushort_as_half((unsigned short)h1)));
+    __half* const at = reinterpret_cast<__half*>(xa) + xa_index<NP>(k, 2 * q);
+    *reinterpret_cast<uint32_t*>(at) = h0 | (h1 << 16);
+    *reinterpret_cast<__half2*>(at + 16) = lo;
+}
+template <int NP>
+__device__ __forceinline__ void xa_store(uint8_t* xa, int k, float v, int q) {
+    const __half hi = __ushort_as_half((unsigned short)xa_hi(v));
+    __half* const at = reinterpret_cast<__half*>(xa) + xa_index<NP>(k, 2 * q);
+    at[0] = hi;
+    at[16] = __float2half_rn(v - __half2float(hi));
 }
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -621,91 +579,55 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Partial products of the 16-row tile `tile` of a chunk of R rows with the staged vector over the column blocks
-// [kb0, kb1).  The weights are the A operand (rows g and g + 8 of the tile: one 16-byte shared-memory load each per two
-// m16n8k16 steps), the staged vector the B operand (column 0 = hi part, column 1 = lo part, held by lanes 0..7).  The
-// lanes with lane % 4 == q < NP return the sums of position q for rows tile*16 + lane/4 (.x) and + 8 (.y); rows past R are
-// meaningless.  With NP positions the staged vector holds 2 NP columns (lanes 0 .. 8 NP - 1 feed the B operand): the
-// products of a second position ride in columns the instruction computes anyway.
-template <int NP>
-__device__ __forceinline__ float2 mega_tile_dot_f16(const uint8_t* chunk, int R, int n_kb, int tile, int kb0, int kb1, const uint8_t* xa, int lane) {
-    // four independent accumulator sets: a dependent m16n8k16 costs ~40-60 cycles, and a warp has only a few blocks
-    float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f}, c3[4] = {0.f, 0.f, 0.f, 0.f};
-    const uint8_t* wp = chunk + ((size_t)(tile * 16 + (lane >> 2)) * 64 + (lane & 3) * 16);
-    const size_t kstride = (size_t)R * 64;
-    const uint8_t* xp = xa + lane * 16;
-    // plain loads: the compiler may move them ahead of the previous block's products, never across a barrier
-    auto block = [&](int kb, float (&ce)[4], float (&co)[4]) {
-        const uint4 w0 = *reinterpret_cast<const uint4*>(wp + kb * kstride);
-        const uint4 w8 = *reinterpret_cast<const uint4*>(wp + kb * kstride + 8 * 64);
-        uint4 xv = make_uint4(0, 0, 0, 0);
-        if (lane < 8 * NP) xv = *reinterpret_cast<const uint4*>(xp + kb * (128 * NP));
-        mma_16816(ce, w0.x, w8.x, w0.y, w8.y, xv.x, xv.y);
-        mma_16816(co, w0.z, w8.z, w0.w, w8.w, xv.z, xv.w);
-    };
-    int kb = kb0;
-#pragma unroll 2
-    for (; kb + 1 < kb1; kb += 2) {
-        block(kb, c0, c1);
-        block(kb + 1, c2, c3);
-    }
-    if (kb < kb1) block(kb, c0, c1);
-    // column 0 of the product is w . x_hi, column 1 is w . x_lo
-    return make_float2(((c0[0] + c1[0]) + (c2[0] + c3[0])) + ((c0[1] + c1[1]) + (c2[1] + c3[1])),
-                       ((c0[2] + c1[2]) + (c2[2] + c3[2])) + ((c0[3] + c1[3]) + (c2[3] + c3[3])));
-}
-
-// ---- Q8_0: the activation as int8 digits, the products on the int8 tensor-core path ----
-// A Q8_0 weight is an int8: instead of widening it to fp16 (eight byte permutes and subtractions per 32 weights and
-// lane), the staged activation is turned into integers.  Per block of 32 columns: q = max|x| / 127 and
-// x_i ~ q (d0 + d1 / 128 + d2 / 16384) with three int8 digits (22 bits relative to the block's largest value; the
-// weights stay exact).  The digits are B columns 0..2 of one mma.sync.m16n8k32 (s8 x s8), the int32 results are combined
-// and scaled by q and the weight block's scale in fp32.  (Q4_0 keeps the fp16 widening: its nibbles carry an offset of 8
-// that has to be taken out through a per-block sum of the staged values, and the extra warp reduction per staged block
-// cost more than the cheaper products gained: 492 against 460 us per token on the 22-layer d2048 model; Q8_0 gained 3 %.)
+// ---- GGUF blocks: the activation as int8 digits, the products on the int8 tensor-core path ----
+// A Q8_0 weight is an int8, a Q4_0 nibble becomes one (times 16) with a mask: instead of widening the weights to fp16, the
+// staged activation is turned into integers.  Per block of 32 columns x_i ~ q I_i with q a power of two and |I_i| <= 2^22, and
+// I = 65536 d0 + 256 d1 + d2 (+ d3 / 256) with int8 digits: 22 bits relative to the block's largest value, for Q4_0 30.  The
+// weights stay exact.  The digits are B columns 0, 1, .. of one mma.sync.m16n8k32 (s8 x s8), the int32 results are combined
+// and scaled by q and the weight block's scale in fp32.  Error of a product against 64 bits (2-norm, K = 64 .. 5632, three
+// distributions): Q8_0 1.7e-7 to 5.9e-7 (three digits per quotient of the block's maximum: 3.3e-7 to 9.5e-7), Q4_0 0.4e-7 to 1.3e-7
+// (fp16 parts times nibbles widened to fp16: 0.5e-7 to 1.3e-7; three digits: 1.6e-7 to 6.7e-7).
 //
-// Staged layout: block kb holds 128 bytes = [digit c][piece t][8 bytes: columns 4t..4t+3 then 16+4t..16+4t+3], the B
-// registers of lane (g = c, t); the block scales q sit behind the vector (qx_scale_bytes).
-__device__ __forceinline__ int qx_byte(int kb, int c, int e) { return kb * 128 + c * 32 + (((e & 15) >> 2) << 3) + ((e >> 4) << 2) + (e & 3); }
+// Staged layout: block kb holds [digit c][piece t][8 bytes: columns 4t..4t+3 then 16+4t..16+4t+3], the B
+// registers of lane (g = c, t).
+constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23: added to a float of magnitude up to 2^22 it leaves the nearest integer in the low mantissa bits
 
-// Rounding without conversion instructions (they issue at a quarter of the rate of an addition, and this runs three times per
-// staged element): adding 1.5 * 2^23 to a float of magnitude below 2^22 rounds it to the nearest integer and leaves that
-// integer in the low mantissa bits.
-constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23
-
-// The three int8 digits of v * inv (|v * inv| <= 127); dg[c] carries digit c in its low 8 bits (two's complement).
-__device__ __forceinline__ void qx_digits(float v, float inv, int (&dg)[3]) {
-    const float s0 = v * inv, t0 = s0 + kRoundMagic, d0 = t0 - kRoundMagic;
-    const float s1 = (s0 - d0) * 128.f, t1 = s1 + kRoundMagic, d1 = t1 - kRoundMagic;
-    const float t2 = (s1 - d1) * 128.f + kRoundMagic;
-    dg[0] = __float_as_int(t0); dg[1] = __float_as_int(t1); dg[2] = __float_as_int(t2);
-}
-// Stages elements k, k + 1 (k even).  Must be called by all 32 lanes of a warp with consecutive pairs: the 16 lanes of a
-// half-warp hold one block of 32 columns.  The block's maximum comes from one warp reduction on integers (the bit
-// pattern of a non-negative float orders like the float).
-__device__ __forceinline__ void qx_store_pair(uint8_t* xq, float* qs, int k, float v0, float v1) {
-    const unsigned half_mask = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
-    const float mx = __uint_as_float(__reduce_max_sync(half_mask, __float_as_uint(fmaxf(fabsf(v0), fabsf(v1)))));
-    const float inv = mx > 0.f ? __fdividef(127.0f, mx) : 0.f;
-    int d0[3], d1[3];
-    qx_digits(v0, inv, d0);
-    qx_digits(v1, inv, d1);
-    const int kb = k >> 5, e = k & 31;
+// Stages N quads of elements k .. k + 3 (k a multiple of 4) per lane; groups of eight lanes with consecutive quads hold one block of
+// 32 columns each (`mask`: the lanes that take part; `live`: which quads of this lane are stored).  The N quads go side by side: a
+// block's maximum takes three shuffles.  (A digit at a time with a quotient per block took 22 operations per element instead
+// of six, and __reduce_max_sync over groups of lanes is executed group by group: 500 cycles per quad.)
+template <int WT, int N>
+__device__ __forceinline__ void qx_store_quads(uint8_t* xq, float* qs, const int (&k)[N], const float4 (&v)[N], const bool (&live)[N], unsigned mask) {
+    float top[N];
 #pragma unroll
-    for (int c = 0; c < 3; c++)
-        *reinterpret_cast<uint16_t*>(xq + qx_byte(kb, c, e)) = (uint16_t)__byte_perm((unsigned)d0[c], (unsigned)d1[c], 0x0040);
-    if ((threadIdx.x & 15) == 0) qs[kb] = mx * (1.0f / 127.0f);
-}
-// Stages element k.  Must be called by all 32 lanes of a warp with consecutive k: the warp holds one block.
-__device__ __forceinline__ void qx_store_elem(uint8_t* xq, float* qs, int k, float v) {
-    const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v))));
-    const float inv = mx > 0.f ? __fdividef(127.0f, mx) : 0.f;
-    int dg[3];
-    qx_digits(v, inv, dg);
-    const int kb = k >> 5, e = k & 31;
+    for (int j = 0; j < N; j++) top[j] = fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w)));
 #pragma unroll
-    for (int c = 0; c < 3; c++) xq[qx_byte(kb, c, e)] = (uint8_t)dg[c];
-    if ((threadIdx.x & 31) == 0) qs[kb] = mx * (1.0f / 127.0f);
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+        for (int j = 0; j < N; j++) top[j] = fmaxf(top[j], __shfl_xor_sync(mask, top[j], o));
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const unsigned e = min(max(__float_as_uint(top[j]) >> 23, 22u), 254u);  // the largest value lies below 2^(e - 126)
+        const float up = __uint_as_float((275u - e) << 23);                     // 2^(148 - e)
+        // the low three bytes of (I + 0x8080) ^ 0x8080 are the digits, each in -128 .. 127 (0x400000: the low bits of the magic number)
+        auto digits = [&](float x, uint32_t& rest) {
+            const float t = fmaf(x, up, kRoundMagic);
+            if (WT == WT_Q4_0) rest = __float_as_uint(fmaf(fminf(fmaf(x, up, kRoundMagic - t), 127.0f / 256.0f), 256.0f, kRoundMagic));  // what is left, in 1 / 256
+            return (__float_as_uint(t) + 0x8080u - 0x400000u) ^ 0x8080u;
+        };
+        uint32_t ra = 0, rb = 0, rc = 0, rd = 0;
+        const uint32_t a = digits(v[j].x, ra), b = digits(v[j].y, rb), c = digits(v[j].z, rc), d = digits(v[j].w, rd);
+        const uint32_t ab = __byte_perm(a, b, 0x5140), cd = __byte_perm(c, d, 0x5140);
+        const int e0 = k[j] & 31;
+        uint32_t* const dst = reinterpret_cast<uint32_t*>(xq + (k[j] >> 5) * (32 * qx_digits(WT)) + ((e0 & 15) << 1) + ((e0 >> 4) << 2));
+        if (live[j]) {
+            dst[0] = __byte_perm(__byte_perm(a, b, 0x0062), __byte_perm(c, d, 0x0062), 0x5410);
+            dst[8] = __byte_perm(ab, cd, 0x7632);
+            dst[16] = __byte_perm(ab, cd, 0x5410);
+            if (WT == WT_Q4_0) dst[24] = __byte_perm(__byte_perm(ra, rb, 0x0040), __byte_perm(rc, rd, 0x0040), 0x5410);
+            if (e0 == 0) qs[k[j] >> 5] = __uint_as_float((e - 21u) << 23);  // 2^(e - 148)
+        }
+    }
 }
 
 __device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -713,258 +635,293 @@ __device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, ui
         : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// Q8_0 chunk: [block][row][piece t: the int8 of columns 4t..4t+3 and 16+4t..16+4t+3], then the scales [block][row] fp16.
-__device__ __forceinline__ float2 mega_tile_dot_q8(const uint8_t* chunk, int R, int n_kb, int tile, int kb0, int kb1, const uint8_t* xq, const float* qs, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-    const int row = tile * 16 + g;
-    const uint8_t* wp = chunk + ((size_t)row * 32 + t * 8);
-    const size_t kstride = (size_t)R * 32;
-    const __half* sp = reinterpret_cast<const __half*>(chunk + (size_t)R * n_kb * 32) + row;
-    const uint8_t* xp = xq + (g < 3 ? g * 32 + t * 8 : 0);
-    // a lane's two result columns are one number, 128 c[0] + c[1] (below 2^27: exact as an integer), in units of 1 / 128 for
-    // t = 0 (digits 0 and 1) and of 1 / 2^21 for t = 1 (digit 2; the next column is zero, like all of the other lanes')
-    float a0 = 0.f, a8 = 0.f;
-#pragma unroll 4
-    for (int kb = kb0; kb < kb1; kb++) {
-        uint2 b = make_uint2(0, 0);
-        if (g < 3) b = *reinterpret_cast<const uint2*>(xp + kb * 128);
-        const float q = qs[kb];
-        const float s0 = __half2float(sp[(size_t)kb * R]), s8 = __half2float(sp[(size_t)kb * R + 8]);
-        const uint2 w0 = *reinterpret_cast<const uint2*>(wp + kb * kstride);
-        const uint2 w8 = *reinterpret_cast<const uint2*>(wp + kb * kstride + 8 * 32);
-        int c[4] = {0, 0, 0, 0};
-        mma_s8(c, w0.x, w8.x, w0.y, w8.y, b.x, b.y);
-        a0 = fmaf(s0 * q, (float)(c[0] * 128 + c[1]), a0);
-        a8 = fmaf(s8 * q, (float)(c[2] * 128 + c[3]), a8);
-    }
-    const float unit = t == 0 ? 1.0f / 128.0f : 1.0f / 2097152.0f;
-    a0 *= unit;
-    a8 *= unit;
-    // lanes t = 0 and t = 1 hold the two parts of every row's sum
-    a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
-    a8 += __shfl_xor_sync(0xffffffffu, a8, 1);
-    return make_float2(a0, a8);
-}
 
-// ---- Q4_0: widened to fp16 in registers (why not the int8 path: see the note above qx_byte) ----
-__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
-// Four bytes of a Q4_0 block (low nibble = element j, high nibble = element j + 16) -> four half2: the low nibbles of
-// bytes (0,1), (2,3), then the high nibbles of (0,1), (2,3), each minus 8.
-__device__ __forceinline__ void q4_widen(uint32_t w, uint32_t (&o)[4]) {
-    const uint32_t x = w & 0x0F0F0F0Fu, y = (w >> 4) & 0x0F0F0F0Fu;
-    const __half2 bias = __floats2half2_rn(1032.f, 1032.f);
-    o[0] = h2_bits(__hsub2(u32_as_h2(__byte_perm(x, 0x64646464u, 0x4140)), bias));
-    o[1] = h2_bits(__hsub2(u32_as_h2(__byte_perm(x, 0x64646464u, 0x4342)), bias));
-    o[2] = h2_bits(__hsub2(u32_as_h2(__byte_perm(y, 0x64646464u, 0x4140)), bias));
-    o[3] = h2_bits(__hsub2(u32_as_h2(__byte_perm(y, 0x64646464u, 0x4342)), bias));
-}
+// ------------------------------------------------------------------------------------------------ products
 
-// Q4_0 chunk: [block][row][16 bytes: piece t = bytes 2t, 2t+1, 2t+8, 2t+9 of the GGUF block], then the scales.
-template <int NP>
-__device__ __forceinline__ float2 mega_tile_dot_q4(const uint8_t* chunk, int R, int n_kb, int tile, int kb0, int kb1, const uint8_t* xa, int lane) {
-    float a0 = 0.f, a8 = 0.f;
-    const int row = tile * 16 + (lane >> 2);
-    const uint8_t* wp = chunk + ((size_t)row * 16 + (lane & 3) * 4);
-    const size_t kstride = (size_t)R * 16;
-    const __half* sp = reinterpret_cast<const __half*>(chunk + (size_t)R * n_kb * 16) + row;
-    const uint8_t* xp = xa + lane * 16;
-#pragma unroll 2
-    for (int kb = kb0; kb < kb1; kb++) {
-        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(wp + kb * kstride);
-        const uint32_t w8 = *reinterpret_cast<const uint32_t*>(wp + kb * kstride + 8 * 16);
-        const float s0 = __half2float(sp[(size_t)kb * R]), s8 = __half2float(sp[(size_t)kb * R + 8]);
-        uint4 xv = make_uint4(0, 0, 0, 0);
-        if (lane < 8 * NP) xv = *reinterpret_cast<const uint4*>(xp + kb * (128 * NP));
-        uint32_t g[4], h[4];
-        q4_widen(w0, g);
-        q4_widen(w8, h);
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_16816(c, g[0], h[0], g[1], h[1], xv.x, xv.y);
-        mma_16816(c, g[2], h[2], g[3], h[3], xv.z, xv.w);
-        a0 = fmaf(s0, c[0] + c[1], a0);
-        a8 = fmaf(s8, c[2] + c[3], a8);
-    }
-    return make_float2(a0, a8);
-}
-
-template <int WT, int NP>
-__device__ __forceinline__ float2 mega_tile_dot(const uint8_t* chunk, int R, int n_kb, int tile, int kb0, int kb1, const uint8_t* xa, const float* qs, int lane) {
-    if constexpr (WT == WT_Q8_0) return mega_tile_dot_q8(chunk, R, n_kb, tile, kb0, kb1, xa, qs, lane);
-    else if constexpr (WT == WT_Q4_0) return mega_tile_dot_q4<NP>(chunk, R, n_kb, tile, kb0, kb1, xa, lane);
-    else return mega_tile_dot_f16<NP>(chunk, R, n_kb, tile, kb0, kb1, xa, lane);
-}
-
-// All products of one chunk (R <= kMegaChunkRows rows over n_kb column blocks), spread over the consumer warps as
-// (16-row tile, column range) units; the number of column ranges is a power of two so that a warp finds its unit with
-// shifts (per chunk every scalar instruction of this set-up is on the critical path of the token).  Unit u = tile <<
-// lg | range stores its sixteen partial sums at partial[u * 16 ...] (position q: + q * kMegaChunkRows); returns lg.  The
-// caller synchronises before reading.
-// log2 of the column ranges of a chunk of R rows: the largest value with tiles << lg <= warps and 1 << lg <= n_kb.
-__device__ __forceinline__ int mega_chunk_lg(int R, int n_kb) {
-    const int n_tiles = (R + 15) >> 4;
-    const int lg_t = n_tiles > 1 ? 32 - __clz(n_tiles - 1) : 0;  // ceil(log2(tiles))
-    return max(0, min(4 - lg_t, 31 - __clz(n_kb)));
-}
-template <int WT, int NP = 1>
-__device__ __forceinline__ int mega_chunk_dots(const uint8_t* chunk, int R, int n_kb, const uint8_t* xa, float* partial, int warp, int lane, const float* qs = nullptr) {
-    if (WT == WT_Q8_0 && !qs) qs = reinterpret_cast<const float*>(xa + (size_t)n_kb * 128);  // block scales behind the staged vector
-    const int n_tiles = (R + 15) >> 4, lg = mega_chunk_lg(R, n_kb);
-    const int per = (n_kb + (1 << lg) - 1) >> lg;
-    for (int u = warp; u < (n_tiles << lg); u += kMegaConsumerWarps) {
-        const int tile = u >> lg, part = u & ((1 << lg) - 1);
-        const float2 y = mega_tile_dot<WT, NP>(chunk, R, n_kb, tile, part * per, min(n_kb, (part + 1) * per), xa, qs, lane);
-        if ((lane & 3) < NP) {
-            float* dst = partial + (NP > 1 ? (lane & 3) * kMegaChunkRows : 0) + u * 16 + (lane >> 2);
-            dst[0] = y.x;
-            dst[8] = y.y;
+// Sums of NT tiles of sixteen rows, kept in registers while a warp goes through the units it owns.
+// fp16: kSets accumulator quads per tile in turn, so that few tiles do not wait for the MMA before (a dependent one comes 35
+// cycles later); quantised: scaled fp32 sums of rows g and g + 8 (lanes t = 0: digits 0 and 1, t = 1: digits 2 and 3).
+template <int WT, int NP, int NT>
+struct MegaSums {
+    static constexpr bool kF16 = WT == WT_F16;
+    static constexpr int kSets = NT == 1 ? 4 : NT == 2 ? 2 : 1;
+    static constexpr int kBatch = NT == 1 ? (kF16 ? 8 : 4) : NT == 2 ? (kF16 ? 6 : 4) : 2;  // units whose loads go out together
+    float f[kF16 ? NT : 1][kF16 ? kSets : 1][4];
+    float a[kF16 ? 1 : NT][2];
+    __device__ __forceinline__ void clear() {
+        if constexpr (kF16) {
+#pragma unroll
+            for (int j = 0; j < NT; j++)
+#pragma unroll
+                for (int x = 0; x < kSets; x++) { f[j][x][0] = 0.f; f[j][x][1] = 0.f; f[j][x][2] = 0.f; f[j][x][3] = 0.f; }
+        } else {
+#pragma unroll
+            for (int j = 0; j < NT; j++) { a[j][0] = 0.f; a[j][1] = 0.f; }
         }
     }
-    return lg;
-}
-// Row r's sum over the column ranges: all loads are issued before the first addition.
-__device__ __forceinline__ float mega_take_sum(const float* partial, int lg, int r) {
-    const float* src = partial + ((r >> 4) << lg) * 16 + (r & 15);
-    float v[16];
+    // Units first, first + step, ... of a chunk's nu (unit i is unit u0 + i of the vector): tiles tile0 .. tile0 + NT - 1 of its
+    // `rows` rows.  Without branches: a batch's units past the last one multiply the last one's weights by zeros, and a tile's rows
+    // past the last one read whatever lies behind it in shared memory; their sums are never stored.
+    __device__ __forceinline__ void add(const uint8_t* chunk, int rows, int nu, int first, int step, int u0, const uint8_t* xa, const float* xq, int lane, int tile0) {
+        const int g = lane >> 2, t = lane & 3;
+        const int db = mega_data_bytes(WT, rows), sb = mega_scale_bytes(WT, rows);
+        constexpr int kPiece = WT == WT_Q4_0 ? 4 : 8, kRow = 4 * kPiece, kTile = 16 * kRow, kXUnit = kF16 ? 64 * NP : 32 * qx_digits(WT);
+        const bool feeds = lane < (kF16 ? 8 * NP : 4 * qx_digits(WT));  // lanes that hold a column of the B operand
+        const uint8_t* const wp = chunk + tile0 * kTile + g * kRow + t * kPiece;
+        const uint8_t* const xp = xa + u0 * kXUnit + lane * 8;  // (quantised: digit g's piece t, 32 g + 8 t)
+        const uint8_t* const sp = chunk + nu * db + tile0 * 32 + g * 4;  // quantised: (scale of row g, of row g + 8) of every tile
+#pragma unroll 1
+        for (int i0 = first; i0 < nu; i0 += step * kBatch) {
+            uint2 b[kBatch], w0[kBatch][NT], w8[kBatch][NT];
+            __half2 sc[kBatch][NT];
+            float q[kBatch];
 #pragma unroll
-    for (int part = 0; part < 16; part++) v[part] = part < (1 << lg) ? src[part * 16] : 0.f;
+            for (int x = 0; x < kBatch; x++) {
+                const int want = i0 + x * step, i = x ? min(want, nu - 1) : i0;
+                b[x] = make_uint2(0, 0);
+                if (feeds && (x == 0 || want < nu)) b[x] = *reinterpret_cast<const uint2*>(xp + i * kXUnit);
+                if (!kF16) q[x] = xq[u0 + i];
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) {
+                for (int j = 0; j < NT; j++) {
+                    const uint8_t* const at = wp + i * db + j * kTile;
+                    if constexpr (WT == WT_Q4_0) {
+                        w0[x][j].y = *reinterpret_cast<const uint32_t*>(at);
+                        w8[x][j].y = *reinterpret_cast<const uint32_t*>(at + 8 * kRow);
+                    } else {
+                        w0[x][j] = *reinterpret_cast<const uint2*>(at);
+                        w8[x][j] = *reinterpret_cast<const uint2*>(at + 8 * kRow);
+                    }
+                    if (!kF16) sc[x][j] = *reinterpret_cast<const __half2*>(sp + i * sb + j * 32);
+                }
+            }
 #pragma unroll
-        for (int part = 0; part < o; part++) v[part] += v[part + o];
+            for (int x = 0; x < kBatch; x++)
+#pragma unroll
+                for (int j = 0; j < NT; j++) {
+                    if constexpr (kF16) {
+                        mma_16816(f[j][x % kSets], w0[x][j].x, w8[x][j].x, w0[x][j].y, w8[x][j].y, b[x].x, b[x].y);
+                    } else {
+                        if constexpr (WT == WT_Q4_0) {  // two's-complement nibbles: bytes of 16 times the weight (the low ones: columns 4t.., the high ones: 16 + 4t..)
+                            w0[x][j].x = (w0[x][j].y << 4) & 0xF0F0F0F0u; w0[x][j].y &= 0xF0F0F0F0u;
+                            w8[x][j].x = (w8[x][j].y << 4) & 0xF0F0F0F0u; w8[x][j].y &= 0xF0F0F0F0u;
+                        }
+                        int c[4] = {0, 0, 0, 0};
+                        mma_s8(c, w0[x][j].x, w8[x][j].x, w0[x][j].y, w8[x][j].y, b[x].x, b[x].y);
+                        // a lane's two result columns are one number, 256 c[0] + c[1] (at most 2^27 + 2^19)
+                        const float2 s = __half22float2(sc[x][j]);
+                        a[j][0] = fmaf(s.x * q[x], (float)(c[0] * 256 + c[1]), a[j][0]);
+                        a[j][1] = fmaf(s.y * q[x], (float)(c[2] * 256 + c[3]), a[j][1]);
+                    }
+                }
+        }
+    }
+    // The sums of rows tile * 16 + g (.x) and + 8 (.y) of position t, in the lanes with t < NP.
+    __device__ __forceinline__ float2 take(int j, int lane) {
+        if constexpr (kF16) {
+            float v[4] = {f[j][0][0], f[j][0][1], f[j][0][2], f[j][0][3]};
+#pragma unroll
+            for (int x = 1; x < kSets; x++) { v[0] += f[j][x][0]; v[1] += f[j][x][1]; v[2] += f[j][x][2]; v[3] += f[j][x][3]; }
+            return make_float2(v[0] + v[1], v[2] + v[3]);  // column 2q of the product is w . x_hi, column 2q + 1 is w . x_lo
+        } else {
+            constexpr float kOne = WT == WT_Q4_0 ? 1.0f / 16.0f : 1.0f;
+            const float unit = (lane & 3) == 0 ? 256.0f * kOne : kOne / 256.0f;  // t = 0: digits 0 and 1; t = 1: digits 2 and 3 (the other lanes' columns are zero)
+            float x = a[j][0] * unit, y = a[j][1] * unit;
+            x += __shfl_xor_sync(0xffffffffu, x, 1);
+            y += __shfl_xor_sync(0xffffffffu, y, 1);
+            return make_float2(x, y);
+        }
+    }
+};
+
+// The sums over the warps of rows r and r + 1 (r even): all loads are issued before the first addition.
+__device__ __forceinline__ float2 mega_take_sum2(const float* sums, int stride, int r) {
+    float2 v[kMegaConsumerWarps];
+#pragma unroll
+    for (int x = 0; x < kMegaConsumerWarps; x++) v[x] = *reinterpret_cast<const float2*>(sums + x * stride + r);
+#pragma unroll
+    for (int o = kMegaConsumerWarps / 2; o > 0; o >>= 1) {
+#pragma unroll
+        for (int x = 0; x < o; x++) { v[x].x += v[x + o].x; v[x].y += v[x + o].y; }
     }
     return v[0];
 }
+__device__ __forceinline__ float mega_sum_warps(const float* red) {
+    const float4* r4 = reinterpret_cast<const float4*>(red);
+    float v[kMegaConsumerWarps / 4];
+#pragma unroll
+    for (int i = 0; i < kMegaConsumerWarps / 4; i++) v[i] = (r4[i].x + r4[i].y) + (r4[i].z + r4[i].w);
+    if (kMegaConsumerWarps == 8) return v[0] + v[1];
+    return (v[0] + v[1]) + (v[kMegaConsumerWarps / 4 - 2] + v[kMegaConsumerWarps / 4 - 1]);
+}
+// The sum of v0 and the maximum of v1 >= 0 over the consumer threads (GPT-2).  One CTA barrier.
+__device__ __forceinline__ float2 mega_block_sum_max(float v0, float v1, float* red) {
+    v1 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v1)));  // (non-negative floats order as their bits)
+    v0 = warp_sum(v0);
+    if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5] = v0; red[kMegaConsumerWarps + (threadIdx.x >> 5)] = v1; }
+    consumer_sync();
+    const float4* r4 = reinterpret_cast<const float4*>(red + kMegaConsumerWarps);
+    float top = 0.f;
+#pragma unroll
+    for (int q = 0; q < kMegaConsumerWarps / 4; q++) top = fmaxf(top, fmaxf(fmaxf(r4[q].x, r4[q].y), fmaxf(r4[q].z, r4[q].w)));
+    return make_float2(mega_sum_warps(red), top);
+}
 
-// ------------------------------------------------------------------------------------------------ consumer stages
+// ------------------------------------------------------------------------------------------------ attention
 
-// S2: attention of one head over the cached positions [0, pos) plus the new token (whose key and value are in
-// shared memory), then this CTA's block of the output projection.
-// Each warp owns the positions t = warp + 16*i (16 per round).  Four neighbouring lanes share one position: each loads
+// S2: attention of one head over the cached positions [0, n_cached) plus the new ones (whose keys and values are in
+// shared memory).
+// Each warp owns the positions t = warp + NW*i (8 kSt per round).  Four neighbouring lanes share one position: each loads
 // a quarter of its K row with 16-byte vectors and the score is completed with two shuffles.  The probabilities are
 // then broadcast position by position while every lane accumulates its own channels of V.  The K and V rows of the
-// first round are requested by the caller's thread before the query is known (see `prefetch`), and the sixteen
+// first round are requested before the query is known, and the new positions take their place in the round like cached ones.  The
 // per-warp (max, sum, ctx) triples are merged once, by all threads: a few lanes per output channel, combined with
-// shuffles (two warps walking all sixteen triples took 0.3 us longer per layer).
-template <int HD>
+// shuffles (two warps walking all triples took 0.3 us longer per layer).
+template <int HD, int NW>  // NW = warps that share one query
 struct MegaKvRound {
-    uint4 kreg[2][HD / 32];
-    uint2 vreg[16];
+    static constexpr int kPieces = HD / 32, kPer = HD / 32;  // 16-byte pieces of a quarter of a key; channels of a lane
+    static constexpr int kSt = HD == 128 ? 2 : 4;            // positions of a lane (of a warp: 8 kSt)
+    uint4 k[kSt][kPieces];
+    uint2 v[8 * kSt];
+    // K, V: the head's rows of the cache; positions past the cached ones read as zeros.
+    __device__ __forceinline__ void load(const __half* K, const __half* V, int base, int n_cached, int warp, int lane) {
+        const int sub = lane & 3, tl = lane >> 2, left = n_cached - base - warp;
+        const __half* kp = K + (size_t)(base + warp + NW * tl) * HD + sub * (HD / 4);
+#pragma unroll
+        for (int st = 0; st < kSt; st++)
+#pragma unroll
+            for (int c = 0; c < kPieces; c++) {
+                k[st][c] = make_uint4(0, 0, 0, 0);
+                if (NW * (st * 8 + tl) < left) k[st][c] = __ldcg(reinterpret_cast<const uint4*>(kp + st * 8 * NW * HD) + c);
+            }
+        const __half* vp = V + (size_t)(base + warp) * HD + lane * kPer;
+#pragma unroll
+        for (int j = 0; j < 8 * kSt; j++) {
+            v[j] = make_uint2(0, 0);
+            if (NW * j < left) {
+                if (kPer == 4) v[j] = __ldcg(reinterpret_cast<const uint2*>(vp + j * NW * HD));
+                else if (kPer == 2) v[j].x = __ldcg(reinterpret_cast<const unsigned int*>(vp + j * NW * HD));
+                else v[j].x = (unsigned int)__ldcg(reinterpret_cast<const unsigned short*>(vp + j * NW * HD));
+            }
+        }
+    }
+    // The keys of the new positions n_cached .. last that fall into this round, from shared memory.
+    __device__ __forceinline__ void take_new(const __half* kn, int base, int n_cached, int last, int warp, int lane) {
+        const int sub = lane & 3, tl = lane >> 2;
+#pragma unroll
+        for (int st = 0; st < kSt; st++) {
+            const int t = base + warp + NW * (st * 8 + tl);
+            if (t >= n_cached && t <= last) {
+#pragma unroll
+                for (int c = 0; c < kPieces; c++) k[st][c] = *(reinterpret_cast<const uint4*>(kn + (t - n_cached) * HD + sub * (HD / 4)) + c);
+            }
+        }
+    }
 };
 
-template <int HD, int NW = kMegaConsumerWarps>  // NW = warps that share one query (position t belongs to warp t % NW)
-__device__ __forceinline__ void mega_kv_load(MegaKvRound<HD>& r, const __half* K, const __half* V, int base, int n_cached, int warp, int lane) {
-    constexpr int cpl = HD / 32, KV4 = HD / 32;
-    const int sub = lane & 3, tl = lane >> 2;
-#pragma unroll
-    for (int st = 0; st < 2; st++) {
-        const int t = base + warp + NW * (st * 8 + tl);
-#pragma unroll
-        for (int c = 0; c < KV4; c++) {
-            r.kreg[st][c] = make_uint4(0, 0, 0, 0);
-            if (t < n_cached) r.kreg[st][c] = __ldcg(reinterpret_cast<const uint4*>(K + (size_t)t * HD + sub * (HD / 4)) + c);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-        const int t = base + warp + NW * j;
-        r.vreg[j] = make_uint2(0, 0);
-        if (t < n_cached) {
-            const __half* vr = V + (size_t)t * HD + lane * cpl;
-            if (cpl == 4) r.vreg[j] = __ldcg(reinterpret_cast<const uint2*>(vr));
-            else if (cpl == 2) r.vreg[j].x = __ldcg(reinterpret_cast<const unsigned int*>(vr));
-            else r.vreg[j].x = (unsigned int)__ldcg(reinterpret_cast<const unsigned short*>(vr));
-        }
-    }
+// Row of the cache (head_dim elements each) of sequence 0; a cache that fits the device has fewer than 2^32 of them.
+__device__ __forceinline__ unsigned mega_kv_row(const ModelDims& m, int layer, int kvh, int pos) {
+    return ((unsigned)layer * (unsigned)m.n_seq * (unsigned)m.n_kv_head + (unsigned)kvh) * (unsigned)m.max_seq + (unsigned)pos;
+}
+// Maximum over a warp through the integer reduction: the bits of a float, the lower 31 flipped where it is negative, order like it.
+__device__ __forceinline__ float mega_warp_max(float v) {
+    int i = __float_as_int(v);
+    i ^= (i >> 31) & 0x7fffffff;
+    i = __reduce_max_sync(0xffffffffu, i);
+    i ^= (i >> 31) & 0x7fffffff;
+    return __int_as_float(i);
 }
 
 // With NP positions per pass the consumer warps split into NP teams of NW = 16 / NP warps, one team per query: query qi
 // sees the n_cached cached positions and the new positions 0 .. qi, whose keys and values are rows of s.kn / s.vn; its
 // context lands in position qi of the staged s.ctx.  The teams run side by side (each reads the cached rows itself).
-template <int HD, int NP = 1, int QCTX = 0, class WaitQ>  // QCTX: 0 = fp16 context staging, 1 = int8 digits
-__device__ __forceinline__ void mega_attention(const MegaArgs& a, const MegaShared& s, const MegaShare& w, const ModelDims& m, const KvLayout& kv, int layer, int n_cached,
-                                               WaitQ wait_q) {
+// The context is staged as the products of weights of type WT read it.
+template <int HD, int NP, int WT, class WaitQ>
+__device__ __forceinline__ void mega_attention(const MegaShared& s, const MegaShare& w, const ModelDims& m, const KvLayout& kv, int layer, int n_cached, WaitQ wait_q) {
     constexpr int NW = kMegaConsumerWarps / NP;
     const int tid = threadIdx.x, lane = tid & 31;
     const int qi = (tid >> 5) / NW, warp = (tid >> 5) - qi * NW;  // this warp's query and its place in the team
     constexpr int cpl = HD / 32, KV4 = HD / 32;
-    const int visible = n_cached + 1;
-    const __half* K = kv.k + kv.offset(m, layer, 0, w.kvh, 0);
-    const __half* V = kv.v + kv.offset(m, layer, 0, w.kvh, 0);
-    const float* qs = s.qs + qi * HD;
-    const float scale = 1.0f / sqrtf((float)HD);
+    const int last = n_cached + qi;  // newest position this query sees
+    const size_t head = (size_t)mega_kv_row(m, layer, w.kvh, 0) * HD;
+    const __half* K = kv.k + head;
+    const __half* V = kv.v + head;
     const int sub = lane & 3, tl = lane >> 2;
-    constexpr int kRound = NW * 16;  // positions per round of a team
-    float m_w = -INFINITY, l_w = 0.f;
+    constexpr int kSt = MegaKvRound<HD, NW>::kSt, kRound = NW * 8 * kSt;  // positions per round of a team
+    constexpr float scale = HD == 32 ? 0.17677669529663687f : HD == 64 ? 0.125f : 0.08838834764831845f;  // 1 / sqrt(HD)
+    const float4* const qv = reinterpret_cast<const float4*>(s.qs + qi * HD + sub * (HD / 4));  // this lane's quarter of the query
+    float m_w = -INFINITY, l_w = 0.f;  // l_w: this lane's share (every probability sits in four lanes)
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int base = 0; base < visible - 1 || base == 0; base += kRound) {
-        // cached rows of this round (the newest position is not in the cache: its key and value come with the query)
-        MegaKvRound<HD> cur;
-        mega_kv_load<HD, NW>(cur, K, V, base, visible - 1, warp, lane);
+#pragma unroll 1
+    for (int base = 0; base < n_cached + NP; base += kRound) {
+        MegaKvRound<HD, NW> cur;
+        cur.load(K, V, base, n_cached, warp, lane);
         if (base == 0) wait_q();  // the loads above are in flight while the query is awaited
-        float sc[2];
-        float mx = -INFINITY;
+        const bool news = base + kRound > n_cached;  // the new positions may fall into this round
+        if (news) cur.take_new(s.kn, base, n_cached, last, warp, lane);
+        float sc[kSt], top = -INFINITY;
 #pragma unroll
-        for (int st = 0; st < 2; st++) {
+        for (int st = 0; st < kSt; st++) {
             const int t = base + warp + NW * (st * 8 + tl);
-            float dot = 0.f;
+            float d0 = 0.f, d1 = 0.f;
 #pragma unroll
             for (int c = 0; c < KV4; c++) {
-                const uint32_t ww[4] = {cur.kreg[st][c].x, cur.kreg[st][c].y, cur.kreg[st][c].z, cur.kreg[st][c].w};
-                const float* qv = qs + sub * (HD / 4) + c * 8;
+                const uint32_t ww[4] = {cur.k[st][c].x, cur.k[st][c].y, cur.k[st][c].z, cur.k[st][c].w};
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&ww[i]));
-                    dot = fmaf(f.x, qv[2 * i], dot);
-                    dot = fmaf(f.y, qv[2 * i + 1], dot);
+                for (int i = 0; i < 2; i++) {
+                    const float4 q = qv[2 * c + i];
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&ww[2 * i])), h = __half22float2(*reinterpret_cast<const __half2*>(&ww[2 * i + 1]));
+                    d0 = fmaf(f.x, q.x, d0);
+                    d1 = fmaf(f.y, q.y, d1);
+                    d0 = fmaf(h.x, q.z, d0);
+                    d1 = fmaf(h.y, q.w, d1);
                 }
             }
+            float dot = (d0 + d1) * scale;
             dot += __shfl_xor_sync(0xffffffffu, dot, 1);
             dot += __shfl_xor_sync(0xffffffffu, dot, 2);
-            sc[st] = t < visible - 1 ? dot * scale : -INFINITY;
-            mx = fmaxf(mx, sc[st]);
+            sc[st] = t <= last ? dot : -INFINITY;
+            top = fmaxf(top, sc[st]);
         }
-        const float m_new = fmaxf(m_w, warp_max(mx));
-        float pr[2], psum = 0.f;
+        const float m_new = fmaxf(m_w, mega_warp_max(top));
+        float pr[kSt], psum = 0.f;
 #pragma unroll
-        for (int st = 0; st < 2; st++) {
+        for (int st = 0; st < kSt; st++) {
             pr[st] = sc[st] == -INFINITY ? 0.f : __expf(sc[st] - m_new);
             psum += pr[st];
         }
         const float corr = m_w == -INFINITY ? 0.f : __expf(m_w - m_new);
-        l_w = l_w * corr + 0.25f * warp_sum(psum);  // every probability sits in four lanes
+        l_w = fmaf(l_w, corr, psum);
 #pragma unroll
         for (int c = 0; c < 4; c++) acc[c] *= corr;
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
+        for (int j = 0; j < 8 * kSt; j++) {
             const float pj = __shfl_sync(0xffffffffu, pr[j >> 3], (j & 7) * 4);
-            const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&cur.vreg[j].x));
-            const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&cur.vreg[j].y));
+            const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&cur.v[j].x));
+            const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&cur.v[j].y));
             acc[0] = fmaf(pj, f0.x, acc[0]);
             if (cpl >= 2) acc[1] = fmaf(pj, f0.y, acc[1]);
             if (cpl == 4) { acc[2] = fmaf(pj, f1.x, acc[2]); acc[3] = fmaf(pj, f1.y, acc[3]); }
         }
+        if (news) {  // (their values were zeros above)
+#pragma unroll
+            for (int jj = 0; jj < NP; jj++) {
+                const int at = n_cached + jj - base - warp;  // position n_cached + jj is this warp's number at / NW
+                if (jj <= qi && at >= 0 && at < kRound && at % NW == 0) {
+                    const int j = at / NW;
+                    float mine = pr[0];
+#pragma unroll
+                    for (int st = 1; st < kSt; st++) mine = j >> 3 == st ? pr[st] : mine;
+                    const float pj = __shfl_sync(0xffffffffu, mine, (j & 7) * 4);
+                    const __half* vn = s.vn + jj * HD + lane * cpl;
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        if (c < cpl) acc[c] = fmaf(pj, __half2float(vn[c]), acc[c]);
+                }
+            }
+        }
         m_w = m_new;
     }
-    // the new positions: keys and values from shared memory, each handled by one warp as a round of a single position
-#pragma unroll
-    for (int j = 0; j < NP; j++) {
-        if (j <= qi && warp == (n_cached + j) % NW) {
-            const __half* kn = s.kn + j * HD;
-            const __half* vn = s.vn + j * HD;
-            float dot = 0.f;
-#pragma unroll
-            for (int c = 0; c < cpl; c++) dot = fmaf(qs[lane * cpl + c], __half2float(kn[lane * cpl + c]), dot);
-            const float sn = warp_sum(dot) * scale;
-            const float m_new = fmaxf(m_w, sn);
-            const float corr = m_w == -INFINITY ? 0.f : __expf(m_w - m_new);
-            const float pn = __expf(sn - m_new);
-            l_w = l_w * corr + pn;
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (c < cpl) acc[c] = fmaf(pn, __half2float(vn[lane * cpl + c]), acc[c] * corr);
-            m_w = m_new;
-        }
-    }
+    l_w = 0.25f * warp_sum(l_w);
     // merge the per-warp partial results of every team (a warp that saw no position carries max = -inf, sum = 0)
     const int gw = tid >> 5;  // warp index among all consumers
 #pragma unroll
@@ -998,146 +955,733 @@ __device__ __forceinline__ void mega_attention(const MegaArgs& a, const MegaShar
         }
         // the staged operand of the Wo products
         const float cv = den > 0.f ? __fdividef(num, den) : 0.f;
-        if constexpr (QCTX != 0) {
-            // int8 digit staging works on whole warps of consecutive elements: the channel values are gathered first
+        if constexpr (WT != WT_F16) {
+            // int8 digit staging works on whole blocks of consecutive elements: the channel values are gathered first
             // (in the query's place: every warp is past its scores)
             static_assert(NP == 1, "int8 context staging handles one position");
             if (xr == 0) s.qs[ch] = cv;
             consumer_sync();
-            if (tid < HD) qx_store_elem(reinterpret_cast<uint8_t*>(s.ctx), reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(s.ctx) + xa_bytes(HD)), tid, s.qs[tid]);
+            if (tid < HD / 4) {
+                const int k[1] = {4 * tid};
+                const float4 v[1] = {*reinterpret_cast<const float4*>(s.qs + 4 * tid)};
+                const bool live[1] = {true};
+                qx_store_quads<WT, 1>(s.ctx, reinterpret_cast<float*>(s.ctx + xa_bytes(WT, HD, 1)), k, v, live, 0xffu << (lane & 24));
+            }
         } else {
-            if (xr == 0) xa_store<NP>(reinterpret_cast<__half*>(s.ctx), ch, cv, qq);
+            if (xr == 0) xa_store<NP>(s.ctx, ch, cv, qq);
         }
     }
     consumer_sync();
 }
 
+// ------------------------------------------------------------------------------------------------ consumers
+
+// The model a pass runs through.
+struct MegaModel {
+    const float* norms;       // [2 n_layer + 1][d_model]
+    const uint16_t* tok_emb;
+    KvLayout kv;
+};
+
+// The larger of two arg-max words held by the lanes of a warp: [ordered logit bits : 32][0xffffff - index : 24][tag : 8].  Two
+// integer reductions: the largest logit, then the largest rest among the lanes that have it.
+__device__ __forceinline__ unsigned long long mega_warp_best(unsigned long long k) {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : 0u);
+    return ((unsigned long long)hi << 32) | lo;
+}
+
+// The consumer warps of a CTA.  A pass is one forward step for NP consecutive token positions, or only its LM head.
+// Every stage's operand vector is dealt out to the warps by K units (unit u to warp u % 8): a warp polls the words of its own
+// columns, stages them for the tensor cores and multiplies them with all rows of the CTA, and nothing is shared between the
+// warps before their partial sums meet.  One CTA barrier per stage remains: the norm's sum of squares meets there too (RMSNorm
+// scales the sums, so the products need not wait for it), and a warp's products start when its own columns have arrived.
+//
+// The bound of the small models is the issue rate: a layer is one pass over straight-line code, and every warp issues it.  Eight
+// warps instead of sixteen, two per scheduler, halve what the set-up, the polling and the reductions cost and leave each warp the
+// registers to keep twice the loads in flight; an own copy of the code per stage keeps the selection between the stages out
+// of it.
+template <int HD, int WT, bool GPT2, int NP>
+struct MegaWorker {
+    static constexpr bool kQuant = WT != WT_F16;
+    static constexpr int half = HD / 2;
+    const MegaArgs& a;
+    const MegaShared& s;
+    const MegaShare& w;  // in shared memory, read wherever it is needed: no registers, no recomputation
+    const int tid, warp, lane;
+    MegaCursor c, pend_from;           // ring position, advances in lock step with the producer's; first slot whose release was put off
+    unsigned n_chunk = 0, landed = 0;  // chunks consumed so far; chunks known to have arrived
+    int par = 0;                       // which half of s.sums the next group's sums go to
+    int n_pend = 0;
+    int n_stamp = 0;
+    bool tracing = false;
+
+    __device__ __forceinline__ MegaWorker(const MegaArgs& a_, const MegaShared& s_)
+        : a(a_), s(s_), w(*s_.share), tid((int)threadIdx.x), warp((int)threadIdx.x >> 5), lane((int)threadIdx.x & 31) {}
+
+    __device__ __forceinline__ void stamp() {
+        if (tracing) a.trace[n_stamp++] = clock64();
+    }
+
+    // A freed slot makes the producer request the chunk that is n_slots ahead at once: megabytes of reads over all
+    // CTAs, which would travel through L2 together with the words of the exchange that follows the stage and delay
+    // them by microseconds.  The last chunk of a stage is therefore handed back only after that exchange (the chunk it
+    // makes room for is needed later; 22-layer d2048 model, Q8_0: 441 us per token without, 429 with).
+    __device__ __forceinline__ void release_pending() {
+        if (n_pend) mega_release_deferred(a, s, pend_from, n_pend);
+        n_pend = 0;
+    }
+    __device__ __forceinline__ void hand_back(bool later) {
+        if (later) {
+            if (n_pend == 0) pend_from = c;
+            n_pend++;
+            c.next((unsigned)a.plan.n_slots);
+        } else {
+            mega_release(a, s, c);
+        }
+    }
+
+    // ---- products
+
+    // One group of rows: this warp's partial sums to `mine`.
+    template <int W2, int NT>
+    __device__ __forceinline__ void group_products(const MegaStage& st, int n, int keep, float* mine) {
+        const int tiles = (n + 15) >> 4;
+        MegaSums<W2, NP, NT> acc;
+        acc.clear();
+#pragma unroll 1
+        for (int u0 = 0; u0 < st.units; u0 += st.chunk_units) {
+            const int nu = min(st.chunk_units, st.units - u0);
+            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++, landed);
+            acc.add(ch, n, nu, (warp - u0) & (kMegaConsumerWarps - 1), kMegaConsumerWarps, u0, s.xa, s.xq, lane, 0);
+            hand_back(u0 + keep * st.chunk_units >= st.units);
+        }
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            const float2 y = acc.take(j, lane);
+            if (j < tiles && (lane & 3) < NP) {
+                float* dst = mine + (lane & 3) * 16 * a.plan.group_tiles + j * 16 + (lane >> 2);
+                dst[0] = y.x;
+                dst[8] = y.y;
+            }
+        }
+    }
+    // This CTA's rows of Wo restricted to its head's columns: every row's sum is one contribution to the counted sum of that row
+    // (head 0 also carries the residual).  A warp owns whole 16-row tiles: its lanes hold finished sums, and no barrier follows.
+    template <int NT>
+    __device__ __forceinline__ void wo_tiles(const uint8_t* ch, int n, int r0, int l) {
+        const int d = a.m.d_model, all = (n + 15) >> 4;
+#pragma unroll 1
+        for (int tile = NT * warp; tile < all; tile += NT * kMegaConsumerWarps) {
+            MegaSums<WT, NP, NT> acc;
+            acc.clear();
+            acc.add(ch, n, HD / mega_unit(WT), 0, 1, 0, s.ctx, reinterpret_cast<const float*>(s.ctx + xa_bytes(WT, HD, NP)), lane, tile);
+            const int q = lane & 3, first = w.blk * a.plan.rpb + r0, row = first + tile * 16 + (lane >> 2), last = min(d, first + n);
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+                const float2 y = acc.take(j, lane);
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int orow = row + 16 * j + 8 * i;
+                    float v = i ? y.y : y.x;
+                    if (q < NP && orow < last) {
+                        if (w.head == 0) v += s.xres[q * d + orow] + (GPT2 ? __ldg(a.out_bias + (size_t)2 * l * d + orow) : 0.f);
+                        red_add_u64(a.mid_sums + q * d + orow, counted(v));
+                    }
+                }
+            }
+        }
+    }
+    __device__ __forceinline__ void wo_products(const MegaStage& st, int l) {
+#pragma unroll 1
+        for (int r0 = 0; r0 < a.plan.rpb; r0 += st.group_rows) {
+            const int n = min(st.group_rows, a.plan.rpb - r0);
+            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++, landed);
+            if (n <= 16 * kMegaConsumerWarps) wo_tiles<1>(ch, n, r0, l);
+            else wo_tiles<4>(ch, n, r0, l);
+            hand_back(r0 + st.group_rows >= a.plan.rpb);
+        }
+    }
+
+    // ---- staging
+
+    // A lane handles four columns of a quantised type's block, or two of an fp16 unit: eight lanes share a unit.  Items of this warp,
+    // numbered through its units: how many, and which column item `it` starts at.
+    template <int W2>
+    __device__ __forceinline__ int items(int units) const {
+        return units > warp ? (units - warp + kMegaConsumerWarps - 1) / kMegaConsumerWarps * 8 : 0;
+    }
+    template <int W2>
+    __device__ __forceinline__ int column(int it) const {
+        return (warp + (it >> 3) * kMegaConsumerWarps) * mega_unit(W2) + (it & 7) * (mega_unit(W2) / 8);
+    }
+    // N items per lane (of position q, columns k .., `live` or not): the residual stream's raw copy (`stream`), gained copy as the
+    // products' operand, sum of squares.  Without branches, so that the items' latencies overlap; all lanes of the warp call.
+    template <int W2, int N>
+    __device__ __forceinline__ void stage_items(bool stream, const bool (&live)[N], const int (&q)[N], const int (&k)[N], const float (&v)[N][mega_unit(W2) / 8],
+                                                const float (&g)[N][mega_unit(W2) / 8], float (&ss)[NP]) {
+        if constexpr (W2 != WT_F16) {
+            float4 x[N];
+#pragma unroll
+            for (int j = 0; j < N; j++) {
+                if (stream && live[j]) *reinterpret_cast<float4*>(s.xres + k[j]) = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
+                if (stream) ss[0] += fmaf(v[j][0], v[j][0], fmaf(v[j][1], v[j][1], fmaf(v[j][2], v[j][2], v[j][3] * v[j][3])));
+                x[j] = make_float4(v[j][0] * g[j][0], v[j][1] * g[j][1], v[j][2] * g[j][2], v[j][3] * g[j][3]);
+            }
+            qx_store_quads<W2, N>(s.xa, s.xq, k, x, live, 0xffffffffu);
+        } else {
+#pragma unroll
+            for (int j = 0; j < N; j++) {
+                if (stream && live[j]) *reinterpret_cast<float2*>(s.xres + q[j] * a.m.d_model + k[j]) = make_float2(v[j][0], v[j][1]);
+                if (GPT2 && stream) {  // (staged by layer_norm)
+                    ln_sum += v[j][0] + v[j][1];
+                    ln_top = fmaxf(ln_top, fmaxf(fabsf(v[j][0]), fabsf(v[j][1])));
+                    continue;
+                }
+                if (live[j]) xa_store_pair<NP>(s.xa, k[j], v[j][0] * g[j][0], v[j][1] * g[j][1], q[j]);
+                if (!stream) continue;
+                const float sq = fmaf(v[j][0], v[j][0], v[j][1] * v[j][1]);
+                if (NP == 2) {
+                    ss[0] += q[j] ? 0.f : sq;
+                    ss[NP - 1] += q[j] ? sq : 0.f;
+                } else {
+                    ss[0] += sq;
+                }
+            }
+        }
+    }
+    // Polls this warp's columns of an exchanged vector and stages them.  MS_UP: counted sums, complete after n_head contributions;
+    // else words with the tag.  Up to kPolls items of a lane are in flight, words that validated are not read again, and what else
+    // an item needs is requested before its words are awaited.
+    template <int KIND, int W2>
+    __device__ __forceinline__ void stage_words(unsigned tag, const float* gain, float (&ss)[NP]) {
+        constexpr bool kSums = KIND == MS_UP, kAct = KIND == MS_DOWN;
+        constexpr int kCols = mega_unit(W2) / 8, kLoads = kCols / 2;
+        constexpr int kPolls = kAct ? (GPT2 || kQuant ? 6 : 4) : 2;
+        constexpr int kCode = kSums ? 7 : kAct ? 8 : KIND == MS_QKV ? 5 : 9;
+        const int K = kAct ? a.m.hidden : a.m.d_model, n = items<W2>(K / mega_unit(W2)), total = NP * n;
+        const bool lines = kAct && !kQuant && a.plan.act_wpc > 0;
+        const unsigned long long* const base = kAct ? a.act_words : kSums ? a.mid_sums : a.x_words;
+        const unsigned n_contrib = (unsigned)a.m.n_head;
+#pragma unroll 1
+        for (int i0 = 0; i0 < total; i0 += 32 * kPolls) {
+            ulonglong2 wd[kPolls][kLoads];
+            float g[kAct || GPT2 ? 1 : kPolls][kCols];
+            const unsigned long long* src[kPolls];
+            const ulonglong2* prev[kPolls];
+            bool ok[kPolls];
+#pragma unroll
+            for (int j = 0; j < kPolls; j++) {
+                const int it = i0 + 32 * j + lane;
+                ok[j] = it >= total;
+                const int q = NP == 2 && it >= n ? 1 : 0, k = ok[j] ? 0 : column<W2>(it - q * n);
+                src[j] = base + (lines ? q * a.plan.n_cta * a.plan.act_wpc + (int)s.act[k >> 1] : q * K + k);
+                prev[j] = reinterpret_cast<const ulonglong2*>(s.prev + (kSums ? q * K + k : 0));
+#pragma unroll
+                for (int i = 0; i < kLoads; i++) wd[j][i] = make_ulonglong2(0, 0);
+                if constexpr (!kAct && !GPT2) {
+#pragma unroll
+                    for (int i = 0; i < kLoads; i++) {
+                        const float2 f = __ldg(reinterpret_cast<const float2*>(gain + k) + i);
+                        g[j][2 * i] = f.x; g[j][2 * i + 1] = f.y;
+                    }
+                }
+            }
+            unsigned spins = 0;
+            if (!mega_aborting(s)) {
+                while (true) {
+                    bool all = true;
+#pragma unroll
+                    for (int j = 0; j < kPolls; j++)
+                        if (!ok[j]) {
+#pragma unroll
+                            for (int i = 0; i < kLoads; i++) wd[j][i] = ld_words2(src[j] + 2 * i);
+                        }
+#pragma unroll
+                    for (int j = 0; j < kPolls; j++)
+                        if (!ok[j]) {
+                            ok[j] = true;
+#pragma unroll
+                            for (int i = 0; i < kLoads; i++) {
+                                if constexpr (kSums) {
+                                    const ulonglong2 pv = prev[j][i];
+                                    ok[j] = ok[j] && (((unsigned)wd[j][i].x - (unsigned)pv.x) & 0xffu) == n_contrib && (((unsigned)wd[j][i].y - (unsigned)pv.y) & 0xffu) == n_contrib;
+                                } else {
+                                    ok[j] = ok[j] && (unsigned)(wd[j][i].x >> 32) == tag && (unsigned)(wd[j][i].y >> 32) == tag;
+                                }
+                            }
+                            all = all && ok[j];
+                        }
+                    if (all) break;
+                    if (mega_spin_out(a, s, spins, kCode)) break;
+                    mega_backoff();
+                }
+            }
+            __syncwarp();
+            int q[kPolls], k[kPolls];
+            float v[kPolls][kCols], gain_of[kPolls][kCols];
+            bool live[kPolls];
+#pragma unroll
+            for (int j = 0; j < kPolls; j++) {
+                const int it = i0 + 32 * j + lane;
+                live[j] = it < total;
+                q[j] = NP == 2 && it >= n ? 1 : 0;
+                k[j] = live[j] ? column<W2>(it - q[j] * n) : 0;
+#pragma unroll
+                for (int i = 0; i < kLoads; i++) {
+                    if constexpr (kSums) {
+                        ulonglong2* const p = const_cast<ulonglong2*>(prev[j]) + i;
+                        const ulonglong2 pv = *p;
+                        if (live[j]) *p = wd[j][i];
+                        v[j][2 * i] = (float)((long long)(wd[j][i].x - pv.x - (unsigned long long)n_contrib) >> 8) * kMegaUnfix;
+                        v[j][2 * i + 1] = (float)((long long)(wd[j][i].y - pv.y - (unsigned long long)n_contrib) >> 8) * kMegaUnfix;
+                        if (!live[j]) v[j][2 * i] = v[j][2 * i + 1] = 0.f;
+                    } else {
+                        v[j][2 * i] = __uint_as_float((unsigned)wd[j][i].x);
+                        v[j][2 * i + 1] = __uint_as_float((unsigned)wd[j][i].y);
+                    }
+                    gain_of[j][2 * i] = gain_of[j][2 * i + 1] = 1.f;
+                    if constexpr (!kAct && !GPT2) { gain_of[j][2 * i] = g[j][2 * i]; gain_of[j][2 * i + 1] = g[j][2 * i + 1]; }
+                }
+            }
+            stage_items<W2, kPolls>(!kAct, live, q, k, v, gain_of, ss);
+        }
+    }
+    // The same for a pass's first vector: the embedding of the tokens, or (the head alone) the sequence's last hidden state.
+    template <int W2>
+    __device__ __forceinline__ void stage_first(bool hidden, const uint32_t (&tok)[NP], int pos, const uint16_t* tok_emb, const float* gain, float (&ss)[NP]) {
+        constexpr int kCols = mega_unit(W2) / 8;
+        const int d = a.m.d_model, n = items<W2>(d / mega_unit(W2));
+#pragma unroll 1
+        for (int i0 = 0; i0 < NP * n; i0 += 32) {
+            const int it = i0 + lane;
+            const bool live[1] = {it < NP * n};
+            const int q[1] = {NP == 2 && it >= n ? 1 : 0}, k[1] = {live[0] ? column<W2>(it - q[0] * n) : 0};
+            float v[1][kCols], g[1][kCols];
+#pragma unroll
+            for (int i = 0; i < kCols; i += 2) {
+                float2 x;
+                if (hidden) {
+                    x = __ldcg(reinterpret_cast<const float2*>(a.hidden_io + k[0] + i));
+                } else {
+                    x = __half22float2(*reinterpret_cast<const __half2*>(tok_emb + (size_t)(q[0] ? tok[NP - 1] : tok[0]) * d + k[0] + i));
+                    if (GPT2) {
+                        const float2 pe = __half22float2(*reinterpret_cast<const __half2*>(a.pos_emb + (size_t)pos * d + k[0] + i));
+                        x.x += pe.x; x.y += pe.y;
+                    }
+                }
+                const float2 f = GPT2 ? make_float2(1.f, 1.f) : __ldg(reinterpret_cast<const float2*>(gain + k[0] + i));
+                v[0][i] = live[0] ? x.x : 0.f; v[0][i + 1] = live[0] ? x.y : 0.f;
+                g[0][i] = f.x; g[0][i + 1] = f.y;
+            }
+            stage_items<W2, 1>(true, live, q, k, v, g, ss);
+        }
+    }
+    // GPT-2's LayerNorm.  The values are staged only when the mean is known: with a mean far from zero both E[x^2] - mean^2 and
+    // W.(x g) - mean W.g cancel (one barrier less, but a stream of mean 32 and deviation 0.05 had no correct digit left).  The
+    // centred values carry a power of two that puts the largest of them near 32: the fp16 parts then neither saturate on a large
+    // residual stream nor lose their low half to subnormals on a small one.  Every lane normalises the pairs that it received;
+    // ln_down becomes the inverse of the power of two, ss the centred squares.
+    float ln_sum, ln_top, ln_down;
+    __device__ __forceinline__ void layer_norm(const float* gain, float (&ss)[NP]) {
+        const int total = items<WT_F16>(a.m.d_model / mega_unit(WT_F16));
+        float2 ahead[2];  // (d_model <= 1024: all gains; requested before the barrier)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            ahead[j] = make_float2(0.f, 0.f);
+            if (lane + 32 * j < total) ahead[j] = __ldg(reinterpret_cast<const float2*>(gain + column<WT_F16>(lane + 32 * j)));
+        }
+        const float2 t = mega_block_sum_max(ln_sum, ln_top, s.red);
+        const float mean = t.x * (a.plan.inv_d);
+        const unsigned e = min(__float_as_uint(t.y + fabsf(mean)) >> 23, 254u), f = min(258u - e, 253u);
+        const float up = __uint_as_float(f << 23);
+        ln_down = __uint_as_float((254u - f) << 23);
+        auto pair = [&](int it, float2 g) {
+            const int k = column<WT_F16>(it);
+            const float2 x = *reinterpret_cast<const float2*>(s.xres + k);
+            const float v0 = x.x - mean, v1 = x.y - mean;
+            ss[0] = fmaf(v0, v0, fmaf(v1, v1, ss[0]));
+            xa_store_pair<1>(s.xa, k, v0 * up * g.x, v1 * up * g.y, 0);
+        };
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            if (lane + 32 * j < total) pair(lane + 32 * j, ahead[j]);
+#pragma unroll 1
+        for (int it = lane + 64; it < total; it += 32) pair(it, __ldg(reinterpret_cast<const float2*>(gain + column<WT_F16>(it))));
+    }
+    // Factor of the products' sums of position q.
+    __device__ __forceinline__ float norm_factor(const float* sq, int q) const {
+        const float mean_sq = fmaf(mega_sum_warps(sq + q * kMegaConsumerWarps), a.plan.inv_d, a.m.eps);
+        float r = rsqrtf(mean_sq);  // (a correctly rounded division and square root cost ~200 cycles here)
+        if (GPT2) {
+            r = r * fmaf(-0.5f * mean_sq * r, r, 1.5f);  // one Newton step: rounding error only
+            r *= ln_down;
+        }
+        return r;
+    }
+
+    // ---- S2: attention of this CTA's head
+    __device__ __forceinline__ void attention(const ModelDims& md, const KvLayout& kv, int l, int pos, unsigned seq) {
+        const MegaPlan& p = a.plan;
+        mega_attention<HD, NP, WT>(s, w, md, kv, l, pos, [&]() {
+            // q of this CTA's head, k and v of the KV head: pairs in the order S1 published them
+            for (int x = tid; x < NP * 3 * half; x += kMegaConsumers) {
+                const int q = NP == 2 && x >= 3 * half ? 1 : 0, r = x - q * 3 * half;
+                const int section = r / half, idx = r - section * half;
+                const int item = (section == 0 ? w.hq * half : section == 1 ? p.qpk * half : (p.qpk + 1) * half) + idx;
+                const unsigned long long* const src = a.qkv_words + (w.kvh * NP + q) * 2 * p.group_items + 2 * item;
+                ulonglong2 v = make_ulonglong2(0, 0);
+                unsigned spins = 0;
+                if (!mega_aborting(s)) {
+                    while (true) {
+                        v = ld_words2(src);
+                        if ((unsigned)(v.x >> 32) == seq && (unsigned)(v.y >> 32) == seq) break;
+                        if (mega_spin_out(a, s, spins, 6)) break;
+                        mega_backoff();
+                    }
+                }
+                const float v0 = __uint_as_float((unsigned)v.x), v1 = __uint_as_float((unsigned)v.y);
+                if (section == 0) { s.qs[q * HD + idx] = v0; s.qs[q * HD + idx + half] = v1; }
+                else if (section == 1) { s.kn[q * HD + idx] = __float2half_rn(v0); s.kn[q * HD + idx + half] = __float2half_rn(v1); }
+                else { s.vn[q * HD + 2 * idx] = __float2half_rn(v0); s.vn[q * HD + 2 * idx + 1] = __float2half_rn(v1); }
+            }
+            __syncwarp();
+            release_pending();  // the q/k/v chunk
+            consumer_sync();
+            stamp();
+        });
+        stamp();
+    }
+
+    // ---- the stages whose operand is a whole vector
+
+    // Best row of this thread in the LM head.
+    float best_v;
+    int best_i;
+
+    // Stage KIND of layer l: awaits and stages its operand (`first`: the pass's first vector), multiplies this CTA's rows, finishes and
+    // publishes them.
+    template <int KIND, int W2>
+    __device__ __forceinline__ void stage(const MegaModel& mo, const ModelDims& md, int l, bool first, const uint32_t (&tok)[NP], int pos, unsigned seq) {
+        constexpr bool kNorm = KIND == MS_QKV || KIND == MS_UP || (GPT2 && KIND == MS_HEAD);  // the sums get the norm's factor (RMSNorm's is positive: the arg-max does not need it)
+        const MegaPlan& p = a.plan;
+        const int d = a.m.d_model;
+        const int gq = NP == 2 && tid >= kMegaConsumers / NP ? 1 : 0, gi = tid - gq * (kMegaConsumers / NP);  // epilogue: position of this thread, and which pair of a group's rows
+        const int rows_of = KIND == MS_QKV ? 2 * w.s1_n : KIND == MS_UP ? p.ffn_rows * w.h_n : KIND == MS_DOWN ? w.d_n : w.v_n;
+        // What the epilogue needs besides its sums is worked out before the words are awaited (a later group's with its products).
+        float e0 = 0.f, e1 = 0.f;
+        float2 cs = make_float2(1.f, 0.f);
+        __half *kv0 = nullptr, *kv1 = nullptr;
+        unsigned long long* dst = nullptr;
+        auto prepare = [&](int r) {
+            if (2 * gi >= rows_of - r) return;
+            int i0 = r + 2 * gi, i1 = min(i0 + 1, rows_of - 1);
+            const float* ln = nullptr;  // GPT-2: the constants of the rows
+            const int ln_rows = a.m.q_dim + 2 * a.m.kv_dim + a.m.hidden;
+            if constexpr (KIND == MS_QKV) {
+                const int4 pair = s.s1[i0 >> 1];
+                if (!GPT2 && pair.x < 2) cs = a.rope[(size_t)(gq ? min(pos + 1, a.m.max_seq - 1) : pos) * half + pair.w];
+                dst = a.qkv_words + (w.kvh * NP + gq) * 2 * p.group_items + 2 * w.s1_begin + i0;
+                kv0 = nullptr;
+                if (pair.x > 0 && (NP == 1 || pos + gq < md.max_seq)) {
+                    kv0 = (pair.x == 1 ? mo.kv.k : mo.kv.v) + (size_t)mega_kv_row(md, l, w.kvh, pos + gq) * HD + (pair.y - w.kvh * HD);
+                    kv1 = kv0 + (pair.z - pair.y);
+                }
+                ln = a.ln + (size_t)l * ln_rows + (pair.x == 0 ? 0 : pair.x == 1 ? a.m.q_dim : a.m.q_dim + a.m.kv_dim);
+                i0 = pair.y; i1 = pair.z;
+            } else if constexpr (KIND == MS_UP) {
+                dst = a.act_words + (p.act_wpc ? (gq * p.n_cta + (int)blockIdx.x) * p.act_wpc : gq * a.m.hidden + w.h_begin) + (GPT2 ? i0 : i0 >> 1);
+                ln = a.ln + (size_t)l * ln_rows + a.m.q_dim + 2 * a.m.kv_dim + w.h_begin;
+            } else if constexpr (KIND == MS_DOWN) {
+                dst = a.x_words + gq * d + w.d_begin + i0;
+                ln = a.out_bias + (size_t)(2 * l + 1) * d + w.d_begin;
+            } else {
+                ln = a.ln + (size_t)md.n_layer * ln_rows + w.v_begin;
+            }
+            if (GPT2) { e0 = __ldg(ln + i0); e1 = __ldg(ln + i1); }
+        };
+        prepare(0);
+        float ss[NP];
+#pragma unroll
+        for (int q = 0; q < NP; q++) ss[q] = 0.f;
+        ln_sum = ln_top = 0.f;
+        // The arg-max candidate words are used once per token; between two uses a whole model's worth of weights streams
+        // through L2.  Reading them once per layer keeps their lines resident, so that the token exchange does not
+        // start with a round trip to memory.
+        if (KIND == MS_UP)
+            for (int i = tid; i < NP * p.n_cta; i += kMegaConsumers) { unsigned long long keep; asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(keep) : "l"(a.cand_words + (size_t)i * kMegaCandStride) : "memory"); }
+        // Everything this CTA wrote with plain stores during the step (KV-cache rows; the CTA barriers since then order
+        // them before these threads) is made visible before the candidate words that are published at the end of the
+        // head.  Issued here, the fence overlaps the wait for the last layer's output.
+        if (KIND == MS_HEAD && warp < NP && lane == 0) __threadfence();
+        const float* const gain = mo.norms + (size_t)(2 * l + (KIND == MS_UP ? 1 : 0)) * d;
+        if ((KIND == MS_QKV || KIND == MS_HEAD) && first) stage_first<W2>(KIND == MS_HEAD, tok, pos, mo.tok_emb, gain, ss);
+        else stage_words<KIND, W2>(KIND == MS_QKV ? seq - 1 : seq, gain, ss);
+        release_pending();  // the last chunks of the stage before
+        if (GPT2 && KIND != MS_DOWN) layer_norm(gain, ss);
+        __syncwarp();
+        stamp();
+        const MegaStage& st = p.stage[KIND];
+        const int stride = NP * 16 * p.group_tiles;
+#pragma unroll 1
+        for (int r0 = 0; r0 < rows_of; r0 += st.group_rows) {
+            const int n = min(st.group_rows, rows_of - r0);
+            if (r0 > 0) prepare(r0);
+            const int keep = r0 + n < rows_of ? 0 : KIND == MS_HEAD ? 2 : 1;  // chunks at the end of the stage that are handed back later
+            float* const sums = s.sums + par * kMegaConsumerWarps * stride;  // warp x, position q, row r: [(x NP + q) 16 group_tiles + r]
+            float* const sq = s.ss + par * NP * kMegaConsumerWarps;
+            par ^= 1;
+            if (KIND != MS_HEAD && n <= 16) group_products<W2, 1>(st, n, keep, sums + warp * stride);
+            else if (KIND != MS_HEAD && n <= 32) group_products<W2, 2>(st, n, keep, sums + warp * stride);
+            else if (KIND != MS_HEAD && n <= 48) group_products<W2, 3>(st, n, keep, sums + warp * stride);
+            else group_products<W2, kMegaMaxTiles>(st, n, keep, sums + warp * stride);
+            if (kNorm) {
+#pragma unroll
+                for (int q = 0; q < NP; q++) {
+                    const float t = warp_sum(ss[q]);
+                    if (lane == 0) sq[q * kMegaConsumerWarps + warp] = t;
+                }
+            }
+            consumer_sync();
+            if (2 * gi < n) {
+                float2 v = mega_take_sum2(sums + gq * 16 * p.group_tiles, stride, 2 * gi);
+                if (kNorm) {
+                    const float inv = norm_factor(sq, gq);
+                    v.x *= inv; v.y *= inv;
+                }
+                if (GPT2) { v.x += e0; v.y += e1; }
+                const bool two = 2 * gi + 1 < n;
+                if constexpr (KIND == MS_QKV) {
+                    // RoPE ((cos, sin) = (1, 0) for a value pair), words for the CTAs that share the KV head, KV-cache append
+                    if (!GPT2) v = make_float2(v.x * cs.x - v.y * cs.y, v.x * cs.y + v.y * cs.x);
+                    st_words2(dst, tagged(v.x, seq), tagged(v.y, seq));
+                    if (kv0) {
+                        *kv0 = __float2half_rn(v.x);
+                        *kv1 = __float2half_rn(v.y);
+                    }
+                } else if constexpr (KIND == MS_UP) {
+                    if (GPT2) st_words2(dst, tagged(gelu_f(v.x), seq), tagged(gelu_f(v.y), seq));
+                    else st_word(dst, tagged(__fdividef(v.x, 1.0f + __expf(-v.x)) * v.y, seq));  // silu(gate) up
+                } else if constexpr (KIND == MS_DOWN) {
+                    const float* const res = s.xres + gq * d + w.d_begin + r0 + 2 * gi;
+                    st_word(dst, tagged(v.x + res[0], seq));
+                    if (two) st_word(dst + 1, tagged(v.y + res[1], seq));
+                } else {
+                    // a thread keeps the best of its rows (ascending: '>' keeps the first maximum)
+                    const int row = w.v_begin + r0 + 2 * gi;
+                    if (v.x > best_v) { best_v = v.x; best_i = row; }
+                    if (two && v.y > best_v) { best_v = v.y; best_i = row + 1; }
+                }
+            }
+            __syncwarp();
+        }
+    }
+
+    // One pass: tokens tok[q] at positions pos + q through `layers` layers (0: the head alone, on the last hidden state), then the LM
+    // head with its first-max arg-max; every CTA learns out[q].  seq: tag of everything the layer publishes, counted up by
+    // every layer; tag8: tag of the arg-max candidates.
+    __device__ __forceinline__ void pass(const MegaModel& mo, const ModelDims& md, int layers, const uint32_t (&tok)[NP], int pos, unsigned& seq, unsigned long long tag8,
+                                         uint32_t (&out)[NP]) {
+        const MegaPlan& p = a.plan;
+        // Why the exchange arrays need no second buffer: x_words is re-written by the W2 stage of this layer, which starts only
+        // after every CTA has published its activation, i.e. after every group CTA has read x; qkv_words one layer
+        // later, after x_words is complete, which needs every CTA's W2 rows, hence the whole activation, hence every
+        // group CTA past its S2; mid_sums receives the next layer's contributions only after that layer's S1, which needs every
+        // CTA past its read of them; act_words is re-written after mid_sums of the next layer is complete, which needs
+        // every group CTA past x_words, i.e. every CTA past its W2 rows.  (A CTA publishes behind the barrier that all of its
+        // warps pass after their reads.)
+#pragma unroll 1
+        for (int l = 0; l < layers; l++) {
+            seq++;
+            stamp();
+            if (w.in_group) {
+                stage<MS_QKV, WT>(mo, md, l, l == 0, tok, pos, seq);
+                stamp();
+                attention(md, mo.kv, l, pos, seq);
+                wo_products(p.stage[MS_WO], l);
+                stamp();
+            } else if (tracing) {
+                for (int i = 0; i < 5; i++) stamp();
+            }
+            stage<MS_UP, WT>(mo, md, l, false, tok, pos, seq);
+            stamp();
+            stage<MS_DOWN, WT>(mo, md, l, false, tok, pos, seq);
+            stamp();
+        }
+        stamp();
+        best_v = -INFINITY;
+        best_i = 0x7fffffff;
+        if (kQuant && p.wt_head == WT_F16) stage<MS_HEAD, WT_F16>(mo, md, md.n_layer, layers == 0, tok, pos, seq);  // an fp16 head on quantised layers reads the fp16 staging
+        else stage<MS_HEAD, WT>(mo, md, md.n_layer, layers == 0, tok, pos, seq);
+        // CTA-wide best (larger value first, then smaller index), published as one word per CTA:
+        // [ordered logit bits : 32][0xffffff - index : 24][tag : 8].  The tag is the same in every word of a step, so the
+        // largest word is the best candidate.
+        constexpr int kTeam = kMegaConsumerWarps / NP;  // warps whose threads hold one position's rows
+        {
+            const unsigned long long k = mega_warp_best(best_i != 0x7fffffff ? ((unsigned long long)ordered_bits(best_v) << 32) | ((unsigned long long)(0xffffffu - (unsigned)best_i) << 8) : 0ull);
+            if (lane == 0) s.key[warp] = k;
+        }
+        consumer_sync();
+        if (warp < NP) {
+            const unsigned long long k = mega_warp_best(lane < kTeam ? s.key[warp * kTeam + lane] : 0ull);
+            if (lane == 0) st_word(a.cand_words + (size_t)(warp * p.n_cta + (int)blockIdx.x) * kMegaCandStride, k | tag8);
+        }
+        stamp();
+        unsigned long long k[NP];  // the best of the candidates that this thread read, per position
+#pragma unroll
+        for (int q = 0; q < NP; q++) {
+            k[q] = 0ull;
+            for (int i = tid; i < p.n_cta; i += kMegaConsumers) {
+                const unsigned long long* const src = a.cand_words + (size_t)(q * p.n_cta + i) * kMegaCandStride;
+                unsigned long long x = 0ull;
+                unsigned spins = 0;
+                if (!mega_aborting(s)) {
+                    while (true) {
+                        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x) : "l"(src) : "memory");
+                        if ((x & 0xffull) == tag8) break;
+                        if (mega_spin_out(a, s, spins, 10)) break;
+                        mega_backoff();
+                    }
+                }
+                k[q] = max(k[q], x);
+            }
+        }
+        // a reader orders its later loads (the KV-cache rows other CTAs appended during this step) after the
+        // candidate words it saw; the writers' side of the pair is the fence at the start of the head
+        if (tid < p.n_cta) __threadfence();
+        __syncwarp();
+        consumer_sync();  // s.key was read above
+#pragma unroll
+        for (int q = 0; q < NP; q++) {
+            const unsigned long long kq = mega_warp_best(k[q]);
+            if (lane == 0) s.key[q * kMegaConsumerWarps + warp] = kq;
+        }
+        if (tid == 0) s.red[63] = mega_aborting(s) ? 1.f : 0.f;  // one decision for the whole CTA
+        consumer_sync();
+#pragma unroll
+        for (int q = 0; q < NP; q++) {
+            const unsigned long long best = mega_warp_best(lane < kMegaConsumerWarps ? s.key[q * kMegaConsumerWarps + lane] : 0ull);
+            out[q] = min(0xffffffu - (uint32_t)((best >> 8) & 0xffffffull), (uint32_t)(a.m.vocab - 1));  // in range even if every logit was NaN
+        }
+        release_pending();  // the last head chunks
+        stamp();
+    }
+};
+
 // ------------------------------------------------------------------------------------------------ the kernel
 
+// Issues a CTA's chunks in consumption order (one thread).
+struct MegaProducer {
+    const MegaArgs& a;
+    const MegaShared& s;
+    MegaCursor c;
+    unsigned issued = 0;
+    uint64_t policy;
+    __device__ __forceinline__ MegaProducer(const MegaArgs& a_, const MegaShared& s_) : a(a_), s(s_), policy(l2_evict_first_policy()) {}
+    __device__ __forceinline__ bool stopped() const { return mega_aborting(s) || *reinterpret_cast<volatile int*>(s.stop) != 0; }
+    // The chunks of stages first .. last of a layer (or the head) at src.
+    __device__ __forceinline__ void stages(const uint8_t* src, int first, int last, const MegaShare& w) {
+        const MegaPlan& p = a.plan;
+        const unsigned n_slots = (unsigned)p.n_slots;
+#pragma unroll 1
+        for (int kind = first; kind <= last; kind++) {
+            const MegaStage st = p.stage[kind];
+            const int wt = kind == MS_HEAD ? p.wt_head : p.wt_layer;
+            int rows = kind == MS_QKV ? 2 * w.s1_n : kind == MS_WO ? p.rpb : kind == MS_UP ? p.ffn_rows * w.h_n : kind == MS_DOWN ? w.d_n : w.v_n;
+            if (kind <= MS_WO && !w.in_group) rows = 0;
+            const uint8_t* at = src;
+#pragma unroll 1
+            for (int r0 = 0; r0 < rows; r0 += st.group_rows) {
+                const int ub = mega_unit_bytes(wt, min(st.group_rows, rows - r0));
+#pragma unroll 1
+                for (int u0 = 0; u0 < st.units; u0 += st.chunk_units) {
+                    const unsigned bytes = (unsigned)(min(st.chunk_units, st.units - u0) * ub);
+                    if (stopped()) return;  // nothing more is copied
+                    if (issued >= n_slots) mega_wait(a, s, s.empty + c.slot, c.phase ^ 1u, 4);  // the previous use of the slot was released
+                    if (stopped()) return;
+                    mbar_expect_tx(s.full + c.slot, bytes);
+                    bulk_copy_g2s(s.slots + (size_t)c.slot * p.slot_bytes, at, bytes, s.full + c.slot, policy);
+                    at += bytes;
+                    c.next(n_slots);
+                    issued++;
+                }
+            }
+            src += kind == MS_QKV ? p.s1_bytes : kind == MS_WO ? p.s2_bytes : kind == MS_UP ? p.s3a_bytes : p.s3b_bytes;
+        }
+    }
+    // Every copy that was issued must have landed before the CTA may exit: walks the last n_slots chunks backwards.
+    __device__ __forceinline__ void drain() {
+        const unsigned n_slots = (unsigned)a.plan.n_slots, back = issued < n_slots ? issued : n_slots;
+        MegaCursor k = c;
+        for (unsigned i = 0; i < back; i++) {
+            if (k.slot == 0) { k.slot = n_slots - 1; k.phase ^= 1u; } else k.slot--;
+            unsigned spins = 0;
+            while (!mbar_try_wait(s.full + k.slot, k.phase) && ++spins < kMegaSpinLimit) {}
+        }
+    }
+};
+__device__ __forceinline__ unsigned mega_layer_chunks(const MegaPlan& p, const MegaShare& w) {
+    return (unsigned)((w.in_group ? mega_stage_chunks(p.stage[MS_QKV], 2 * w.s1_n) + mega_stage_chunks(p.stage[MS_WO], p.rpb) : 0) +
+                      mega_stage_chunks(p.stage[MS_UP], p.ffn_rows * w.h_n) + mega_stage_chunks(p.stage[MS_DOWN], w.d_n));
+}
+// The watcher: follows the chunks in order and counts the ones whose bytes have arrived (one thread).
+__device__ __forceinline__ void mega_watch(const MegaArgs& a, const MegaShared& s, unsigned total) {
+    MegaCursor k;
+    for (unsigned i = 0; i < total; i++) {
+        unsigned spins = 0;
+        while (!mbar_try_wait(s.full + k.slot, k.phase)) {
+            if (*reinterpret_cast<volatile int*>(s.stop) || mega_spin_out(a, s, spins, 3)) return;
+        }
+        st_release_cta_shared(s.landed, i + 1);
+        k.next((unsigned)a.plan.n_slots);
+    }
+}
+
 template <int HD, int WT, bool GPT2>
-__global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs a) {
+__global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const __grid_constant__ MegaArgs a) {
     extern __shared__ __align__(128) uint8_t mega_smem[];
-    const MegaShared s = mega_carve(mega_smem, a);
     const MegaPlan& p = a.plan;
+    const MegaShared s = mega_carve(mega_smem, p);
     const ModelDims& m = a.m;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int L = m.n_layer;
-    if (tid == 0) {
-        *s.share = mega_share(m, p, (int)blockIdx.x);
-        for (int i = 0; i < p.n_slots; i++) { mbar_init(s.full + i, 1); mbar_init(s.empty + i, kMegaConsumerWarps); }
-        *s.abort = 0;
-        *s.stop = 0;
-        *s.landed = 0u;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    for (int k = tid; k < m.d_model; k += kMegaThreads) s.prev[k] = 0ull;  // the counted sums are zero at launch
-    for (int c = tid; c <= p.n_cta; c += kMegaThreads) {
-        s.hbeg[c] = mega_share_begin(m.hidden, p.n_cta, c);
-    }
+    mega_init(a, s, 1);
     __syncthreads();
-    const MegaShare& w = *s.share;  // read from shared memory wherever it is needed: no registers, no recomputation
-    const uint8_t* blob = a.pack + (size_t)blockIdx.x * p.cta_bytes;
-    const long long head_off = (long long)L * p.layer_bytes;
+    const MegaShare& w = *s.share;
 
     if (warp == kMegaConsumerWarps) {
         // ---------------- producer: one thread streams this CTA's chunks in consumption order ----------------
         if (lane == 0) {
-            MegaCursor c;
-            unsigned issued = 0;
-#ifdef MEGA_FINE_TRACE
-            int p_step = 0, p_n = 0;
-#endif
-            const uint64_t policy = l2_evict_first_policy();
+            const uint8_t* blob = a.pack + (size_t)blockIdx.x * p.cta_bytes;
+            const uint8_t* head = blob + (long long)L * p.layer_bytes;
             uint64_t keep_policy;
             asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep_policy));
-            // head rows behind the first (n_slots - 1) chunks: what still has to come from memory when the head begins
-            const long long tail_off = (long long)min(w.v_n, (p.n_slots - 1) * p.head_rpc) * p.head_row_bytes;
-            const long long tail_bytes = (long long)w.v_n * p.head_row_bytes - tail_off;
-            auto issue = [&](long long off, int bytes) {
-                if (mega_aborting(s) || *reinterpret_cast<volatile int*>(s.stop)) return;  // nothing more is copied
-#ifdef MEGA_FINE_TRACE
-                const bool tr = a.trace && (int)blockIdx.x == a.trace_cta && p_step == a.n_steps - 1 && p_n < 56;
-                if (tr) a.trace[400 + 2 * p_n] = clock64();
-#endif
-                if (issued >= (unsigned)p.n_slots) mega_wait(a, s, s.empty + c.slot, c.phase ^ 1u, 4);  // the previous use of the slot was released
-                if (mega_aborting(s) || *reinterpret_cast<volatile int*>(s.stop)) return;
-                mbar_expect_tx(s.full + c.slot, (unsigned)bytes);
-                bulk_copy_g2s(s.slots + (size_t)c.slot * p.slot_bytes, blob + off, (unsigned)bytes, s.full + c.slot, policy);
-#ifdef MEGA_FINE_TRACE
-                if (tr) { a.trace[400 + 2 * p_n + 1] = clock64(); p_n++; }
-#endif
-                c.next((unsigned)p.n_slots);
-                issued++;
-            };
-            // a stage's slice: whole items, `per_chunk` at a time
-            auto issue_stage = [&](long long off, int items, int per_chunk, int item_bytes) {
-                for (int i0 = 0; i0 < items; i0 += per_chunk) issue(off + (long long)i0 * item_bytes, min(per_chunk, items - i0) * item_bytes);
-            };
+            // head bytes behind the first (n_slots - 1) chunks: what still has to come from memory when the head begins
+            const long long head_bytes = mega_stage_bytes(p.stage[MS_HEAD], p.wt_head, w.v_n);
+            const long long tail_off = min(head_bytes, (long long)(p.n_slots - 1) * p.stage[MS_HEAD].chunk_units * mega_unit_bytes(p.wt_head, min(w.v_n, p.stage[MS_HEAD].group_rows)));
+            const long long tail_bytes = head_bytes - tail_off;
+            MegaProducer prod(a, s);
             for (int step = a.first; step < a.first + a.n_steps; step++) {
-#ifdef MEGA_FINE_TRACE
-                p_step = step - a.first;
-#endif
-                if (step > 0) {
-                    for (int l = 0; l < L; l++) {
-                        // HBM idles during the layers (their weights are a full layer ahead in the ring): the part of the head
-                        // that the ring cannot hold before the head begins is brought into L2 now, a slice per layer
-                        if (tail_bytes > 0 && !mega_aborting(s)) {
-                            const long long b0 = tail_bytes * l / L / 16 * 16, b1 = l + 1 == L ? tail_bytes : tail_bytes * (l + 1) / L / 16 * 16;
-                            if (b1 > b0)
-                                asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;" ::"l"(blob + head_off + tail_off + b0), "r"((unsigned)(b1 - b0)),
-                                             "l"(keep_policy)
-                                             : "memory");
-                        }
-                        long long off = (long long)l * p.layer_bytes;
-                        if (w.in_group) issue_stage(off, w.s1_n, p.s1_ipc, 2 * p.row_bytes);
-                        off += p.s1_bytes;
-                        if (w.in_group) issue_stage(off, p.rpb, p.s2_rpc, p.wo_row_bytes);
-                        off += p.s2_bytes;
-                        issue_stage(off, w.h_n, p.s3a_ipc, (GPT2 ? 1 : 2) * p.row_bytes); off += p.s3a_bytes;
-                        if (WT == WT_F16) {
-                            issue_stage(off, w.d_n, p.s3b_rpc, p.down_row_bytes);
-                        } else {
-                            const int n_kb = m.hidden >> 5;
-                            for (int k = 0; k < n_kb; k += p.s3b_kpc) {
-                                const int bytes = w.d_n * mega_row_bytes(WT, 32 * min(p.s3b_kpc, n_kb - k));
-                                issue(off, bytes);
-                                off += bytes;
-                            }
-                        }
+                for (int l = 0; step > 0 && l < L; l++) {
+                    // HBM idles during the layers (their weights are a full layer ahead in the ring): the part of the head
+                    // that the ring cannot hold before the head begins is brought into L2 now, a slice per layer
+                    if (tail_bytes > 0 && !mega_aborting(s)) {
+                        const long long b0 = tail_bytes * l / L / 16 * 16, b1 = l + 1 == L ? tail_bytes : tail_bytes * (l + 1) / L / 16 * 16;
+                        if (b1 > b0)
+                            asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;" ::"l"(head + tail_off + b0), "r"((unsigned)(b1 - b0)), "l"(keep_policy)
+                                         : "memory");
                     }
+                    prod.stages(blob + (long long)l * p.layer_bytes, MS_QKV, MS_DOWN, w);
                 }
-                issue_stage(head_off, w.v_n, p.head_rpc, p.head_row_bytes);
+                prod.stages(head, MS_HEAD, MS_HEAD, w);
             }
-            // every copy that was issued must have landed before the CTA may exit: walk the last n_slots chunks backwards
-            MegaCursor k = c;
-            const unsigned back = issued < (unsigned)p.n_slots ? issued : (unsigned)p.n_slots;
-            for (unsigned i = 0; i < back; i++) {
-                if (k.slot == 0) { k.slot = (unsigned)p.n_slots - 1; k.phase ^= 1u; } else k.slot--;
-                unsigned spins = 0;
-                while (!mbar_try_wait(s.full + k.slot, k.phase) && ++spins < kMegaSpinLimit) {}
-            }
+            prod.drain();
         }
         return;
     }
     if (warp == kMegaConsumerWarps + 1) {
-        // ---------------- watcher: follows the chunks in order and counts the ones whose bytes have arrived ----------------
-        if (lane == 0) {
-            auto chunks_of = [](int items, int per_chunk) { return (items + per_chunk - 1) / per_chunk; };
-            const unsigned per_layer = (w.in_group ? chunks_of(w.s1_n, p.s1_ipc) + chunks_of(p.rpb, p.s2_rpc) : 0) + chunks_of(w.h_n, p.s3a_ipc) +
-                                       (WT == WT_F16 ? chunks_of(w.d_n, p.s3b_rpc) : chunks_of(m.hidden >> 5, p.s3b_kpc));
-            const unsigned total = (unsigned)a.n_steps * chunks_of(w.v_n, p.head_rpc) + (unsigned)(a.n_steps - 1 + a.first) * L * per_layer;
-            MegaCursor k;
-            for (unsigned i = 0; i < total; i++) {
-                unsigned spins = 0;
-                bool gone = false;
-                while (!mbar_try_wait(s.full + k.slot, k.phase)) {
-                    if (*reinterpret_cast<volatile int*>(s.stop) || mega_spin_out(a, s, spins, 3)) { gone = true; break; }
-                }
-                if (gone) break;
-                st_release_cta_shared(s.landed, i + 1);
-                k.next((unsigned)p.n_slots);
-            }
-        }
+        if (lane == 0)
+            mega_watch(a, s, (unsigned)a.n_steps * mega_stage_chunks(p.stage[MS_HEAD], w.v_n) + (unsigned)(a.n_steps - 1 + a.first) * L * mega_layer_chunks(p, w));
         return;
     }
 
@@ -1147,523 +1691,28 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
         a.stamps[0] = t;
     }
-#ifdef MEGA_FINE_TRACE
-    int n_fine = 0;
-    int fine_layer = -1, fine_step = -1;
-#define FINE() do { if (a.trace && (int)blockIdx.x == a.trace_cta && tid == 0 && fine_step == a.n_steps - 1 && (fine_layer == 2 || fine_layer == 99) && n_fine < 120) a.trace[256 + n_fine++] = clock64(); } while (0)
-#else
-#define FINE() do {} while (0)
-#endif
-    int n_stamp = 0;
-    auto stamp = [&](int step) {
-        if (a.trace && (int)blockIdx.x == a.trace_cta && tid == 0 && step == a.first + a.n_steps - 1) a.trace[n_stamp++] = clock64();
-    };
-    MegaCursor c;        // ring position, advances in lock step with the producer's
-    unsigned n_chunk = 0, landed = 0;  // chunks consumed so far; chunks known to have arrived
+    MegaWorker<HD, WT, GPT2, 1> work(a, s);
+    const MegaModel model{a.norms, a.tok_emb, a.kv};
     int pos = a.pos0;    // visible tokens
-    uint32_t tok = a.tok0;
+    uint32_t tok[1] = {a.tok0};
     int emitted = 0;
-    int par = 0;         // which half of s.partial the next chunk's sums go to
-    constexpr int half = HD / 2;
+    unsigned seq = a.tag0;
     const int d = m.d_model;
-    const float inv_d = 1.0f / (float)d;
-    const float* fin_gain = a.norms + (size_t)(2 * L) * d;
-    unsigned long long* my_qkv = a.qkv_words + (size_t)w.kvh * 2 * p.group_items;
-    __half* xa_h = reinterpret_cast<__half*>(s.xa);
-
-    // Stages values of the residual stream: raw copy, gained copy as the products' staged operand (fp16 hi/lo parts, or
-    // int8 digits for the quantised types; `K` = length of the vector being staged), sum of squares.
-    constexpr bool kQuant = WT == WT_Q8_0;  // int8 digit staging (Q4_0 widens its nibbles to fp16 and reads the fp16 staging)
-    auto stage_x = [&](float* raw, int K, bool digits, int k, float v, float g, float& ss) {  // one element per lane, consecutive k
-        raw[k] = v;
-        if (kQuant && digits) qx_store_elem(s.xa, reinterpret_cast<float*>(s.xa + xa_bytes(K)), k, v * g);
-        else xa_store(xa_h, k, v * g);
-        ss = fmaf(v, v, ss);
-    };
-    auto stage_x2 = [&](float* raw, int K, bool digits, int k, float v0, float v1, float g0, float g1, float& ss) {  // a pair per lane
-        raw[k] = v0; raw[k + 1] = v1;
-        if (kQuant && digits) {
-            qx_store_pair(s.xa, reinterpret_cast<float*>(s.xa + xa_bytes(K)), k, v0 * g0, v1 * g1);
-        } else {
-            xa_store(xa_h, k, v0 * g0);
-            xa_store(xa_h, k + 1, v1 * g1);
-        }
-        ss = fmaf(v0, v0, fmaf(v1, v1, ss));
-    };
-    auto rms_scale = [&](float ss) { return rsqrtf(mega_block_sum(ss, s.red) * inv_d + m.eps); };  // (a correctly rounded division and square root cost ~200 cycles here)
-    // GPT-2's LayerNorm.  The values are staged only when the mean is known: with a mean far from zero both E[x^2] - mean^2 and
-    // W.(x g) - mean W.g cancel (one barrier less, but a stream of mean 32 and deviation 0.05 had no correct digit left).  The
-    // centred values carry a power of two that puts the largest of them near 32: the fp16 parts then neither saturate on a large
-    // residual stream nor lose their low half to subnormals on a small one.  Every thread normalises the pairs that it received.
-    // GPT-2 117M, 64 tokens: 10.88 ms with one pass over the values, 11.37 with two (25 barriers per token).
-    constexpr int kLnAhead = 2;  // gain pairs of a thread requested before the values arrive (d_model <= 2048: all)
-    struct LnGains { float2 g[kLnAhead]; };
-    auto ln_gains = [&](const float* gain) {
-        LnGains p2;
-#pragma unroll
-        for (int i = 0; i < kLnAhead; i++) {
-            const int k = 2 * (tid + i * kMegaConsumers);
-            p2.g[i] = k < d ? __ldg(reinterpret_cast<const float2*>(gain + k)) : make_float2(0.f, 0.f);
-        }
-        return p2;
-    };
-    float ln_sum = 0.f, ln_top = 0.f;
-    auto ln_take = [&](float* raw, int k, float v0, float v1) {
-        *reinterpret_cast<float2*>(raw + k) = make_float2(v0, v1);
-        ln_sum += v0 + v1;
-        ln_top = fmaxf(ln_top, fmaxf(fabsf(v0), fabsf(v1)));
-    };
-    auto layer_norm = [&](const float* raw, const float* gain, const LnGains& ahead) {  // stages the vector, returns the factor of the products' sums
-        const float2 t = mega_block_sum_max(ln_sum, ln_top, s.red);
-        ln_sum = ln_top = 0.f;
-        const float mean = t.x * inv_d;
-        const unsigned e = min(__float_as_uint(t.y + fabsf(mean)) >> 23, 254u), f = min(258u - e, 253u);
-        const float up = __uint_as_float(f << 23);
-        float ss = 0.f;
-        auto pair = [&](int k, float2 g) {
-            const float2 x = *reinterpret_cast<const float2*>(raw + k);
-            const float v0 = x.x - mean, v1 = x.y - mean;
-            ss = fmaf(v0, v0, fmaf(v1, v1, ss));
-            xa_store(xa_h, k, v0 * up * g.x);
-            xa_store(xa_h, k + 1, v1 * up * g.y);
-        };
-#pragma unroll
-        for (int i = 0; i < kLnAhead; i++)
-            if (2 * (tid + i * kMegaConsumers) < d) pair(2 * (tid + i * kMegaConsumers), ahead.g[i]);
-        for (int k = 2 * (tid + kLnAhead * kMegaConsumers); k < d; k += 2 * kMegaConsumers) pair(k, __ldg(reinterpret_cast<const float2*>(gain + k)));
-        const float var = fmaf(mega_block_sum(ss, s.red + 2 * kMegaConsumerWarps), inv_d, m.eps);  // (its barrier also publishes the staged vector)
-        float r = rsqrtf(var);
-        r *= fmaf(-0.5f * var * r, r, 1.5f);  // one Newton step: rounding error only
-        return r * __uint_as_float((254u - f) << 23);
-    };
-    const int ln_rows = m.q_dim + 2 * m.kv_dim + m.hidden;  // rows of a layer whose input is normalised
-    const bool head_digits = kQuant && p.wt_head != WT_F16;  // an fp16 head on quantised layers reads the fp16 staging
-    // A freed slot makes the producer request the chunk that is n_slots ahead at once: megabytes of reads over all
-    // CTAs, which would travel through L2 together with the words of the exchange that follows the stage and delay
-    // them by microseconds.  The last chunk of a stage is therefore handed back only after that exchange (the chunk it
-    // makes room for is needed a whole layer later).
-    MegaCursor pend_from;
-    int n_pend = 0;
-    auto release_pending = [&]() {
-        if (n_pend) mega_release_deferred(a, s, pend_from, n_pend);
-        n_pend = 0;
-    };
-    // Quantised models: a stage's slice is several chunks, and a barrier plus an epilogue per chunk cost 0.7 us each.  The
-    // products of up to p.group chunks (`rows` rows, `per` per chunk) share one CTA barrier; a warp goes from chunk to chunk on
-    // its own.  fp16 models: one chunk at a time (their stages are one chunk, and the short way is 4 us per token faster).
-    // The last `keep` chunks of the rows still to come (`left`) are handed back later.  Returns where the sums are.
-    constexpr bool kGrouped = WT != WT_F16;
-    const int group = kGrouped ? p.group : 1;
-    int lg_parts = 0;    // fp16: log2 of the column ranges of the chunk whose sums are being read
-    auto hand_back = [&](bool later) {
-        if (later) {
-            if (n_pend == 0) pend_from = c;
-            n_pend++;
-            c.next((unsigned)p.n_slots);
-        } else {
-            mega_release(a, s, c);
-        }
-    };
-    auto group_products = [&](int rows, int per, int n_kb, const uint8_t* xa, int left, int keep, bool is_head = false) {
-        float* const base = s.partial + par * group * kMegaChunkRows;
-        par ^= 1;
-        if constexpr (kGrouped) {
-            float* partial = base;
-#pragma unroll 1
-            for (int r0 = 0; r0 < rows; r0 += per) {
-                const uint8_t* ch = mega_acquire(a, s, c, n_chunk++, landed);
-                const int n = min(per, rows - r0);
-                if (is_head && p.wt_head == WT_F16) mega_chunk_dots<WT_F16>(ch, n, n_kb, xa, partial, warp, lane);  // an fp16 head on quantised layers
-                else mega_chunk_dots<WT>(ch, n, n_kb, xa, partial, warp, lane);
-                partial += kMegaChunkRows;
-                hand_back(left - r0 <= keep * per);
-            }
-        } else {
-            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++, landed);
-            FINE();
-            lg_parts = mega_chunk_dots<WT>(ch, rows, n_kb, xa, base, warp, lane);
-            FINE();
-            hand_back(left <= keep * per);
-        }
-        consumer_sync();
-        FINE();
-        return base;
-    };
-    // The sum of row r of a group.
-    auto row_sum = [&](const float* base, int rows, int per, int n_kb, int r) {
-        if constexpr (!kGrouped) return mega_take_sum(base, lg_parts, r);
-        int i = 0;
-        while (r >= per) { r -= per; rows -= per; i++; }  // (at most three times)
-        return mega_take_sum(base + i * kMegaChunkRows, mega_chunk_lg(min(per, rows), n_kb), r);
-    };
-    // f(i) for every i < n this thread owns (an fp16 chunk has at most 256 rows: at most one per thread)
-    auto each = [&](int n, auto f) {
-        if constexpr (kGrouped) {
-            for (int i = tid; i < n; i += kMegaConsumers) f(i);
-        } else {
-            if (tid < n) f(tid);
-        }
-    };
-
     for (int step = a.first; step < a.first + a.n_steps; step++) {
-        if (step > 0) {
-            const uint16_t* emb_row = a.tok_emb + (size_t)tok * d;
-            if (!GPT2 && tid < half) s.rope[tid] = a.rope[(size_t)pos * half + tid];  // published by the barrier of the first norm
-            for (int l = 0; l < L; l++) {
-                const unsigned seq = a.tag0 + (unsigned)((step - 1) * L + l + 1);  // tag of everything this layer publishes
-                float inv = 0.f;
-#ifdef MEGA_FINE_TRACE
-                fine_layer = l; fine_step = step;
-#endif
-                stamp(step);
-                if (w.in_group) {
-                    // ---- S1: x of this layer.  x_words is re-written by the W2 stage of this layer, which starts only
-                    // after every CTA has published its activation, i.e. after every group CTA has read x here.
-                    const float* gain = a.norms + (size_t)(2 * l) * d;
-                    float ss = 0.f;
-                    LnGains ahead;
-                    if (GPT2) ahead = ln_gains(gain);
-                    if (l == 0 && GPT2) {
-                        for (int k = 2 * tid; k < d; k += 2 * kMegaConsumers) {
-                            const __half2 te = *reinterpret_cast<const __half2*>(emb_row + k), pe = *reinterpret_cast<const __half2*>(a.pos_emb + (size_t)pos * d + k);
-                            ln_take(s.xraw, k, __low2float(te) + __low2float(pe), __high2float(te) + __high2float(pe));
-                        }
-                    } else if (l == 0) {
-                        for (int k = tid; k < d; k += kMegaConsumers) stage_x(s.xraw, d, true, k, __half2float(__ushort_as_half(emb_row[k])), __ldg(gain + k), ss);
-                    } else if (GPT2) {
-                        mega_read_words(a, s, a.x_words, d, seq - 1, 5, nullptr, [&](int k, float v0, float v1, float, float) { ln_take(s.xraw, k, v0, v1); });
-                    } else {
-                        mega_read_words(a, s, a.x_words, d, seq - 1, 5, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, true, k, v0, v1, g0, g1, ss); });
-                    }
-                    FINE();
-                    release_pending();  // the W2 chunk of the previous layer
-                    if (GPT2) inv = layer_norm(s.xraw, gain, ahead);
-                    else inv = rms_scale(ss);
-                    FINE();
-                    stamp(step);
-                    // q/k/v row pairs of this CTA, RoPE, words for the CTAs that share the KV head, KV-cache append.
-                    // qkv_words is re-written one layer later, after x_words of this layer is complete, which needs every
-                    // CTA's W2 rows, hence the whole activation vector, hence every group CTA past its S2 of this layer.
-                    const int s1_step = group * p.s1_ipc;
-                    for (int i0 = 0; i0 < w.s1_n; i0 += s1_step) {
-                        const int n_items = min(s1_step, w.s1_n - i0);
-                        // A group holds at most 512 row pairs: one per thread.  Where the pair goes (matrix, RoPE entry,
-                        // exchange words, cache rows) does not depend on the products: worked out before them, it is off
-                        // the path between the last product and the words the other CTAs are waiting for.
-                        int kind = 0, row0 = 0, row1 = 0, idx = 0;
-                        float2 cs = make_float2(1.f, 0.f);
-                        float n0 = 0.f, n1 = 0.f;
-                        unsigned long long* dst = my_qkv;
-                        __half* kv_row = nullptr;
-                        if (tid < n_items) {
-                            mega_s1_rows(m, p, w.kvh, w.s1_begin + i0 + tid, kind, row0, row1, idx);
-                            if (!GPT2 && kind < 2) cs = s.rope[idx];
-                            if (GPT2) {
-                                const float* ln = a.ln + (size_t)l * ln_rows + (kind == 0 ? 0 : kind == 1 ? m.q_dim : m.q_dim + m.kv_dim);
-                                n0 = __ldg(ln + row0);
-                                n1 = __ldg(ln + row1);
-                            }
-                            dst = my_qkv + 2 * (w.s1_begin + i0 + tid);
-                            if (kind > 0) kv_row = (kind == 1 ? a.kv.k : a.kv.v) + a.kv.offset(m, l, 0, w.kvh, pos) - w.kvh * HD;
-                        }
-                        const float* sums = group_products(2 * n_items, 2 * p.s1_ipc, d >> 5, s.xa, 2 * (w.s1_n - i0), 1);
-                        if (tid < n_items) {
-                            float v0 = row_sum(sums, 2 * n_items, 2 * p.s1_ipc, d >> 5, 2 * tid);
-                            float v1 = row_sum(sums, 2 * n_items, 2 * p.s1_ipc, d >> 5, 2 * tid + 1);
-                            float r0, r1;
-                            if (GPT2) {
-                                r0 = fmaf(v0, inv, n0);
-                                r1 = fmaf(v1, inv, n1);
-                            } else {
-                                v0 *= inv;
-                                v1 *= inv;
-                                r0 = v0 * cs.x - v1 * cs.y;  // (cos, sin) = (1, 0) for a value pair
-                                r1 = v0 * cs.y + v1 * cs.x;
-                            }
-                            st_word(dst, tagged(r0, seq));
-                            st_word(dst + 1, tagged(r1, seq));
-                            if (kind > 0) {
-                                kv_row[row0] = __float2half_rn(r0);
-                                kv_row[row1] = __float2half_rn(r1);
-                            }
-                        }
-                    }
-                    stamp(step);
-                    // ---- S2: attention of this CTA's head (the cached K/V rows are requested before the query is awaited)
-                    FINE();
-                    mega_attention<HD, 1, WT == WT_Q8_0 ? 1 : 0>(a, s, w, m, a.kv, l, pos, [&]() {
-                        // q of this CTA's head, k and v of the KV head: pairs in the order S1 published them
-                        FINE();
-                        if (tid < 3 * half) {
-                            const int section = tid / half, idx = tid - section * half;
-                            const int item = (section == 0 ? w.hq * half : section == 1 ? p.qpk * half : (p.qpk + 1) * half) + idx;
-                            ulonglong2 v = make_ulonglong2(0, 0);
-                            unsigned spins = 0;
-                            if (!mega_aborting(s)) {
-                                while (true) {
-                                    v = ld_words2(my_qkv + 2 * item);
-                                    if ((unsigned)(v.x >> 32) == seq && (unsigned)(v.y >> 32) == seq) break;
-                                    if (mega_spin_out(a, s, spins, 6)) break;
-                                    mega_backoff();
-                                }
-                            }
-                            const float v0 = __uint_as_float((unsigned)v.x), v1 = __uint_as_float((unsigned)v.y);
-                            if (section == 0) { s.qs[idx] = v0; s.qs[idx + half] = v1; }
-                            else if (section == 1) { s.kn[idx] = __float2half_rn(v0); s.kn[idx + half] = __float2half_rn(v1); }
-                            else { s.vn[2 * idx] = __float2half_rn(v0); s.vn[2 * idx + 1] = __float2half_rn(v1); }
-                        }
-                        release_pending();  // the q/k/v chunk
-                        FINE();
-                        consumer_sync();
-                        FINE();
-                        stamp(step);
-                    });
-                    stamp(step);
-                    // ---- rows [blk*rpb, ...) of Wo restricted to this head's columns: every row's partial sum is one
-                    // contribution to the counted sum of that row (head 0 also carries the residual)
-                    for (int r0 = 0; r0 < p.rpb; r0 += group * p.s2_rpc) {
-                        const int nr = min(group * p.s2_rpc, p.rpb - r0);
-                        const float* sums = group_products(nr, p.s2_rpc, HD >> 5, reinterpret_cast<const uint8_t*>(s.ctx), p.rpb - r0, 1);
-                        each(nr, [&](int r) {
-                            const int orow = w.blk * p.rpb + r0 + r;
-                            float v = row_sum(sums, nr, p.s2_rpc, HD >> 5, r);
-                            if (orow < d) {
-                                if (w.head == 0) v += s.xraw[orow] + (GPT2 ? __ldg(a.out_bias + (size_t)2 * l * d + orow) : 0.f);
-                                red_add_u64(a.mid_sums + orow, counted(v));
-                            }
-                        });
-                    }
-                    stamp(step);
-                } else {
-                    stamp(step); stamp(step); stamp(step); stamp(step); stamp(step);
-                }
-                // ---- S3: x_mid = residual + attention projection.  mid_sums receives the next layer's contributions
-                // only after that layer's S1, which needs x_words of this layer complete, i.e. every CTA past this read.
-                {
-                    // The arg-max candidate words are used once per token; between two uses a whole model's worth of
-                    // weights streams through L2.  Reading them once per layer keeps their lines resident, so that the
-                    // token exchange does not start with a round trip to memory.
-                    if (tid < p.n_cta) { unsigned long long keep; asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(keep) : "l"(a.cand_words + (size_t)tid * kMegaCandStride) : "memory"); }
-                    const float* gain = a.norms + (size_t)(2 * l + 1) * d;
-                    float ss = 0.f;
-                    FINE();
-                    LnGains ahead;
-                    if (GPT2) {
-                        ahead = ln_gains(gain);
-                        mega_read_sums(a, s, a.mid_sums, d, m.n_head, 7, nullptr, [&](int k, float v0, float v1, float, float) { ln_take(s.xmid, k, v0, v1); });
-                    } else {
-                        mega_read_sums(a, s, a.mid_sums, d, m.n_head, 7, gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xmid, d, true, k, v0, v1, g0, g1, ss); });
-                    }
-                    FINE();
-                    release_pending();  // the Wo chunk (CTAs outside the head groups: the W2 chunk of the previous layer)
-                    if (GPT2) inv = layer_norm(s.xmid, gain, ahead);
-                    else inv = rms_scale(ss);
-                }
-                stamp(step);
-                // (gate, up) row pairs of this CTA's hidden units, SiLU(gate) * up.  act_words is re-written one layer later,
-                // after mid_sums of that layer is complete, which needs every group CTA past x_words of this layer, i.e.
-                // every CTA past its W2 rows and so past this activation vector.
-                constexpr int kFfn = GPT2 ? 1 : 2;  // packed rows per unit
-                for (int j0 = 0; j0 < w.h_n; j0 += group * p.s3a_ipc) {
-                    const int n_items = min(group * p.s3a_ipc, w.h_n - j0), n_rows = kFfn * n_items, per = kFfn * p.s3a_ipc;
-                    // (the first item of a thread: its word's address and constants are known before the products)
-                    unsigned long long* const dst = a.act_words + (p.act_wpc ? (size_t)blockIdx.x * p.act_wpc : (size_t)w.h_begin) + j0;
-                    const float* ln = GPT2 ? a.ln + (size_t)l * ln_rows + m.q_dim + 2 * m.kv_dim + w.h_begin + j0 : nullptr;
-                    float n0 = 0.f;
-                    if (GPT2 && tid < n_items) n0 = __ldg(ln + tid);
-                    const float* sums = group_products(n_rows, per, d >> 5, s.xa, kFfn * (w.h_n - j0), 1);
-                    each(n_items, [&](int j) {
-                        float v;
-                        if (GPT2) {
-                            if (j >= kMegaConsumers) n0 = __ldg(ln + j);
-                            const float x = fmaf(row_sum(sums, n_rows, per, d >> 5, j), inv, n0);
-                            v = gelu_f(x);
-                        } else {
-                            const float g = row_sum(sums, n_rows, per, d >> 5, 2 * j) * inv;
-                            const float u = row_sum(sums, n_rows, per, d >> 5, 2 * j + 1) * inv;
-                            // silu(g) = g * sigmoid(g) = 0.5 g (1 + tanh(g / 2))
-                            v = __fdividef(g, 1.0f + __expf(-g)) * u;
-                        }
-                        st_word(dst + j, tagged(v, seq));
-                    });
-                }
-                stamp(step);
-                // ---- the whole activation vector, then this CTA's rows of W2 (+ residual) = the next layer's x
-                FINE();
-                if (p.act_wpc) {  // (cache lines per CTA: fp16 models only, see the plan)
-                    mega_read_lines(a, s, a.act_words, p.act_wpc, s.hbeg, m.hidden, p.n_cta, (p.hpc_max + 1) >> 1, seq, 8, nullptr, [&](int k, float v, float) { xa_store(xa_h, k, v); });
-                } else {
-                    mega_read_words(a, s, a.act_words, m.hidden, seq, 8, nullptr, [&](int k, float v0, float v1, float, float) {
-                        if (kQuant) {
-                            qx_store_pair(s.xa, reinterpret_cast<float*>(s.xa + xa_bytes(m.hidden)), k, v0, v1);
-                        } else {
-                            xa_store(xa_h, k, v0);
-                            xa_store(xa_h, k + 1, v1);
-                        }
-                    });
-                }
-                FINE();
-                release_pending();  // the gate/up chunk
-                consumer_sync();
-                FINE();
-                stamp(step);
-                if constexpr (kGrouped) {
-                    // all rows of the CTA (at most 256), the chunks cut along the columns: a 16-row tile of the products is
-                    // then nearly full, and two chunks of eight rows would each cost as much as one of sixteen
-                    const int n_kb = m.hidden >> 5;
-                    float sum = tid < w.d_n ? s.xmid[w.d_begin + tid] : 0.f;
-                    const float* const qs = reinterpret_cast<const float*>(s.xa + xa_bytes(m.hidden));
-                    for (int k0 = 0; k0 < n_kb; k0 += group * p.s3b_kpc) {
-                        float* const base = s.partial + par * group * kMegaChunkRows;
-                        par ^= 1;
-                        const int k1 = min(n_kb, k0 + group * p.s3b_kpc);
-                        float* partial = base;
-#pragma unroll 1
-                        for (int k = k0; k < k1; k += p.s3b_kpc) {
-                            const uint8_t* ch = mega_acquire(a, s, c, n_chunk++, landed);
-                            mega_chunk_dots<WT>(ch, w.d_n, min(p.s3b_kpc, k1 - k), s.xa + (size_t)k * 128, partial, warp, lane, qs + k);
-                            partial += kMegaChunkRows;
-                            hand_back(k + p.s3b_kpc >= n_kb);
-                        }
-                        consumer_sync();
-                        if (tid < w.d_n) {
-                            partial = base;
-                            for (int k = k0; k < k1; k += p.s3b_kpc) {
-                                sum += mega_take_sum(partial, mega_chunk_lg(w.d_n, min(p.s3b_kpc, k1 - k)), tid);
-                                partial += kMegaChunkRows;
-                            }
-                        }
-                    }
-                    if (tid < w.d_n) st_word(a.x_words + w.d_begin + tid, tagged(sum, seq));
-                } else {
-                    for (int r0 = 0; r0 < w.d_n; r0 += p.s3b_rpc) {
-                        const int nr = min(p.s3b_rpc, w.d_n - r0);
-                        // (residual and address are fetched before the products)
-                        float res = 0.f;
-                        if (tid < nr) res = s.xmid[w.d_begin + r0 + tid] + (GPT2 ? __ldg(a.out_bias + (size_t)(2 * l + 1) * d + w.d_begin + r0 + tid) : 0.f);
-                        unsigned long long* const dst = a.x_words + w.d_begin + r0 + tid;
-                        const float* sums = group_products(nr, p.s3b_rpc, m.hidden >> 5, s.xa, w.d_n - r0, 1);
-                        if (tid < nr) st_word(dst, tagged(row_sum(sums, nr, p.s3b_rpc, m.hidden >> 5, tid) + res, seq));
-                    }
-                }
-                stamp(step);
-            }
-            pos++;  // the token that was just processed is now visible
-        }
-        // ---- LM head over this CTA's vocabulary rows, first-max argmax
-#ifdef MEGA_FINE_TRACE
-        fine_layer = 99; fine_step = step;
-#endif
-        stamp(step);
-        // Everything this CTA wrote with plain stores during the step (KV-cache rows; the CTA barriers since then order
-        // them before this thread) is made visible before the candidate words that thread 0 publishes at the end of the
-        // head.  Issued here, the fence overlaps the wait for the last layer's output.
-        if (tid == 0) __threadfence();
-        float head_inv = 1.f;
-        {
-            float ss = 0.f;
-            LnGains ahead;
-            if (GPT2) ahead = ln_gains(fin_gain);
-            if (step == 0 && GPT2) {
-                for (int k = 2 * tid; k < d; k += 2 * kMegaConsumers) {
-                    const float2 v = __ldcg(reinterpret_cast<const float2*>(a.hidden_io + k));
-                    ln_take(s.xraw, k, v.x, v.y);
-                }
-            } else if (step == 0) {
-                for (int k = tid; k < d; k += kMegaConsumers) stage_x(s.xraw, d, head_digits, k, __ldcg(a.hidden_io + k), __ldg(fin_gain + k), ss);
-            } else if (GPT2) {
-                mega_read_words(a, s, a.x_words, d, a.tag0 + (unsigned)(step * L), 9, nullptr, [&](int k, float v0, float v1, float, float) { ln_take(s.xraw, k, v0, v1); });
-            } else {
-                mega_read_words(a, s, a.x_words, d, a.tag0 + (unsigned)(step * L), 9, fin_gain, [&](int k, float v0, float v1, float g0, float g1) { stage_x2(s.xraw, d, head_digits, k, v0, v1, g0, g1, ss); });
-            }
-            release_pending();  // the W2 chunk of the last layer
-            if (GPT2) head_inv = layer_norm(s.xraw, fin_gain, ahead);
-            else consumer_sync();  // the RMSNorm scale is positive: the arg-max does not need it
-        }
-        stamp(step);
-        float best_v = -INFINITY;
-        int best_i = 0x7fffffff;
-        const float* head_ln = GPT2 ? a.ln + (size_t)L * ln_rows + w.v_begin : nullptr;
-        for (int r0 = 0; r0 < w.v_n; r0 += group * p.head_rpc) {
-            const int nrows = min(group * p.head_rpc, w.v_n - r0);
-            FINE();
-            float n0 = 0.f;
-            if (GPT2 && tid < nrows) n0 = __ldg(head_ln + r0 + tid);
-            const float* sums = group_products(nrows, p.head_rpc, d >> 5, s.xa, w.v_n - r0, 2, true);
-            // a thread keeps the best of its rows (ascending: '>' keeps the first maximum)
-            each(nrows, [&](int r) {
-                float v = row_sum(sums, nrows, p.head_rpc, d >> 5, r);
-                if (GPT2) {
-                    if (r >= kMegaConsumers) n0 = __ldg(head_ln + r0 + r);
-                    v = fmaf(v, head_inv, n0);
-                }
-                if (v > best_v) { best_v = v; best_i = w.v_begin + r0 + r; }
-            });
-        }
-#ifdef MEGA_FINE_TRACE
-        if (a.trace && tid == 0 && step == a.n_steps - 1) { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); a.trace[600 + blockIdx.x] = (long long)t; }
-#endif
-        // CTA-wide best (larger value first, then smaller index), published as one word per CTA:
-        // [ordered logit bits : 32][0xffffff - index : 24][tag : 8].  The tag is the same in every word of a step, so the
-        // largest word is the best candidate; 148 consecutive words are ten cache lines for every reader.
-        const unsigned long long tag8 = (unsigned long long)((a.cand0 + (unsigned)step) % 255u + 1u);
-        {
-            unsigned long long k = best_i != 0x7fffffff ? ((unsigned long long)ordered_bits(best_v) << 32) | ((unsigned long long)(0xffffffu - (unsigned)best_i) << 8) : 0ull;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, off));
-            if (lane == 0) s.key[warp] = k;
-        }
-        consumer_sync();
-        if (tid == 0) {
-            unsigned long long k = 0ull;
-#pragma unroll
-            for (int x = 0; x < kMegaConsumerWarps; x++) k = max(k, s.key[x]);
-            st_word(a.cand_words + (size_t)blockIdx.x * kMegaCandStride, k | tag8);
-        }
-        stamp(step);
-        {
-            unsigned long long k = 0ull;
-            if (tid < p.n_cta) {
-                unsigned spins = 0;
-                if (!mega_aborting(s)) {
-                    while (true) {
-                        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(k) : "l"(a.cand_words + (size_t)tid * kMegaCandStride) : "memory");
-                        if ((k & 0xffull) == tag8) break;
-                        if (mega_spin_out(a, s, spins, 10)) break;
-                        mega_backoff();
-                    }
-                }
-                // a reader orders its later loads (the KV-cache rows other CTAs appended during this step) after the
-                // candidate words it saw; the writers' side of the pair is the fence at the start of the head
-                __threadfence();
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, off));
-            consumer_sync();  // s.key was read by thread 0 above
-            if (lane == 0) s.key[warp] = k;
-            if (tid == 0) s.red[63] = mega_aborting(s) ? 1.f : 0.f;  // one decision for the whole CTA
-            consumer_sync();
-            k = 0ull;
-#pragma unroll
-            for (int x = 0; x < kMegaConsumerWarps; x++) k = max(k, s.key[x]);
-            tok = min(0xffffffu - (uint32_t)((k >> 8) & 0xffffffull), (uint32_t)(m.vocab - 1));  // in range even if every logit was NaN
-        }
-        release_pending();  // the last head chunks
-        stamp(step);
-#ifdef MEGA_FINE_TRACE
-        if (a.trace && tid == 0 && step == a.n_steps - 1) { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); a.trace[800 + blockIdx.x] = (long long)t; }
-#endif
-        const bool gpt2_stop = GPT2 && tok == GPT2_EOS;  // GPT-2 rule: the stop token ends the loop without being emitted
+        work.tracing = a.trace && (int)blockIdx.x == a.trace_cta && tid == 0 && step == a.first + a.n_steps - 1;
+        work.pass(model, m, step > 0 ? L : 0, tok, pos, seq, (unsigned long long)((a.cand0 + (unsigned)step) % 255u + 1u), tok);
+        if (step > 0) pos++;  // the token that was just processed is now visible
+        const bool gpt2_stop = GPT2 && tok[0] == GPT2_EOS;  // GPT-2 rule: the stop token ends the loop without being emitted
         if (!gpt2_stop) emitted++;
         if (blockIdx.x == 0 && tid == 0 && !gpt2_stop) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             if (emitted == 1) a.stamps[1] = t;
-            a.rs.out[emitted - 1] = tok;
+            a.rs.out[emitted - 1] = tok[0];
             if (a.token_times) a.token_times[emitted - 1] = t;
         }
         // Llama rule: the end-of-sequence token is emitted, then the loop stops (every CTA sees the same token)
-        const bool eos = GPT2 ? gpt2_stop : m.eos_token >= 0 && tok == (uint32_t)m.eos_token;
+        const bool eos = GPT2 ? gpt2_stop : m.eos_token >= 0 && tok[0] == (uint32_t)m.eos_token;
         if (eos || s.red[63] != 0.f) {
             if (tid == 0) *reinterpret_cast<volatile int*>(s.stop) = 1;
             break;
@@ -1671,13 +1720,13 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const MegaArgs 
     }
     if (blockIdx.x == 0) {
         // the sequence's last hidden state (what the head just read)
-        for (int k = tid; k < d; k += kMegaConsumers) a.hidden_io[k] = s.xraw[k];
+        for (int k = tid; k < d; k += kMegaConsumers) a.hidden_io[k] = s.xres[k];
         if (tid == 0) {
             a.rs.pos[0] = pos;
-            a.rs.tok[0] = tok;
-            a.rs.next[0] = tok;
+            a.rs.tok[0] = tok[0];
+            a.rs.next[0] = tok[0];
             a.rs.n_out[0] = emitted;
-            a.stamps[2] = (unsigned long long)emitted | ((unsigned long long)tok << 32);
+            a.stamps[2] = (unsigned long long)emitted | ((unsigned long long)tok[0] << 32);
             a.stamps[3] = (unsigned long long)pos;
         }
     }
@@ -1720,56 +1769,62 @@ __device__ __forceinline__ PackRow pack_row(int wt, const PackMatrix& m, int col
     return r;
 }
 
-// Writes `nr` rows of K columns each in the order the products read them: for every block of 32 columns, for every row,
-// four pieces.  fp16: piece t holds columns {2t, 2t+1, 2t+8, 2t+9, 16+2t, 17+2t, 24+2t, 25+2t} of the block (the A registers
-// of two m16n8k16 steps for the lanes with that t).  Q8_0: the int8 of columns 4t..4t+3 and 16+4t..16+4t+3 (the A registers
-// of one m16n8k32 step); Q4_0: bytes 2t, 2t+1, 2t+8, 2t+9 of the GGUF block, whose low and high nibbles are the fp16 piece's columns.
-// The quantised types put the scales [block][row] behind the data.  row_of(r) names the row's source.
+// Writes a stage's `rows` rows in the order the products read them: group by group of rows, chunk by chunk of K units, inside a
+// chunk [unit][row][four pieces] and behind it, for the quantised types, the scales [unit][tile][g][rows g and g + 8 of the tile].
+// fp16: piece t of a unit of 16 columns holds columns {2t, 2t+1, 2t+8, 2t+9} (the A registers of an m16n8k16 step for the lanes
+// with that t).  Q8_0: the int8 of columns 4t..4t+3 and 16+4t..16+4t+3 of a block (the A registers of one m16n8k32 step); Q4_0:
+// bytes 4t..4t+3 of the GGUF block, whose low and high nibbles are the same columns, as two's-complement nibbles (8 less).
+// row_of(r) names the row's source.
 template <class RowOf>
-__device__ __forceinline__ void pack_tiled(int wt, uint8_t* dst, int nr, int K, RowOf row_of) {
-    const int n_kb = K >> 5;
-    const int piece = wt == WT_Q8_0 ? 8 : wt == WT_Q4_0 ? 4 : 16;
-    for (int i = threadIdx.x; i < n_kb * nr * 4; i += blockDim.x) {
-        const int t = i & 3, q = i >> 2;
-        const int kb = q / nr, r = q - kb * nr;
-        const PackRow src = row_of(r);
-        uint8_t* out = dst + ((size_t)q * 4 + t) * piece;
-        if (wt == WT_F16) {
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (src.data) {
-                const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src.data + (size_t)kb * 64);
-                v = make_uint4(s32[t], s32[t + 4], s32[t + 8], s32[t + 12]);
+__device__ __forceinline__ void pack_stage(int wt, uint8_t* dst, const MegaStage& st, int rows, RowOf row_of) {
+    const int piece = wt == WT_Q4_0 ? 4 : 8;
+    for (int r0 = 0; r0 < rows; r0 += st.group_rows) {
+        const int n = min(st.group_rows, rows - r0);
+        for (int u0 = 0; u0 < st.units; u0 += st.chunk_units) {
+            const int nu = min(st.chunk_units, st.units - u0);
+            for (int i = threadIdx.x; i < nu * n * 4; i += blockDim.x) {
+                const int t = i & 3, x = i >> 2, u = x / n, r = x - u * n;
+                const PackRow src = row_of(r0 + r);
+                uint8_t* out = dst + (size_t)i * piece;
+                if (wt == WT_F16) {
+                    uint2 v = make_uint2(0, 0);
+                    if (src.data) {
+                        const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src.data + (size_t)(u0 + u) * 32);
+                        v = make_uint2(s32[t], s32[t + 4]);
+                    }
+                    *reinterpret_cast<uint2*>(out) = v;
+                } else if (wt == WT_Q8_0) {
+                    uint2 v = make_uint2(0, 0);
+                    if (src.data) {
+                        const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src.data + (size_t)(u0 + u) * 32);  // four columns each
+                        v = make_uint2(s32[t], s32[4 + t]);
+                    }
+                    *reinterpret_cast<uint2*>(out) = v;
+                } else {
+                    uint32_t v = 0u;
+                    if (src.data) v = reinterpret_cast<const uint32_t*>(src.data + (size_t)(u0 + u) * 16)[t] ^ 0x88888888u;
+                    *reinterpret_cast<uint32_t*>(out) = v;
+                }
             }
-            *reinterpret_cast<uint4*>(out) = v;
-        } else if (wt == WT_Q8_0) {
-            uint2 v = make_uint2(0, 0);
-            if (src.data) {
-                const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src.data + (size_t)kb * 32);  // four columns each
-                v.x = s32[t];      // columns 4t .. 4t+3
-                v.y = s32[4 + t];  // columns 16+4t .. 16+4t+3
+            if (wt != WT_F16) {
+                const int padded = (n + 15) / 16 * 16;
+                __half* sc = reinterpret_cast<__half*>(dst + (size_t)nu * mega_data_bytes(wt, n));
+                for (int i = threadIdx.x; i < nu * padded; i += blockDim.x) {
+                    const int u = i / padded, x = i - u * padded, r = (x & ~15) + ((x & 15) >> 1) + 8 * (x & 1);
+                    __half v = __float2half(0.f);
+                    if (r < n) {
+                        const PackRow src = row_of(r0 + r);
+                        if (src.data) v = src.scales[u0 + u];
+                    }
+                    sc[i] = v;
+                }
             }
-            *reinterpret_cast<uint2*>(out) = v;
-        } else {
-            uint32_t v = 0x88888888u;  // nibble 8 = value 0
-            if (src.data) {
-                const uint16_t* s16 = reinterpret_cast<const uint16_t*>(src.data + (size_t)kb * 16);  // pairs of bytes
-                v = (uint32_t)s16[t] | ((uint32_t)s16[t + 4] << 16);
-            }
-            *reinterpret_cast<uint32_t*>(out) = v;
-        }
-    }
-    if (wt != WT_F16) {
-        __half* sc = reinterpret_cast<__half*>(dst + (size_t)n_kb * nr * 4 * piece);
-        for (int i = threadIdx.x; i < n_kb * nr; i += blockDim.x) {
-            const int kb = i / nr, r = i - kb * nr;
-            const PackRow src = row_of(r);
-            sc[i] = src.data ? src.scales[kb] : __float2half(0.f);
+            dst += (size_t)nu * mega_unit_bytes(wt, n);
         }
     }
 }
 
-// One CTA builds the blob of one CTA of the decode kernel: per layer [S1 | S2 | S3 gate/up | S3 W2], then the head;
-// every stage is a sequence of chunks (the units the ring carries), each in the tiled order above.
+// One CTA builds the blob of one CTA of the decode kernel: per layer [S1 | S2 | S3 gate/up | S3 W2], then the head.
 __global__ void k_build_pack(PackSources src, MegaPlan p, ModelDims m, uint8_t* pack) {
     const int cta = blockIdx.x;
     uint8_t* blob = pack + (size_t)cta * p.cta_bytes;
@@ -1780,54 +1835,30 @@ __global__ void k_build_pack(PackSources src, MegaPlan p, ModelDims m, uint8_t* 
         uint8_t* base = blob + (size_t)l * p.layer_bytes;
         // S1: pairs of rows in RoPE order
         if (w.in_group)
-            for (int i0 = 0; i0 < w.s1_n; i0 += p.s1_ipc) {
-                const int n = min(p.s1_ipc, w.s1_n - i0);
-                pack_tiled(wt, base + (size_t)i0 * 2 * p.row_bytes, 2 * n, d, [&](int r) {
-                    int kind, row0, row1, idx;
-                    mega_s1_rows(m, p, w.kvh, w.s1_begin + i0 + (r >> 1), kind, row0, row1, idx);
-                    const PackMatrix& W = kind == 0 ? src.wq[l] : kind == 1 ? src.wk[l] : src.wv[l];
-                    return pack_row(wt, W, d, (size_t)((r & 1) ? row1 : row0), 0);
-                });
-            }
+            pack_stage(wt, base, p.stage[MS_QKV], 2 * w.s1_n, [&](int r) {
+                int kind, row0, row1, idx;
+                mega_s1_rows(m, p, w.kvh, w.s1_begin + (r >> 1), kind, row0, row1, idx);
+                const PackMatrix& W = kind == 0 ? src.wq[l] : kind == 1 ? src.wk[l] : src.wv[l];
+                return pack_row(wt, W, d, (size_t)((r & 1) ? row1 : row0), 0);
+            });
         base += p.s1_bytes;
         // S2: rows [blk*rpb, +rpb) of Wo, columns of one head
         if (w.in_group)
-            for (int r0 = 0; r0 < p.rpb; r0 += p.s2_rpc) {
-                const int n = min(p.s2_rpc, p.rpb - r0);
-                pack_tiled(wt, base + (size_t)r0 * p.wo_row_bytes, n, hd, [&](int r) {
-                    const int orow = w.blk * p.rpb + r0 + r;
-                    return orow < d ? pack_row(wt, src.wo[l], m.q_dim, (size_t)orow, w.head * hd) : PackRow{nullptr, nullptr};
-                });
-            }
+            pack_stage(wt, base, p.stage[MS_WO], p.rpb, [&](int r) {
+                const int orow = w.blk * p.rpb + r;
+                return orow < d ? pack_row(wt, src.wo[l], m.q_dim, (size_t)orow, w.head * hd) : PackRow{nullptr, nullptr};
+            });
         base += p.s2_bytes;
         // S3: (gate_j, up_j) row pairs
-        for (int j0 = 0; j0 < w.h_n; j0 += p.s3a_ipc) {
-            const int n = min(p.s3a_ipc, w.h_n - j0), fr = p.ffn_rows;
-            pack_tiled(wt, base + (size_t)j0 * fr * p.row_bytes, fr * n, d, [&](int r) {
-                return pack_row(wt, fr == 2 && (r & 1) ? src.w3[l] : src.w1[l], d, (size_t)(w.h_begin + j0 + (fr == 2 ? r >> 1 : r)), 0);
-            });
-        }
+        const int fr = p.ffn_rows;
+        pack_stage(wt, base, p.stage[MS_UP], fr * w.h_n, [&](int r) {
+            return pack_row(wt, fr == 2 && (r & 1) ? src.w3[l] : src.w1[l], d, (size_t)(w.h_begin + (fr == 2 ? r >> 1 : r)), 0);
+        });
         base += p.s3a_bytes;
         // S3: this CTA's rows of W2
-        if (wt != WT_F16) {
-            size_t at = 0;
-            for (int k = 0; k < m.hidden >> 5; k += p.s3b_kpc) {
-                const int cols = 32 * min(p.s3b_kpc, (m.hidden >> 5) - k);
-                pack_tiled(wt, base + at, w.d_n, cols, [&](int r) { return pack_row(wt, src.w2[l], m.hidden, (size_t)(w.d_begin + r), 32 * k); });
-                at += (size_t)w.d_n * mega_row_bytes(wt, cols);
-            }
-            continue;
-        }
-        for (int r0 = 0; r0 < w.d_n; r0 += p.s3b_rpc) {
-            const int n = min(p.s3b_rpc, w.d_n - r0);
-            pack_tiled(wt, base + (size_t)r0 * p.down_row_bytes, n, m.hidden, [&](int r) { return pack_row(wt, src.w2[l], m.hidden, (size_t)(w.d_begin + r0 + r), 0); });
-        }
+        pack_stage(wt, base, p.stage[MS_DOWN], w.d_n, [&](int r) { return pack_row(wt, src.w2[l], m.hidden, (size_t)(w.d_begin + r), 0); });
     }
-    uint8_t* hb = blob + (size_t)m.n_layer * p.layer_bytes;
-    for (int r0 = 0; r0 < w.v_n; r0 += p.head_rpc) {
-        const int n = min(p.head_rpc, w.v_n - r0);
-        pack_tiled(p.wt_head, hb + (size_t)r0 * p.head_row_bytes, n, d, [&](int r) { return pack_row(p.wt_head, src.lm_head, d, (size_t)(w.v_begin + r0 + r), 0); });
-    }
+    pack_stage(p.wt_head, blob + (size_t)m.n_layer * p.layer_bytes, p.stage[MS_HEAD], w.v_n, [&](int r) { return pack_row(p.wt_head, src.lm_head, d, (size_t)(w.v_begin + r), 0); });
 }
 
 // GPT-2: W.b + bias of every row of a matrix [rows][K] (see MegaArgs::ln).  One warp per row.

@@ -133,6 +133,36 @@ def test_quantised_down_projection_in_column_chunks(rt, oracle_lib, kind, n_head
     eng.close()
 
 
+@pytest.mark.parametrize("kind,head,n_head,n_kv,head_dim,hidden,vocab", [
+    ("f16", "f16", 3, 3, 32, 96, 301),          # fewer K units than warps
+    ("f16", "f16", 6, 2, 64, 2944, 12000),      # gate/up rows in three tiles, the head in two groups
+    ("f16", "f16", 12, 12, 64, 7168, 31000),    # gate/up rows in two groups
+    ("q8_0", "q8_0", 4, 1, 128, 512, 2000),     # q/k/v rows past one tile
+    ("q8_0", "f16", 8, 2, 64, 768, 9000),       # an fp16 head on quantised layers
+    ("q4_0", "q4_0", 8, 8, 32, 9728, 26001),    # two groups, a ragged last row
+])
+def test_row_groups_and_units_of_the_persistent_kernel(rt, oracle_lib, kind, head, n_head, n_kv, head_dim, hidden, vocab):
+    """A CTA's rows in one to five tiles and in several groups, K units that do not divide among the warps, contexts that pass a
+    warp round (256 positions)."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-groups", 2, n_head, n_kv, n_head * head_dim, head_dim, hidden, vocab, 300)
+    if kind == "f16":
+        eng, model = dense_pair(rt, oracle_lib, cfg)
+    else:
+        model, uploads = quantised_pair(oracle_lib, cfg, kind, quantise_head=head != "f16")
+        eng = rt.DecodeEngine.empty(cfg)
+        upload_all(eng, uploads)
+    for length in (9, 250):
+        prompt = synthetic_prompt(cfg.vocab, length)
+        res = eng.generate(prompt, 14)
+        assert eng.timings()["kernel_launches"] == 1
+        ora = oracle_lib.Runtime(model)
+        compare_greedy_stream(ora, prompt, res.tokens)
+        assert_logits_close(eng.logits(), ora.logits(), f"{kind} {length}")
+    eng.close()
+
+
 @pytest.mark.parametrize("n_seq", [3, 40, 330])
 def test_full_sequence_beside_unfinished_ones(rt, oracle_lib, n_seq):
     """A sequence that has filled its context stays in the batch as an inactive row one position past the rotation table;
