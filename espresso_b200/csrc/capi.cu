@@ -32,7 +32,12 @@ static int32_t fail(int32_t code, const std::string& msg) {
 }
 
 #define ESP_GUARD(engine) \
-    if (!(engine)) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "null engine handle")
+    if (!(engine)) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "null engine handle"); \
+    if ((engine)->impl.streaming()) {  /* called from a generate_steps callback */ \
+        const int32_t settled = const_cast<esp_cuda_engine*>(engine)->impl.stream_settle(); \
+        if (settled) return settled; \
+    } \
+    do {} while (0)
 
 // ---- metadata.json (Sources/ESPCompiler/ESPModelConfigIO.swift:12-59): a flat JSON object ------------
 
@@ -174,7 +179,9 @@ int32_t esp_cuda_generate_batch(esp_cuda_engine* engine, const uint32_t* prompts
 // Step-by-step generation with the caller's callback invoked inline after every token, as the reference's loop does
 // with onStep (Engine.swift:6393-6405): prefill, select the first token, then one decode step per token.  Limits and
 // stop rules as in generate (Llama: the EOS token is emitted, then the loop stops, :6385-6388; GPT-2: 50256 stops
-// without being emitted, :4918-4922).
+// without being emitted, :4918-4922).  Where the persistent kernel serves the model the device runs ahead of the callback
+// (Engine::stream_begin); a callback that uses the engine finds it as the step-by-step loop leaves it, and that loop goes on
+// from there.
 int32_t esp_cuda_generate_steps(esp_cuda_engine* engine, const uint32_t* prompt, int32_t n_prompt, int32_t max_tokens,
                                 esp_cuda_step_callback on_step, void* user, uint32_t* out_tokens, int32_t* n_out,
                                 esp_cuda_generation_result* result) {
@@ -201,9 +208,7 @@ int32_t esp_cuda_generate_steps(esp_cuda_engine* engine, const uint32_t* prompt,
     bool hit_eos = false;
     double first_ms = 0.0;
     uint32_t tok = 0;
-    if ((rc = e.select_greedy(&tok))) return rc;
-    while (true) {
-        if (c.architecture == ESP_CUDA_ARCH_GPT2 && tok == 50256u) { hit_eos = true; break; }
+    auto report = [&] {
         auto t = now();
         const double lat = ms(t_last, t);
         t_last = t;
@@ -212,7 +217,38 @@ int32_t esp_cuda_generate_steps(esp_cuda_engine* engine, const uint32_t* prompt,
         latencies.push_back((float)lat);
         if (on_step) on_step(user, tok, gen, lat);
         gen++;
-        if (c.architecture != ESP_CUDA_ARCH_GPT2 && c.eos_token >= 0 && tok == (uint32_t)c.eos_token) { hit_eos = true; break; }
+    };
+    const bool gpt2 = c.architecture == ESP_CUDA_ARCH_GPT2;
+    auto is_eos = [&] { return !gpt2 && c.eos_token >= 0 && tok == (uint32_t)c.eos_token; };
+    bool by_steps = !e.stream_usable(), reported = false;
+    if (!by_steps) {
+        if ((rc = e.stream_begin(eff))) return rc;
+        bool got = true;
+        while (gen < eff) {
+            if ((rc = e.stream_next(gen, &tok, &got))) return rc;
+            if (!got) break;
+            report();
+            if (esp::force_failure_enabled() && (rc = e.stream_settle())) return rc;
+            if (!e.streaming()) {  // the callback used the engine
+                if (e.stream_error()) return e.stream_error();
+                by_steps = reported = true;
+                break;
+            }
+        }
+        if (!by_steps) {
+            if ((rc = e.stream_end())) return rc;
+            hit_eos = gpt2 ? gen < eff : gen > 0 && is_eos();
+        }
+    } else if ((rc = e.select_greedy(&tok))) {
+        return rc;
+    }
+    while (by_steps) {
+        if (!reported) {
+            if (gpt2 && tok == 50256u) { hit_eos = true; break; }
+            report();
+        }
+        reported = false;
+        if (is_eos()) { hit_eos = true; break; }
         if (gen >= eff || n_prompt + gen >= c.max_seq) break;
         uint32_t next = 0;
         if ((rc = e.decode_step(tok, &next))) return rc;

@@ -381,6 +381,7 @@ Engine::~Engine() {
     if (h_rows_block_) cudaFreeHost(h_rows_block_);
     if (h_next_) cudaFreeHost(h_next_);
     if (h_mega_ctl_) cudaFreeHost(h_mega_ctl_);
+    if (h_stream_) cudaFreeHost(h_stream_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -2299,6 +2300,11 @@ int32_t Engine::build_mega_gpt2() {
 // state, or (feed != null) starting with a forward pass for the token *feed at the current position.  h_mega_ctl_ then
 // holds {.., error, start, first token, {last token, tokens emitted}}.
 int32_t Engine::launch_mega(int n_steps, const uint32_t* feed, bool times) {
+    const int32_t rc = enqueue_mega(n_steps, feed, times, nullptr);
+    return rc ? rc : finish_mega();
+}
+
+int32_t Engine::enqueue_mega(int n_steps, const uint32_t* feed, bool times, unsigned long long* host_words) {
     MegaArgs a{};
     const MegaPlan& p = mega_plan_;
     a.m = m_; a.plan = p; a.pack = d_pack_; a.norms = d_norms_;
@@ -2316,6 +2322,7 @@ int32_t Engine::launch_mega(int n_steps, const uint32_t* feed, bool times) {
     a.rs = rs_;
     a.trace = d_mega_trace_;
     a.token_times = times && n_steps <= m_.max_seq + 1 ? d_token_times_ : nullptr;
+    a.host_words = host_words;
     token_times_n_ = 0;
     a.trace_cta = std::min(mega_trace_cta_, p.n_cta - 1);
     a.n_steps = n_steps;
@@ -2341,6 +2348,11 @@ int32_t Engine::launch_mega(int n_steps, const uint32_t* feed, bool times) {
     ESP_CUDA_TRY(cudaLaunchCooperativeKernel(mega_kernel_for(m_.head_dim, p.wt_layer, m_.arch == ARCH_GPT2), dim3(p.n_cta), dim3(kMegaThreads), args, (size_t)p.smem_bytes, stream_));
     if (times) ESP_CUDA_TRY(cudaEventRecord(ev_end_, stream_));
     ESP_CUDA_TRY(cudaMemcpyAsync(h_mega_ctl_, d_mega_ctl_, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream_));
+    mega_first_ = a.first;
+    return ESP_CUDA_OK;
+}
+
+int32_t Engine::finish_mega() {
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
     launches_last_step_ = 1;
     timings_.kernel_launches = 1;
@@ -2351,7 +2363,7 @@ int32_t Engine::launch_mega(int n_steps, const uint32_t* feed, bool times) {
            << ": 3 = weight chunk, 4 = ring slot, 5/9 = layer output words, 6 = q/k/v words, 7 = attention sums, 8 = activation words, 10 = arg-max words)";
         return fail(ESP_CUDA_ERR_TIMEOUT, os.str());
     }
-    mega_cand_ = (a.cand0 + (unsigned)a.first + (unsigned)(h_mega_ctl_[5] & 0xffffffffull) + 1u) % 255u;  // behind the last step that ran (GPT-2's last one may emit nothing)
+    mega_cand_ = (mega_cand_ + (unsigned)mega_first_ + (unsigned)(h_mega_ctl_[5] & 0xffffffffull) + 1u) % 255u;  // behind the last step that ran (GPT-2's last one may emit nothing)
     mega_dirty_ = false;
     return ESP_CUDA_OK;
 }
@@ -2376,6 +2388,80 @@ int32_t Engine::run_mega(int n_steps, int* emitted, float* device_ms, double* fi
         for (int i = 0; i < n; i++) { latencies_ms_.push_back((float)((double)(tt[i] - prev) / 1e6)); prev = tt[i]; }
     }
     h_visible_[0] = (int)h_mega_ctl_[6];
+    return ESP_CUDA_OK;
+}
+
+// Token-by-token reporting of one greedy loop of sequence 0.  The whole loop is one launch; the kernel writes every token to pinned
+// host memory as it becomes known and goes on, and the host reports it (stream_next) while the next one is computed: a
+// launch and a host round trip per token took 107 us where the kernel needs 64 (6 layers d768).
+// A caller that uses the engine between two tokens (from its callback) must find it as a step-by-step loop would have left it: every
+// entry point first settles the stream, i.e. lets the kernel finish and goes back to the state after the reported token.
+// The reporting loop then goes on step by step.
+bool Engine::stream_usable() const { return mega_usable() && !(cfg_.flags & ESP_CUDA_FLAG_KEEP_LOGITS); }
+
+int32_t Engine::stream_begin(int n_steps) {
+    int32_t rc = check_ready("generate_steps");
+    if (rc) return rc;
+    if (h_visible_[0] <= 0 || n_steps < 1 || n_steps > m_.max_seq) return fail(ESP_CUDA_ERR_STATE, "generate_steps: sequence has no prefilled tokens");
+    if (!h_stream_) {
+        if ((rc = dev_alloc(owned_, &d_stream_hidden_, (size_t)m_.d_model, false))) return rc;
+        ESP_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void**>(&h_stream_), sizeof(unsigned long long) * m_.max_seq, cudaHostAllocPortable));
+    }
+    memset(h_stream_, 0, sizeof(unsigned long long) * n_steps);
+    ESP_CUDA_TRY(cudaMemcpyAsync(d_stream_hidden_, act_.hidden, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_));
+    if ((rc = enqueue_mega(n_steps, nullptr, false, h_stream_))) return rc;
+    streaming_ = true;
+    stream_error_ = ESP_CUDA_OK;
+    stream_visible_ = h_visible_[0];
+    stream_reported_ = 0;
+    return ESP_CUDA_OK;
+}
+
+// Waits for token number i of the loop; *got = false: the loop ended before it.
+int32_t Engine::stream_next(int i, uint32_t* token, bool* got) {
+    volatile unsigned long long* const word = h_stream_ + i;
+    *got = false;
+    bool ended = false;
+    for (unsigned spins = 1; *word == 0ull; spins++) {
+        if (ended) return ESP_CUDA_OK;
+        if (spins % 4096 == 0) {  // (the kernel bounds its own waits: it ends)
+            const cudaError_t e = cudaStreamQuery(stream_);
+            if (e == cudaSuccess) ended = true;  // (one more look at the word)
+            else if (e != cudaErrorNotReady) { streaming_ = false; ESP_CUDA_TRY(e); }
+        }
+    }
+    *token = (uint32_t)(*word & 0xffffffffull);
+    *got = true;
+    stream_reported_ = i + 1;
+    return ESP_CUDA_OK;
+}
+
+int32_t Engine::stream_end() {
+    streaming_ = false;
+    const int32_t rc = finish_mega();
+    if (rc) return rc;
+    h_visible_[0] = (int)h_mega_ctl_[6];
+    return ESP_CUDA_OK;
+}
+
+int32_t Engine::stream_settle() {
+    if (!streaming_) return ESP_CUDA_OK;
+    stream_error_ = stream_rewind();
+    return stream_error_;
+}
+
+int32_t Engine::stream_rewind() {
+    int32_t rc = stream_end();
+    if (rc) return rc;
+    const int fed = stream_reported_ - 1;  // the newest reported token has not been fed
+    h_visible_[0] = stream_visible_ + std::max(0, fed - 1);
+    if (fed <= 0) {
+        ESP_CUDA_TRY(cudaMemcpyAsync(act_.hidden, d_stream_hidden_, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_));
+        return ESP_CUDA_OK;
+    }
+    const uint32_t token = (uint32_t)(h_stream_[fed - 1] & 0xffffffffull);
+    if ((rc = launch_mega(1, &token, false))) return rc;  // the same pass once more: the same cache rows and hidden state
+    h_visible_[0]++;
     return ESP_CUDA_OK;
 }
 

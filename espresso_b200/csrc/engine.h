@@ -80,6 +80,14 @@ public:
                            uint32_t* out_tokens, int32_t* n_out, esp_cuda_generation_result* result);
     int32_t decode_loop(int32_t n_seq, int32_t count, uint32_t* out_tokens, int32_t out_stride, int32_t* n_out,
                         float* device_ms, double* first_token_ms);
+    // Reporting a greedy loop token by token (generate_steps); every other entry point settles it first.
+    bool stream_usable() const;
+    bool streaming() const { return streaming_; }
+    int32_t stream_begin(int n_steps);
+    int32_t stream_next(int i, uint32_t* token, bool* got);
+    int32_t stream_end();
+    int32_t stream_settle();
+    int32_t stream_error() const { return stream_error_; }  // of the last settling
     int32_t stage_trace(int32_t cta, long long* out, int32_t capacity, int32_t* n);
     int32_t token_times(unsigned long long* out_ns, int32_t capacity, int32_t* n);
     int32_t token_latencies(float* out_ms, int32_t capacity, int32_t* n);
@@ -134,6 +142,8 @@ private:
     int32_t build_mega();   // packs the weights for the persistent decode kernel when the model qualifies
     int32_t build_mega_gpt2();
     int32_t launch_mega(int n_steps, const uint32_t* feed, bool times);
+    int32_t enqueue_mega(int n_steps, const uint32_t* feed, bool times, unsigned long long* host_words);
+    int32_t finish_mega();
     bool mega_usable() const;
     int32_t run_mega(int n_steps, int* emitted, float* device_ms, double* first_token_ms);
     int32_t spec_prepare();   // plan, arena and result block of the two-position kernel
@@ -230,6 +240,14 @@ private:
     unsigned mega_spin_limit_ = kMegaSpinLimit;   // attempts per device-side wait (test hook: set_wait_limit)
     unsigned long long* d_mega_ctl_ = nullptr;  // [2] error (i32 in the upper half), [3..4] time stamps, [5] tokens emitted
     unsigned long long* h_mega_ctl_ = nullptr;  // pinned mirror
+    int mega_first_ = 0;  // `first` of the launch in flight
+    // token-by-token reporting (stream_begin)
+    int32_t stream_rewind();
+    bool streaming_ = false;
+    int32_t stream_error_ = 0;
+    int stream_visible_ = 0, stream_reported_ = 0;  // visible tokens at its start, tokens reported so far
+    unsigned long long* h_stream_ = nullptr;  // pinned [max_seq]
+    float* d_stream_hidden_ = nullptr;        // [d_model] hidden state at its start
     long long* d_mega_trace_ = nullptr;
     unsigned long long* d_token_times_ = nullptr;  // [max_seq] emission time of every token of the last persistent loop
     int token_times_n_ = 0;

@@ -140,6 +140,7 @@ struct MegaArgs {
     float* hidden_io;         // [d_model] last hidden state of the sequence (in and out)
     int* error;               // [1] 0 = ok
     unsigned long long* stamps; // [4] globaltimer at kernel start and when the first token is known; {last token : 32}{number of tokens emitted : 32}; visible tokens
+    unsigned long long* host_words;  // optional pinned host memory [n_steps]: {number of tokens emitted : 32}{token : 32} of every token as it becomes known, or null
     unsigned long long* token_times; // optional [n_steps] globaltimer (ns) at which each token became known, or null
     long long* trace;         // optional [kMegaTraceLayer*L + kMegaTraceHead] SM clock stamps of the last step taken by CTA `trace_cta`, or null
     int trace_cta;
@@ -1709,6 +1710,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const __grid_co
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             if (emitted == 1) a.stamps[1] = t;
             a.rs.out[emitted - 1] = tok[0];
+            if (a.host_words) asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(a.host_words + emitted - 1), "l"(((unsigned long long)emitted << 32) | tok[0]) : "memory");
             if (a.token_times) a.token_times[emitted - 1] = t;
         }
         // Llama rule: the end-of-sequence token is emitted, then the loop stops (every CTA sees the same token)

@@ -568,6 +568,44 @@ def test_token_emission_times_of_the_persistent_loop(rt, tmp_models):
     eng.close()
 
 
+@pytest.mark.parametrize("use_at", [(), (0,), (3, 7)])
+@pytest.mark.parametrize("eos", [False, True])
+def test_streamed_tokens_and_a_callback_that_uses_the_engine(rt, tmp_models, use_at, eos):
+    """The tokens reach the callback in order while the device runs ahead; an engine used from inside the callback is in the state
+    after the reported token, and the loop goes on from there, also to its stop rule."""
+    from espresso_b200.model_config import tiny_llama
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = tiny_llama(vocab=515, max_seq=64)
+    d = tmp_models(cfg)
+    prompt = synthetic_prompt(cfg.vocab, 9)
+    eng = rt.DecodeEngine.build(d)
+    plain = [int(t) for t in eng.generate(prompt, 12).tokens]
+    if eos:
+        eng.close()
+        cfg = dataclasses.replace(cfg, eosToken=plain[8])
+        eng = rt.DecodeEngine.build(tmp_models(cfg))
+        plain = plain[:plain.index(plain[8]) + 1]
+    other = rt.DecodeEngine.build(tmp_models(cfg))
+    seen = []
+
+    def on_step(token, index, _ms):
+        seen.append((token, index))
+        if index in use_at:
+            other.prefill(list(prompt) + plain[:index])
+            assert eng.visible_token_count() == len(prompt) + index
+            assert eng.select_greedy_token() == token
+            np.testing.assert_allclose(eng.logits(), other.logits(), atol=2e-2)
+
+    res = eng.generate(prompt, 12, on_step=on_step)
+    assert [t for t, _ in seen] == plain and [i for _, i in seen] == list(range(len(plain)))
+    assert [int(t) for t in res.tokens] == plain
+    assert eng.visible_token_count() == len(prompt) + len(plain) - 1
+    assert eng.generate(prompt, 12).tokens.tolist() == plain
+    eng.close()
+    other.close()
+
+
 @pytest.mark.parametrize("kind", ["f16", "q8_0"])
 def test_persistent_kernel_streams_wide_stages_in_chunks(rt, oracle_lib, tmp_models, kind):
     """d_model 2048 / hidden 5632: every stage slice of the persistent kernel exceeds a ring slot and arrives in chunks
