@@ -34,6 +34,7 @@ struct DecodeAttArgs {
     int parts;
     int layer;
     float* debug;      // optional fp32 capture of row 0's context (already offset), or null
+    L2Ahead ahead;
 };
 
 __host__ __device__ constexpr int da_smem_floats(int HD, int nw, int ranks) { return nw * kDaHeads * (HD + 2) + (ranks > 1 ? ranks * kDaHeads * (HD + 4) : 0); }
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
     const int nh = min(kDaHeads, qpk - h0), head0 = kvh * qpk + h0;
     const int row = (int)blockIdx.y, rank = (int)blockIdx.z, ranks = (int)gridDim.z;
     pdl_launch_dependents();
+    if (warp == 0) l2_request(p.ahead, (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x, gridDim.x * gridDim.y * gridDim.z, lane);
     pdl_wait();
     const int active = __ldcg(p.rs.active + row), pos = __ldcg(p.rs.pos + row), seq = __ldcg(p.rs.seq + row);
     float4 qv[KB][2];

@@ -1871,6 +1871,11 @@ int32_t Engine::launch_head_stream(int rows, int mode, int parts, cudaStream_t s
     return ESP_CUDA_OK;
 }
 
+// How far ahead a launch requests later weights into L2.  Larger budgets get in the way of the operands that the products wait for:
+// us per step of the 22-layer d2048 model at 5 rows / 16 rows (Q8_0 expansion): 738 / 815 without, 713 / 767 at 8 MB, 719 / 773
+// at 16, 754 / 844 at 24.  A layer that L2 does not hold (4096 wide: 436 MB) is bound by HBM itself and only loses (0.5 %).
+constexpr size_t kL2Ahead = (size_t)8 << 20, kL2Lead = (size_t)32 << 20, kL2Layer = (size_t)128 << 20;
+
 // One pass over the model for few rows (see step_path) with the streamed products (stream_gemm.cuh): per layer q/k/v (norm,
 // bias, RoPE and cache append inside), attention, Wo + residual, FFN up (norm and activation inside), W2 + residual.
 int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool profile) {
@@ -1893,6 +1898,34 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
         launches++;
         return launch_prep(rows, src, K, norm, g, b, dst, parts, s);
     };
+    // Weights in the order of their use; a launch requests the next kL2Ahead bytes behind those of the launch after it (L2Ahead), at
+    // most kLead in front of them.
+    std::vector<std::pair<const uint8_t*, size_t>> order;
+    auto weights = [&](const DeviceTensor* W) { order.emplace_back(static_cast<const uint8_t*>(W->shadow16 ? static_cast<const void*>(W->shadow16) : W->data), (size_t)W->rows * W->cols * 2); };
+    if (mode & STEP_FORWARD)
+        for (const LayerTensors& t : layer_tensors_)
+            for (const DeviceTensor* W : {t.wq, t.wk, t.wv, t.wo, t.w1, t.w3, t.w2})
+                if (W) weights(W);
+    if (mode & STEP_HEAD) weights(&tensors_.at("lm_head"));
+    size_t used = 0, requested = 0, at = 0, next = 0;  // bytes of the products launched so far, bytes requested so far; the first matrix not all requested, where it begins
+    const bool look_ahead = rows <= kSgMaxCols && 2 * ((size_t)(2 * q + 2 * kv + (gpt2 ? 2 : 3) * h) * d) <= kL2Layer;
+    auto ahead = [&](size_t budget) {
+        L2Ahead a{};
+        if (!look_ahead) return a;
+        requested = std::max(requested, used);
+        const size_t end = std::min(requested + budget, used + kL2Lead);
+        for (int n = 0; next < order.size() && at < end && n < kL2Ranges;) {
+            const size_t to = std::min(end, at + order[next].second);
+            if (requested < to) {
+                a.p[n] = order[next].first + (requested - at);
+                a.bytes[n++] = (unsigned)(to - requested);  // (whole rows of 64 and more columns, or the budgets' megabytes: multiples of 16)
+                requested = to;
+            }
+            if (to < at + order[next].second) break;
+            at += order[next++].second;
+        }
+        return a;
+    };
     struct Part { const DeviceTensor* W; float* out; int ldo; const float* bias; };
     struct Norm { const float *g, *b; };
     // norm != null: the operand is the normalised residual stream (fused, or through xbuf); else the 16-bit rows of xbuf
@@ -1907,6 +1940,8 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
             a.g[g].M = pt.W->rows; a.g[g].out = pt.out; a.g[g].ldo = pt.ldo; a.g[g].bias = pt.bias;
             g++;
         }
+        for (const Part& pt : ps) used += (size_t)pt.W->rows * K * 2;
+        a.ahead = ahead(kL2Ahead);
         a.n_groups = g; a.K = K; a.rows = rows; a.bf16 = tc_bf16_; a.error = d_tc_error_; a.m = m_; a.rs = rs_; a.kv = kv_; a.eps = m_.eps;
         if (norm) {
             a.hidden = act_.hidden; a.stat = row_stat_; a.stat_tiles = stat_tiles; a.norm = gpt2 ? NORM_LAYER : NORM_RMS; a.norm_g = norm->g; a.norm_b = norm->b;
@@ -1979,7 +2014,7 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
                 launches++;
             } else if (att_ok_hd) {
                 DecodeAttArgs da{};
-                da.m = m_; da.rs = rs_; da.kv = kv_; da.q = act_.q; da.ctx16 = xh_q_; da.bf16 = tc_bf16_; da.parts = parts; da.layer = l;
+                da.m = m_; da.rs = rs_; da.kv = kv_; da.q = act_.q; da.ctx16 = xh_q_; da.bf16 = tc_bf16_; da.parts = parts; da.layer = l; da.ahead = ahead(2 * kL2Ahead);
                 da.debug = cap ? dbg + q + 2 * kv : nullptr;
                 if ((rc = launch_attention_decode(da, rows, s))) return rc;
                 launches++;

@@ -42,6 +42,25 @@ constexpr int kSgMaxSplits = 8;   // portable cluster size
 constexpr int kSgWBytes = kSgRows * kTcBlockK * 2;
 constexpr int kSgSmemBudget = 110 * 1024;
 
+// Weights that later kernels of the step will read, brought into L2 while this one waits for its predecessor (Engine::launch_step_stream
+// says which): HBM would otherwise idle through the hand-over, the operand staging, the exchange and the attention of every stage.  Each CTA requests its
+// share of every range.
+constexpr int kL2Ranges = 4;
+struct L2Ahead {
+    const uint8_t* p[kL2Ranges];
+    unsigned bytes[kL2Ranges];  // multiples of 16; 0 ends the list
+};
+__device__ __forceinline__ void l2_request(const L2Ahead& a, unsigned cta, unsigned n_cta, int lane) {
+    constexpr unsigned kPiece = 8192;
+#pragma unroll 1
+    for (int r = 0; r < kL2Ranges && a.bytes[r]; r++) {
+        const unsigned pieces = (a.bytes[r] + kPiece - 1) / kPiece;
+#pragma unroll 1
+        for (unsigned i = cta + n_cta * (unsigned)lane; i < pieces; i += n_cta * 32u)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.p[r] + (size_t)i * kPiece), "r"(min(kPiece, a.bytes[r] - i * kPiece)) : "memory");
+    }
+}
+
 enum SgEpilogue { SG_STORE = 0, SG_RESIDUAL = 1, SG_QKV = 2, SG_GELU = 3, SG_SWIGLU = 4, SG_HEAD = 5 };
 
 struct SgGroup {
@@ -82,6 +101,7 @@ struct SgArgs {
     float* debug;         // optional capture of batch row 0
     float* logits;        // SG_HEAD: optional [n][M]
     int row_offset;       // SG_HEAD: added to the vocabulary row (shard of a tensor-parallel rank)
+    L2Ahead ahead;
     int finalize;         // SG_HEAD: the last CTA turns the packed maxima into tokens with this head_finalize mode; -1 = a later kernel does
     int* error;
 };
@@ -513,6 +533,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
         const float* bias = gi == 0 ? a.g[0].bias : gi == 1 ? a.g[1].bias : a.g[2].bias;
         if (bias && valid) bias4 = __ldg(reinterpret_cast<const float4*>(bias + m0));
     }
+    if (warp == 0) l2_request(a.ahead, ((unsigned)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x, gridDim.x * gridDim.y * gridDim.z, lane);
     pdl_launch_dependents();  // (only now: a CTA of this kernel must never queue for TMEM behind its successor)
     pdl_wait();
     const uint32_t acc = s_tmem;
@@ -568,7 +589,10 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
                 const int k0 = (kb0 + kb) * kTcBlockK;
                 phase ^= 1u;
                 if (kb >= stages) {
-                    if (norm) sg_norm_gains(a, pre_x, k0, lane);
+                    if (norm) {  // (requested before the wait for the stage)
+                        sg_norm_gains(a, pre_x, k0, lane);
+                        sg_norm_rows(a, pre_x, n0, 0, rows, k0, lane);
+                    }
                     if (!tc_wait_warp(s_empty + xw, phase ^ 1u, a.error)) break;
                     if (elect_one()) load_w(kb, xw);
                 }
@@ -579,7 +603,7 @@ __global__ void __launch_bounds__(kSgThreads, 2) k_gemm_stream(const __grid_cons
                 }
 #pragma unroll 1
                 for (int r0 = 0; r0 < rows; r0 += 16) {
-                    if (kb >= stages || r0 > 0) sg_norm_rows(a, pre_x, n0, r0, rows, k0, lane);
+                    if (r0 > 0) sg_norm_rows(a, pre_x, n0, r0, rows, k0, lane);
                     sg_norm_store<BF16>(a, pre_x, sw + kSgWBytes, s_stat, r0, rows, lane);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
