@@ -4,11 +4,14 @@
 // row state -> first keys and values -> merge.
 //
 // A CTA takes one row and one KV head, so grouped query heads share every load; its NW warps (8, 4 or 2: as many as keep
-// all pairs resident at once) take alternate blocks of sixteen positions.  Both products run on mma.sync.m16n8k16 straight from registers:
+// all pairs resident at once) take alternate blocks of sixteen positions.  Every warp keeps the next da_stages blocks in flight through
+// a ring of its own in shared memory (cp.async): a short context is then requested all at once, and its time is one round trip to
+// memory instead of one per block (operands loaded a block ahead into registers: 256 GPT-2 rows at contexts 64 to 96: 711 -> 650 us per step).  Both
+// products run on mma.sync.m16n8k16:
 //   * scores: the query heads are the A operand.  A row of the MMA is a head's fp16 part: rows 0..7 the rounded queries,
 //     rows 8..15 the rounding remainders (22 bits together), whose results land in the same thread and are added there.  Keys
 //     are the B operand; a lane's 16-byte piece of a key row supplies two MMA steps once the query's dimensions are taken in
-//     the same order, so keys go from global memory to the operand registers as they are.
+//     the same order.
 //   * context: the probabilities, again split into two fp16 parts, are the A operand (the accumulator layout of the scores
 //     is the operand layout), values the B operand: a lane loads the same run of dimensions of four positions and interleaves
 //     them with byte permutes; output dimension n * (HD / 8) + j is column n of tile j.
@@ -37,7 +40,20 @@ struct DecodeAttArgs {
     L2Ahead ahead;
 };
 
-__host__ __device__ constexpr int da_smem_floats(int HD, int nw, int ranks) { return nw * kDaHeads * (HD + 2) + (ranks > 1 ? ranks * kDaHeads * (HD + 4) : 0); }
+// Blocks in flight per warp.  Eight warps share a pair only where pairs are few: they (and the cluster) cover 128 to 1024 positions at
+// once, and more shared memory would keep the next product's CTAs off the SM (5 rows of the 22-layer model: 713 us per step with
+// one block, 716 with two, 750 with three).
+__host__ __device__ constexpr int da_stages(int HD, int nw) { return nw == 8 ? 1 : HD == 128 ? 2 : 3; }
+__host__ __device__ constexpr int da_ring_floats(int HD, int nw) { return da_stages(HD, nw) * kDaBlock * HD; }  // of one warp: keys and values, fp16
+__host__ __device__ constexpr int da_smem_floats(int HD, int nw, int ranks) { return nw * (da_ring_floats(HD, nw) + kDaHeads * 2) + (ranks > 1 ? ranks * kDaHeads * (HD + 4) : 0); }
+
+// Where 16-byte chunk c of row r of a 16-row tile lies (in bytes), so that the lanes of an operand load meet in different banks.
+template <int HD>
+__device__ __forceinline__ int da_key_at(int r, int c) { return r * (HD * 2) + ((HD == 32 ? c : c ^ ((r & 1) << 2)) << 4); }
+template <int HD>
+__device__ __forceinline__ int da_value_at(int r, int c) {
+    return r * (HD * 2) + ((HD == 32 ? c : HD == 64 ? c ^ (r & 7) : c ^ (((r >> 1) & 1) | (((r >> 2) & 1) << 2))) << 4);
+}
 
 // grid = (KV heads x head groups, rows, cluster size); cluster = (1, 1, cluster size)
 template <int HD, int NW>
@@ -46,9 +62,11 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
     constexpr int KB = HD / 32;   // 32-dimension blocks of a key row
     constexpr int NT = HD / 8;    // output tiles = dimensions per lane of a value row
     constexpr int kVw = NT / 2;   // 32-bit words of them
-    extern __shared__ float da_smem[];
-    float* const s_o = da_smem;                                        // [warp][head][HD]
-    float* const s_ml = s_o + NW * kDaHeads * HD;                // [warp][head][max, sum]
+    constexpr int kStages = da_stages(HD, NW), kTileBytes = kDaBlock * HD * 2, kRingFloats = da_ring_floats(HD, NW);
+    static_assert(kRingFloats >= kDaHeads * HD, "a warp parks its contexts in its ring");
+    extern __shared__ __align__(128) float da_smem[];
+    float* const s_o = da_smem;                                  // [warp]: the ring, then [head][HD]
+    float* const s_ml = s_o + NW * kRingFloats;                  // [warp][head][max, sum]
     float* const s_rank = s_ml + NW * kDaHeads * 2;              // rank 0 of a cluster: [rank][head][HD + 2]
     const ModelDims& m = p.m;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -78,46 +96,28 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
     const __half* K = p.kv.k + p.kv.offset(m, p.layer, seq, kvh, 0);
     const __half* V = p.kv.v + p.kv.offset(m, p.layer, seq, kvh, 0);
 
-    // keys base + g and base + g + 8: this lane's 16-byte piece of every 32 dimensions.  (Coherent loads: the product before this
-    // kernel appends to the cache while the kernel is already resident.)
-    uint4 kr[2][KB];
-    auto load_k = [&](int base) {
+    // Positions base .. base + 15 into ring stage st; those past the context read as zeros.  (Coherent copies: the product before
+    // this kernel appends to the cache while the kernel is already resident.)
+    uint8_t* const ring = reinterpret_cast<uint8_t*>(s_o + warp * kRingFloats);
+    const uint32_t ring_at = smem_u32(ring);
+    auto request = [&](int base, int st) {
+        if (base < visible) {
+            constexpr int kChunks = HD / 8;
+            const uint32_t at = ring_at + (uint32_t)(st * 2 * kTileBytes);
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int key = base + 8 * i + g;
-#pragma unroll
-            for (int kb = 0; kb < KB; kb++) {
-                kr[i][kb] = make_uint4(0, 0, 0, 0);
-                if (key < visible) kr[i][kb] = __ldca(reinterpret_cast<const uint4*>(K + (size_t)key * HD + kb * 32 + t * 8));
+            for (int i = 0; i < kDaBlock * kChunks / 32; i++) {
+                const int r = (lane + 32 * i) / kChunks, c = (lane + 32 * i) % kChunks, key = base + r;
+                const size_t src = (size_t)min(key, visible - 1) * HD + c * 8;
+                const int bytes = key < visible ? 16 : 0;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + da_key_at<HD>(r, c)), "l"(K + src), "r"(bytes) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + kTileBytes + da_value_at<HD>(r, c)), "l"(V + src), "r"(bytes) : "memory");
             }
         }
-    };
-    // values of positions base + 2t, 2t + 1, 2t + 8, 2t + 9: dimensions g * NT .. g * NT + NT - 1
-    uint32_t vr[4][kVw];
-    auto load_v = [&](int base) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int key = base + 2 * t + (i & 1) + 8 * (i >> 1);
-            const __half* src = V + (size_t)key * HD + g * NT;
-#pragma unroll
-            for (int w = 0; w < kVw; w++) vr[i][w] = 0u;
-            if (key < visible) {
-                if constexpr (kVw == 2) {
-                    const uint2 x = __ldca(reinterpret_cast<const uint2*>(src));
-                    vr[i][0] = x.x; vr[i][1] = x.y;
-                } else {
-#pragma unroll
-                    for (int w = 0; w < kVw; w += 4) {
-                        const uint4 x = __ldca(reinterpret_cast<const uint4*>(src) + w / 4);
-                        vr[i][w] = x.x; vr[i][w + 1] = x.y; vr[i][w + 2] = x.z; vr[i][w + 3] = x.w;
-                    }
-                }
-            }
-        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int step = used * kRound, first = rank < used ? rank * kRound + warp * kDaBlock : visible;
-    load_k(first);
-    load_v(first);
+#pragma unroll
+    for (int st = 0; st < kStages; st++) request(first + st * step, st);
     // queries, scaled, as (rounded, remainder) fp16 pairs: A registers of the two MMA steps of every 32 dimensions
     uint32_t qa[KB][2][4];
     {
@@ -138,8 +138,35 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
     float o[NT][4], mx = -INFINITY, sum = 0.f;  // head g: o[j][0] + o[j][2] is dimension 2t * NT + j, o[j][1] + o[j][3] (2t + 1) * NT + j
 #pragma unroll
     for (int j = 0; j < NT; j++) { o[j][0] = 0.f; o[j][1] = 0.f; o[j][2] = 0.f; o[j][3] = 0.f; }
+    int st = 0;
 #pragma unroll 1
     for (int base = first; base < visible; base += step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
+        __syncwarp();
+        const uint8_t* const tile = ring + st * 2 * kTileBytes;
+        uint4 kr[2][KB];  // keys base + g and base + g + 8: this lane's 16-byte piece of every 32 dimensions
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int kb = 0; kb < KB; kb++) kr[i][kb] = *reinterpret_cast<const uint4*>(tile + da_key_at<HD>(8 * i + g, kb * 4 + t));
+        uint32_t vr[4][kVw];  // values of positions base + 2t, 2t + 1, 2t + 8, 2t + 9: dimensions g * NT .. g * NT + NT - 1
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = 2 * t + (i & 1) + 8 * (i >> 1);
+            if constexpr (kVw == 2) {
+                const uint2 x = *reinterpret_cast<const uint2*>(tile + kTileBytes + da_value_at<HD>(r, g >> 1) + (g & 1) * 8);
+                vr[i][0] = x.x; vr[i][1] = x.y;
+            } else {
+#pragma unroll
+                for (int w = 0; w < kVw; w += 4) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(tile + kTileBytes + da_value_at<HD>(r, g * (NT / 8) + w / 4));
+                    vr[i][w] = x.x; vr[i][w + 1] = x.y; vr[i][w + 2] = x.z; vr[i][w + 3] = x.w;
+                }
+            }
+        }
+        __syncwarp();
+        request(base + kStages * step, st);
+        st = st + 1 == kStages ? 0 : st + 1;
         float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
         for (int kb = 0; kb < KB; kb++)
@@ -148,7 +175,6 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
                 pf_mma(sc[i], qa[kb][0][0], qa[kb][0][1], qa[kb][0][2], qa[kb][0][3], kr[i][kb].x, kr[i][kb].y);
                 pf_mma(sc[i], qa[kb][1][0], qa[kb][1][1], qa[kb][1][2], qa[kb][1][3], kr[i][kb].z, kr[i][kb].w);
             }
-        load_k(base + step);
         float s[2][2], top = -INFINITY;
 #pragma unroll
         for (int i = 0; i < 2; i++)
@@ -181,13 +207,13 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
             const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
             pf_mma(o[j], pa[0], pa[1], pa[2], pa[3], __byte_perm(vr[0][j >> 1], vr[1][j >> 1], sel), __byte_perm(vr[2][j >> 1], vr[3][j >> 1], sel));
         }
-        load_v(base + step);
     }
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    // ---- merge the warps: every warp parks (max, sum, context) of its heads
+    // ---- merge the warps: every warp parks (max, sum, context) of its heads (the copies still pending are empty)
+    __syncwarp();
     if (g < nh) {
-        float* dst = s_o + (warp * kDaHeads + g) * HD + 2 * t * NT;
+        float* dst = s_o + warp * kRingFloats + g * HD + 2 * t * NT;
 #pragma unroll
         for (int j = 0; j < NT; j++) { dst[j] = o[j][0] + o[j][2]; dst[NT + j] = o[j][1] + o[j][3]; }
         if (t == 0) { s_ml[(warp * kDaHeads + g) * 2] = mx; s_ml[(warp * kDaHeads + g) * 2 + 1] = sum; }
@@ -219,7 +245,7 @@ __global__ void __launch_bounds__(NW * 32, (HD == 128 ? 8 : 16) / NW) k_attentio
     for (int i = threadIdx.x; i < nh * kQuads; i += NW * 32) {
         const int h = i / kQuads, d = (i - h * kQuads) * 4;
         float gm, total;
-        const float4 c = merge(s_ml + h * 2, kDaHeads * 2, s_o + h * HD + d, kDaHeads * HD, NW, gm, total);
+        const float4 c = merge(s_ml + h * 2, kDaHeads * 2, s_o + h * HD + d, kRingFloats, NW, gm, total);
         if (used == 1) {
             store(h, d, c, total);
         } else if (rank < used) {

@@ -297,7 +297,8 @@ static void raise_smem_limits_on_current_device() {
     ESP_CARVE(k_attention); ESP_CARVE(k_prep_rows<0>); ESP_CARVE(k_prep_rows<1>); ESP_CARVE(k_prep_rows<2>); ESP_CARVE(k_prep_rows<4>); ESP_CARVE(k_prep_rows<8>); ESP_CARVE(k_embed_rows); ESP_CARVE(k_rope_append); ESP_CARVE(k_head_done); ESP_CARVE(k_bump);
 #define ESP_DA(HD)                                                                                                         \
     ESP_CARVE((k_attention_decode<HD, 2>)); ESP_CARVE((k_attention_decode<HD, 4>)); ESP_CARVE((k_attention_decode<HD, 8>)); \
-    cudaFuncSetAttribute(k_attention_decode<HD, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, da_smem_floats(HD, 8, 8) * 4);
+    cudaFuncSetAttribute(k_attention_decode<HD, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, da_smem_floats(HD, 8, 8) * 4); \
+    cudaFuncSetAttribute(k_attention_decode<HD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, da_smem_floats(HD, 4, 1) * 4);
     ESP_DA(32) ESP_DA(64) ESP_DA(128)
 #undef ESP_DA
 #undef ESP_CARVE
