@@ -777,10 +777,10 @@ __device__ __forceinline__ float2 mega_block_sum_max(float v0, float v1, float* 
 // first round are requested before the query is known, and the new positions take their place in the round like cached ones.  The
 // per-warp (max, sum, ctx) triples are merged once, by all threads: a few lanes per output channel, combined with
 // shuffles (two warps walking all triples took 0.3 us longer per layer).
-template <int HD, int NW>  // NW = warps that share one query
+template <int HD, int NW, int ST>  // NW = warps that share one query
 struct MegaKvRound {
     static constexpr int kPieces = HD / 32, kPer = HD / 32;  // 16-byte pieces of a quarter of a key; channels of a lane
-    static constexpr int kSt = HD == 128 ? 2 : 4;            // positions of a lane (of a warp: 8 kSt)
+    static constexpr int kSt = ST;  // positions of a lane (of a warp: 8 kSt)
     uint4 k[kSt][kPieces];
     uint2 v[8 * kSt];
     // K, V: the head's rows of the cache; positions past the cached ones read as zeros.
@@ -836,8 +836,8 @@ __device__ __forceinline__ float mega_warp_max(float v) {
 // sees the n_cached cached positions and the new positions 0 .. qi, whose keys and values are rows of s.kn / s.vn; its
 // context lands in position qi of the staged s.ctx.  The teams run side by side (each reads the cached rows itself).
 // The context is staged as the products of weights of type WT read it.
-template <int HD, int NP, int WT, class WaitQ>
-__device__ __forceinline__ void mega_attention(const MegaShared& s, const MegaShare& w, const ModelDims& m, const KvLayout& kv, int layer, int n_cached, WaitQ wait_q) {
+template <int HD, int NP, int WT, int ST, class WaitQ>
+__device__ __forceinline__ void mega_attention_rounds(const MegaShared& s, const MegaShare& w, const ModelDims& m, const KvLayout& kv, int layer, int n_cached, WaitQ wait_q) {
     constexpr int NW = kMegaConsumerWarps / NP;
     const int tid = threadIdx.x, lane = tid & 31;
     const int qi = (tid >> 5) / NW, warp = (tid >> 5) - qi * NW;  // this warp's query and its place in the team
@@ -847,14 +847,14 @@ __device__ __forceinline__ void mega_attention(const MegaShared& s, const MegaSh
     const __half* K = kv.k + head;
     const __half* V = kv.v + head;
     const int sub = lane & 3, tl = lane >> 2;
-    constexpr int kSt = MegaKvRound<HD, NW>::kSt, kRound = NW * 8 * kSt;  // positions per round of a team
+    constexpr int kSt = MegaKvRound<HD, NW, ST>::kSt, kRound = NW * 8 * kSt;  // positions per round of a team
     constexpr float scale = HD == 32 ? 0.17677669529663687f : HD == 64 ? 0.125f : 0.08838834764831845f;  // 1 / sqrt(HD)
     const float4* const qv = reinterpret_cast<const float4*>(s.qs + qi * HD + sub * (HD / 4));  // this lane's quarter of the query
     float m_w = -INFINITY, l_w = 0.f;  // l_w: this lane's share (every probability sits in four lanes)
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
     for (int base = 0; base < n_cached + NP; base += kRound) {
-        MegaKvRound<HD, NW> cur;
+        MegaKvRound<HD, NW, ST> cur;
         cur.load(K, V, base, n_cached, warp, lane);
         if (base == 0) wait_q();  // the loads above are in flight while the query is awaited
         const bool news = base + kRound > n_cached;  // the new positions may fall into this round
@@ -975,6 +975,16 @@ __device__ __forceinline__ void mega_attention(const MegaShared& s, const MegaSh
     consumer_sync();
 }
 
+// Positions per round: 8 of a lane's group times ST times the warps of a query.  fp16 models: short contexts take half rounds (6 layers
+// d768: 1.05 -> 0.87 us per layer and attention up to 128 positions); quantised ones, whose kernel is larger, are slower with a second
+// copy of the code.
+template <int HD, int NP, int WT, class WaitQ>
+__device__ __forceinline__ void mega_attention(const MegaShared& s, const MegaShare& w, const ModelDims& m, const KvLayout& kv, int layer, int n_cached, WaitQ wait_q) {
+    if constexpr (HD == 128) mega_attention_rounds<HD, NP, WT, 2>(s, w, m, kv, layer, n_cached, wait_q);
+    else if (WT == WT_F16 && n_cached + NP <= 16 * (kMegaConsumerWarps / NP)) mega_attention_rounds<HD, NP, WT, 2>(s, w, m, kv, layer, n_cached, wait_q);
+    else mega_attention_rounds<HD, NP, WT, 4>(s, w, m, kv, layer, n_cached, wait_q);
+}
+
 // ------------------------------------------------------------------------------------------------ consumers
 
 // The model a pass runs through.
@@ -1042,6 +1052,13 @@ struct MegaWorker {
         }
     }
 
+    // Brings the count of arrived chunks up to date while there is something else to wait for: the products then find their chunk
+    // without a read.
+    __device__ __forceinline__ void peek() {
+        const unsigned n = ld_acquire_cta_shared(s.landed);
+        landed = __shfl_sync(0xffffffffu, n, 0);
+    }
+
     // ---- products
 
     // One group of rows: this warp's partial sums to `mine`.
@@ -1078,19 +1095,26 @@ struct MegaWorker {
             acc.clear();
             acc.add(ch, n, HD / mega_unit(WT), 0, 1, 0, s.ctx, reinterpret_cast<const float*>(s.ctx + xa_bytes(WT, HD, NP)), lane, tile);
             const int q = lane & 3, first = w.blk * a.plan.rpb + r0, row = first + tile * 16 + (lane >> 2), last = min(d, first + n);
+            float v[2 * NT];
 #pragma unroll
             for (int j = 0; j < NT; j++) {
                 const float2 y = acc.take(j, lane);
+                v[2 * j] = y.x; v[2 * j + 1] = y.y;
+            }
+            if (w.head == 0 && q < NP) {
 #pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    const int orow = row + 16 * j + 8 * i;
-                    float v = i ? y.y : y.x;
-                    if (q < NP && orow < last) {
-                        if (w.head == 0) v += s.xres[q * d + orow] + (GPT2 ? __ldg(a.out_bias + (size_t)2 * l * d + orow) : 0.f);
-                        red_add_u64(a.mid_sums + q * d + orow, counted(v));
-                    }
+                for (int i = 0; i < 2 * NT; i++) {
+                    const int orow = min(row + 8 * i, d - 1);
+                    v[i] += s.xres[q * d + orow] + (GPT2 ? __ldg(a.out_bias + (size_t)2 * l * d + orow) : 0.f);
                 }
             }
+            unsigned long long* const dst = a.mid_sums + (q < NP ? q * d : 0) + row;
+            unsigned long long c64[2 * NT];
+#pragma unroll
+            for (int i = 0; i < 2 * NT; i++) c64[i] = counted(v[i]);
+#pragma unroll
+            for (int i = 0; i < 2 * NT; i++)
+                if (q < NP && row + 8 * i < last) red_add_u64(dst + 8 * i, c64[i]);
         }
     }
     __device__ __forceinline__ void wo_products(const MegaStage& st, int l) {
@@ -1158,7 +1182,9 @@ struct MegaWorker {
     __device__ __forceinline__ void stage_words(unsigned tag, const float* gain, float (&ss)[NP]) {
         constexpr bool kSums = KIND == MS_UP, kAct = KIND == MS_DOWN;
         constexpr int kCols = mega_unit(W2) / 8, kLoads = kCols / 2;
-        constexpr int kPolls = kAct ? (GPT2 || kQuant ? 6 : 4) : 2;
+        // (one round of polls at the widths in use: a second one costs a round trip to L2.  Two positions of the 6-layer model: three
+        // and eight items per lane; with two and four a two-token pass took 113 us instead of 104)
+        constexpr int kPolls = NP == 2 ? (kAct ? 8 : 3) : kAct ? (GPT2 || kQuant ? 6 : 4) : 2;
         constexpr int kCode = kSums ? 7 : kAct ? 8 : KIND == MS_QKV ? 5 : 9;
         const int K = kAct ? a.m.hidden : a.m.d_model, n = items<W2>(K / mega_unit(W2)), total = NP * n;
         const bool lines = kAct && !kQuant && a.plan.act_wpc > 0;
@@ -1348,6 +1374,7 @@ struct MegaWorker {
             }
             __syncwarp();
             release_pending();  // the q/k/v chunk
+            peek();
             consumer_sync();
             stamp();
         });
@@ -1416,6 +1443,7 @@ struct MegaWorker {
         // head.  Issued here, the fence overlaps the wait for the last layer's output.
         if (KIND == MS_HEAD && warp < NP && lane == 0) __threadfence();
         const float* const gain = mo.norms + (size_t)(2 * l + (KIND == MS_UP ? 1 : 0)) * d;
+        peek();
         if ((KIND == MS_QKV || KIND == MS_HEAD) && first) stage_first<W2>(KIND == MS_HEAD, tok, pos, mo.tok_emb, gain, ss);
         else stage_words<KIND, W2>(KIND == MS_QKV ? seq - 1 : seq, gain, ss);
         release_pending();  // the last chunks of the stage before
