@@ -57,7 +57,7 @@ constexpr int kMegaTraceHead = 4;                  // stamps of the head
 constexpr int kMegaSlots = 4, kMegaSlotMax = 64 * 1024;  // ring slots and the most bytes of one (Q8_0, 22 layers of d2048: 4 slots of 44 KB 371 us per token, 5 of 35 KB 395, 7 of 25 KB 447)
 constexpr int kMegaRingMin = 96 * 1024;  // less than that is consumed faster than a refill takes to arrive
 constexpr int kMegaMaxTiles = 5;                   // 16-row tiles whose sums a warp keeps in registers
-// Which exchanges give every CTA cache lines of its own (see mega_read_lines) is the plan's choice (act_wpc > 0).
+// Which exchanges give every CTA cache lines of its own is the plan's choice (act_wpc > 0).
 // Measured on the 6-layer d768 model against compact arrays: arg-max candidates -4.6 us per token, activation vector
 // -1.4 us, layer output x +0.3 us (five words per CTA: three times as many lines to poll for little contention saved).
 // On the 22-layer d2048 model, whose activation vector needs two polling rounds either way, lines per CTA cost 1.8 us

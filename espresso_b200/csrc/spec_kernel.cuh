@@ -6,7 +6,7 @@
 // The kernel is the persistent decode kernel (mega_kernel.cuh) widened to two token positions per pass:
 //   * the products run on mma.sync with the weights as the A operand; the staged activations of the second position
 //     occupy two more of the eight B columns the instruction computes anyway, so the weights are read from the ring
-//     once for both positions and the per-position sums are bit-identical to the single-position kernel's;
+//     once for both positions and every position is summed in the single-position kernel's order;
 //   * every exchange (tagged words, counted sums, arg-max candidates) carries one value per position;
 //   * attention runs once per query; the second query also sees the first new position, whose key and value sit in
 //     shared memory beside its own.
