@@ -1398,7 +1398,7 @@ struct MegaWorker {
         const int rows_of = KIND == MS_QKV ? 2 * w.s1_n : KIND == MS_UP ? p.ffn_rows * w.h_n : KIND == MS_DOWN ? w.d_n : w.v_n;
         // What the epilogue needs besides its sums is worked out before the words are awaited (a later group's with its products).
         float e0 = 0.f, e1 = 0.f;
-        float2 cs = make_float2(1.f, 0.f);
+        float2 cs;
         __half *kv0 = nullptr, *kv1 = nullptr;
         unsigned long long* dst = nullptr;
         auto prepare = [&](int r) {
@@ -1408,6 +1408,7 @@ struct MegaWorker {
             const int ln_rows = a.m.q_dim + 2 * a.m.kv_dim + a.m.hidden;
             if constexpr (KIND == MS_QKV) {
                 const int4 pair = s.s1[i0 >> 1];
+                cs = make_float2(1.f, 0.f);  // (a later group's value pair must not keep the angle of an earlier one's key)
                 if (!GPT2 && pair.x < 2) cs = a.rope[(size_t)(gq ? min(pos + 1, a.m.max_seq - 1) : pos) * half + pair.w];
                 dst = a.qkv_words + (w.kvh * NP + gq) * 2 * p.group_items + 2 * w.s1_begin + i0;
                 kv0 = nullptr;

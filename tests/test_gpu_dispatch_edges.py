@@ -163,6 +163,47 @@ def test_row_groups_and_units_of_the_persistent_kernel(rt, oracle_lib, kind, hea
     eng.close()
 
 
+@pytest.mark.parametrize("kind,n_head,n_kv,head_dim,hidden", [
+    ("f16", 4, 4, 128, 32),      # 96 rows in two groups; a CTA's second group takes over from the keys
+    ("f16", 10, 5, 128, 64),     # grouped heads, 86 rows: groups of 48 and 38
+    ("q8_0", 26, 26, 128, 256),
+])
+def test_query_key_value_rows_in_several_groups(rt, oracle_lib, kind, n_head, n_kv, head_dim, hidden):
+    """A thread of the persistent kernel finishes a rotated pair in one row group and a value pair in the next: decode and the
+    two-position pass, the cache that they leave included."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = _model("edge-qkv-groups", 2, n_head, n_kv, n_head * head_dim, head_dim, hidden, 600, 64)
+    cfg = dataclasses.replace(cfg, ropeTheta=10.0)  # (the upper pairs of a key turn visibly within a few positions)
+    n_cta, qpk = hidden // 2, n_head // n_kv  # (fewer CTAs than SMs: one pair of FFN units each)
+    items = (qpk + 2) * head_dim // 2
+    rows = 2 * -(-items // (min(n_cta // n_head, items // qpk) * qpk))
+    assert 80 < rows <= 160  # five 16-row tiles per group
+    if kind == "f16":
+        eng, model = dense_pair(rt, oracle_lib, cfg)
+    else:
+        model, uploads = quantised_pair(oracle_lib, cfg, kind)
+        eng = rt.DecodeEngine.empty(cfg)
+        upload_all(eng, uploads)
+    prompt = synthetic_prompt(cfg.vocab, 9)
+    ora = oracle_lib.Runtime(model)
+    res = eng.generate(prompt, 14)
+    assert eng.timings()["kernel_launches"] == 1
+    compare_greedy_stream(ora, prompt, res.tokens)
+    assert_logits_close(eng.logits(), ora.logits(), "decode")
+    if kind == "f16":
+        follow = [int(t) for t in synthetic_prompt(cfg.vocab, 8, stream=1)]
+        eng.prefill(prompt)
+        assert ora.prefill(prompt) == 0
+        for i in range(0, len(follow), 2):
+            eng.verify2(follow[i], follow[i + 1])
+            assert eng.timings()["kernel_launches"] == 1
+            eng.commit(2)
+            assert ora.advance(follow[i]) == 0 and ora.advance(follow[i + 1]) == 0
+            assert_logits_close(eng.logits(), ora.logits(), f"pair {i // 2}")
+    eng.close()
+
+
 @pytest.mark.parametrize("n_seq", [3, 40, 330])
 def test_full_sequence_beside_unfinished_ones(rt, oracle_lib, n_seq):
     """A sequence that has filled its context stays in the batch as an inactive row one position past the rotation table;
