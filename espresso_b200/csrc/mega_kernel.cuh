@@ -45,6 +45,7 @@
 #include <algorithm>
 
 #include "decode_kernels.cuh"
+#include "mega_units.h"
 
 namespace esp {
 
@@ -661,8 +662,8 @@ struct MegaSums {
         }
     }
     // Units first, first + step, ... of a chunk's nu (unit i is unit u0 + i of the vector): tiles tile0 .. tile0 + NT - 1 of its
-    // `rows` rows.  Without branches: a batch's units past the last one multiply the last one's weights by zeros, and a tile's rows
-    // past the last one read whatever lies behind it in shared memory; their sums are never stored.
+    // `rows` rows.  Without branches: a batch's units past the last one multiply the weights of its first one by zeros, and a
+    // tile's rows past the last one read whatever lies behind it in shared memory; their sums are never stored.
     __device__ __forceinline__ void add(const uint8_t* chunk, int rows, int nu, int first, int step, int u0, const uint8_t* xa, const float* xq, int lane, int tile0) {
         const int g = lane >> 2, t = lane & 3;
         const int db = mega_data_bytes(WT, rows), sb = mega_scale_bytes(WT, rows);
@@ -678,9 +679,9 @@ struct MegaSums {
             float q[kBatch];
 #pragma unroll
             for (int x = 0; x < kBatch; x++) {
-                const int want = i0 + x * step, i = x ? min(want, nu - 1) : i0;
+                const int i = mega_batch_unit(i0, x, step, nu);
                 b[x] = make_uint2(0, 0);
-                if (feeds && (x == 0 || want < nu)) b[x] = *reinterpret_cast<const uint2*>(xp + i * kXUnit);
+                if (feeds && (x == 0 || i0 + x * step < nu)) b[x] = *reinterpret_cast<const uint2*>(xp + i * kXUnit);
                 if (!kF16) q[x] = xq[u0 + i];
 #pragma unroll
                 for (int j = 0; j < NT; j++) {

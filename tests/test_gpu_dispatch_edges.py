@@ -204,6 +204,32 @@ def test_query_key_value_rows_in_several_groups(rt, oracle_lib, kind, n_head, n_
     eng.close()
 
 
+def test_quantised_engines_of_different_widths_take_turns(rt, oracle_lib):
+    """A launch finds in shared memory what the other engine's kernel left there: every engine repeats its tokens and logits."""
+    from espresso_b200.synthetic import synthetic_prompt
+
+    engines = []
+    for kind, n_head, n_kv, hidden in (("q8_0", 8, 4, 1536), ("q8_0", 32, 4, 5632), ("q4_0", 32, 4, 5632)):
+        cfg = _model("edge-turns", 2, n_head, n_kv, 64 * n_head, 64, hidden, 2000, 64)
+        model, uploads = quantised_pair(oracle_lib, cfg, kind)
+        eng = rt.DecodeEngine.empty(cfg)
+        upload_all(eng, uploads)
+        prompt = synthetic_prompt(cfg.vocab, 11)
+        tokens = eng.generate(prompt, 10).tokens
+        assert eng.timings()["kernel_launches"] == 1
+        logits = eng.logits()
+        ora = oracle_lib.Runtime(model)
+        compare_greedy_stream(ora, prompt, tokens)
+        assert_logits_close(logits, ora.logits(), kind)
+        engines.append((eng, prompt, tokens, logits))
+    for turn in range(12):
+        eng, prompt, tokens, logits = engines[(turn * 5 + turn // 3) % 3]
+        np.testing.assert_array_equal(eng.generate(prompt, 10).tokens, tokens)
+        np.testing.assert_array_equal(eng.logits(), logits)
+    for eng, *_ in engines:
+        eng.close()
+
+
 @pytest.mark.parametrize("n_seq", [3, 40, 330])
 def test_full_sequence_beside_unfinished_ones(rt, oracle_lib, n_seq):
     """A sequence that has filled its context stays in the batch as an inactive row one position past the rotation table;
