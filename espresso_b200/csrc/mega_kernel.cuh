@@ -1003,6 +1003,10 @@ __device__ __forceinline__ unsigned long long mega_warp_best(unsigned long long 
     return ((unsigned long long)hi << 32) | lo;
 }
 
+// The candidate of a CTA in which a wait ran out: it went on with operands that never arrived, and what it published is
+// complete by its tags.  No logit orders as high (a NaN is never a best row), so every CTA finds the mark as the largest candidate.
+constexpr unsigned long long kMegaGaveUp = 0xffffffffffffff00ull;
+
 // The consumer warps of a CTA.  A pass is one forward step for NP consecutive token positions, or only its LM head.
 // Every stage's operand vector is dealt out to the warps by K units (unit u to warp u % 8): a warp polls the words of its own
 // columns, stages them for the tensor cores and multiplies them with all rows of the CTA, and nothing is shared between the
@@ -1510,8 +1514,9 @@ struct MegaWorker {
 
     // One pass: tokens tok[q] at positions pos + q through `layers` layers (0: the head alone, on the last hidden state), then the LM
     // head with its first-max arg-max; every CTA learns out[q].  seq: tag of everything the layer publishes, counted up by
-    // every layer; tag8: tag of the arg-max candidates.
-    __device__ __forceinline__ void pass(const MegaModel& mo, const ModelDims& md, int layers, const uint32_t (&tok)[NP], int pos, unsigned& seq, unsigned long long tag8,
+    // every layer; tag8: tag of the arg-max candidates.  False (in every thread of the CTA): a wait ran out in this CTA, or in another
+    // one before it published its candidate, and out[q] means nothing.
+    __device__ __forceinline__ bool pass(const MegaModel& mo, const ModelDims& md, int layers, const uint32_t (&tok)[NP], int pos, unsigned& seq, unsigned long long tag8,
                                          uint32_t (&out)[NP]) {
         const MegaPlan& p = a.plan;
         // Why the exchange arrays need no second buffer: x_words is re-written by the W2 stage of this layer, which starts only
@@ -1554,7 +1559,8 @@ struct MegaWorker {
         }
         consumer_sync();
         if (warp < NP) {
-            const unsigned long long k = mega_warp_best(lane < kTeam ? s.key[warp * kTeam + lane] : 0ull);
+            unsigned long long k = mega_warp_best(lane < kTeam ? s.key[warp * kTeam + lane] : 0ull);
+            if (mega_aborting(s)) k = kMegaGaveUp;
             if (lane == 0) st_word(a.cand_words + (size_t)(warp * p.n_cta + (int)blockIdx.x) * kMegaCandStride, k | tag8);
         }
         stamp();
@@ -1589,13 +1595,16 @@ struct MegaWorker {
         }
         if (tid == 0) s.red[63] = mega_aborting(s) ? 1.f : 0.f;  // one decision for the whole CTA
         consumer_sync();
+        bool valid = s.red[63] == 0.f;
 #pragma unroll
         for (int q = 0; q < NP; q++) {
             const unsigned long long best = mega_warp_best(lane < kMegaConsumerWarps ? s.key[q * kMegaConsumerWarps + lane] : 0ull);
+            valid = valid && (best | 0xffull) != (kMegaGaveUp | 0xffull);
             out[q] = min(0xffffffu - (uint32_t)((best >> 8) & 0xffffffull), (uint32_t)(a.m.vocab - 1));  // in range even if every logit was NaN
         }
         release_pending();  // the last head chunks
         stamp();
+        return valid;
     }
 };
 
@@ -1731,7 +1740,10 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const __grid_co
     const int d = m.d_model;
     for (int step = a.first; step < a.first + a.n_steps; step++) {
         work.tracing = a.trace && (int)blockIdx.x == a.trace_cta && tid == 0 && step == a.first + a.n_steps - 1;
-        work.pass(model, m, step > 0 ? L : 0, tok, pos, seq, (unsigned long long)((a.cand0 + (unsigned)step) % 255u + 1u), tok);
+        if (!work.pass(model, m, step > 0 ? L : 0, tok, pos, seq, (unsigned long long)((a.cand0 + (unsigned)step) % 255u + 1u), tok)) {
+            if (tid == 0) *reinterpret_cast<volatile int*>(s.stop) = 1;
+            break;
+        }
         if (step > 0) pos++;  // the token that was just processed is now visible
         const bool gpt2_stop = GPT2 && tok[0] == GPT2_EOS;  // GPT-2 rule: the stop token ends the loop without being emitted
         if (!gpt2_stop) emitted++;
@@ -1745,7 +1757,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const __grid_co
         }
         // Llama rule: the end-of-sequence token is emitted, then the loop stops (every CTA sees the same token)
         const bool eos = GPT2 ? gpt2_stop : m.eos_token >= 0 && tok[0] == (uint32_t)m.eos_token;
-        if (eos || s.red[63] != 0.f) {
+        if (eos) {
             if (tid == 0) *reinterpret_cast<volatile int*>(s.stop) = 1;
             break;
         }

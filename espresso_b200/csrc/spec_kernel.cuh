@@ -117,11 +117,10 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_spec_mega(const __grid_cons
             md.n_layer = M.m.n_layer; md.n_seq = M.m.n_seq; md.max_seq = M.m.max_seq;
             const uint32_t in[NP] = {mi ? current : prev, mi ? proposed : current};
             uint32_t o[NP];
-            work.pass(MegaModel{M.norms, M.tok_emb, M.kv}, md, md.n_layer, in, mi ? P : P - 1, seq, (unsigned long long)(n_heads % 255 + 1), o);
+            gave_up = !work.pass(MegaModel{M.norms, M.tok_emb, M.kv}, md, md.n_layer, in, mi ? P : P - 1, seq, (unsigned long long)(n_heads % 255 + 1), o);
             ++n_heads;
             if (mi == 0) { proposed = o[1]; draft_visible = P + 1; }
             else { next = o[0]; future = o[1]; }
-            gave_up = s.red[63] != 0.f;
         }
         if (gave_up) break;
         if (sa.verify_only) {

@@ -181,6 +181,39 @@ def test_device_wait_that_runs_out_reports_a_timeout(rt, oracle_lib, tmp_models)
     eng.close()
 
 
+@pytest.mark.parametrize("at", [0, 5])
+def test_no_token_is_reported_from_a_pass_that_gave_up(rt, tmp_models, at):
+    """Token by token, a device-side wait runs out (from the first pass on, or in a call made by the callback at token `at`):
+    what has been reported until then is a prefix of the good stream, and the call returns the timeout."""
+    from espresso_b200.model_config import tiny_llama
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = tiny_llama(vocab=512, max_seq=64, n_layer=2)
+    prompt = synthetic_prompt(cfg.vocab, 9)
+    eng = rt.DecodeEngine.build(tmp_models(cfg))
+    good = [int(t) for t in eng.generate(prompt, 20).tokens]
+    for _ in range(4):
+        seen = []
+
+        def on_step(token, index, _ms):
+            seen.append(token)
+            if at and index == at:
+                eng.set_wait_limit(2)
+
+        if not at:
+            eng.set_wait_limit(2)
+        with pytest.raises(rt.RealModelInferenceError) as err:
+            eng.generate(prompt, 20, on_step=on_step)
+        assert err.value.status == 5 and "gave up waiting" in err.value.message  # ESP_CUDA_ERR_TIMEOUT
+        assert seen == good[:len(seen)] and len(seen) < 20
+        eng.set_wait_limit(0)
+        eng.reset()
+        seen = []
+        assert list(eng.generate(prompt, 20, on_step=lambda token, _index, _ms: seen.append(token)).tokens) == good
+        assert seen == good
+    eng.close()
+
+
 def test_per_token_latencies_and_step_callback(rt, oracle_lib, tmp_models):
     """GenerationResult.tokenLatenciesMs and the inline onStep callback (Engine.swift:17-55, 6393-6405): the device-driven
     loops report one latency per token, and the token-by-token form calls back once per token with the same stream."""
