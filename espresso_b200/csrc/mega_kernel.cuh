@@ -594,19 +594,26 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 // registers of lane (g = c, t).
 constexpr float kRoundMagic = 12582912.0f;  // 1.5 * 2^23: added to a float of magnitude up to 2^22 it leaves the nearest integer in the low mantissa bits
 
+// Maximum that keeps a NaN.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
 // Stages N quads of elements k .. k + 3 (k a multiple of 4) per lane; groups of eight lanes with consecutive quads hold one block of
 // 32 columns each (`mask`: the lanes that take part; `live`: which quads of this lane are stored).  The N quads go side by side: a
 // block's maximum takes three shuffles.  (A digit at a time with a quotient per block took 22 operations per element instead
 // of six, and __reduce_max_sync over groups of lanes is executed group by group: 500 cycles per quad.)
+// An Inf or a NaN has no digits: it makes the block's scale NaN, and so every row's sum, as a product with the value itself would.
 template <int WT, int N>
 __device__ __forceinline__ void qx_store_quads(uint8_t* xq, float* qs, const int (&k)[N], const float4 (&v)[N], const bool (&live)[N], unsigned mask) {
     float top[N];
 #pragma unroll
-    for (int j = 0; j < N; j++) top[j] = fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w)));
+    for (int j = 0; j < N; j++) top[j] = max_nan(max_nan(fabsf(v[j].x), fabsf(v[j].y)), max_nan(fabsf(v[j].z), fabsf(v[j].w)));
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-        for (int j = 0; j < N; j++) top[j] = fmaxf(top[j], __shfl_xor_sync(mask, top[j], o));
+        for (int j = 0; j < N; j++) top[j] = max_nan(top[j], __shfl_xor_sync(mask, top[j], o));
 #pragma unroll
     for (int j = 0; j < N; j++) {
         const unsigned e = min(max(__float_as_uint(top[j]) >> 23, 22u), 254u);  // the largest value lies below 2^(e - 126)
@@ -627,7 +634,7 @@ __device__ __forceinline__ void qx_store_quads(uint8_t* xq, float* qs, const int
             dst[8] = __byte_perm(ab, cd, 0x7632);
             dst[16] = __byte_perm(ab, cd, 0x5410);
             if (WT == WT_Q4_0) dst[24] = __byte_perm(__byte_perm(ra, rb, 0x0040), __byte_perm(rc, rd, 0x0040), 0x5410);
-            if (e0 == 0) qs[k[j] >> 5] = __uint_as_float((e - 21u) << 23);  // 2^(e - 148)
+            if (e0 == 0) qs[k[j] >> 5] = top[j] < INFINITY ? __uint_as_float((e - 21u) << 23) : __uint_as_float(0x7fffffffu);  // 2^(e - 148)
         }
     }
 }

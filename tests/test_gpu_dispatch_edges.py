@@ -230,6 +230,27 @@ def test_quantised_engines_of_different_widths_take_turns(rt, oracle_lib):
         eng.close()
 
 
+@pytest.mark.parametrize("kind", ["f16", "q8_0", "q4_0"])
+@pytest.mark.parametrize("gain", [1e20, float("nan")])
+def test_values_that_overflow_stay_visible(rt, oracle_lib, kind, gain):
+    """Gains that overflow the FFN activation: the persistent kernel's last hidden state is not finite, whatever the weights' type."""
+    from espresso_b200.synthetic import synthetic_prompt, synthetic_tensors
+
+    cfg = _model("edge-overflow", 1, 4, 2, 256, 64, 512, 320, 32)
+    if kind != "f16":
+        _, uploads = quantised_pair(oracle_lib, cfg, kind)
+    else:
+        uploads = [(n, "f16", t.astype(np.float16)) for n, t in synthetic_tensors(cfg, 1234)]
+    gains = np.full(cfg.dModel, gain, np.float32)
+    eng = rt.DecodeEngine.empty(cfg)
+    upload_all(eng, [(n, "f32", gains) if n.endswith("rms_ffn") else (n, k, t) for n, k, t in uploads])
+    eng.prefill(synthetic_prompt(cfg.vocab, 5))
+    eng.decode(3)
+    assert eng.timings()["kernel_launches"] == 1
+    assert np.isnan(eng.logits()).all()
+    eng.close()
+
+
 @pytest.mark.parametrize("n_seq", [3, 40, 330])
 def test_full_sequence_beside_unfinished_ones(rt, oracle_lib, n_seq):
     """A sequence that has filled its context stays in the batch as an inactive row one position past the rotation table;
