@@ -31,10 +31,14 @@ static int32_t fail(int32_t code, const std::string& msg) {
     return code;
 }
 
+// Calls that are answered from what the host knows, also while a token-by-token loop runs on the device.
+#define ESP_HANDLE(engine) \
+    if (!(engine)) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "null engine handle")
+// All other calls find the state after the reported token.
 #define ESP_GUARD(engine) \
-    if (!(engine)) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "null engine handle"); \
+    ESP_HANDLE(engine); \
     if ((engine)->impl.streaming()) {  /* called from a generate_steps callback */ \
-        const int32_t settled = const_cast<esp_cuda_engine*>(engine)->impl.stream_settle(); \
+        const int32_t settled = (engine)->impl.stream_settle(); \
         if (settled) return settled; \
     } \
     do {} while (0)
@@ -131,7 +135,7 @@ int32_t esp_cuda_destroy(esp_cuda_engine* engine) {
     return ESP_CUDA_OK;
 }
 int32_t esp_cuda_get_config(const esp_cuda_engine* engine, esp_cuda_config* out) {
-    ESP_GUARD(engine);
+    ESP_HANDLE(engine);
     if (!out) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "null output");
     *out = engine->impl.config();
     return ESP_CUDA_OK;
@@ -143,7 +147,7 @@ int32_t esp_cuda_advance(esp_cuda_engine* engine, uint32_t token) { ESP_GUARD(en
 int32_t esp_cuda_select_greedy(esp_cuda_engine* engine, uint32_t* token) { ESP_GUARD(engine); return engine->impl.select_greedy(token); }
 int32_t esp_cuda_decode_step(esp_cuda_engine* engine, uint32_t token, uint32_t* next) { ESP_GUARD(engine); return engine->impl.decode_step(token, next); }
 int32_t esp_cuda_visible_token_count(const esp_cuda_engine* engine, int32_t seq, int32_t* count) {
-    ESP_GUARD(engine);
+    ESP_HANDLE(engine);
     if (!count || seq < 0 || seq >= engine->impl.config().max_batch) return fail(ESP_CUDA_ERR_INVALID_ARGUMENT, "bad sequence index");
     *count = engine->impl.visible(seq);
     return ESP_CUDA_OK;
@@ -269,7 +273,7 @@ int32_t esp_cuda_generate_steps(esp_cuda_engine* engine, const uint32_t* prompt,
 }
 
 int32_t esp_cuda_token_latencies(esp_cuda_engine* engine, float* out_ms, int32_t capacity, int32_t* n) {
-    ESP_GUARD(engine);
+    ESP_HANDLE(engine);
     return engine->impl.token_latencies(out_ms, capacity, n);
 }
 
@@ -400,13 +404,13 @@ int32_t esp_cuda_generate_two_token(esp_cuda_engine* engine, esp_cuda_engine* dr
     return ESP_CUDA_OK;
 }
 
-int32_t esp_cuda_get_timings(esp_cuda_engine* engine, esp_cuda_timings* out) { ESP_GUARD(engine); return engine->impl.get_timings(out); }
+int32_t esp_cuda_get_timings(esp_cuda_engine* engine, esp_cuda_timings* out) { ESP_HANDLE(engine); return engine->impl.get_timings(out); }
 int32_t esp_cuda_stage_trace(esp_cuda_engine* engine, int32_t cta, int64_t* out, int32_t capacity, int32_t* n) {
     ESP_GUARD(engine);
     return engine->impl.stage_trace(cta, reinterpret_cast<long long*>(out), capacity, n);
 }
 int32_t esp_cuda_token_times(esp_cuda_engine* engine, uint64_t* out_ns, int32_t capacity, int32_t* n) {
-    ESP_GUARD(engine);
+    ESP_HANDLE(engine);
     return engine->impl.token_times(reinterpret_cast<unsigned long long*>(out_ns), capacity, n);
 }
 int32_t esp_cuda_set_debug_layer(esp_cuda_engine* engine, int32_t layer) { ESP_GUARD(engine); return engine->impl.set_debug_layer(layer); }

@@ -2385,13 +2385,13 @@ int32_t Engine::enqueue_mega(int n_steps, const uint32_t* feed, bool times, unsi
     if (times) ESP_CUDA_TRY(cudaEventRecord(ev_end_, stream_));
     ESP_CUDA_TRY(cudaMemcpyAsync(h_mega_ctl_, d_mega_ctl_, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream_));
     mega_first_ = a.first;
+    launches_last_step_ = 1;
+    timings_.kernel_launches = 1;
     return ESP_CUDA_OK;
 }
 
 int32_t Engine::finish_mega() {
     ESP_CUDA_TRY(cudaStreamSynchronize(stream_));
-    launches_last_step_ = 1;
-    timings_.kernel_launches = 1;
     const int err = reinterpret_cast<int*>(h_mega_ctl_ + 2)[1];
     if (err != 0) {
         std::ostringstream os;
@@ -2430,8 +2430,9 @@ int32_t Engine::run_mega(int n_steps, int* emitted, float* device_ms, double* fi
 // Token-by-token reporting of one greedy loop of sequence 0.  The whole loop is one launch; the kernel writes every token to pinned
 // host memory as it becomes known and goes on, and the host reports it (stream_next) while the next one is computed: a
 // launch and a host round trip per token took 107 us where the kernel needs 64 (6 layers d768).
-// A caller that uses the engine between two tokens (from its callback) must find it as a step-by-step loop would have left it: every
-// entry point first settles the stream, i.e. lets the kernel finish and goes back to the state after the reported token.
+// A caller that uses the engine between two tokens (from its callback) must find it as a step-by-step loop would have left it: an
+// entry point that needs the device's state first settles the stream, i.e. lets the kernel finish and goes back to the state after
+// the reported token.  Questions that the host can answer (visible tokens, configuration, timings) do not.
 // The reporting loop then goes on step by step.
 bool Engine::stream_usable() const { return mega_usable() && !(cfg_.flags & ESP_CUDA_FLAG_KEEP_LOGITS); }
 

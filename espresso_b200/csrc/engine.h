@@ -80,7 +80,7 @@ public:
                            uint32_t* out_tokens, int32_t* n_out, esp_cuda_generation_result* result);
     int32_t decode_loop(int32_t n_seq, int32_t count, uint32_t* out_tokens, int32_t out_stride, int32_t* n_out,
                         float* device_ms, double* first_token_ms);
-    // Reporting a greedy loop token by token (generate_steps); every other entry point settles it first.
+    // Reporting a greedy loop token by token (generate_steps); an entry point that needs the device's state settles it first.
     bool stream_usable() const;
     bool streaming() const { return streaming_; }
     int32_t stream_begin(int n_steps);
@@ -104,7 +104,7 @@ public:
     int32_t run_spec(Engine& draft, uint32_t prev, uint32_t current, int gen0, int eff, int max_seq, uint32_t* out_tokens, int* stats);
 
     const esp_cuda_config& config() const { return cfg_; }
-    int visible(int seq) const { return h_visible_[seq]; }
+    int visible(int seq) const { return streaming_ && seq == 0 ? stream_visible_ + std::max(0, stream_reported_ - 1) : h_visible_[seq]; }
     bool finalized() const { return finalized_; }
 
 private:

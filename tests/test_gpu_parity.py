@@ -606,6 +606,34 @@ def test_streamed_tokens_and_a_callback_that_uses_the_engine(rt, tmp_models, use
     other.close()
 
 
+def test_questions_from_a_callback_do_not_wait_for_the_device(rt, tmp_models):
+    """The visible count, the configuration and the timings are known to the host: a callback that asks for them at every token gets the
+    step-by-step loop's answers and does not wait for the tokens that the device is still working on."""
+    import time
+
+    from espresso_b200.model_config import llama_6l
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = llama_6l()
+    eng = rt.DecodeEngine.build(tmp_models(cfg))
+    prompt = synthetic_prompt(cfg.vocab, 9)
+    plain = eng.generate(prompt, 200).tokens.tolist()  # about 12 ms on the device
+    seen, waited, answers = [], [], []
+
+    def on_step(token, index, _ms):
+        t = time.perf_counter()
+        answers.append((eng.visible_token_count(), eng.timings()["kernel_launches"], eng.token_latencies_ms().size, eng.token_times_ns().size))
+        waited.append(time.perf_counter() - t)
+        seen.append(token)
+
+    begin = time.perf_counter()
+    assert eng.generate(prompt, 200, on_step=on_step).tokens.tolist() == plain and seen == plain
+    whole = time.perf_counter() - begin
+    assert answers == [(len(prompt) + i, 1, 200, 0) for i in range(200)]
+    assert max(waited) < whole / 4  # the first answer used to take as long as the remaining tokens together
+    eng.close()
+
+
 @pytest.mark.parametrize("kind", ["f16", "q8_0"])
 def test_persistent_kernel_streams_wide_stages_in_chunks(rt, oracle_lib, tmp_models, kind):
     """d_model 2048 / hidden 5632: every stage slice of the persistent kernel exceeds a ring slot and arrives in chunks
