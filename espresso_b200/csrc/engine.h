@@ -142,7 +142,7 @@ private:
     int32_t build_mega();   // packs the weights for the persistent decode kernel when the model qualifies
     int32_t build_mega_gpt2();
     int32_t launch_mega(int n_steps, const uint32_t* feed, bool times);
-    int32_t enqueue_mega(int n_steps, const uint32_t* feed, bool times, unsigned long long* host_words);
+    int32_t enqueue_mega(int n_steps, const uint32_t* feed, bool times, unsigned long long* host_words, const unsigned* stop_request);
     int32_t finish_mega();
     bool mega_usable() const;
     int32_t run_mega(int n_steps, int* emitted, float* device_ms, double* first_token_ms);
@@ -246,7 +246,7 @@ private:
     bool streaming_ = false;
     int32_t stream_error_ = 0;
     int stream_visible_ = 0, stream_reported_ = 0;  // visible tokens at its start, tokens reported so far
-    unsigned long long* h_stream_ = nullptr;  // pinned [max_seq]
+    unsigned long long* h_stream_ = nullptr;  // pinned [max_seq] tokens, [1] request to end
     float* d_stream_hidden_ = nullptr;        // [d_model] hidden state at its start
     long long* d_mega_trace_ = nullptr;
     unsigned long long* d_token_times_ = nullptr;  // [max_seq] emission time of every token of the last persistent loop

@@ -137,11 +137,12 @@ struct MegaArgs {
     unsigned long long* act_words;  // [hidden] or [n_cta][act_wpc]; tagged: FFN activation
     unsigned long long* qkv_words;  // [n_kv_head][2 * group_items] tagged: post-RoPE q / k / v of one token
     unsigned long long* mid_sums;   // [d_model] counted: residual + attention projection
-    unsigned long long* cand_words; // [n_cta][kMegaCandStride] {logit bits, index, 8-bit tag} of each CTA's best row in word 0
+    unsigned long long* cand_words; // [n_cta][kMegaCandStride] {logit bits, index, 8-bit tag} of each CTA's best row in word 0, {request, 8-bit tag} in word 1
     float* hidden_io;         // [d_model] last hidden state of the sequence (in and out)
     int* error;               // [1] 0 = ok
     unsigned long long* stamps; // [4] globaltimer at kernel start and when the first token is known; {last token : 32}{number of tokens emitted : 32}; visible tokens
     unsigned long long* host_words;  // optional pinned host memory [n_steps]: {number of tokens emitted : 32}{token : 32} of every token as it becomes known, or null
+    const unsigned* stop_request;    // optional pinned host word: not zero = the loop ends after the token at hand, or null
     unsigned long long* token_times; // optional [n_steps] globaltimer (ns) at which each token became known, or null
     long long* trace;         // optional [kMegaTraceLayer*L + kMegaTraceHead] SM clock stamps of the last step taken by CTA `trace_cta`, or null
     int trace_cta;
@@ -293,6 +294,7 @@ struct MegaShared {
     int* abort;    // [1] a wait gave up: no more waiting in this CTA
     int* stop;     // [1] the loop ended early (EOS): the producer stops issuing
     unsigned* landed;  // [1] number of chunks whose bytes have arrived (written by the watcher warp)
+    unsigned* asked;   // [1] CTA 0: the host wants the loop to end (written by the producer warp)
 };
 
 // The areas sit at offsets the host computed once (mega_layout): an address is the base plus a kernel-argument
@@ -318,6 +320,7 @@ __device__ __forceinline__ MegaShared mega_carve(uint8_t* base, const MegaPlan& 
     s.abort = reinterpret_cast<int*>(base + p.off_flags);
     s.stop = s.abort + 1;
     s.landed = reinterpret_cast<unsigned*>(s.abort + 2);
+    s.asked = s.landed + 1;
     s.share = reinterpret_cast<MegaShare*>(base + p.off_share);
     s.act = reinterpret_cast<uint16_t*>(base + p.off_act);
     s.s1 = reinterpret_cast<int4*>(base + p.off_s1);
@@ -441,6 +444,7 @@ __device__ __forceinline__ void mega_init(const MegaArgs& a, const MegaShared& s
         *s.abort = 0;
         *s.stop = 0;
         *s.landed = 0u;
+        *s.asked = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int k = tid; k < np * m.d_model; k += kMegaThreads) s.prev[k] = 0ull;  // the counted sums are zero at launch
@@ -1038,6 +1042,7 @@ struct MegaWorker {
     int n_pend = 0;
     int n_stamp = 0;
     bool tracing = false;
+    bool asked = false;                // the host wants the loop to end: the same pass tells every CTA
 
     __device__ __forceinline__ MegaWorker(const MegaArgs& a_, const MegaShared& s_)
         : a(a_), s(s_), w(*s_.share), tid((int)threadIdx.x), warp((int)threadIdx.x >> 5), lane((int)threadIdx.x & 31) {}
@@ -1568,26 +1573,28 @@ struct MegaWorker {
         if (warp < NP) {
             unsigned long long k = mega_warp_best(lane < kTeam ? s.key[warp * kTeam + lane] : 0ull);
             if (mega_aborting(s)) k = kMegaGaveUp;
-            if (lane == 0) st_word(a.cand_words + (size_t)(warp * p.n_cta + (int)blockIdx.x) * kMegaCandStride, k | tag8);
+            const unsigned long long ask = *reinterpret_cast<volatile unsigned*>(s.asked);
+            if (lane == 0) st_words2(a.cand_words + (size_t)(warp * p.n_cta + (int)blockIdx.x) * kMegaCandStride, k | tag8, (ask << 8) | tag8);
         }
         stamp();
-        unsigned long long k[NP];  // the best of the candidates that this thread read, per position
+        unsigned long long k[NP], ask = 0ull;  // the best of the candidates that this thread read, per position; their requests
 #pragma unroll
         for (int q = 0; q < NP; q++) {
             k[q] = 0ull;
             for (int i = tid; i < p.n_cta; i += kMegaConsumers) {
                 const unsigned long long* const src = a.cand_words + (size_t)(q * p.n_cta + i) * kMegaCandStride;
-                unsigned long long x = 0ull;
+                ulonglong2 x = make_ulonglong2(0, 0);
                 unsigned spins = 0;
                 if (!mega_aborting(s)) {
                     while (true) {
-                        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x) : "l"(src) : "memory");
-                        if ((x & 0xffull) == tag8) break;
+                        x = ld_words2(src);
+                        if ((x.x & 0xffull) == tag8 && (x.y & 0xffull) == tag8) break;
                         if (mega_spin_out(a, s, spins, 10)) break;
                         mega_backoff();
                     }
                 }
-                k[q] = max(k[q], x);
+                k[q] = max(k[q], x.x);
+                ask |= x.y >> 8;
             }
         }
         // a reader orders its later loads (the KV-cache rows other CTAs appended during this step) after the
@@ -1600,9 +1607,11 @@ struct MegaWorker {
             const unsigned long long kq = mega_warp_best(k[q]);
             if (lane == 0) s.key[q * kMegaConsumerWarps + warp] = kq;
         }
-        if (tid == 0) s.red[63] = mega_aborting(s) ? 1.f : 0.f;  // one decision for the whole CTA
+        if (tid == 0) s.red[63] = mega_aborting(s) ? 1.f : ask ? 2.f : 0.f;  // one decision for the whole CTA (thread 0 reads CTA 0's word)
         consumer_sync();
-        bool valid = s.red[63] == 0.f;
+        const float decision = s.red[63];
+        bool valid = decision != 1.f;
+        asked = decision == 2.f;
 #pragma unroll
         for (int q = 0; q < NP; q++) {
             const unsigned long long best = mega_warp_best(lane < kMegaConsumerWarps ? s.key[q * kMegaConsumerWarps + lane] : 0ull);
@@ -1708,11 +1717,11 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const __grid_co
             const long long tail_off = min(head_bytes, (long long)(p.n_slots - 1) * p.stage[MS_HEAD].chunk_units * mega_unit_bytes(p.wt_head, min(w.v_n, p.stage[MS_HEAD].group_rows)));
             const long long tail_bytes = head_bytes - tail_off;
             MegaProducer prod(a, s);
-            for (int step = a.first; step < a.first + a.n_steps; step++) {
+            for (int step = a.first; step < a.first + a.n_steps && !prod.stopped(); step++) {  // (nothing for the steps behind the one that ended the loop)
                 for (int l = 0; step > 0 && l < L; l++) {
                     // HBM idles during the layers (their weights are a full layer ahead in the ring): the part of the head
                     // that the ring cannot hold before the head begins is brought into L2 now, a slice per layer
-                    if (tail_bytes > 0 && !mega_aborting(s)) {
+                    if (tail_bytes > 0 && !prod.stopped()) {
                         const long long b0 = tail_bytes * l / L / 16 * 16, b1 = l + 1 == L ? tail_bytes : tail_bytes * (l + 1) / L / 16 * 16;
                         if (b1 > b0)
                             asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;" ::"l"(head + tail_off + b0), "r"((unsigned)(b1 - b0)), "l"(keep_policy)
@@ -1721,6 +1730,13 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const __grid_co
                     prod.stages(blob + (long long)l * p.layer_bytes, MS_QKV, MS_DOWN, w);
                 }
                 prod.stages(head, MS_HEAD, MS_HEAD, w);
+                // The ring is full and the consumers are a few chunks into the head: the one moment of a token at which a read of
+                // host memory (a microsecond or two) holds nothing up.
+                if (a.stop_request && blockIdx.x == 0) {
+                    unsigned v;
+                    asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(a.stop_request) : "memory");
+                    if (v) *reinterpret_cast<volatile unsigned*>(s.asked) = 1u;
+                }
             }
             prod.drain();
         }
@@ -1764,7 +1780,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) k_decode_mega(const __grid_co
         }
         // Llama rule: the end-of-sequence token is emitted, then the loop stops (every CTA sees the same token)
         const bool eos = GPT2 ? gpt2_stop : m.eos_token >= 0 && tok[0] == (uint32_t)m.eos_token;
-        if (eos) {
+        if (eos || work.asked) {
             if (tid == 0) *reinterpret_cast<volatile int*>(s.stop) = 1;
             break;
         }

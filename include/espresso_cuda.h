@@ -225,8 +225,10 @@ ESP_CUDA_API int32_t esp_cuda_generate_batch(esp_cuda_engine* engine, const uint
                                              int32_t* n_out, esp_cuda_generation_result* result);
 /* The same generation, token by token, with `on_step(user, token, index, latency_ms)` called inline on the caller's
  * thread as each token becomes known: the reference's onStep callback (Engine.swift:6393-6405, GenerationStep
- * :57-83).  on_step may be NULL.  The device may be computing later tokens meanwhile; a call on this engine from inside the
- * callback finds the state after the reported token (and costs the loop its head start). */
+ * :57-83).  on_step may be NULL.  The device may be computing later tokens meanwhile.  From inside the callback,
+ * esp_cuda_get_config, _visible_token_count, _get_timings, _token_latencies and _token_times answer at once; every other call on
+ * this engine finds the state after the reported token: it waits until the device has ended the token at hand and one or two
+ * behind it, which are computed again, and from there on the loop takes one launch per token. */
 typedef void (*esp_cuda_step_callback)(void* user, uint32_t token, int32_t index, double latency_ms);
 ESP_CUDA_API int32_t esp_cuda_generate_steps(esp_cuda_engine* engine, const uint32_t* prompt, int32_t n_prompt,
                                              int32_t max_tokens, esp_cuda_step_callback on_step, void* user,

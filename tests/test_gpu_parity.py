@@ -568,7 +568,7 @@ def test_token_emission_times_of_the_persistent_loop(rt, tmp_models):
     eng.close()
 
 
-@pytest.mark.parametrize("use_at", [(), (0,), (3, 7)])
+@pytest.mark.parametrize("use_at", [(), (0,), (3, 7), (11,)])
 @pytest.mark.parametrize("eos", [False, True])
 def test_streamed_tokens_and_a_callback_that_uses_the_engine(rt, tmp_models, use_at, eos):
     """The tokens reach the callback in order while the device runs ahead; an engine used from inside the callback is in the state
@@ -587,17 +587,19 @@ def test_streamed_tokens_and_a_callback_that_uses_the_engine(rt, tmp_models, use
         eng = rt.DecodeEngine.build(tmp_models(cfg))
         plain = plain[:plain.index(plain[8]) + 1]
     other = rt.DecodeEngine.build(tmp_models(cfg))
-    seen = []
+    seen, found = [], []
 
-    def on_step(token, index, _ms):
+    def on_step(token, index, _ms):  # (what it raises does not reach the caller of generate)
         seen.append((token, index))
         if index in use_at:
             other.prefill(list(prompt) + plain[:index])
-            assert eng.visible_token_count() == len(prompt) + index
-            assert eng.select_greedy_token() == token
-            np.testing.assert_allclose(eng.logits(), other.logits(), atol=2e-2)
+            found.append((index, token, eng.select_greedy_token(), eng.visible_token_count(), eng.logits(), other.logits()))
 
     res = eng.generate(prompt, 12, on_step=on_step)
+    assert [f[0] for f in found] == [i for i in use_at if i < len(plain)]
+    for index, token, selected, visible, logits, expected in found:
+        assert selected == token and visible == len(prompt) + index
+        np.testing.assert_allclose(logits, expected, atol=2e-2)
     assert [t for t, _ in seen] == plain and [i for _, i in seen] == list(range(len(plain)))
     assert [int(t) for t in res.tokens] == plain
     assert eng.visible_token_count() == len(prompt) + len(plain) - 1
@@ -631,6 +633,38 @@ def test_questions_from_a_callback_do_not_wait_for_the_device(rt, tmp_models):
     whole = time.perf_counter() - begin
     assert answers == [(len(prompt) + i, 1, 200, 0) for i in range(200)]
     assert max(waited) < whole / 4  # the first answer used to take as long as the remaining tokens together
+    eng.close()
+
+
+@pytest.mark.parametrize("at", [0, 40])
+def test_a_call_from_a_callback_ends_the_look_ahead_within_a_few_tokens(rt, tmp_models, at):
+    """A callback that needs the device's state waits for the token at hand and the one behind it, not for the whole loop."""
+    import time
+
+    from espresso_b200.model_config import llama_6l
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = llama_6l()
+    eng = rt.DecodeEngine.build(tmp_models(cfg))
+    prompt = synthetic_prompt(cfg.vocab, 9)
+    plain = eng.generate(prompt, 240).tokens.tolist()
+    begin = time.perf_counter()
+    eng.generate(prompt, 240)
+    whole = time.perf_counter() - begin  # about 15 ms
+    eng.prefill(prompt)
+    eng.select_greedy_token()  # (the first one of an engine captures its graph)
+    selected, waited = [], []
+
+    def on_step(token, index, _ms):
+        if index == at:
+            t = time.perf_counter()
+            selected.append((eng.select_greedy_token(), token))
+            waited.append(time.perf_counter() - t)
+
+    assert eng.generate(prompt, 240, on_step=on_step).tokens.tolist() == plain
+    assert len(selected) == 1 and selected[0][0] == selected[0][1]
+    print(f"call at token {at}: {waited[0] * 1e3:.2f} ms, whole loop {whole * 1e3:.2f} ms")
+    assert waited[0] < whole / 4
     eng.close()
 
 
