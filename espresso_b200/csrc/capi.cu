@@ -184,8 +184,8 @@ int32_t esp_cuda_generate_batch(esp_cuda_engine* engine, const uint32_t* prompts
 // with onStep (Engine.swift:6393-6405): prefill, select the first token, then one decode step per token.  Limits and
 // stop rules as in generate (Llama: the EOS token is emitted, then the loop stops, :6385-6388; GPT-2: 50256 stops
 // without being emitted, :4918-4922).  Where the persistent kernel serves the model the device runs ahead of the callback
-// (Engine::stream_begin); a callback that uses the engine finds it as the step-by-step loop leaves it, and that loop goes on
-// from there.
+// (Engine::stream_begin); a callback that needs the engine's device state finds it as the step-by-step loop leaves it, and that
+// loop goes on from there.
 int32_t esp_cuda_generate_steps(esp_cuda_engine* engine, const uint32_t* prompt, int32_t n_prompt, int32_t max_tokens,
                                 esp_cuda_step_callback on_step, void* user, uint32_t* out_tokens, int32_t* n_out,
                                 esp_cuda_generation_result* result) {

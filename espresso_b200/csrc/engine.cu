@@ -2428,14 +2428,18 @@ int32_t Engine::run_mega(int n_steps, int* emitted, float* device_ms, double* fi
     return ESP_CUDA_OK;
 }
 
-// Token-by-token reporting of one greedy loop of sequence 0.  The whole loop is one launch; the kernel writes every token to pinned
-// host memory as it becomes known and goes on, and the host reports it (stream_next) while the next one is computed: a
-// launch and a host round trip per token took 107 us where the kernel needs 64 (6 layers d768).
+// Token-by-token reporting of one greedy loop of sequence 0.  A launch computes up to kStreamTokens tokens; the kernel writes every
+// token to pinned host memory as it becomes known and goes on, and the host reports it (stream_next) while the next one is
+// computed: a launch and a host round trip per token took 107 us where the kernel needs 62 (6 layers d768).
+// The kernel occupies every SM: whatever else wants the GPU, another engine in the callback or in another thread, gets it between
+// two launches, after 4 ms here (15 with 240 tokens in one launch).  A launch more costs 20 us, 0.4 % of 64 of the shortest tokens.
 // A caller that uses the engine between two tokens (from its callback) must find it as a step-by-step loop would have left it: an
 // entry point that needs the device's state first settles the stream, i.e. asks the kernel to end and goes back to the state after the
 // reported token.  The kernel looks for the request once per token and ends one or two tokens on (6 layers d768, 200 tokens to go:
 // 12.4 ms until the first such call returned, now 0.2 ms; 22 layers d2048 Q8_0, 100 tokens: 37 and 0.85 ms).  Questions that the host can answer (visible tokens, configuration, timings) do not.
 // The reporting loop then goes on step by step.
+constexpr int kStreamTokens = 64;
+
 bool Engine::stream_usable() const { return mega_usable() && !(cfg_.flags & ESP_CUDA_FLAG_KEEP_LOGITS); }
 
 int32_t Engine::stream_begin(int n_steps) {
@@ -2449,7 +2453,9 @@ int32_t Engine::stream_begin(int n_steps) {
     memset(h_stream_, 0, sizeof(unsigned long long) * n_steps);
     h_stream_[m_.max_seq] = 0ull;
     ESP_CUDA_TRY(cudaMemcpyAsync(d_stream_hidden_, act_.hidden, sizeof(float) * m_.d_model, cudaMemcpyDeviceToDevice, stream_));
-    if ((rc = enqueue_mega(n_steps, nullptr, false, h_stream_, reinterpret_cast<unsigned*>(h_stream_ + m_.max_seq)))) return rc;
+    stream_total_ = n_steps;
+    stream_launched_ = std::min(n_steps, kStreamTokens);
+    if ((rc = enqueue_mega(stream_launched_, nullptr, false, h_stream_, reinterpret_cast<unsigned*>(h_stream_ + m_.max_seq)))) return rc;
     streaming_ = true;
     stream_error_ = ESP_CUDA_OK;
     stream_visible_ = h_visible_[0];
@@ -2473,9 +2479,19 @@ int32_t Engine::stream_next(int i, uint32_t* token, bool* got) {
     *token = (uint32_t)(*word & 0xffffffffull);
     *got = true;
     stream_reported_ = i + 1;
+    const bool eos = m_.arch != ARCH_GPT2 && m_.eos_token >= 0 && *token == (uint32_t)m_.eos_token;
+    if (i + 1 < stream_launched_ || i + 1 == stream_total_ || eos) return ESP_CUDA_OK;
+    // the launch's last token: the next launch feeds it while it is reported
+    int32_t rc = stream_end();
+    if (rc) return rc;
+    const int n = std::min(stream_total_ - stream_launched_, kStreamTokens);
+    if ((rc = enqueue_mega(n, token, false, h_stream_ + stream_launched_, reinterpret_cast<unsigned*>(h_stream_ + m_.max_seq)))) return rc;
+    stream_launched_ += n;
+    streaming_ = true;
     return ESP_CUDA_OK;
 }
 
+// Waits for the launch in flight; the loop has ended when no other one is enqueued.
 int32_t Engine::stream_end() {
     streaming_ = false;
     const int32_t rc = finish_mega();

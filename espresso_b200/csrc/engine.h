@@ -246,6 +246,7 @@ private:
     bool streaming_ = false;
     int32_t stream_error_ = 0;
     int stream_visible_ = 0, stream_reported_ = 0;  // visible tokens at its start, tokens reported so far
+    int stream_total_ = 0, stream_launched_ = 0;    // tokens of the loop, tokens of the launches up to the one in flight
     unsigned long long* h_stream_ = nullptr;  // pinned [max_seq] tokens, [1] request to end
     float* d_stream_hidden_ = nullptr;        // [d_model] hidden state at its start
     long long* d_mega_trace_ = nullptr;

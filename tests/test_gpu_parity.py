@@ -668,6 +668,74 @@ def test_a_call_from_a_callback_ends_the_look_ahead_within_a_few_tokens(rt, tmp_
     eng.close()
 
 
+@pytest.mark.parametrize("arch", ["llama", "gpt2"])
+def test_streamed_tokens_past_one_launch(rt, arch):
+    """A launch of the token loop ends after 64 tokens and the next one takes over: the stream, the stop rules at and beside the seam
+    and the state behind it are those of the loop in one launch.  The model's choice after t is t + 1, so the stop token 50256 comes
+    where the prompt says."""
+    from espresso_b200.model_config import tiny_gpt2, tiny_llama
+    from espresso_b200.synthetic import synthetic_tensors
+
+    cfg = tiny_gpt2(vocab=50257, max_seq=160) if arch == "gpt2" else dataclasses.replace(tiny_llama(vocab=50257, max_seq=160), eosToken=50256)
+    embedding = np.random.default_rng(5).standard_normal((cfg.vocab, cfg.dModel)).astype(np.float16)
+    eng = rt.DecodeEngine.empty(cfg)
+    for name, t in synthetic_tensors(cfg, 1234):
+        t = embedding if name == "embeddings/token" else np.roll(embedding, 1, axis=0) if name == "lm_head" else t
+        eng.load_tensor(name, "f16", np.ascontiguousarray(t))
+    eng.finalize()
+    for stop in (62, 63, 64, 65, 127, 128, 200):
+        last = 50255 - stop
+        prompt = [17, 4, last]
+        want = [last + 1 + i for i in range(min(140, stop + (arch == "llama")))]
+        seen = []
+        res = eng.generate(prompt, 140, on_step=lambda token, index, _ms: seen.append((token, index)))
+        assert seen == [(t, i) for i, t in enumerate(want)] and res.tokens.tolist() == want
+        assert res.stoppedOnEOS == (stop < 140)
+        state = (eng.visible_token_count(), eng.select_greedy_token(), eng.logits())
+        assert eng.generate(prompt, 140).tokens.tolist() == want
+        assert state[:2] == (eng.visible_token_count(), eng.select_greedy_token())
+        np.testing.assert_array_equal(state[2], eng.logits())
+    for at in (62, 63, 64, 100):  # a callback that uses the engine beside the seam
+        found = []
+        prompt = [17, 4, 40000]
+        eng.generate(prompt, 140, on_step=lambda token, index, _ms: found.append((token, eng.select_greedy_token(), eng.visible_token_count())) if index == at else None)
+        assert found == [(40001 + at, 40001 + at, 3 + at)]
+        assert eng.visible_token_count() == 3 + 139
+    eng.close()
+
+
+def test_another_engine_gets_the_gpu_between_launches_of_a_stream(rt, tmp_models):
+    """A callback that waits for work of another engine on the same GPU waits for one launch of the token loop, not for all of it."""
+    import time
+
+    from espresso_b200.model_config import llama_6l
+    from espresso_b200.synthetic import synthetic_prompt
+
+    cfg = llama_6l()
+    eng, other = rt.DecodeEngine.build(tmp_models(cfg)), rt.DecodeEngine.build(tmp_models(cfg))
+    prompt = synthetic_prompt(cfg.vocab, 9)
+    for e in (eng, other):
+        plain = e.generate(prompt, 240).tokens.tolist()
+        e.prefill(prompt)
+        e.select_greedy_token()
+    begin = time.perf_counter()
+    eng.generate(prompt, 240)
+    whole = time.perf_counter() - begin  # about 15 ms
+    waited, got = [], []
+
+    def on_step(token, index, _ms):
+        if index == 0:
+            t = time.perf_counter()
+            got.append(other.select_greedy_token())
+            waited.append(time.perf_counter() - t)
+
+    assert eng.generate(prompt, 240, on_step=on_step).tokens.tolist() == plain and got == plain[:1]
+    print(f"the other engine waited {waited[0] * 1e3:.2f} ms, whole loop {whole * 1e3:.2f} ms")
+    assert waited[0] < whole / 2
+    eng.close()
+    other.close()
+
+
 @pytest.mark.parametrize("kind", ["f16", "q8_0"])
 def test_persistent_kernel_streams_wide_stages_in_chunks(rt, oracle_lib, tmp_models, kind):
     """d_model 2048 / hidden 5632: every stage slice of the persistent kernel exceeds a ring slot and arrives in chunks
