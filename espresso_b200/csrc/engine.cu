@@ -2564,7 +2564,6 @@ int32_t Engine::spec_prepare() {
         if (probe.smem_bytes <= smem_max) { p = probe; break; }
     }
     if (p.n_slots == 0) return fail(ESP_CUDA_ERR_STATE, "two-token kernel: the model's working set does not fit shared memory");
-    if (kSpecNP * m_.hidden > 4096) p.act_wpc = 0;  // two positions no longer fit one polling round
     const void* kern = spec_kernel_for(m_.head_dim);
     ESP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem_bytes));
     int occ = 0;

@@ -59,10 +59,12 @@ constexpr int kMegaSlots = 4, kMegaSlotMax = 64 * 1024;  // ring slots and the m
 constexpr int kMegaRingMin = 96 * 1024;  // less than that is consumed faster than a refill takes to arrive
 constexpr int kMegaMaxTiles = 5;                   // 16-row tiles whose sums a warp keeps in registers
 // Which exchanges give every CTA cache lines of its own is the plan's choice (act_wpc > 0).
-// Measured on the 6-layer d768 model against compact arrays: arg-max candidates -4.6 us per token, activation vector
-// -1.4 us, layer output x +0.3 us (five words per CTA: three times as many lines to poll for little contention saved).
-// On the 22-layer d2048 model, whose activation vector needs two polling rounds either way, lines per CTA cost 1.8 us
-// per layer.  So: candidates always, the activation vector when all of it is polled in one round, x never.
+// The arg-max candidates always have them (-4.6 us per token of the 6-layer d768 model against a compact array), the layer output x
+// never (+0.3 us: five words per CTA, three times as many lines to poll for little contention saved).  The activation vector has them
+// up to the width that a lane polls in one round.  us per token of six fp16 layers, lines / compact: d256 hidden 1280 54.7 / 60.5, d512
+// 512 53.7 / 56.5, 1408 57.2 / 58.3, GPT-2 d384 1536 65.6 / 67.9; d512 2048 57.9 / 58.7, d768 2048 60.7 / 60.0; wider, where the padding only
+// adds lines to poll: d768 3072 68.9 / 68.3, 4096 77.0 / 74.0, d1024 4096 81.8 / 80.1, d1536 4096 117.1 / 115.6, GPT-2 d768 3072 73.4 / 72.6.
+constexpr int kMegaLinesMost = 2048;
 constexpr int kMegaLineWords = 16;  // 8-byte words of a 128-byte cache line
 constexpr int kMegaCandStride = kMegaLineWords;  // 8-byte words between the arg-max candidates of two CTAs: a cache line each
 constexpr float kMegaFix = 4294967296.0f;          // counted sums: fixed point with 32 fractional bits
@@ -381,9 +383,9 @@ inline bool mega_plan(const ModelDims& m, int wt_layer, int wt_head, int sms, in
     p.wt_layer = wt_layer;
     p.wt_head = wt_head;
     p.ffn_rows = m.arch == ARCH_GPT2 ? 1 : 2;
-    // Exchange arrays: the activation vector gets cache lines per CTA where a lane polls all of its pairs in one round (four
-    // 16-byte loads); the layer output stays compact (see kMegaLineWords).
-    p.act_wpc = !quant && m.hidden <= 4096 ? ceil_div(p.hpc_max, kMegaLineWords) * kMegaLineWords : 0;
+    // Exchange arrays: the activation vector gets cache lines per CTA where a lane polls all of its pairs in one round (see
+    // kMegaLinesMost; two positions share one round of twice as many loads); the layer output stays compact.
+    p.act_wpc = !quant && m.hidden <= kMegaLinesMost ? ceil_div(p.hpc_max, kMegaLineWords) * kMegaLineWords : 0;
     // Row groups: as equal as whole tiles allow.
     const int rows[5] = {2 * p.s1_max, p.rpb, p.ffn_rows * p.hpc_max, p.dpc_max, p.vpc_max};
     for (int k = 0; k < 5; k++) {

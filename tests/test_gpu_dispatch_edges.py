@@ -135,6 +135,8 @@ def test_quantised_down_projection_in_column_chunks(rt, oracle_lib, kind, n_head
 
 @pytest.mark.parametrize("kind,head,n_head,n_kv,head_dim,hidden,vocab", [
     ("f16", "f16", 3, 3, 32, 96, 301),          # fewer K units than warps
+    ("f16", "f16", 4, 4, 64, 2048, 600),        # the widest activation vector with cache lines of its own per CTA
+    ("f16", "f16", 4, 4, 64, 2080, 600),        # the narrowest compact one
     ("f16", "f16", 6, 2, 64, 2944, 12000),      # gate/up rows in three tiles, the head in two groups
     ("f16", "f16", 12, 12, 64, 7168, 31000),    # gate/up rows in two groups
     ("q8_0", "q8_0", 4, 1, 128, 512, 2000),     # q/k/v rows past one tile
