@@ -1567,6 +1567,7 @@ struct MegaWorker {
         // [ordered logit bits : 32][0xffffff - index : 24][tag : 8].  The tag is the same in every word of a step, so the
         // largest word is the best candidate.
         constexpr int kTeam = kMegaConsumerWarps / NP;  // warps whose threads hold one position's rows
+        constexpr bool kAsks = NP == 1;  // (the two-token loop is never asked to end, and a second word costs it 0.2 %)
         {
             const unsigned long long k = mega_warp_best(best_i != 0x7fffffff ? ((unsigned long long)ordered_bits(best_v) << 32) | ((unsigned long long)(0xffffffu - (unsigned)best_i) << 8) : 0ull);
             if (lane == 0) s.key[warp] = k;
@@ -1575,8 +1576,9 @@ struct MegaWorker {
         if (warp < NP) {
             unsigned long long k = mega_warp_best(lane < kTeam ? s.key[warp * kTeam + lane] : 0ull);
             if (mega_aborting(s)) k = kMegaGaveUp;
-            const unsigned long long ask = *reinterpret_cast<volatile unsigned*>(s.asked);
-            if (lane == 0) st_words2(a.cand_words + (size_t)(warp * p.n_cta + (int)blockIdx.x) * kMegaCandStride, k | tag8, (ask << 8) | tag8);
+            unsigned long long* const dst = a.cand_words + (size_t)(warp * p.n_cta + (int)blockIdx.x) * kMegaCandStride;
+            if (kAsks && lane == 0) st_words2(dst, k | tag8, ((unsigned long long)*reinterpret_cast<volatile unsigned*>(s.asked) << 8) | tag8);
+            if (!kAsks && lane == 0) st_word(dst, k | tag8);
         }
         stamp();
         unsigned long long k[NP], ask = 0ull;  // the best of the candidates that this thread read, per position; their requests
@@ -1589,8 +1591,9 @@ struct MegaWorker {
                 unsigned spins = 0;
                 if (!mega_aborting(s)) {
                     while (true) {
-                        x = ld_words2(src);
-                        if ((x.x & 0xffull) == tag8 && (x.y & 0xffull) == tag8) break;
+                        if (kAsks) x = ld_words2(src);
+                        else asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x.x) : "l"(src) : "memory");
+                        if ((x.x & 0xffull) == tag8 && (!kAsks || (x.y & 0xffull) == tag8)) break;
                         if (mega_spin_out(a, s, spins, 10)) break;
                         mega_backoff();
                     }
