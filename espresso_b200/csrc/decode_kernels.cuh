@@ -201,11 +201,6 @@ __device__ __forceinline__ void fma_vec16(const uint4& w, const __half* srow, in
 // staged as fp16 (scaled by a power of two so that |x| < 1, see stage_vector) and summed per 32-element block in
 // packed fp16; each block sum is then widened and multiplied by the block scale in fp32.  The dequantised
 // weight values themselves stay exactly fp32(d) * q.
-__device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));  // (a & b) | c
-    return d;
-}
 __device__ __forceinline__ __half2 u32_as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 
 // 16 bytes = 16 int8 of one Q8_0 block half; xh = the matching 16 staged activations (two 16-byte groups).

@@ -2194,8 +2194,6 @@ int32_t Engine::launch_step_wide(int rows, int mode, cudaStream_t s) {
     return ESP_CUDA_OK;
 }
 
-static int pad128(long long v) { return (int)((v + 127) / 128 * 128); }
-
 // Carves the exchange arena of a persistent kernel for `np` token positions: every array starts on a cache line.
 // Returns the words needed; with `a` != null (a->x_words = arena base) it also sets the pointers.
 static size_t mega_arena_layout(const ModelDims& m, const MegaPlan& p, int np, MegaArgs* a) {
