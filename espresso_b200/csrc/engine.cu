@@ -2339,6 +2339,7 @@ int32_t Engine::launch_mega(int n_steps, const uint32_t* feed, bool times) {
 }
 
 int32_t Engine::enqueue_mega(int n_steps, const uint32_t* feed, bool times, unsigned long long* host_words, const unsigned* stop_request) {
+    ESP_CUDA_TRY(cudaSetDevice(cfg_.device));  // (a callback between two launches of a streamed loop may have made another device current)
     MegaArgs a{};
     const MegaPlan& p = mega_plan_;
     a.m = m_; a.plan = p; a.pack = d_pack_; a.norms = d_norms_;
