@@ -610,7 +610,7 @@ __device__ __forceinline__ void qx_store_quads(uint8_t* xq, float* qs, const int
         for (int j = 0; j < N; j++) top[j] = max_nan(top[j], __shfl_xor_sync(mask, top[j], o));
 #pragma unroll
     for (int j = 0; j < N; j++) {
-        const unsigned e = min(max(__float_as_uint(top[j]) >> 23, 22u), 254u);  // the largest value lies below 2^(e - 126)
+        const unsigned e = max(__float_as_uint(top[j]) >> 23, 22u);  // the largest value lies below 2^(e - 126)
         const float up = __uint_as_float((275u - e) << 23);                     // 2^(148 - e)
         // the low three bytes of (I + 0x8080) ^ 0x8080 are the digits, each in -128 .. 127 (0x400000: the low bits of the magic number)
         auto digits = [&](float x, uint32_t& rest) {
@@ -628,7 +628,7 @@ __device__ __forceinline__ void qx_store_quads(uint8_t* xq, float* qs, const int
             dst[8] = __byte_perm(ab, cd, 0x7632);
             dst[16] = __byte_perm(ab, cd, 0x5410);
             if (WT == WT_Q4_0) dst[24] = __byte_perm(__byte_perm(ra, rb, 0x0040), __byte_perm(rc, rd, 0x0040), 0x5410);
-            if (e0 == 0) qs[k[j] >> 5] = top[j] < INFINITY ? __uint_as_float((e - 21u) << 23) : __uint_as_float(0x7fffffffu);  // 2^(e - 148)
+            if (e0 == 0) qs[k[j] >> 5] = fmaf(top[j], 0.f, __uint_as_float((e - 21u) << 23));  // 2^(e - 148), or NaN
         }
     }
 }
