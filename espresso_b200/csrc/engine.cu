@@ -1900,7 +1900,7 @@ int32_t Engine::launch_step_stream(int rows, int mode, cudaStream_t s, bool prof
         return launch_prep(rows, src, K, norm, g, b, dst, parts, s);
     };
     // Weights in the order of their use; a launch requests the next kL2Ahead bytes behind those of the launch after it (L2Ahead), at
-    // most kLead in front of them.
+    // most kL2Lead in front of them.
     std::vector<std::pair<const uint8_t*, size_t>> order;
     auto weights = [&](const DeviceTensor* W) { order.emplace_back(static_cast<const uint8_t*>(W->shadow16 ? static_cast<const void*>(W->shadow16) : W->data), (size_t)W->rows * W->cols * 2); };
     if (mode & STEP_FORWARD)

@@ -28,17 +28,17 @@
 // Inside a CTA the columns of a stage's operand belong to the warps (MegaWorker): a warp awaits, stages and multiplies its own.
 // Products.  The fp16->fp32 conversion rate of the CUDA cores (measured: 20-26 weights per clock per SM from shared
 // memory) would make the row products the longest link of the chain, so they are issued as m16n8k16 tensor-core
-// instructions: sixteen weight rows are the A operand, and the fp32 activation vector, split exactly into two fp16
-// vectors (x = hi + lo, |error| <= 2^-22 |x|), occupies columns 0 and 1 of the B operand; the accumulators are fp32.  The
-// pack stores every chunk in the order the A fragments are read.
+// instructions: sixteen weight rows are the A operand, and the fp32 activation vector, split into two fp16 vectors (x = hi + lo,
+// off by at most 2^-22 |x|, or 2^-25 where the low part is subnormal; |x| up to 65504), occupies columns 0 and 1 of the B operand; the
+// accumulators are fp32.  The pack stores every chunk in the order the A fragments are read.
 // GGUF Q8_0 / Q4_0 matrices travel through the ring as their blocks (32 or 16 bytes per row and block of 32 columns,
 // the fp16 scales behind them): 34/32 or 18/32 bytes per weight from HBM, never an fp16 copy; the activation becomes int8
 // digits (qx_store_quads) and a block one int8 m16n8k32 step, scaled in fp32 (value = fp32(d) * q as in the GGUF definition).
-// A warp's time per 16-row tile and block, weights in shared memory: 40 cycles per scheduler for Q8_0 and 56 for Q4_0 widened to
-// fp16, most of it shared-memory wavefronts (one per scale) and conversions.
+// A warp's time per 16-row tile and block with the weights in shared memory was 40 cycles per scheduler for Q8_0 and 56 for Q4_0
+// nibbles widened to fp16, most of it shared-memory wavefronts (one per scale) and conversions; hence the nibbles as int8.
 //
-// us per token (16 warps that staged and synchronised together, multiplying row tiles -> this): 6 layers d768 fp16 77.6 -> 64,
-// GPT-2 117M 169.5 -> 143, 22 layers d2048 Q8_0 482 -> 369, Q4_0 477 -> 388.
+// us per token (16 warps that staged and synchronised together, multiplying row tiles -> this): 6 layers d768 fp16 77.6 -> 61,
+// GPT-2 117M 169.5 -> 135, 22 layers d2048 Q8_0 482 -> 361, Q4_0 477 -> 376.
 // Every wait (mbarrier, tagged word, counted sum) is bounded: when a limit is hit the kernel records an error code,
 // stops waiting everywhere and runs to completion; the host reports a timeout.
 #pragma once
@@ -496,7 +496,7 @@ struct MegaCursor {
 };
 
 // A consumer does not test the slot's mbarrier itself: that test costs ~280 cycles per call on this part even when the
-// phase completed long ago.  The producer warp's second lane follows the chunks in order, waits on each barrier and
+// phase completed long ago.  The watcher warp (one thread) follows the chunks in order, waits on each barrier and
 // publishes the count of landed chunks in a plain shared-memory word (release), which the consumers read (acquire).
 __device__ __forceinline__ unsigned ld_acquire_cta_shared(const unsigned* p) {
     unsigned v;
@@ -834,7 +834,7 @@ __device__ __forceinline__ float mega_warp_max(float v) {
     return __int_as_float(i);
 }
 
-// With NP positions per pass the consumer warps split into NP teams of NW = 16 / NP warps, one team per query: query qi
+// With NP positions per pass the consumer warps split into NP teams of NW = kMegaConsumerWarps / NP warps, one team per query: query qi
 // sees the n_cached cached positions and the new positions 0 .. qi, whose keys and values are rows of s.kn / s.vn; its
 // context lands in position qi of the staged s.ctx.  The teams run side by side (each reads the cached rows itself).
 // The context is staged as the products of weights of type WT read it.
@@ -1189,8 +1189,9 @@ struct MegaWorker {
     __device__ __forceinline__ void stage_words(unsigned tag, const float* gain, float (&ss)[NP]) {
         constexpr bool kSums = KIND == MS_UP, kAct = KIND == MS_DOWN;
         constexpr int kCols = mega_unit(W2) / 8, kLoads = kCols / 2;
-        // (one round of polls at the widths in use: a second one costs a round trip to L2.  Two positions of the 6-layer model: three
-        // and eight items per lane; with two and four a two-token pass took 113 us instead of 104)
+        // One round of polls holds d_model 1024 and hidden 2048 (GPT-2: 3072), of quantised types 2048 and 6144, for two positions 768
+        // and 2048; a wider vector takes another round, a round trip to L2 each.  (Two positions of the 6-layer model with two and
+        // four items per lane instead of three and eight: a two-token pass took 113 us instead of 104.)
         constexpr int kPolls = NP == 2 ? (kAct ? 8 : 3) : kAct ? (GPT2 || kQuant ? 6 : 4) : 2;
         constexpr int kCode = kSums ? 7 : kAct ? 8 : KIND == MS_QKV ? 5 : 9;
         const int K = kAct ? a.m.hidden : a.m.d_model, n = items<W2>(K / mega_unit(W2)), total = NP * n;

@@ -256,9 +256,9 @@ ESP_CUDA_API int32_t esp_cuda_get_timings(esp_cuda_engine* engine, esp_cuda_timi
  * before the step. */
 /* SM clock stamps taken by one CTA of the persistent decode kernel during the last token of the most recent
  * decode loop (the fine-grained counterpart of the per-layer DecodeKernelProfile, DecodeForwardPass.swift:212-320).
- * Per layer 14 stamps: S1 begin, norm done, weights arrived, rows done, barrier passed; S2 weights arrived, done,
- * barrier passed; S3 norm done, weights arrived, gate/up done, weights arrived, down done, barrier passed; then
- * 4 for the head: begin, norm done, rows done, barrier passed.  *n = 0 when the model does not use that kernel.
+ * Per layer 10 stamps: begin; operand staged, q/k/v published; q/k/v received, attention done; Wo done; operand staged, gate/up
+ * published; activation staged, layer output published (a CTA outside the head groups stamps the first five stages at once); then 4 for
+ * the head: begin, operand staged, candidate published, token known.  *n = 0 when the model does not use that kernel.
  * `cta` selects which CTA records the NEXT loop. */
 ESP_CUDA_API int32_t esp_cuda_stage_trace(esp_cuda_engine* engine, int32_t cta, int64_t* out, int32_t capacity, int32_t* n);
 /* Emission time (GPU global timer, nanoseconds) of every token of the most recent decode loop that ran as the

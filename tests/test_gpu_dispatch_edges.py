@@ -144,8 +144,8 @@ def test_quantised_down_projection_in_column_chunks(rt, oracle_lib, kind, n_head
     ("q4_0", "q4_0", 8, 8, 32, 9728, 26001),    # two groups, a ragged last row
 ])
 def test_row_groups_and_units_of_the_persistent_kernel(rt, oracle_lib, kind, head, n_head, n_kv, head_dim, hidden, vocab):
-    """A CTA's rows in one to five tiles and in several groups, K units that do not divide among the warps, contexts that pass a
-    warp round (256 positions)."""
+    """A CTA's gate/up and head rows in one to five tiles and in several groups (q/k/v rows: the test below), K units that do not divide
+    among the warps, contexts that pass a warp round (256 positions)."""
     from espresso_b200.synthetic import synthetic_prompt
 
     cfg = _model("edge-groups", 2, n_head, n_kv, n_head * head_dim, head_dim, hidden, vocab, 300)
